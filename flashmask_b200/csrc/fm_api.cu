@@ -33,7 +33,6 @@ int bwd_mma_tile_shape(int d, int dv, int* tile_m, int* tile_n);
 int bwd_mma_launch(const AttnKParams& p, int dtype, cudaStream_t s);
 int bwd_preprocess_launch(const AttnKParams& p, int dtype, cudaStream_t s);
 int bwd_dsink_launch(const AttnKParams& p, cudaStream_t s);
-bool fwd_sm100_supported(const fm_attn_args* a);
 int fwd_sm100_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s);
 bool bwd_sm100_supported(const fm_attn_args* a);
 int bwd_sm100_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s);
@@ -43,6 +42,14 @@ int bwd_sm100_fused_status(int* out, bool reset);
 size_t bwd_sm100_fused_accum_bytes(const fm_attn_args* a);
 int bwd_sm100_persist_status(int* out, bool reset);
 size_t bwd_sm100_workspace_bytes(const fm_attn_args* a);
+
+bool fwd_pair_supported(const fm_attn_args* a);
+int fwd_pair_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s);
+int fwd_pair_status(int* out, bool reset);
+bool bwd_pair_supported(const fm_attn_args* a);
+size_t bwd_pair_workspace_bytes(const fm_attn_args* a);
+int bwd_pair_launch(const AttnKParams& p, const fm_attn_args* a, void* ws, cudaStream_t s);
+int bwd_pair_status(int* out, bool reset);
 
 int fwd_sm100_status(int* out, bool reset);
 int bwd_sm100_status(int* out, bool reset);
@@ -70,11 +77,14 @@ static Options read_options() {
 static Options g_opt = read_options();
 int option_order_classes() { return g_opt.order_classes; }
 
-// Kernel variant of the forward for (d, dv): the tcgen05 kernels cover head dims up to
-// 128 (multiples of 8); FLASHMASK_B200_FWD=mma forces the warp-MMA variant (A/B runs).
+// Head dims of the CTA-pair kernels.
+static bool pair_dims(int d, int dv) { return (d == 256 && dv == 256) || ((d == 512 || d == 576) && dv == 512); }
+
+// Kernel variant of the forward for (d, dv): the tcgen05 kernels cover head dims up to 128 (multiples of 8),
+// 192 / 128 and, on CTA pairs, 256, 512 and 576 / 512; FLASHMASK_B200_FWD=mma forces the warp-MMA variant (A/B runs).
 static bool fwd_uses_sm100(int d, int dv) {
   const bool small = d <= 128 && dv <= 128 && d % 8 == 0 && dv % 8 == 0;
-  if (!small && !(d == 192 && dv == 128) && !(d == 256 && dv == 256)) return false;
+  if (!small && !(d == 192 && dv == 128) && !pair_dims(d, dv)) return false;
   return !g_opt.fwd_mma;
 }
 
@@ -129,6 +139,7 @@ int fill_kparams(const fm_attn_args* a, AttnKParams* p, bool backward) {
   p->md.nblk_pad = fm_mask_nblk_pad(a->Sk, a->tile_n > 0 ? a->tile_n : 64);
   p->md.BHm = p->md.mask_B * p->md.Hm;
   p->md.Sq = a->Sq; p->md.Sk = a->Sk;
+  p->mask_tile = a->ncols ? a->tile_n : 0;
   if (a->ncols) { p->fwd_order = a->fwd_order; p->dq_order = a->dq_order; p->dkdv_order = a->dkdv_order; }
   if (backward) {
     p->d_o = a->d_o; p->dq = a->dq; p->dk = a->dk; p->dv = a->dv_out; p->dsink = a->dsink;
@@ -170,6 +181,12 @@ static bool bwd_uses_fused(const fm_attn_args* a) {
   return bwd_uses_sm100(a->d, a->dv) && exact && !a->deterministic && !g_opt.bwd_split;
 }
 
+// The CTA-pair backward (256, 512, 576 / 512) keeps P and dS of a chunk of query rows in the caller's workspace;
+// without one (fm_bwd_static_scratch) and past its index range the warp-MMA kernels serve these head dims.
+static bool bwd_uses_pair(const fm_attn_args* a) {
+  return pair_dims(a->d, a->dv) && !g_opt.bwd_mma && bwd_pair_supported(a);
+}
+
 // preprocess -> main kernels of the selected variant -> dsink, on one stream
 static int run_bwd_kernels(const fm_attn_args* a, const AttnKParams& p, cudaStream_t s) {
   int rc = bwd_preprocess_launch(p, a->dtype, s);
@@ -191,6 +208,10 @@ static int run_bwd_kernels(const fm_attn_args* a, const AttnKParams& p, cudaStre
     // masks they are 5-12 % slower than the one-unit kernels, which is why both exist.)
     const bool persist = p.dq_order && p.dkdv_order && g_opt.bwd_persist && a->d <= 128;   // 192 / 128: one-unit kernels only
     rc = persist ? bwd_sm100_persist_launch(p, a, s) : bwd_sm100_launch(p, a, s);
+  } else if (p.pair_ws) {
+    FM_REQUIRE((((uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)a->d_o) & 15) == 0,
+               FM_ERR_INVALID_ARGUMENT, "backward: q/k/v/d_o must be 16-byte aligned");
+    rc = bwd_pair_launch(p, a, p.pair_ws, s);
   } else {
     rc = bwd_mma_launch(p, a->dtype, s);
   }
@@ -210,6 +231,7 @@ extern "C" int fm_fwd_tile_shape(int d, int dv, int* tile_m, int* tile_n) {
 extern "C" int fm_bwd_tile_shape(int d, int dv, int* tile_m, int* tile_n) {
   FM_REQUIRE(tile_m && tile_n, FM_ERR_INVALID_ARGUMENT, "fm_bwd_tile_shape: NULL output");
   if (bwd_uses_sm100(d, dv)) { *tile_m = 64; *tile_n = 128; return FM_OK; }
+  if (pair_dims(d, dv) && !g_opt.bwd_mma) { *tile_m = 128; *tile_n = 128; return FM_OK; }
   int rc = bwd_mma_tile_shape(d, dv, tile_m, tile_n);
   if (rc != FM_OK) set_error("fm_bwd_tile_shape: unsupported head dims (d=%d, dv=%d)", d, dv);
   return rc;
@@ -238,16 +260,15 @@ static int fwd_impl(const fm_attn_args* a, const BlockScore& bs, void* stream) {
                bs.block_ld, p.block_cols);
     p.block_logit = bs.block_logit; p.block_bos = bs.block_bos; p.block_ld = bs.block_ld;
     p.block_log2 = bs.block_size == 32 ? 5 : (bs.block_size == 64 ? 6 : 7);
-    // the tcgen05 kernels have compile-time variants for it; the warp-MMA kernels (head dims 256 and up,
-    // or FLASHMASK_B200_FWD=mma) a run-time branch
-    if (fwd_uses_sm100(a->d, a->dv) && fwd_sm100_supported(a)) return fwd_sm100_launch(p, a, (cudaStream_t)stream);
-    FM_REQUIRE(!fwd_uses_sm100(a->d, a->dv), FM_ERR_INVALID_ARGUMENT, "fm_fwd_block_score: q/k/v must be 16-byte aligned");
-    return fwd_mma_launch(p, a->dtype, (cudaStream_t)stream);
   }
-  if (fwd_uses_sm100(a->d, a->dv) && fwd_sm100_supported(a)) return fwd_sm100_launch(p, a, (cudaStream_t)stream);
-  FM_REQUIRE(!fwd_uses_sm100(a->d, a->dv), FM_ERR_INVALID_ARGUMENT,
-             "fm_fwd: q/k/v must be 16-byte aligned");
-  return fwd_mma_launch(p, a->dtype, (cudaStream_t)stream);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (!fwd_uses_sm100(a->d, a->dv)) return fwd_mma_launch(p, a->dtype, s);
+  FM_REQUIRE((((uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v) & 15) == 0, FM_ERR_INVALID_ARGUMENT,
+             "forward: q/k/v must be 16-byte aligned");
+  // Past the CTA-pair kernels' key limit, and for block scores at 512 and 576, the warp-MMA kernels serve.
+  if (pair_dims(a->d, a->dv))
+    return fwd_pair_supported(a) && !(bs.block_logit && a->d > 256) ? fwd_pair_launch(p, a, s) : fwd_mma_launch(p, a->dtype, s);
+  return fwd_sm100_launch(p, a, s);
 }
 
 extern "C" int fm_fwd(const fm_attn_args* a, void* stream) { return fwd_impl(a, BlockScore{}, stream); }
@@ -371,6 +392,7 @@ static size_t bwd_stat_operand_bytes(const fm_attn_args* a) {
 
 extern "C" size_t fm_bwd_workspace_bytes(const fm_attn_args* a) {
   if (!a || a->B <= 0 || a->Hq <= 0 || a->Sq <= 0) return 0;
+  if (a->Sk > 0 && a->Hkv > 0 && bwd_uses_pair(a)) return bwd_row_stat_bytes(a) + bwd_pair_workspace_bytes(a);
   return bwd_row_stat_bytes(a) +
          (bwd_uses_fused(a) ? bwd_sm100_fused_accum_bytes(a) + bwd_stat_operand_bytes(a) : 0);
 }
@@ -410,6 +432,7 @@ extern "C" int fm_bwd(const fm_attn_args* a, void* stream) {
     p.stat_dp = p.stat_s + (size_t)a->B * a->Hq * p.Sq_r * 8;
     p.bwd_flags = a->bwd_flags;
   }
+  if (bwd_uses_pair(a)) p.pair_ws = reinterpret_cast<uint8_t*>(a->workspace) + bwd_row_stat_bytes(a);
   cudaStream_t s = (cudaStream_t)stream;
   attach_bwd_tables(a, &p);
   return run_bwd_kernels(a, p, s);
@@ -422,11 +445,15 @@ extern "C" int fm_kernel_status(int* status, int reset) {
   if (rc != FM_OK) return rc;
   rc = bwd_sm100_status(&bw, reset != 0);
   if (rc != FM_OK) return rc;
-  int bp = 0, bf = 0;
+  int bp = 0, bf = 0, fp = 0, bpair = 0;
+  rc = fwd_pair_status(&fp, reset != 0);
+  if (rc != FM_OK) return rc;
+  rc = bwd_pair_status(&bpair, reset != 0);
+  if (rc != FM_OK) return rc;
   rc = bwd_sm100_persist_status(&bp, reset != 0);
   if (rc != FM_OK) return rc;
   rc = bwd_sm100_fused_status(&bf, reset != 0);
-  *status = f ? f : (bw ? bw : (bp ? bp : bf));
+  *status = f ? f : (bw ? bw : (bp ? bp : (bf ? bf : (fp ? fp : bpair))));
   return rc;
 }
 

@@ -14,6 +14,7 @@ struct AttnKParams {
   // one-kernel backward only: the row statistics as 16-bit GEMM operands, [B,Hq,Sq_r,8] each:
   // (-c_hi, -c_lo, 0 x 6) with c = LSE*log2e / scale_log2, and (-d_hi, -d_lo, 0 x 6) with d = rowsum(O dO)
   uint16_t* stat_s; uint16_t* stat_dp;
+  void* pair_ws;    // CTA-pair backward: workspace of P, dS and fp32 sums (nullptr: that variant is not used)
   int bwd_flags;    // FM_BWD_DQ_CARRY: the accumulator holds earlier sums; FM_BWD_DQ_LEAVE: dq is not written
   int64_t q_b, q_s, q_h, k_b, k_s, k_h, v_b, v_s, v_h, o_b, o_s, o_h;
   int64_t do_b, do_s, do_h, dq_b, dq_s, dq_h, dk_b, dk_s, dk_h, dv_b, dv_s, dv_h;
@@ -21,6 +22,7 @@ struct AttnKParams {
   int Sq_r;  // Sq rounded up to the row tile, stride of the per-row workspaces
   float scale, scale_log2;
   MaskDesc md;
+  int mask_tile;    // key columns per entry of md.minmax (0: no mask)
   // optional longest-work-first launch orders (unit ids over (mask_b, mask_h, unit)); nullptr = index order
   const int32_t* fwd_order; const int32_t* dq_order; const int32_t* dkdv_order;
   // state behind a backward table: [0] next table entry, [1] CTAs that left, [2] 1 when the persistent

@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(256) bwd_dkdv_mma_kernel(const AttnKParams p) 
   const int j0 = n * BC;
   const int off = p.Sk - p.Sq;
   const int n_q_tiles = (p.Sq + BR - 1) / BR;
+  const int mask_tile = p.mask_tile ? p.mask_tile : BC;   // the reductions may cover wider tiles than BC
   const int bh_mask = md.ncols ? ((md.mask_B == 1 ? 0 : b) * md.Hm + (hk * G) / (p.Hq / md.Hm)) : 0;
   const uint32_t sK = smem_u32(smem + Cfg::OFF_K), sV = smem_u32(smem + Cfg::OFF_V);
   const uint32_t sQ = smem_u32(smem + Cfg::OFF_Q), sdO = smem_u32(smem + Cfg::OFF_DO);
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(256) bwd_dkdv_mma_kernel(const AttnKParams p) 
     const float* gDps = p.dpsum + ((int64_t)b * p.Hq + hq) * p.Sq_r;
     for (int m = m_lo; m < n_q_tiles; ++m) {
       const int ms = m * BR, me = min(ms + BR, p.Sq);
-      const int cls = classify_tile(md, bh_mask, n, ms, me, BC);
+      const int cls = classify_tile(md, bh_mask, n * BC / mask_tile, ms, me, mask_tile);
       if (cls == FM_TILE_SKIP) continue;
       __syncthreads();  // previous tile's phase B finished with sQ/sdO/sP/sdS
       bwd_load_tile_async<BR, D, 256>(sQ, gQ + (int64_t)ms * p.q_s, p.q_s, me - ms, p.d, tid);
@@ -296,6 +297,7 @@ __global__ void __launch_bounds__(256) bwd_dq_mma_kernel(const AttnKParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_q_tiles = (p.Sq + BR - 1) / BR;
+  const int mask_tile = p.mask_tile ? p.mask_tile : BC;   // the reductions may cover wider tiles than BC
   const int m = n_q_tiles - 1 - blockIdx.x, hq = blockIdx.y, b = blockIdx.z;
   const int hk = hq / (p.Hq / p.Hkv);
   const MaskDesc& md = p.md;
@@ -334,7 +336,7 @@ __global__ void __launch_bounds__(256) bwd_dq_mma_kernel(const AttnKParams p) {
   if (md.causal) n_hi = max(0, min(nb, (me + off + BC - 1) / BC));
   const int c0 = warp * (D / 8);
   for (int n = n_hi - 1; n >= 0; --n) {
-    const int cls = classify_tile(md, bh_mask, n, ms, me, BC);
+    const int cls = classify_tile(md, bh_mask, n * BC / mask_tile, ms, me, mask_tile);
     if (cls == FM_TILE_SKIP) continue;
     const int j0 = n * BC;
     __syncthreads();

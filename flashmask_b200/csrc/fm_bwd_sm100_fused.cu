@@ -118,21 +118,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
-// Barrier over the `n` threads of named barrier `id` that also ANDs a predicate: every thread of the
-// group gets the same answer, so a bounded wait that gave up in one warp takes the whole group out of
-// its loop together and no warp is left alone at a later barrier.
-__device__ __forceinline__ bool group_all(bool ok, int id, int n) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, %2, %3, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)ok), "r"(id), "r"(n)
-      : "memory");
-  return r != 0;
-}
 // Tiled reduction shared -> global through a 2-D tensor map: the box at (x, y) of the fp32 tensor gets
 // the staged box added to it by the copy engine; completion is tracked by this thread's bulk groups.
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* tmap, uint32_t src_smem, int x, int y) {
@@ -144,13 +129,6 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
-// Shared-memory descriptor of a K-major operand WITHOUT swizzle: 8-row x 16-byte core matrices; `lbo` = bytes
-// between the two core matrices of one k-step (K columns 0..7 and 8..15), `sbo` = bytes between 8-row groups.
-__device__ __forceinline__ uint64_t make_sdesc_noswz(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
 
 // Four k-steps (K = 64) of D[tmem] (+)= A[smem] * B[smem]: A K-major (advances 32 bytes per
 // step inside its 128-byte rows), B MN-major (advances 16 rows = 2048 bytes per step).

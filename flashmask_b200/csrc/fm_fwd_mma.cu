@@ -59,6 +59,7 @@ fwd_mma_kernel(const AttnKParams p) {
   const int ms = t * BR, me = min(ms + BR, p.Sq);
   const int off = p.Sk - p.Sq;
   const int nb = (p.Sk + BC - 1) / BC;
+  const int mask_tile = p.mask_tile ? p.mask_tile : BC;
 
   const uint16_t* gq = reinterpret_cast<const uint16_t*>(p.q) + b * p.q_b + (int64_t)ms * p.q_s + hq * p.q_h;
   const uint16_t* gk = reinterpret_cast<const uint16_t*>(p.k) + b * p.k_b + hk * p.k_h;
@@ -84,7 +85,8 @@ fwd_mma_kernel(const AttnKParams p) {
   const int col_a = (lane >> 4);                                    // chunk offset (0/1)
 
   for (int n = n_hi - 1; n >= 0; --n) {
-    const int cls = classify_tile(md, bh_mask, n, ms, me, BC);
+    // (the reductions may cover wider tiles than this kernel's: their class is then the wider tile's)
+    const int cls = classify_tile(md, bh_mask, n * BC / mask_tile, ms, me, mask_tile);
     if (cls == FM_TILE_SKIP) continue;
     __syncthreads();  // all warps finished reading the previous K/V tile
     const int j0 = n * BC;

@@ -292,6 +292,22 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// Barrier over the `n` threads of named barrier `id` that also ANDs a predicate: every thread of the
+// group gets the same answer, so a bounded wait that gave up in one warp takes the whole group out of
+// its loop together and no warp is left alone at a later barrier.
+__device__ __forceinline__ bool group_all(bool ok, int id, int n) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)ok), "r"(id), "r"(n)
+      : "memory");
+  return r != 0;
+}
+
 // ---------------------------------------------------------------------------
 // descriptors
 // ---------------------------------------------------------------------------
@@ -313,6 +329,15 @@ __host__ __device__ constexpr uint32_t make_idesc(bool is_bf16, int M, int N, in
 __device__ __forceinline__ uint64_t make_sdesc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
   return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16) |
          ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (2ull << 61);
+}
+
+// Shared-memory descriptor of an operand WITHOUT swizzle, made of 8-row x 16-byte core matrices of 128
+// contiguous bytes.  K-major: `lbo` = bytes between the core matrices of neighbouring 8-element K groups,
+// `sbo` = bytes between 8-row groups.  MN-major (the 16 contiguous bytes are 8 MN elements, the 8 rows of a
+// core matrix are K): `sbo` = bytes between 8-element MN groups, `lbo` = bytes between 8-row K groups.
+__device__ __forceinline__ uint64_t make_sdesc_noswz(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16) |
+         ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
 // Block maxima of one row of a 128-column tile (reference: the fused block-score epilogue,
@@ -385,6 +410,29 @@ __device__ __forceinline__ float block_scores(const uint32_t* sr, int rel0, floa
   return all;
 }
 
+// Merges group g (eight consecutive blocks) of a row's accumulators into the row of the output at `dst`: 32
+// contiguous bytes loaded, maximised and stored when they are 16-byte aligned (`vec`) and whole.
+template <int STRIDE>
+__device__ __forceinline__ void block_flush(float* dst, float* acc, int g, bool vec, int n_cols) {
+  float* gp = dst + g * 8;
+  float* a = acc + (g & 1) * 8 * STRIDE;
+  if (vec && g * 8 + 7 < n_cols) {
+    float4 o0 = *reinterpret_cast<const float4*>(gp), o1 = *reinterpret_cast<const float4*>(gp + 4);
+    o0.x = fmaxf(o0.x, a[0 * STRIDE]); o0.y = fmaxf(o0.y, a[1 * STRIDE]);
+    o0.z = fmaxf(o0.z, a[2 * STRIDE]); o0.w = fmaxf(o0.w, a[3 * STRIDE]);
+    o1.x = fmaxf(o1.x, a[4 * STRIDE]); o1.y = fmaxf(o1.y, a[5 * STRIDE]);
+    o1.z = fmaxf(o1.z, a[6 * STRIDE]); o1.w = fmaxf(o1.w, a[7 * STRIDE]);
+    *reinterpret_cast<float4*>(gp) = o0;
+    *reinterpret_cast<float4*>(gp + 4) = o1;
+  } else {
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (g * 8 + c < n_cols) gp[c] = fmaxf(gp[c], a[c * STRIDE]);
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) a[c * STRIDE] = __int_as_float(0xff800000);
+}
+
 // host: driver entry point for tensor-map encoding, resolved once
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
@@ -393,9 +441,10 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 EncodeTiledFn get_encode_tiled();
 
 // [B, S, H, D] tensor (element strides sb, ss, sh; innermost contiguous) as a
-// 4-D map (D, H, S, B) with a 64 x 1 x rows x 1 box and 128-byte swizzle.
+// 4-D map (D, H, S, B) with a cols x 1 x rows x 1 box: 64 columns with 128-byte
+// swizzle, or 32 columns with 64-byte swizzle.
 int make_bshd_tmap(CUtensorMap* out, const void* base, int dtype, int B, int S, int H, int D, int64_t sb,
-                   int64_t ss, int64_t sh, int box_rows);
+                   int64_t ss, int64_t sh, int box_rows, int box_cols = 64);
 
 }  // namespace sm100
 }  // namespace fm

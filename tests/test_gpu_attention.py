@@ -174,6 +174,21 @@ def test_masks_d256(kind):
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("d,dv", [(576, 512), (512, 512)])
+@pytest.mark.parametrize("kind", MASKS)
+def test_masks_pair_kernels_two_slices(kind, d, dv):
+    """Every mask family through the CTA-pair kernels at the head dims whose V / O have two 256-column slices (and,
+    at 576, whose dQ / dK have a 64-column rest): lengths off every tile, Sq != Sk, one CTA of a pair without rows,
+    rows and keys long enough to wrap every ring, sink, GQA and MQA."""
+    _run(kind, 1, 129, 129, 2, 1, d, dv, sink=True, seed=81)
+    _run(kind, 2, 300, 300, 4, 2, d, dv, seed=82)
+    _run(kind, 1, 1411, 1411, 2, 1, d, dv, sink=True, seed=83)
+    if kind in ("causal_doc", "none_causal"):
+        _run(kind, 1, 203, 333, 2, 1, d, dv, seed=84)
+        _run(kind, 1, 333, 203, 2, 2, d, dv, seed=85)
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("kind", MASKS)
 def test_masks_d64(kind, fwd_variant):
     """Every mask family through the 64-column variants: GQA, rows long enough to wrap the K/V ring."""
