@@ -56,6 +56,7 @@ SIGNATURES = {
     "fm_bwd_tile_shape": (C.c_int, [C.c_int, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "fm_reload_options": (C.c_int, []),
     "fm_launch_count": (C.c_ulonglong, []),
+    "fm_fwd_workspace_bytes": (C.c_size_t, [C.POINTER(AttnArgs)]),
     "fm_fwd": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "fm_fwd_block_score": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p]),
     "fm_launch_order_ints": (C.c_int64, [C.POINTER(AttnArgs), C.c_int]),

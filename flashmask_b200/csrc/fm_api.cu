@@ -18,6 +18,16 @@ void set_error(const char* fmt, ...) {
   va_end(ap);
 }
 
+int sm_count() {
+  static std::atomic<int> cached[64];        // zero-initialised: 0 = not asked yet
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  if (dev < 64 && (n = cached[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+  if (dev < 64) cached[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 static std::atomic<unsigned long long> g_launches{0};
 void count_launches(int n) { g_launches.fetch_add((unsigned long long)n, std::memory_order_relaxed); }
 
@@ -34,6 +44,7 @@ int bwd_mma_launch(const AttnKParams& p, int dtype, cudaStream_t s);
 int bwd_preprocess_launch(const AttnKParams& p, int dtype, cudaStream_t s);
 int bwd_dsink_launch(const AttnKParams& p, cudaStream_t s);
 int fwd_sm100_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s);
+size_t fwd_sm100_workspace_bytes(const fm_attn_args* a);
 bool bwd_sm100_supported(const fm_attn_args* a);
 int bwd_sm100_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s);
 int bwd_sm100_persist_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s);
@@ -269,6 +280,11 @@ static int fwd_impl(const fm_attn_args* a, const BlockScore& bs, void* stream) {
   if (pair_dims(a->d, a->dv))
     return fwd_pair_supported(a) && !(bs.block_logit && a->d > 256) ? fwd_pair_launch(p, a, s) : fwd_mma_launch(p, a->dtype, s);
   return fwd_sm100_launch(p, a, s);
+}
+
+extern "C" size_t fm_fwd_workspace_bytes(const fm_attn_args* a) {
+  if (!a || a->B <= 0 || a->Hq <= 0 || a->Hkv <= 0 || a->Hq % a->Hkv || a->Sq <= 0 || a->Sk <= 0) return 0;
+  return fwd_uses_sm100(a->d, a->dv) ? fwd_sm100_workspace_bytes(a) : 0;
 }
 
 extern "C" int fm_fwd(const fm_attn_args* a, void* stream) { return fwd_impl(a, BlockScore{}, stream); }

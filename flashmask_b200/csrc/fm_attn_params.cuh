@@ -33,6 +33,9 @@ struct AttnKParams {
   // masked, scaled scores, combined into block_logit[b][head][row][block] with fmax; block ids are
   // relative to block_bos[b][row] (the first key of the row's document) when that is given
   float* block_logit; const int32_t* block_bos;
+  // forward over packed heads / split keys: log2(heads packed per query), parts of a row block's K tiles, partial results
+  int pack_log2, n_split;
+  float* part_o; float* part_lse;
   int block_log2, block_cols, block_ld;   // log2(block size), ceil(Sk / block size), row stride
 };
 
@@ -55,6 +58,8 @@ struct OrderJob { int axis, block_rows, n_units, n_other, rep_h, rep_b, heads, i
 struct OrderJobs { OrderJob job[3]; };
 // Builds up to three tables in one launch (one CTA each).
 int launch_order_build(const MaskDesc& md, int tile_n, const OrderJobs& jobs, int n_jobs, cudaStream_t s);
+// Multiprocessors of the current device.
+int sm_count();
 // Work classes requested through the environment when the library was loaded (0: the default).
 int option_order_classes();
 

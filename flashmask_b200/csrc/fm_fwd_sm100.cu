@@ -88,7 +88,11 @@ __device__ __forceinline__ float neg_inf() { return __int_as_float(0xff800000); 
 
 // BLOCK_SCORE: 0, or the block size (32 / 64 / 128) of the block-score side output; BLOCK_BOS: document
 // starts are given, so a block may straddle two tiles.
-template <int D, int DV, bool IS_BF16, int BLOCK_SCORE, bool BLOCK_BOS>
+// SPLIT: the variant for calls that leave most of the chip idle otherwise (few query rows against many keys).
+// The rows of a CTA are (query, head of the GQA group) pairs, 2^pack_log2 heads per query, so that the heads
+// sharing a K / V tile share its loads; the K tiles of a row block are dealt to n_split CTAs, whose partial
+// results (fp32 O / l and m + log2 l) fwd_combine_kernel merges.
+template <int D, int DV, bool IS_BF16, int BLOCK_SCORE, bool BLOCK_BOS, bool SPLIT>
 __global__ void __launch_bounds__(384, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const AttnKParams p) {
@@ -110,9 +114,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (tid == 0) FPROF(0);
   // descriptor fetches start before anything else: the first loads wait on them
   if (warp == 8 && lane == 0) { tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); }
-  const int n_tiles = (p.Sq + ROWS - 1) / ROWS;
-  int t = n_tiles - 1 - blockIdx.x, hq = blockIdx.y, b = blockIdx.z;
-  if (p.fwd_order) {
+  const int lg = SPLIT ? p.pack_log2 : 0;
+  const int n_rows = p.Sq << lg;             // row x of the launch: query x >> lg, head hq + (x & (2^lg - 1))
+  const int n_tiles = (n_rows + ROWS - 1) / ROWS;
+  int t = n_tiles - 1 - (SPLIT ? blockIdx.x / p.n_split : blockIdx.x), hq = blockIdx.y << lg, b = blockIdx.z;
+  if (!SPLIT && p.fwd_order) {
     const OrderedCta c = ordered_cta(p.fwd_order, p.Hq);
     t = c.unit; hq = c.head; b = c.b;
   }
@@ -122,10 +128,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int bh_mask = md.ncols ? ((md.mask_B == 1 ? 0 : b) * md.Hm + hq / (p.Hq / md.Hm)) : 0;
   const int ms = t * ROWS;
   const int off = p.Sk - p.Sq;
+  // queries [q_lo(s), q_hi(s)) of sub-tile s
+  auto q_lo = [&](int s) { return (ms + 128 * s) >> lg; };
+  auto q_hi = [&](int s) { return min(((ms + 128 * s + 127) >> lg) + 1, p.Sq); };
   // first K tile right of everything these rows can see, and whether the diagonal tile is loaded ahead of the list
   const int nb = (p.Sk + 127) / 128;
-  const int n_hi = md.causal ? max(0, min(nb, (min(ms + ROWS, p.Sq) + off + 127) / 128)) : nb;
-  const bool spec = Cfg::SPEC && BLOCK_SCORE == 0 && md.causal && n_hi > 0;
+  const int n_hi = md.causal ? max(0, min(nb, (q_hi(1) + off + 127) / 128)) : nb;
+  const bool spec = Cfg::SPEC && BLOCK_SCORE == 0 && !SPLIT && md.causal && n_hi > 0;
 
   if (tid == 0) misc[4] = 0;
   if (warp == 8 && lane == 0) {
@@ -142,7 +151,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       mbar_arrive_expect_tx(bar(Cfg::B_QFULL + s), Cfg::Q_BYTES);
       for (int dc = 0; dc < D / 64; ++dc)
         tma_load_4d(sQ + s * Cfg::Q_BYTES + dc * Cfg::SUB, &tm_q, bar(Cfg::B_QFULL + s), dc * 64, hq,
-                    ms + 128 * s, b);
+                    q_lo(s), b);
     }
     if (spec) {
       const int j0 = (n_hi - 1) * 128;
@@ -170,13 +179,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int n = base - lane;
       uint32_t f0 = 0, f1 = 0;
       if (n >= 0) {
-        f0 = tile_flags(mst, 0, n, ms, min(ms + 128, p.Sq), 128);
-        if (ms + 128 < p.Sq) f1 = tile_flags(mst, 0, n, ms + 128, min(ms + 256, p.Sq), 128);
+        f0 = tile_flags(mst, 0, n, q_lo(0), q_hi(0), 128);
+        if (ms + 128 < n_rows) f1 = tile_flags(mst, 0, n, q_lo(1), q_hi(1), 128);
         if (spec && n == n_hi - 1 && (f0 | f1) == 0) {
           // the diagonal tile is already on its way into slots 0 / 1, so it is the first list entry whatever its
           // class: an invisible one is computed with the element mask (every score masked, P = 0)
           f0 = FM_TF_ACTIVE | FM_TF_CAUSAL | FM_TF_RAGGED | (md.ncols ? FM_TF_BOUNDS : 0u);
-          if (ms + 128 < p.Sq) f1 = f0;
+          if (ms + 128 < n_rows) f1 = f0;
         }
       }
       const bool keep = (f0 | f1) != 0;
@@ -194,7 +203,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = (uint32_t)misc[0];
-  const int cnt = misc[1];
+  int cnt = misc[1];
+  if constexpr (SPLIT) {
+    // this CTA's share of the tiles
+    const int part = blockIdx.x % p.n_split, lo = cnt * part / p.n_split;
+    cnt = cnt * (part + 1) / p.n_split - lo;
+    list += lo;
+  }
   WaitCtx wc{misc + 4, global_timer_ns() + 2000000000ull};
   if (tid == 0) { FPROF(1); FPROF_VAL(7, (long long)cnt); }
   if (cnt == 0) {
@@ -206,15 +221,24 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       mbar_wait(bar(Cfg::B_QFULL + 1), 0u, wc);
     }
     if (warp == 9) tmem_dealloc(tmem, 512);
-    uint16_t* go = reinterpret_cast<uint16_t*>(p.o) + b * p.o_b + (int64_t)ms * p.o_s + hq * p.o_h;
-    for (int x = tid; x < ROWS * (DV / 8); x += Cfg::NTHREADS) {
-      const int rr = x / (DV / 8), cc = x % (DV / 8);
-      if (ms + rr < p.Sq && cc * 8 < p.dv_dim)
-        *reinterpret_cast<uint4*>(go + (int64_t)rr * p.o_s + cc * 8) = make_uint4(0u, 0u, 0u, 0u);
+    if constexpr (SPLIT) {
+      if (p.n_split > 1) {
+        // an empty part: the merge skips it
+        for (int x = ms + tid; x < min(ms + ROWS, n_rows); x += Cfg::NTHREADS)
+          p.part_lse[(((int64_t)b * p.Hq + hq + (x & ((1 << lg) - 1))) * p.Sq + (x >> lg)) * p.n_split + blockIdx.x % p.n_split] = neg_inf();
+        return;
+      }
     }
-    const float empty_lse = p.sink ? p.sink[hq] : neg_inf();
-    for (int rr = tid; rr < ROWS; rr += Cfg::NTHREADS)
-      if (ms + rr < p.Sq) p.lse[((int64_t)b * p.Hq + hq) * p.Sq + ms + rr] = empty_lse;
+    uint16_t* go = reinterpret_cast<uint16_t*>(p.o) + b * p.o_b + hq * p.o_h;
+    for (int x = tid; x < ROWS * (DV / 8); x += Cfg::NTHREADS) {
+      const int row = ms + x / (DV / 8), cc = x % (DV / 8);
+      if (row < n_rows && cc * 8 < p.dv_dim)
+        *reinterpret_cast<uint4*>(go + (int64_t)(row >> lg) * p.o_s + (row & ((1 << lg) - 1)) * p.o_h + cc * 8) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    for (int row = ms + tid; row < min(ms + ROWS, n_rows); row += Cfg::NTHREADS) {
+      const int h = hq + (row & ((1 << lg) - 1));
+      p.lse[((int64_t)b * p.Hq + h) * p.Sq + (row >> lg)] = p.sink ? p.sink[h] : neg_inf();
+    }
     return;
   }
   const int cnt_s[2] = {misc[2], misc[3]};
@@ -224,7 +248,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     setmaxnreg_inc<216>();
     const int s = warp >> 2;
     const int r = tid & 127;                   // row inside the sub-tile == TMEM lane
-    const int row = ms + 128 * s + r;
+    const int prow = ms + 128 * s + r;         // row of the launch
+    const int row = prow >> lg;                // its query
+    const int head = hq + (prow & ((1 << lg) - 1));
     const uint32_t lane_field = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t tS = tmem + lane_field + 128u * s;
     const uint32_t tP = tS + 64u;
@@ -323,8 +349,28 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (ok) {
       const float m_fin = (m_run == neg_inf()) ? 0.f : m_run;
       float l_tot = l_run;
-      if (p.sink) l_tot += fast_exp2(p.sink[hq] * kLog2e - m_fin);
+      if (p.sink && !(SPLIT && p.n_split > 1)) l_tot += fast_exp2(p.sink[head] * kLog2e - m_fin);
       const float inv = l_tot > 0.f ? 1.f / l_tot : 0.f;
+      if (SPLIT && p.n_split > 1) {
+        // partial result of this share of the tiles, in fp32: 4 * DV contiguous bytes per row
+        const int64_t at = (((int64_t)b * p.Hq + head) * p.Sq + row) * p.n_split + blockIdx.x % p.n_split;
+        if (prow < n_rows) p.part_lse[at] = l_tot > 0.f ? m_fin + log2f(l_tot) : neg_inf();
+#pragma unroll
+        for (int c = 0; c < DV / 32; ++c) {
+          uint32_t orr[32];
+          if (n_done > 0) {
+            tmem_ld32(tO + 32 * c, orr);
+            tc_wait_ld();
+            if (prow < n_rows) {
+#pragma unroll
+              for (int j = 0; j < 32; j += 4)
+                *reinterpret_cast<float4*>(p.part_o + at * DV + 32 * c + j) =
+                    make_float4(__uint_as_float(orr[j]) * inv, __uint_as_float(orr[j + 1]) * inv,
+                                __uint_as_float(orr[j + 2]) * inv, __uint_as_float(orr[j + 3]) * inv);
+            }
+          }
+        }
+      } else {
       uint8_t* stage = smem + Cfg::OFF_Q + s * Cfg::Q_BYTES;   // Q is no longer needed
 #pragma unroll
       for (int c = 0; c < DV / 32; ++c) {
@@ -347,20 +393,22 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           *reinterpret_cast<uint4*>(stage + r * (DV * 2) + ((chunk ^ (r & (DV / 8 - 1))) << 4)) = v;
         }
       }
-      if (row < p.Sq)
-        p.lse[((int64_t)b * p.Hq + hq) * p.Sq + row] = l_tot > 0.f ? (m_fin + log2f(l_tot)) * kLn2 : neg_inf();
+      if (prow < n_rows)
+        p.lse[((int64_t)b * p.Hq + head) * p.Sq + row] = l_tot > 0.f ? (m_fin + log2f(l_tot)) * kLn2 : neg_inf();
       __syncwarp();   // each warp stores the 32 rows it staged itself: no cross-warp dependency
       const int rbase = ms + 128 * s;
-      uint16_t* go = reinterpret_cast<uint16_t*>(p.o) + b * p.o_b + (int64_t)rbase * p.o_s + hq * p.o_h;
+      uint16_t* go = reinterpret_cast<uint16_t*>(p.o) + b * p.o_b + hq * p.o_h;
       constexpr int CH = DV / 8;                         // chunks per row
       const int wrow = (warp & 3) * 32;
 #pragma unroll 4
       for (int idx = lane; idx < 32 * CH; idx += 32) {
         const int rr = wrow + idx / CH, cc = idx % CH;
-        if (rbase + rr < p.Sq && cc * 8 < p.dv_dim) {
+        const int x = rbase + rr;
+        if (x < n_rows && cc * 8 < p.dv_dim) {
           const uint4 v = *reinterpret_cast<const uint4*>(stage + rr * (DV * 2) + ((cc ^ (rr & (CH - 1))) << 4));
-          *reinterpret_cast<uint4*>(go + (int64_t)rr * p.o_s + cc * 8) = v;
+          *reinterpret_cast<uint4*>(go + (int64_t)(x >> lg) * p.o_s + (x & ((1 << lg) - 1)) * p.o_h + cc * 8) = v;
         }
+      }
       }
     }
     if (tid == 0) FPROF(5);
@@ -496,6 +544,50 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (warp == 9) tmem_dealloc(tmem, 512);
 }
 
+// Merges the n_split partial results of every query row: one warp per (batch, head, query), lane l owns columns
+// [l DV / 32, (l + 1) DV / 32).  The partials were written a moment ago and are read from the L2.
+template <int DV, bool IS_BF16>
+__global__ void __launch_bounds__(256) fwd_combine_kernel(const AttnKParams p) {
+  constexpr int PER = DV / 32;
+  const int lane = threadIdx.x & 31;
+  const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);       // (b * Hq + h) * Sq + i
+  if (row >= (int64_t)p.B * p.Hq * p.Sq) return;
+  const int i = (int)(row % p.Sq), h = (int)(row / p.Sq % p.Hq), b = (int)(row / p.Sq / p.Hq);
+  const float* lse = p.part_lse + row * p.n_split;
+  const float mine = lane < p.n_split ? lse[lane] : neg_inf();            // n_split <= 32
+  float m = mine;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (m == neg_inf()) m = 0.f;
+  const float w_mine = exp2f(mine - m);
+  float l = w_mine;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+  float acc[PER];
+#pragma unroll
+  for (int c = 0; c < PER; ++c) acc[c] = 0.f;
+  const float* src = p.part_o + row * p.n_split * DV + lane * PER;
+  for (int s = 0; s < p.n_split; ++s) {
+    const float w = __shfl_sync(0xffffffffu, w_mine, s);
+    if (w == 0.f) continue;                                               // (an empty part's O is not written)
+    if constexpr (PER == 4) {
+      const float4 v = *reinterpret_cast<const float4*>(src + s * DV);
+      acc[0] += w * v.x; acc[1] += w * v.y; acc[2] += w * v.z; acc[3] += w * v.w;
+    } else {
+      const float2 v = *reinterpret_cast<const float2*>(src + s * DV);
+      acc[0] += w * v.x; acc[1] += w * v.y;
+    }
+  }
+  if (p.sink) l += exp2f(p.sink[h] * kLog2e - m);
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+  if (lane == 0) p.lse[row] = l > 0.f ? (m + log2f(l)) * kLn2 : neg_inf();
+  if (lane * PER < p.dv_dim) {
+    uint32_t* out = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(p.o) + b * p.o_b + (int64_t)i * p.o_s + h * p.o_h + lane * PER);
+#pragma unroll
+    for (int c = 0; c < PER; c += 2) out[c / 2] = pack2<IS_BF16>(acc[c] * inv, acc[c + 1] * inv);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------
@@ -522,12 +614,12 @@ EncodeTiledFn get_encode_tiled() {
 }
 
 int make_bshd_tmap(CUtensorMap* out, const void* base, int dtype, int B, int S, int H, int D, int64_t sb,
-                   int64_t ss, int64_t sh, int box_rows, int box_cols) {
+                   int64_t ss, int64_t sh, int box_rows, int box_cols, int box_heads) {
   EncodeTiledFn enc = get_encode_tiled();
   FM_REQUIRE(enc != nullptr, FM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
   const cuuint64_t strides[3] = {(cuuint64_t)sh * 2, (cuuint64_t)ss * 2, (cuuint64_t)(sb > 0 ? sb : ss * S) * 2};
-  const cuuint32_t box[4] = {(cuuint32_t)box_cols, 1, (cuuint32_t)box_rows, 1};
+  const cuuint32_t box[4] = {(cuuint32_t)box_cols, (cuuint32_t)box_heads, (cuuint32_t)box_rows, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUresult r = enc(out, dtype == FM_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                          4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -564,29 +656,81 @@ int bounded_wait_selftest_launch(uint64_t budget_ns, cudaStream_t s) {
   return FM_OK;
 }
 
-template <int D, int DV, bool IS_BF16, int BLOCK_SCORE, bool BLOCK_BOS>
+// Split plan of a call (SPLIT above): heads packed per query, parts, bytes of partial results.
+//
+// The plan is for calls without a mask tensor (the tiles a mask leaves are not known to the host) whose row blocks
+// do not fill the chip.  Packing is taken where it saves row blocks.  The number of parts minimises
+// waves x (tiles per part + 4): an unsplit tile step is 1 to 1.7 us and entry, list build and epilogue of a CTA cost
+// about four of them.  512 queries against 16384 keys (32 / 8 heads, d = 128): 64 CTAs of 128 tiles -> 128 of 64,
+// 231 -> 125 us; one query of 8 sequences against 8192 keys: 256 CTAs -> 128 packed ones, 220 -> 69 us.
+struct FwdSplitPlan { int pack_log2, n_split; size_t bytes; };
+static FwdSplitPlan fwd_split_plan(const fm_attn_args* a) {
+  FwdSplitPlan pl{0, 1, 0};
+  if (a->ncols != 0 || a->d > 128 || a->dv > 128) return pl;
+  const int G = a->Hq / a->Hkv, n_sm = sm_count();
+  auto blocks = [&](int64_t rows) { return (rows + 255) / 256; };
+  int64_t units = blocks(a->Sq) * a->Hq * a->B;
+  if (units >= 4 * n_sm && blocks(a->Sq) > 1) return pl;
+  if ((G & (G - 1)) == 0 && G <= 128 && blocks((int64_t)a->Sq * G) < blocks(a->Sq) * G) {
+    while ((1 << pl.pack_log2) < G) ++pl.pack_log2;
+    units = blocks((int64_t)a->Sq * G) * a->Hkv * a->B;
+  }
+  const int tiles = (a->Sk + 127) / 128;
+  double best = 1e30;
+  for (int s = 1; s <= 32 && s <= tiles && (s == 1 || units < n_sm); ++s) {
+    const double cost = (double)((units * s + n_sm - 1) / n_sm) * ((double)tiles / s + 4) + (s > 1 ? 3 : 0);
+    if (cost < best) { best = cost; pl.n_split = s; }
+  }
+  if (pl.n_split > 1) pl.bytes = (size_t)a->B * a->Hq * a->Sq * pl.n_split * (((a->d <= 64 && a->dv <= 64) ? 64 : 128) + 1) * sizeof(float);
+  return pl;
+}
+
+size_t fwd_sm100_workspace_bytes(const fm_attn_args* a) { return fwd_split_plan(a).bytes; }
+
+template <int D, int DV, bool IS_BF16, int BLOCK_SCORE, bool BLOCK_BOS, bool SPLIT = false>
 static int launch_fwd_sm100(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s) {
   using Cfg = FwdSm100Cfg<D, DV>;
   FM_REQUIRE((a->Sk + 127) / 128 <= Cfg::LIST_MAX, FM_ERR_UNSUPPORTED,
              "forward: Sk=%d exceeds the %d keys this kernel variant indexes", a->Sk, Cfg::LIST_MAX * 128);
   CUtensorMap tq, tk, tv;
   int rc;
-  if ((rc = make_bshd_tmap(&tq, a->q, a->dtype, a->B, a->Sq, a->Hq, a->d, a->q_stride[0], a->q_stride[1], a->q_stride[2], 128))) return rc;
+  if ((rc = make_bshd_tmap(&tq, a->q, a->dtype, a->B, a->Sq, a->Hq, a->d, a->q_stride[0], a->q_stride[1], a->q_stride[2], 128 >> p.pack_log2, 64, 1 << p.pack_log2))) return rc;
   if ((rc = make_bshd_tmap(&tk, a->k, a->dtype, a->B, a->Sk, a->Hkv, a->d, a->k_stride[0], a->k_stride[1], a->k_stride[2], 128))) return rc;
   if ((rc = make_bshd_tmap(&tv, a->v, a->dtype, a->B, a->Sk, a->Hkv, a->dv, a->v_stride[0], a->v_stride[1], a->v_stride[2], 128))) return rc;
-  auto kern = fwd_sm100_kernel<D, DV, IS_BF16, BLOCK_SCORE, BLOCK_BOS>;
+  auto kern = fwd_sm100_kernel<D, DV, IS_BF16, BLOCK_SCORE, BLOCK_BOS, SPLIT>;
   constexpr int smem_bytes = BLOCK_BOS ? Cfg::SMEM_BS : Cfg::SMEM;
   FM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-  dim3 grid((p.Sq + Cfg::ROWS - 1) / Cfg::ROWS, p.Hq, p.B);
+  dim3 grid(((p.Sq << p.pack_log2) + Cfg::ROWS - 1) / Cfg::ROWS, p.Hq >> p.pack_log2, p.B);
+  if (SPLIT) grid.x *= p.n_split;
   kern<<<grid, Cfg::NTHREADS, smem_bytes, s>>>(tq, tk, tv, p);
   count_launches(1);
   FM_CUDA_TRY(cudaGetLastError());
+  if (SPLIT && p.n_split > 1) {
+    fwd_combine_kernel<DV, IS_BF16><<<(unsigned)(((int64_t)p.B * p.Hq * p.Sq + 7) / 8), 256, 0, s>>>(p);
+    count_launches(1);
+    FM_CUDA_TRY(cudaGetLastError());
+  }
   return FM_OK;
 }
 
-int fwd_sm100_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s) {
+int fwd_sm100_launch(const AttnKParams& p_in, const fm_attn_args* a, cudaStream_t s) {
+  AttnKParams p = p_in;
   const bool bf = a->dtype == FM_DTYPE_BF16;
   const bool small = a->d <= 64 && a->dv <= 64;
+  if (!p.block_logit) {
+    FwdSplitPlan pl = fwd_split_plan(a);
+    if (pl.bytes && (!a->workspace || a->workspace_bytes < pl.bytes || ((uintptr_t)a->workspace & 15))) pl.n_split = 1;
+    p.pack_log2 = pl.pack_log2;
+    p.n_split = pl.n_split;
+    if (pl.n_split > 1) {
+      p.part_o = reinterpret_cast<float*>(a->workspace);
+      p.part_lse = p.part_o + (size_t)p.B * p.Hq * p.Sq * pl.n_split * (small ? 64 : 128);
+    }
+    if (pl.n_split > 1 || pl.pack_log2) {
+      if (small) return bf ? launch_fwd_sm100<64, 64, true, 0, false, true>(p, a, s) : launch_fwd_sm100<64, 64, false, 0, false, true>(p, a, s);
+      return bf ? launch_fwd_sm100<128, 128, true, 0, false, true>(p, a, s) : launch_fwd_sm100<128, 128, false, 0, false, true>(p, a, s);
+    }
+  }
 #define FM_FWD_DISPATCH(BSZ, BOS)                                                                         \
   do {                                                                                                    \
     if (a->d == 192)                                                                                      \

@@ -441,10 +441,10 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 EncodeTiledFn get_encode_tiled();
 
 // [B, S, H, D] tensor (element strides sb, ss, sh; innermost contiguous) as a
-// 4-D map (D, H, S, B) with a cols x 1 x rows x 1 box: 64 columns with 128-byte
+// 4-D map (D, H, S, B) with a cols x heads x rows x 1 box: 64 columns with 128-byte
 // swizzle, or 32 columns with 64-byte swizzle.
 int make_bshd_tmap(CUtensorMap* out, const void* base, int dtype, int B, int S, int H, int D, int64_t sb,
-                   int64_t ss, int64_t sh, int box_rows, int box_cols = 64);
+                   int64_t ss, int64_t sh, int box_rows, int box_cols = 64, int box_heads = 1);
 
 }  // namespace sm100
 }  // namespace fm

@@ -228,6 +228,10 @@ def _flash_attn_fwd(q, k, v, startend_row_indices=None, softmax_scale=None, caus
         a.fwd_order = _launch_order(a, info, _lib.FM_ORDER_FWD, q)
     if block_logit is None:
         assert block_bos is None, "block_bos requires block_logit (it drives its relative bucketing)"
+        nbytes = _lib.load().fm_fwd_workspace_bytes(C.byref(a))
+        if nbytes:
+            ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+            a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
         _lib.check(_lib.load().fm_fwd(C.byref(a), _stream(q)), "fm_fwd")
         return out, lse
     assert not pack_gqa, "block_logit requires pack_gqa=False: it is indexed by the query head and the query row"

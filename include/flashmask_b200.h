@@ -189,7 +189,12 @@ FM_API unsigned long long fm_launch_count(void);
 /* Forward: O = softmax(QK^T*scale + M [, sink]) V and LSE.
  * Replaces _flash_attn_fwd (flashmask/cute/ops/fwd.py:52-882) +
  * FlashAttentionForwardSm100 (flashmask/cute/flash_fwd_sm100.py:1485-2104).
- * Uses no workspace. */
+ * Workspace (args->workspace, 16-byte aligned) is optional: with at least
+ * fm_fwd_workspace_bytes(args) bytes a call with few query rows against many
+ * keys may deal the K tiles of a row block to several CTAs and merge their fp32
+ * partial results; without it every row block is one CTA's.  0 bytes: the call
+ * would not be split. */
+FM_API size_t fm_fwd_workspace_bytes(const fm_attn_args* args);
 FM_API int fm_fwd(const fm_attn_args* args, void* stream);
 
 /* fm_fwd with the fused block-score side output: besides O and LSE, for every
@@ -204,7 +209,7 @@ FM_API int fm_fwd(const fm_attn_args* args, void* stream);
  * ids are relative to that column: block j of a row covers the columns
  * [bos + j * block_size, bos + (j + 1) * block_size); NULL means bos = 0.
  * block_size is 32, 64 or 128; block_ld >= ceil(Sk / block_size); O and LSE
- * are bitwise those of fm_fwd.  Every head dim fm_fwd takes is served.
+ * are bitwise those of fm_fwd without a workspace.  Every head dim fm_fwd takes is served.
  * Replaces the block_logit / block_size / block_bos arguments of
  * _flash_attn_fwd (flashmask/cute/ops/fwd.py:75-77,605-658) and the fused
  * epilogue of flashmask/cute/flash_fwd_sm100.py:4256-4371. */

@@ -189,6 +189,22 @@ def test_masks_pair_kernels_two_slices(kind, d, dv):
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("kind", ["none_causal", "none_full"])
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,d,dv,sink", [
+    (1, 1, 2048, 8, 1, 128, 128, True),       # one query, every head of the group in one row block
+    (2, 1, 2304, 4, 2, 64, 64, False),
+    (1, 33, 4097, 8, 1, 128, 128, False),     # packed rows end inside the second sub-tile, one key in the last tile
+    (1, 129, 2050, 6, 2, 96, 80, True),       # three heads per group: split, not packed; padded head dims
+    (1, 300, 700, 4, 1, 128, 128, False),     # packed, too few keys to split
+    (1, 4, 5000, 128, 1, 64, 64, False)])     # 128 heads per query: one query per sub-tile
+def test_few_queries_many_keys(kind, B, Sq, Sk, Hq, Hkv, d, dv, sink):
+    """The forward that packs the heads of a group into the rows of a CTA and deals the K tiles of a row block to
+    several CTAs (calls without a mask tensor that would leave most of the chip idle)."""
+    _run(kind, B, Sq, Sk, Hq, Hkv, d, dv, sink=sink, seed=91)
+    _run(kind, B, Sq, Sk, Hq, Hkv, d, dv, sink=sink, seed=92, dtype=torch.float16)
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("kind", MASKS)
 def test_masks_d64(kind, fwd_variant):
     """Every mask family through the 64-column variants: GQA, rows long enough to wrap the K/V ring."""
