@@ -5,7 +5,9 @@
 Every ``csrc/*.cu`` is compiled to an object under ``build/`` (in parallel,
 skipped when the object is newer than all sources and headers) and linked into
 ``flashmask_b200/libflashmask_b200.so``.  The host C++ solver sources
-(``csrc/*.cpp``) go through the same nvcc invocation.
+(``csrc/*.cpp``) go through the same nvcc invocation.  ``csrc/torch/fm_torch.cpp``,
+the native host path of the operator, is compiled against torch into
+``flashmask_b200/_host.so`` and finds the library beside itself.
 """
 from __future__ import annotations
 
@@ -21,6 +23,8 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OUT = os.path.join(PKG, "libflashmask_b200.so")
+HOST_SRC = os.path.join(CSRC, "torch", "fm_torch.cpp")
+HOST_OUT = os.path.join(PKG, "_host.so")
 OBJ = os.path.join(ROOT, "build", "obj")
 
 NVCC_FLAGS = [
@@ -42,6 +46,22 @@ def _stale(obj: str, deps) -> bool:
         return True
     t = os.path.getmtime(obj)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _host_command():
+    """g++ invocation of the native host path (no device code, no pybind beyond torch's own)."""
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension as ce
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for d in ce.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include"),
+                                   os.path.join(ROOT, "include")]:
+        cmd += ["-isystem", d]
+    return cmd + [HOST_SRC, "-o", HOST_OUT, f"-L{lib}", f"-L{PKG}", "-ltorch", "-ltorch_cpu", "-ltorch_python",
+                  "-lc10", "-lc10_cuda", "-l:libflashmask_b200.so", "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -81,6 +101,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    hdr = os.path.join(ROOT, "include", "flashmask_b200.h")
+    if force or _stale(HOST_OUT, [HOST_SRC, hdr, os.path.abspath(__file__)]):
+        r = subprocess.run(_host_command(), capture_output=True, text=True)
+        if verbose or r.returncode:
+            sys.stderr.write(r.stdout + r.stderr)
+        if r.returncode:
+            raise RuntimeError(f"g++ failed on {HOST_SRC}")
     return OUT
 
 

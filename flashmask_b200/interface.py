@@ -20,7 +20,26 @@ from .ops import _check_shapes, _flash_attn_bwd, _flash_attn_fwd, fwd_tile_shape
 __all__ = ["flashmask_attention", "FlashMaskFunc", "sliding_window_indices"]
 
 
+_host = None
+
+
+def _native_host():
+    """The native host path (csrc/torch/fm_torch.cpp): checks, allocations, autograd node and library calls."""
+    global _host
+    if _host is None:
+        try:
+            from . import _host as ext
+        except ImportError as e:
+            raise RuntimeError("flashmask_b200/_host.so is missing or does not load: build it with "
+                               "`python -m flashmask_b200.build`. There is no fallback path.") from e
+        _host = ext
+    return _host
+
+
 class FlashMaskFunc(torch.autograd.Function):
+    """The operator as a Python autograd function over ops.py; ``flashmask_attention`` runs the same calls
+    natively."""
+
     @staticmethod
     def forward(ctx, q, k, v, startend_row_indices, softmax_scale, causal, learnable_sink,
                 deterministic):
@@ -106,6 +125,6 @@ def flashmask_attention(query, key, value, startend_row_indices: Optional[torch.
                                           softmax_scale=softmax_scale, sink=sink,
                                           deterministic=deterministic, group=group)
     else:
-        out, lse = FlashMaskFunc.apply(query, key, value, startend_row_indices, softmax_scale, causal,
-                                       sink, deterministic)
+        out, lse = _native_host().attention(query, key, value, startend_row_indices, sink, softmax_scale,
+                                            bool(causal), -1 if deterministic is None else int(bool(deterministic)))
     return (out, lse) if want_lse else out
