@@ -33,8 +33,10 @@ struct AttnKParams {
   // masked, scaled scores, combined into block_logit[b][head][row][block] with fmax; block ids are
   // relative to block_bos[b][row] (the first key of the row's document) when that is given
   float* block_logit; const int32_t* block_bos;
-  // forward over packed heads / split keys: log2(heads packed per query), parts of a row block's K tiles, partial results
-  int pack_log2, n_split;
+  // forward over packed heads / split keys: log2(heads packed per query), CTAs a row block's K tiles are dealt to,
+  // whether the two sub-tiles of a CTA hold the same rows and take its tiles in turn (two partial results per CTA
+  // then), partial results
+  int pack_log2, n_split, alternate;
   float* part_o; float* part_lse;
   int block_log2, block_cols, block_ld;   // log2(block size), ceil(Sk / block size), row stride
 };

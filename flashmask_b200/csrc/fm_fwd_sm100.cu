@@ -92,6 +92,9 @@ __device__ __forceinline__ float neg_inf() { return __int_as_float(0xff800000); 
 // The rows of a CTA are (query, head of the GQA group) pairs, 2^pack_log2 heads per query, so that the heads
 // sharing a K / V tile share its loads; the K tiles of a row block are dealt to n_split CTAs, whose partial
 // results (fp32 O / l and m + log2 l) fwd_combine_kernel merges.
+// p.alternate (SPLIT, all rows of the launch fit one sub-tile): both sub-tiles hold the same rows and take the CTA's
+// K tiles in turn, each with its own running maximum, sum and O, merged like two parts.  With the second sub-tile
+// idle, scores, softmax and P V of one tile after the other form one dependent chain; two chains overlap.
 template <int D, int DV, bool IS_BF16, int BLOCK_SCORE, bool BLOCK_BOS, bool SPLIT>
 __global__ void __launch_bounds__(384, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -128,9 +131,14 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int bh_mask = md.ncols ? ((md.mask_B == 1 ? 0 : b) * md.Hm + hq / (p.Hq / md.Hm)) : 0;
   const int ms = t * ROWS;
   const int off = p.Sk - p.Sq;
+  const bool alt = SPLIT && p.alternate;
+  const int sub_rows = alt ? 0 : 128;        // first row of sub-tile 1 against that of sub-tile 0
   // queries [q_lo(s), q_hi(s)) of sub-tile s
-  auto q_lo = [&](int s) { return (ms + 128 * s) >> lg; };
-  auto q_hi = [&](int s) { return min(((ms + 128 * s + 127) >> lg) + 1, p.Sq); };
+  auto q_lo = [&](int s) { return (ms + sub_rows * s) >> lg; };
+  auto q_hi = [&](int s) { return min(((ms + sub_rows * s + 127) >> lg) + 1, p.Sq); };
+  // partial result of sub-tile s: its place among the parts of a row
+  const int n_parts = SPLIT ? p.n_split << (alt ? 1 : 0) : 1;
+  auto part_of = [&](int s) { return (int)(blockIdx.x % p.n_split) * (alt ? 2 : 1) + (alt ? s : 0); };
   // first K tile right of everything these rows can see, and whether the diagonal tile is loaded ahead of the list
   const int nb = (p.Sk + 127) / 128;
   const int n_hi = md.causal ? max(0, min(nb, (q_hi(1) + off + 127) / 128)) : nb;
@@ -222,10 +230,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     if (warp == 9) tmem_dealloc(tmem, 512);
     if constexpr (SPLIT) {
-      if (p.n_split > 1) {
-        // an empty part: the merge skips it
-        for (int x = ms + tid; x < min(ms + ROWS, n_rows); x += Cfg::NTHREADS)
-          p.part_lse[(((int64_t)b * p.Hq + hq + (x & ((1 << lg) - 1))) * p.Sq + (x >> lg)) * p.n_split + blockIdx.x % p.n_split] = neg_inf();
+      if (n_parts > 1) {
+        // empty parts: the merge skips them
+        for (int s = 0; s <= (alt ? 1 : 0); ++s)
+          for (int x = ms + tid; x < min(ms + ROWS, n_rows); x += Cfg::NTHREADS)
+            p.part_lse[(((int64_t)b * p.Hq + hq + (x & ((1 << lg) - 1))) * p.Sq + (x >> lg)) * n_parts + part_of(s)] = neg_inf();
         return;
       }
     }
@@ -248,7 +257,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     setmaxnreg_inc<216>();
     const int s = warp >> 2;
     const int r = tid & 127;                   // row inside the sub-tile == TMEM lane
-    const int prow = ms + 128 * s + r;         // row of the launch
+    const int prow = ms + sub_rows * s + r;    // row of the launch
+    const bool no_rows = SPLIT && prow - lane >= n_rows;   // the whole warp: it keeps pace with the barriers only
     const int row = prow >> lg;                // its query
     const int head = hq + (prow & ((1 << lg) - 1));
     const uint32_t lane_field = (uint32_t)((warp & 3) * 32) << 16;
@@ -287,7 +297,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     auto bs_flush = [&](int g) { block_flush<BS_ACC_STRIDE>(bs_dst, bs_acc, g, bs_vec, p.block_cols); };
     for (int i = 0; i < cnt && ok; ++i) {
       const uint32_t e = list[i];
-      const uint32_t flags = (e >> (16 + 4 * s)) & 0xFu;
+      uint32_t flags = (e >> (16 + 4 * s)) & 0xFu;
+      if constexpr (SPLIT) { if (alt) flags = (i & 1) == s ? (e >> 16) & 0xFu : 0u; }
       const bool any_bounds = (((e >> 16) | (e >> 20)) & FM_TF_BOUNDS) != 0;
       const int bslot = nbnd % Cfg::NBND;
       const uint32_t bpar = (uint32_t)(nbnd / Cfg::NBND) & 1u;
@@ -320,12 +331,14 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         ok = __all_sync(0xffffffffu, mbar_wait(bar(Cfg::B_SFULL + s), (uint32_t)n_done & 1u, wc));
         if (!ok) break;
         if (tid == 0 && n_done == 0) FPROF(2);
+        if (!no_rows) {
 #define FM_N_UNIT n_done
 #define FM_N_TOT n_done
 #include "fm_fwd_sm100_tile.inc"
 #undef FM_N_UNIT
 #undef FM_N_TOT
-        tc_wait_st();
+          tc_wait_st();
+        }
         tc_fence_before();
         mbar_arrive(bar(Cfg::B_PFULL + s));
         ++n_done;
@@ -349,11 +362,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (ok) {
       const float m_fin = (m_run == neg_inf()) ? 0.f : m_run;
       float l_tot = l_run;
-      if (p.sink && !(SPLIT && p.n_split > 1)) l_tot += fast_exp2(p.sink[head] * kLog2e - m_fin);
+      if (p.sink && n_parts == 1) l_tot += fast_exp2(p.sink[head] * kLog2e - m_fin);
       const float inv = l_tot > 0.f ? 1.f / l_tot : 0.f;
-      if (SPLIT && p.n_split > 1) {
+      if (SPLIT && n_parts > 1) {
         // partial result of this share of the tiles, in fp32: 4 * DV contiguous bytes per row
-        const int64_t at = (((int64_t)b * p.Hq + head) * p.Sq + row) * p.n_split + blockIdx.x % p.n_split;
+        const int64_t at = (((int64_t)b * p.Hq + head) * p.Sq + row) * n_parts + part_of(s);
         if (prow < n_rows) p.part_lse[at] = l_tot > 0.f ? m_fin + log2f(l_tot) : neg_inf();
 #pragma unroll
         for (int c = 0; c < DV / 32; ++c) {
@@ -494,13 +507,33 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           tc_commit(bar(Cfg::B_ODONE + s));
           ++npv[s];
         };
-        if (cnt > 0) {
+        if (alt) {
+          // tile i belongs to sub-tile i & 1; its scores are issued before the P V of the tile ahead of it
+          auto pv_then_qk = [&](auto sub, int i) {
+            issue_pv(sub, i);
+            if (ok) tc_commit(bar(Cfg::B_KVEMPTY + (2 * i + 1) % Cfg::NSTAGE));
+            if (ok && i + 2 < cnt) {
+              issue_qk(sub, i + 2);
+              if (ok) tc_commit(bar(Cfg::B_KVEMPTY + (2 * i + 4) % Cfg::NSTAGE));
+            }
+          };
+          issue_qk(std::integral_constant<int, 0>{}, 0);
+          if (ok) tc_commit(bar(Cfg::B_KVEMPTY + 0));
+          if (ok && cnt > 1) {
+            issue_qk(std::integral_constant<int, 1>{}, 1);
+            if (ok) tc_commit(bar(Cfg::B_KVEMPTY + 2 % Cfg::NSTAGE));
+          }
+          for (int i = 0; i < cnt && ok; i += 2) {
+            pv_then_qk(std::integral_constant<int, 0>{}, i);
+            if (ok && i + 1 < cnt) pv_then_qk(std::integral_constant<int, 1>{}, i + 1);
+          }
+        } else if (cnt > 0) {
           const uint32_t e = list[0];
           if ((e >> 16) & 0xFu) issue_qk(std::integral_constant<int, 0>{}, 0);
           if ((e >> 20) & 0xFu) issue_qk(std::integral_constant<int, 1>{}, 0);
           if (ok) tc_commit(bar(Cfg::B_KVEMPTY + 0));
         }
-        for (int i = 0; i < cnt && ok; ++i) {
+        for (int i = 0; i < cnt && ok && !alt; ++i) {
           const uint32_t e = list[i];
           const uint32_t en = (i + 1 < cnt) ? list[i + 1] : 0u;
           // the sub-tile whose P is ready first goes first (sub-tile 0 when both or neither are)
@@ -544,7 +577,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (warp == 9) tmem_dealloc(tmem, 512);
 }
 
-// Merges the n_split partial results of every query row: one warp per (batch, head, query), lane l owns columns
+// Merges the partial results of every query row: one warp per (batch, head, query), lane l owns columns
 // [l DV / 32, (l + 1) DV / 32).  The partials were written a moment ago and are read from the L2.
 template <int DV, bool IS_BF16>
 __global__ void __launch_bounds__(256) fwd_combine_kernel(const AttnKParams p) {
@@ -553,8 +586,9 @@ __global__ void __launch_bounds__(256) fwd_combine_kernel(const AttnKParams p) {
   const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);       // (b * Hq + h) * Sq + i
   if (row >= (int64_t)p.B * p.Hq * p.Sq) return;
   const int i = (int)(row % p.Sq), h = (int)(row / p.Sq % p.Hq), b = (int)(row / p.Sq / p.Hq);
-  const float* lse = p.part_lse + row * p.n_split;
-  const float mine = lane < p.n_split ? lse[lane] : neg_inf();            // n_split <= 32
+  const int n_parts = p.n_split << p.alternate;                            // <= 32
+  const float* lse = p.part_lse + row * n_parts;
+  const float mine = lane < n_parts ? lse[lane] : neg_inf();
   float m = mine;
 #pragma unroll
   for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -566,8 +600,8 @@ __global__ void __launch_bounds__(256) fwd_combine_kernel(const AttnKParams p) {
   float acc[PER];
 #pragma unroll
   for (int c = 0; c < PER; ++c) acc[c] = 0.f;
-  const float* src = p.part_o + row * p.n_split * DV + lane * PER;
-  for (int s = 0; s < p.n_split; ++s) {
+  const float* src = p.part_o + row * n_parts * DV + lane * PER;
+  for (int s = 0; s < n_parts; ++s) {
     const float w = __shfl_sync(0xffffffffu, w_mine, s);
     if (w == 0.f) continue;                                               // (an empty part's O is not written)
     if constexpr (PER == 4) {
@@ -662,10 +696,15 @@ int bounded_wait_selftest_launch(uint64_t budget_ns, cudaStream_t s) {
 // do not fill the chip.  Packing is taken where it saves row blocks.  The number of parts minimises
 // waves x (tiles per part + 4): an unsplit tile step is 1 to 1.7 us and entry, list build and epilogue of a CTA cost
 // about four of them.  512 queries against 16384 keys (32 / 8 heads, d = 128): 64 CTAs of 128 tiles -> 128 of 64,
-// 231 -> 125 us; one query of 8 sequences against 8192 keys: 256 CTAs -> 128 packed ones, 220 -> 69 us.
-struct FwdSplitPlan { int pack_log2, n_split; size_t bytes; };
+// 231 -> 143 us; one query of 8 sequences against 8192 keys: 256 CTAs -> 128 packed ones, 220 -> 69 us.
+//
+// Where all rows of a block fit one sub-tile (packed decoding, up to 128 rows) both sub-tiles take its tiles in turn
+// // (p.alternate) from two tiles on: two chains of scores, softmax and P V instead of one, and a step is counted as 0.6
+// of an unalternated one.  8 sequences against 8192 keys (32 / 8 heads): 69 -> 56 us (4.8 TB/s of K / V); one
+// sequence against 32768 keys 39 us (3.4 TB/s).
+struct FwdSplitPlan { int pack_log2, n_split; bool alternate; size_t bytes; };
 static FwdSplitPlan fwd_split_plan(const fm_attn_args* a) {
-  FwdSplitPlan pl{0, 1, 0};
+  FwdSplitPlan pl{0, 1, false, 0};
   if (a->ncols != 0 || a->d > 128 || a->dv > 128) return pl;
   const int G = a->Hq / a->Hkv, n_sm = sm_count();
   auto blocks = [&](int64_t rows) { return (rows + 255) / 256; };
@@ -676,12 +715,15 @@ static FwdSplitPlan fwd_split_plan(const fm_attn_args* a) {
     units = blocks((int64_t)a->Sq * G) * a->Hkv * a->B;
   }
   const int tiles = (a->Sk + 127) / 128;
+  pl.alternate = ((int64_t)a->Sq << pl.pack_log2) <= 128 && tiles >= 2;
+  const double step = pl.alternate ? 0.6 : 1.0;
   double best = 1e30;
-  for (int s = 1; s <= 32 && s <= tiles && (s == 1 || units < n_sm); ++s) {
-    const double cost = (double)((units * s + n_sm - 1) / n_sm) * ((double)tiles / s + 4) + (s > 1 ? 3 : 0);
+  for (int s = 1; s <= (pl.alternate ? 16 : 32) && s <= tiles && (s == 1 || units < n_sm); ++s) {
+    const double cost = (double)((units * s + n_sm - 1) / n_sm) * (step * tiles / s + 4) + (s > 1 ? 3 : 0);
     if (cost < best) { best = cost; pl.n_split = s; }
   }
-  if (pl.n_split > 1) pl.bytes = (size_t)a->B * a->Hq * a->Sq * pl.n_split * (((a->d <= 64 && a->dv <= 64) ? 64 : 128) + 1) * sizeof(float);
+  const size_t parts = (size_t)pl.n_split << pl.alternate;
+  if (parts > 1) pl.bytes = (size_t)a->B * a->Hq * a->Sq * parts * (((a->d <= 64 && a->dv <= 64) ? 64 : 128) + 1) * sizeof(float);
   return pl;
 }
 
@@ -705,7 +747,7 @@ static int launch_fwd_sm100(const AttnKParams& p, const fm_attn_args* a, cudaStr
   kern<<<grid, Cfg::NTHREADS, smem_bytes, s>>>(tq, tk, tv, p);
   count_launches(1);
   FM_CUDA_TRY(cudaGetLastError());
-  if (SPLIT && p.n_split > 1) {
+  if (SPLIT && (p.n_split << p.alternate) > 1) {
     fwd_combine_kernel<DV, IS_BF16><<<(unsigned)(((int64_t)p.B * p.Hq * p.Sq + 7) / 8), 256, 0, s>>>(p);
     count_launches(1);
     FM_CUDA_TRY(cudaGetLastError());
@@ -719,14 +761,16 @@ int fwd_sm100_launch(const AttnKParams& p_in, const fm_attn_args* a, cudaStream_
   const bool small = a->d <= 64 && a->dv <= 64;
   if (!p.block_logit) {
     FwdSplitPlan pl = fwd_split_plan(a);
-    if (pl.bytes && (!a->workspace || a->workspace_bytes < pl.bytes || ((uintptr_t)a->workspace & 15))) pl.n_split = 1;
+    if (pl.bytes && (!a->workspace || a->workspace_bytes < pl.bytes || ((uintptr_t)a->workspace & 15))) { pl.n_split = 1; pl.alternate = false; }
     p.pack_log2 = pl.pack_log2;
     p.n_split = pl.n_split;
-    if (pl.n_split > 1) {
+    p.alternate = pl.alternate;
+    const int parts = pl.n_split << pl.alternate;
+    if (parts > 1) {
       p.part_o = reinterpret_cast<float*>(a->workspace);
-      p.part_lse = p.part_o + (size_t)p.B * p.Hq * p.Sq * pl.n_split * (small ? 64 : 128);
+      p.part_lse = p.part_o + (size_t)p.B * p.Hq * p.Sq * parts * (small ? 64 : 128);
     }
-    if (pl.n_split > 1 || pl.pack_log2) {
+    if (parts > 1 || pl.pack_log2) {
       if (small) return bf ? launch_fwd_sm100<64, 64, true, 0, false, true>(p, a, s) : launch_fwd_sm100<64, 64, false, 0, false, true>(p, a, s);
       return bf ? launch_fwd_sm100<128, 128, true, 0, false, true>(p, a, s) : launch_fwd_sm100<128, 128, false, 0, false, true>(p, a, s);
     }

@@ -205,6 +205,20 @@ def test_few_queries_many_keys(kind, B, Sq, Sk, Hq, Hkv, d, dv, sink):
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,d,dv", [
+    (1, 1, 129, 4, 1, 128, 128),      # two tiles: one per sub-tile
+    (2, 1, 300, 4, 4, 64, 64),        # an odd number of tiles, one row
+    (1, 32, 641, 4, 1, 128, 128),     # 128 packed rows: a full sub-tile
+    (1, 33, 641, 4, 1, 128, 128),     # 132: past it, so one tile serves both sub-tiles again
+    (1, 128, 1500, 3, 1, 64, 48),     # 128 rows unpacked, several diagonal tiles
+    (3, 2, 9000, 16, 2, 96, 96)])     # several CTAs per row block, some of them with an odd share
+def test_rows_of_one_sub_tile(B, Sq, Sk, Hq, Hkv, d, dv):
+    """Calls whose rows fit one sub-tile of a CTA: the two sub-tiles take the K tiles in turn and are merged."""
+    for kind in ("none_causal", "none_full"):
+        _run(kind, B, Sq, Sk, Hq, Hkv, d, dv, sink=True, seed=93)
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("kind", MASKS)
 def test_masks_d64(kind, fwd_variant):
     """Every mask family through the 64-column variants: GQA, rows long enough to wrap the K/V ring."""
