@@ -394,6 +394,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const AttnKParams p
   constexpr int RPW = 32 / LPR;                       // rows per warp
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane / LPR, ln = lane % LPR;
+  grid_dep_trigger();
   const int row = (blockIdx.x * 8 + warp) * RPW + sub, hq = blockIdx.y, b = blockIdx.z;
   float acc = 0.f, lse2 = 0.f;
   if (row < p.Sq) {

@@ -233,6 +233,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
   tc_fence_after();
   const uint32_t tmem = (uint32_t)misc[0];
   const int cnt = misc[1];
+  if constexpr (MODE == MODE_DKDV) {
+    grid_dep_wait();                    // row statistics of the preprocess kernel
+    grid_dep_trigger();                 // the dQ kernel reads nothing of this one: it fills the SMs this one leaves
+  }
   WaitCtx wc{misc + 4, global_timer_ns() + 2000000000ull};
   if (tid == 0) { PROF(1); PROF_VAL(10, (long long)cnt * ((MODE == MODE_DKDV) ? p.Hq / p.Hkv : 1)); }
   if (cnt == 0) {
@@ -257,6 +261,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
         if (row0 + rr < p.Sq && cc * 8 < p.d)
           *reinterpret_cast<uint4*>(gq + (int64_t)rr * p.dq_s + cc * 8) = make_uint4(0u, 0u, 0u, 0u);
       }
+      grid_dep_wait();
     }
     return;
   }
@@ -294,8 +299,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
     } else {
       const int i = row0 + r;
       if (i < p.Sq) {
-        lse2_row = p.lse_log2[((int64_t)b * p.Hq + hq0) * p.Sq_r + i];
-        dps_row = p.dpsum[((int64_t)b * p.Hq + hq0) * p.Sq_r + i];
+        // from the L2: this kernel does not wait for the one that wrote them (the dK / dV kernel before it did)
+        lse2_row = __ldcg(p.lse_log2 + ((int64_t)b * p.Hq + hq0) * p.Sq_r + i);
+        dps_row = __ldcg(p.dpsum + ((int64_t)b * p.Hq + hq0) * p.Sq_r + i);
       }
     }
 
@@ -585,6 +591,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
     if (tid == 0) atomicExch(&g_bwd_status, FM_ERR_TIMEOUT);
   }
   if (warp == 9) tmem_dealloc(tmem, 512);
+  if constexpr (MODE == MODE_DQ) grid_dep_wait();      // not complete before the dK / dV kernel is
 }
 
 // ---------------------------------------------------------------------------
@@ -620,11 +627,9 @@ static int launch_bwd_sm100(const AttnKParams& p, const fm_attn_args* a, cudaStr
   auto k2 = bwd_sm100_kernel<MODE_DQ, IS_BF16, D, DV>;
   FM_CUDA_TRY(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
   FM_CUDA_TRY(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
-  k1<<<dim3((p.Sk + 127) / 128, p.Hkv, p.B), Cfg::NTHREADS, Cfg::SMEM, s>>>(k128, v128, q64, do64, p);
-  FM_CUDA_TRY(cudaGetLastError());
-  k2<<<dim3((p.Sq + 127) / 128, p.Hq, p.B), Cfg::NTHREADS, Cfg::SMEM, s>>>(q128, do128, k64, v64, p);
+  FM_CUDA_TRY(launch_dependent(k1, dim3((p.Sk + 127) / 128, p.Hkv, p.B), dim3(Cfg::NTHREADS), Cfg::SMEM, s, k128, v128, q64, do64, p));
+  FM_CUDA_TRY(launch_dependent(k2, dim3((p.Sq + 127) / 128, p.Hq, p.B), dim3(Cfg::NTHREADS), Cfg::SMEM, s, q128, do128, k64, v64, p));
   count_launches(2);
-  FM_CUDA_TRY(cudaGetLastError());
   return FM_OK;
 }
 

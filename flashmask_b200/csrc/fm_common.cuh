@@ -27,6 +27,23 @@ int cuda_fail(cudaError_t e, const char* what);
     if (_e != cudaSuccess) return ::fm::cuda_fail(_e, #expr); \
   } while (0)
 
+// Programmatic launches: kernel B of a call may start while kernel A before it drains.  A opens the door with
+// grid_dep_trigger() (only kernels that the same call always follows with another of its own do), B is launched with
+// launch_dependent() and calls grid_dep_wait() before it touches what A writes, or before it ends when it needs
+// nothing of A; either way B is complete only after A is.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 #define FM_REQUIRE(cond, code, ...)     \
   do {                                  \
     if (!(cond)) {                      \

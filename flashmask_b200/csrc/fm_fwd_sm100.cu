@@ -218,6 +218,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     cnt = cnt * (part + 1) / p.n_split - lo;
     list += lo;
   }
+  if constexpr (SPLIT) { if (n_parts > 1) grid_dep_trigger(); }     // the merge follows
   WaitCtx wc{misc + 4, global_timer_ns() + 2000000000ull};
   if (tid == 0) { FPROF(1); FPROF_VAL(7, (long long)cnt); }
   if (cnt == 0) {
@@ -584,6 +585,7 @@ __global__ void __launch_bounds__(256) fwd_combine_kernel(const AttnKParams p) {
   constexpr int PER = DV / 32;
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);       // (b * Hq + h) * Sq + i
+  grid_dep_wait();
   if (row >= (int64_t)p.B * p.Hq * p.Sq) return;
   const int i = (int)(row % p.Sq), h = (int)(row / p.Sq % p.Hq), b = (int)(row / p.Sq / p.Hq);
   const int n_parts = p.n_split << p.alternate;                            // <= 32
@@ -748,9 +750,8 @@ static int launch_fwd_sm100(const AttnKParams& p, const fm_attn_args* a, cudaStr
   count_launches(1);
   FM_CUDA_TRY(cudaGetLastError());
   if (SPLIT && (p.n_split << p.alternate) > 1) {
-    fwd_combine_kernel<DV, IS_BF16><<<(unsigned)(((int64_t)p.B * p.Hq * p.Sq + 7) / 8), 256, 0, s>>>(p);
+    FM_CUDA_TRY(launch_dependent(fwd_combine_kernel<DV, IS_BF16>, dim3((unsigned)(((int64_t)p.B * p.Hq * p.Sq + 7) / 8)), dim3(256), 0, s, p));
     count_launches(1);
-    FM_CUDA_TRY(cudaGetLastError());
   }
   return FM_OK;
 }
