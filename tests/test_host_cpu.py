@@ -75,6 +75,22 @@ def test_kernel_variant_routing_needs_no_gpu():
         assert got == has, (d, dv, got)
 
 
+def test_pair_backward_workspace_is_bounded():
+    """The CTA-pair backward keeps P and dS of at least 256 rows of a kv group: up to 8 GiB, and none at all (the
+    kernels without a workspace serve the call) where that would not do."""
+    lib = _lib.load()
+    sizes = {}
+    for Hq, Sk in ((16, 16384), (128, 65536), (128, 131072), (16, 262144), (64, 262144)):
+        a = _lib.AttnArgs()
+        a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.Hm, a.mask_B, a.d, a.dv = 1, 4096, Sk, Hq, 1, 1, 1, 576, 512
+        stats = 2 * 4 * Hq * 4096
+        n = lib.fm_bwd_workspace_bytes(ctypes.byref(a)) - stats
+        sizes[Hq, Sk] = n
+        assert n == 0 or n <= (8 << 30) + Sk * (576 + 512) * 4
+        assert (n == 0) == (Hq * Sk * 4 * 256 > 8 << 30), (Hq, Sk, n)
+    assert sizes[128, 131072] == 0 and sizes[128, 65536] > 8 << 30
+
+
 def test_struct_layout_matches_header():
     # 18 int32/float + 15 pointers/size_t + 24 int64
     assert ctypes.sizeof(_lib.AttnArgs) == 18 * 4 + 15 * 8 + 24 * 8 + 3 * 8
