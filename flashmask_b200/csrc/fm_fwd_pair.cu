@@ -11,8 +11,8 @@
 // delivers 68 B/clk per SM to all SMs together; the pair reads 32.
 //
 // Bound: the tensor pipe (2048 cycles per 128 keys and pair at d = 256, 3328 at 576; softmax 1024 exp2 cycles).
-// Measured at S = 16384, 16 heads, causal: 256/256 2.67 ms (one CTA, S computed twice) -> 1.94 ms = 1136 TFLOP/s;
-// 576/512 29.9 ms (warp MMA) -> 4.76 ms = 982 TFLOP/s of the mathematics, 1500 executed.
+// Measured at S = 16384, 16 heads, causal: 256/256 2.67 ms (one CTA, S computed twice) -> 1.47 ms = 1500 TFLOP/s;
+// 576/512 29.9 ms (warp MMA) -> 4.56 ms = 1025 TFLOP/s of the mathematics, 1560 executed.
 //
 // Warp roles of each CTA (384 threads): 0-3 / 4-7 softmax warpgroups 0 / 1: thread r of a warpgroup owns row r
 // and 64 of the tile's 128 keys, the pair of threads exchanges the row maximum through shared memory; 8 TMA

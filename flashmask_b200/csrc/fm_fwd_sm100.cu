@@ -698,11 +698,11 @@ int bounded_wait_selftest_launch(uint64_t budget_ns, cudaStream_t s) {
 // do not fill the chip.  Packing is taken where it saves row blocks.  The number of parts minimises
 // waves x (tiles per part + 4): an unsplit tile step is 1 to 1.7 us and entry, list build and epilogue of a CTA cost
 // about four of them.  512 queries against 16384 keys (32 / 8 heads, d = 128): 64 CTAs of 128 tiles -> 128 of 64,
-// 231 -> 143 us; one query of 8 sequences against 8192 keys: 256 CTAs -> 128 packed ones, 220 -> 69 us.
+// 231 -> 152 us; one query of 8 sequences against 8192 keys: 256 CTAs -> 128 packed ones, 220 -> 69 us.
 //
 // Where all rows of a block fit one sub-tile (packed decoding, up to 128 rows) both sub-tiles take its tiles in turn
 // // (p.alternate) from two tiles on: two chains of scores, softmax and P V instead of one, and a step is counted as 0.6
-// of an unalternated one.  8 sequences against 8192 keys (32 / 8 heads): 69 -> 56 us (4.8 TB/s of K / V); one
+// of an unalternated one.  8 sequences against 8192 keys (32 / 8 heads): 69 -> 54 us (5.0 TB/s of K / V); one
 // sequence against 32768 keys 39 us (3.4 TB/s).
 struct FwdSplitPlan { int pack_log2, n_split; bool alternate; size_t bytes; };
 static FwdSplitPlan fwd_split_plan(const fm_attn_args* a) {
