@@ -514,3 +514,38 @@ def test_forward_and_backward_replay_from_a_cuda_graph(d):
     for g_, w_ in zip(got, want):
         assert torch.equal(g_, w_)
     assert _kernel_status() == 0
+
+
+@pytest.mark.parametrize("Sq,Sk,kind", [(700, 700, "causal_doc"), (512, 512, "none_causal"), (4, 3000, "none_causal")])
+def test_overlapping_kernels_of_a_call_replay_from_a_cuda_graph(Sq, Sk, kind):
+    """The programmatic launches inside a call (split forward + merge; dK / dV + dQ kernel of the deterministic
+    backward) under capture: replays on new inputs are bitwise eager calls."""
+    from flashmask_b200.ops import _flash_attn_bwd, _flash_attn_fwd
+    causal, idx = True, None
+    if kind == "causal_doc":
+        idx = torch.full((1, 1, Sk, 1), Sk, dtype=torch.int32, device="cuda")
+        idx[:, :, :300] = 300
+    g = torch.Generator(device="cuda").manual_seed(5)
+    new = lambda *shape: torch.randn(*shape, generator=g, device="cuda", dtype=torch.bfloat16)
+    ins = [new(1, Sq, 4, 128), new(1, Sk, 2, 128), new(1, Sk, 2, 128), new(1, Sq, 4, 128)]
+
+    def call(q, k, v, do):
+        out, lse = _flash_attn_fwd(q, k, v, idx, causal=causal)
+        return [out, lse, *_flash_attn_bwd(q, k, v, out, do, lse, idx, causal=causal, deterministic=True)[:3]]
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call(*ins)
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = call(*ins)
+    for _ in range(3):
+        for t in ins:
+            t.copy_(new(*t.shape))
+        graph.replay()
+        for a, b in zip(got, call(*ins)):
+            assert torch.equal(a, b)
+    assert _kernel_status() == 0
