@@ -45,7 +45,6 @@ int bwd_preprocess_launch(const AttnKParams& p, int dtype, cudaStream_t s);
 int bwd_dsink_launch(const AttnKParams& p, cudaStream_t s);
 int fwd_sm100_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s);
 size_t fwd_sm100_workspace_bytes(const fm_attn_args* a);
-bool bwd_sm100_supported(const fm_attn_args* a);
 int bwd_sm100_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s);
 int bwd_sm100_persist_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s);
 int bwd_sm100_fused_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s);
@@ -100,6 +99,17 @@ static bool fwd_uses_sm100(int d, int dv) {
 }
 
 static bool stride_ok(const int64_t* s) { return s[0] % 8 == 0 && s[1] % 8 == 0 && s[2] % 8 == 0; }
+
+// The tcgen05 kernels read q, k, v and d_o through tensor maps, which have no stride 0: a tensor that repeats along
+// a dimension (an expanded batch, one key head shown as several) is served by the warp-MMA kernels, which compute
+// their addresses.  (The torch hosts copy such a tensor instead and keep the faster kernels.)
+static bool mappable(const int64_t* s, int B, int S, int H) {
+  return (B == 1 || s[0] > 0) && (S == 1 || s[1] > 0) && (H == 1 || s[2] > 0);
+}
+static bool operands_mappable(const fm_attn_args* a, bool backward) {
+  return mappable(a->q_stride, a->B, a->Sq, a->Hq) && mappable(a->k_stride, a->B, a->Sk, a->Hkv) &&
+         mappable(a->v_stride, a->B, a->Sk, a->Hkv) && (!backward || mappable(a->do_stride, a->B, a->Sq, a->Hq));
+}
 
 static int validate_common(const fm_attn_args* a, const char* who) {
   FM_REQUIRE(a != nullptr, FM_ERR_INVALID_ARGUMENT, "%s: args is NULL", who);
@@ -182,28 +192,32 @@ static bool bwd_uses_sm100(int d, int dv) {
   return !g_opt.bwd_mma;
 }
 
+// Kernel family of a backward call.
 // The one-kernel backward (five GEMMs per tile pair, dQ summed into an fp32 accumulator in an order
 // that is not fixed) serves the tcgen05 head dims whenever the call does not ask for deterministic
 // gradients; the two-kernel variant gives every output element one owner and a fixed order.
 // Measured on 8K-128K masks it is 5-22 % faster at d = dv = 64 and d = dv = 128; head dims that only
 // partly fill a 64-column box measured slower (d = 96: +25 %), so they keep the two-kernel variant.
-static bool bwd_uses_fused(const fm_attn_args* a) {
-  const bool exact = a->d == a->dv && (a->d == 64 || a->d == 128);
-  return bwd_uses_sm100(a->d, a->dv) && exact && !a->deterministic && !g_opt.bwd_split;
-}
-
 // The CTA-pair backward (256, 512, 576 / 512) keeps P and dS of a chunk of query rows in the caller's workspace;
 // without one (fm_bwd_static_scratch) and past its index range the warp-MMA kernels serve these head dims.
-static bool bwd_uses_pair(const fm_attn_args* a) {
-  return pair_dims(a->d, a->dv) && !g_opt.bwd_mma && bwd_pair_supported(a);
+enum BwdKernels { BWD_ONE_KERNEL, BWD_TWO_KERNELS, BWD_PAIR, BWD_WARP_MMA };
+// By geometry and options alone: what the workspace is sized for.
+static BwdKernels bwd_kernels_by_geometry(const fm_attn_args* a) {
+  const bool exact = a->d == a->dv && (a->d == 64 || a->d == 128);
+  if (bwd_uses_sm100(a->d, a->dv)) return exact && !a->deterministic && !g_opt.bwd_split ? BWD_ONE_KERNEL : BWD_TWO_KERNELS;
+  return pair_dims(a->d, a->dv) && !g_opt.bwd_mma && bwd_pair_supported(a) ? BWD_PAIR : BWD_WARP_MMA;
+}
+static BwdKernels bwd_kernels(const fm_attn_args* a) {
+  return operands_mappable(a, true) ? bwd_kernels_by_geometry(a) : BWD_WARP_MMA;
 }
 
 // preprocess -> main kernels of the selected variant -> dsink, on one stream
-static int run_bwd_kernels(const fm_attn_args* a, const AttnKParams& p, cudaStream_t s) {
+static int run_bwd_kernels(const fm_attn_args* a, BwdKernels kernels, const AttnKParams& p, cudaStream_t s) {
+  FM_REQUIRE((((uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)a->d_o) & 15) == 0,
+             FM_ERR_INVALID_ARGUMENT, "backward: q/k/v/d_o must be 16-byte aligned");
   int rc = bwd_preprocess_launch(p, a->dtype, s);
   if (rc != FM_OK) return rc;
-  if (bwd_uses_sm100(a->d, a->dv)) {
-    FM_REQUIRE(bwd_sm100_supported(a), FM_ERR_INVALID_ARGUMENT, "backward: q/k/v/d_o must be 16-byte aligned");
+  if (kernels == BWD_ONE_KERNEL || kernels == BWD_TWO_KERNELS) {
     if (p.dq_accum) {
       rc = bwd_sm100_fused_launch(p, a, s);
       if (rc != FM_OK) return rc;
@@ -220,8 +234,6 @@ static int run_bwd_kernels(const fm_attn_args* a, const AttnKParams& p, cudaStre
     const bool persist = p.dq_order && p.dkdv_order && g_opt.bwd_persist && a->d <= 128;   // 192 / 128: one-unit kernels only
     rc = persist ? bwd_sm100_persist_launch(p, a, s) : bwd_sm100_launch(p, a, s);
   } else if (p.pair_ws) {
-    FM_REQUIRE((((uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)a->d_o) & 15) == 0,
-               FM_ERR_INVALID_ARGUMENT, "backward: q/k/v/d_o must be 16-byte aligned");
     rc = bwd_pair_launch(p, a, p.pair_ws, s);
   } else {
     rc = bwd_mma_launch(p, a->dtype, s);
@@ -273,9 +285,9 @@ static int fwd_impl(const fm_attn_args* a, const BlockScore& bs, void* stream) {
     p.block_log2 = bs.block_size == 32 ? 5 : (bs.block_size == 64 ? 6 : 7);
   }
   cudaStream_t s = (cudaStream_t)stream;
-  if (!fwd_uses_sm100(a->d, a->dv)) return fwd_mma_launch(p, a->dtype, s);
   FM_REQUIRE((((uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v) & 15) == 0, FM_ERR_INVALID_ARGUMENT,
              "forward: q/k/v must be 16-byte aligned");
+  if (!fwd_uses_sm100(a->d, a->dv) || !operands_mappable(a, false)) return fwd_mma_launch(p, a->dtype, s);
   // Past the CTA-pair kernels' key limit, and for block scores at 512 and 576, the warp-MMA kernels serve.
   if (pair_dims(a->d, a->dv))
     return fwd_pair_supported(a) && !(bs.block_logit && a->d > 256) ? fwd_pair_launch(p, a, s) : fwd_mma_launch(p, a->dtype, s);
@@ -406,15 +418,21 @@ static size_t bwd_stat_operand_bytes(const fm_attn_args* a) {
   return (size_t)a->B * a->Hq * round_up(a->Sq, 128) * 32;
 }
 
+static size_t bwd_workspace_bytes(const fm_attn_args* a, BwdKernels kernels) {
+  size_t n = bwd_row_stat_bytes(a);
+  if (kernels == BWD_PAIR) n += bwd_pair_workspace_bytes(a);
+  if (kernels == BWD_ONE_KERNEL) n += bwd_sm100_fused_accum_bytes(a) + bwd_stat_operand_bytes(a);
+  return n;
+}
+
+// (by geometry: a host may ask before it knows its tensors)
 extern "C" size_t fm_bwd_workspace_bytes(const fm_attn_args* a) {
-  if (!a || a->B <= 0 || a->Hq <= 0 || a->Sq <= 0) return 0;
-  if (a->Sk > 0 && a->Hkv > 0 && bwd_uses_pair(a)) return bwd_row_stat_bytes(a) + bwd_pair_workspace_bytes(a);
-  return bwd_row_stat_bytes(a) +
-         (bwd_uses_fused(a) ? bwd_sm100_fused_accum_bytes(a) + bwd_stat_operand_bytes(a) : 0);
+  if (!a || a->B <= 0 || a->Hq <= 0 || a->Sq <= 0 || a->Sk <= 0 || a->Hkv <= 0) return 0;
+  return bwd_workspace_bytes(a, bwd_kernels_by_geometry(a));
 }
 
 extern "C" int fm_bwd_accumulates(const fm_attn_args* a) {
-  return (a && a->d > 0 && a->dv > 0 && bwd_uses_fused(a)) ? 1 : 0;
+  return (a && a->d > 0 && a->dv > 0 && bwd_kernels(a) == BWD_ONE_KERNEL) ? 1 : 0;
 }
 
 extern "C" int fm_bwd(const fm_attn_args* a, void* stream) {
@@ -431,7 +449,8 @@ extern "C" int fm_bwd(const fm_attn_args* a, void* stream) {
   if (rc != FM_OK) return rc;
   FM_REQUIRE(a->ncols == 0 || a->tile_n == tn, FM_ERR_INVALID_ARGUMENT,
              "fm_bwd: minmax was prepared for tile_n=%d, this variant needs %d", a->tile_n, tn);
-  const size_t need = fm_bwd_workspace_bytes(a);
+  const BwdKernels kernels = bwd_kernels(a);
+  const size_t need = bwd_workspace_bytes(a, kernels);
   FM_REQUIRE(a->workspace && a->workspace_bytes >= need, FM_ERR_WORKSPACE,
              "fm_bwd: workspace too small (%zu bytes given, %zu needed)", a->workspace_bytes, need);
   FM_REQUIRE(((uintptr_t)a->workspace & 255) == 0, FM_ERR_WORKSPACE, "fm_bwd: workspace must be 256-byte aligned");
@@ -441,17 +460,17 @@ extern "C" int fm_bwd(const fm_attn_args* a, void* stream) {
   const size_t rows = (size_t)a->B * a->Hq * p.Sq_r;
   p.dpsum = reinterpret_cast<float*>(a->workspace);
   p.lse_log2 = p.dpsum + rows;
-  if (bwd_uses_fused(a)) {
+  if (kernels == BWD_ONE_KERNEL) {
     uint8_t* w = reinterpret_cast<uint8_t*>(a->workspace) + bwd_row_stat_bytes(a);
     p.dq_accum = reinterpret_cast<float*>(w);
     p.stat_s = reinterpret_cast<uint16_t*>(w + bwd_sm100_fused_accum_bytes(a));
     p.stat_dp = p.stat_s + (size_t)a->B * a->Hq * p.Sq_r * 8;
     p.bwd_flags = a->bwd_flags;
   }
-  if (bwd_uses_pair(a)) p.pair_ws = reinterpret_cast<uint8_t*>(a->workspace) + bwd_row_stat_bytes(a);
+  if (kernels == BWD_PAIR) p.pair_ws = reinterpret_cast<uint8_t*>(a->workspace) + bwd_row_stat_bytes(a);
   cudaStream_t s = (cudaStream_t)stream;
   attach_bwd_tables(a, &p);
-  return run_bwd_kernels(a, p, s);
+  return run_bwd_kernels(a, kernels, p, s);
 }
 
 extern "C" int fm_kernel_status(int* status, int reset) {
@@ -539,5 +558,5 @@ extern "C" int fm_bwd_static_scratch(const fm_attn_args* a, void* stream) {
   p.dpsum = scratch;
   p.lse_log2 = scratch + rows;
   attach_bwd_tables(a, &p);
-  return run_bwd_kernels(a, p, (cudaStream_t)stream);
+  return run_bwd_kernels(a, bwd_kernels(a), p, (cudaStream_t)stream);
 }

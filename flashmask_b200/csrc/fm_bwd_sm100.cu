@@ -597,13 +597,6 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
 // ---------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------
-bool bwd_sm100_supported(const fm_attn_args* a) {
-  const bool small = a->d <= 128 && a->dv <= 128 && a->d % 8 == 0 && a->dv % 8 == 0;
-  if (!small && !(a->d == 192 && a->dv == 128)) return false;
-  if (((uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)a->d_o) & 15) return false;
-  return true;
-}
-
 template <bool IS_BF16, int D, int DV>
 static int launch_bwd_sm100(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s) {
   using Cfg = BwdSm100Cfg<D>;

@@ -592,11 +592,10 @@ static int launch_fwd_pair(const AttnKParams& p, const fm_attn_args* a, cudaStre
   return FM_OK;
 }
 
-// d = dv = 256, 512, and 576 / 512, up to 2048 K tiles, 16-byte aligned operands.
+// d = dv = 256, 512, and 576 / 512, up to 2048 K tiles.
 bool fwd_pair_supported(const fm_attn_args* a) {
   const bool dims = (a->d == 256 && a->dv == 256) || ((a->d == 512 || a->d == 576) && a->dv == 512);
-  return dims && (a->Sk + 127) / 128 <= FwdPairCfg<256>::LIST_MAX &&
-         (((uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v) & 15) == 0;
+  return dims && (a->Sk + 127) / 128 <= FwdPairCfg<256>::LIST_MAX;
 }
 
 // (with p.block_logit: d = 256 only)

@@ -653,8 +653,12 @@ int make_bshd_tmap(CUtensorMap* out, const void* base, int dtype, int B, int S, 
                    int64_t ss, int64_t sh, int box_rows, int box_cols, int box_heads) {
   EncodeTiledFn enc = get_encode_tiled();
   FM_REQUIRE(enc != nullptr, FM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  // a dimension of one element may carry any stride, 0 included: it gets the dense one
+  const int64_t th = H > 1 ? sh : D, ts = S > 1 ? ss : th * H, tb = B > 1 ? sb : ts * S;
+  FM_REQUIRE(th > 0 && ts > 0 && tb > 0, FM_ERR_INVALID_ARGUMENT,
+             "tensor map: strides must be positive (batch %lld, row %lld, head %lld)", (long long)tb, (long long)ts, (long long)th);
   const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
-  const cuuint64_t strides[3] = {(cuuint64_t)sh * 2, (cuuint64_t)ss * 2, (cuuint64_t)(sb > 0 ? sb : ss * S) * 2};
+  const cuuint64_t strides[3] = {(cuuint64_t)th * 2, (cuuint64_t)ts * 2, (cuuint64_t)tb * 2};
   const cuuint32_t box[4] = {(cuuint32_t)box_cols, (cuuint32_t)box_heads, (cuuint32_t)box_rows, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUresult r = enc(out, dtype == FM_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,

@@ -35,7 +35,15 @@ int dtype_code(const Tensor& t) {
   return FM_DTYPE_FP16;
 }
 
-Tensor rows(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
+// Whether t repeats along a dimension (stride 0: an expanded tensor).
+bool repeats(const Tensor& t) {
+  for (int i = 0; i < 3; ++i)
+    if (t.size(i) > 1 && t.stride(i) == 0) return true;
+  return false;
+}
+
+// t as the kernels' tensor maps can describe it: rows contiguous, nothing repeated.
+Tensor rows(const Tensor& t) { return t.stride(-1) == 1 && !repeats(t) ? t : t.contiguous(); }
 
 void strides(int64_t* out, const Tensor& t) { for (int i = 0; i < 3; ++i) out[i] = t.stride(i); }
 
@@ -121,6 +129,15 @@ bool kv_shared(const Tensor& k, const Tensor& v) {
          k.strides() == v.strides();
 }
 
+// Key and value as the kernels read them; a value that is a view of the key's storage stays one.
+std::pair<Tensor, Tensor> kv_rows(const Tensor& k, const Tensor& v) {
+  if (k.stride(-1) == 1 && repeats(k) && kv_shared(k, v)) {
+    const Tensor kc = k.contiguous();
+    return {kc, kc.slice(3, 0, v.size(3))};
+  }
+  return {rows(k), rows(v)};
+}
+
 class FlashMask : public torch::autograd::Function<FlashMask> {
  public:
   static variable_list forward(AutogradContext* ctx, const Variable& q_in, const Variable& k_in, const Variable& v_in,
@@ -128,7 +145,8 @@ class FlashMask : public torch::autograd::Function<FlashMask> {
                                double scale, bool causal, int deterministic) {
     const c10::cuda::CUDAGuard guard(q_in.device());
     void* stream = c10::cuda::getCurrentCUDAStream(q_in.get_device()).stream();
-    const Tensor q = rows(q_in), k = rows(k_in), v = rows(v_in);
+    const Tensor q = rows(q_in);
+    const auto [k, v] = kv_rows(k_in, v_in);
     const int d = (int)q.size(3), dv = (int)v.size(3);
     int tm = 0, tn = 0;
     check(fm_fwd_tile_shape(d, dv, &tm, &tn), "fm_fwd_tile_shape");

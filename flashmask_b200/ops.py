@@ -123,6 +123,21 @@ def _last_dim_contiguous(t: torch.Tensor) -> torch.Tensor:
     return t if t.stride(-1) == 1 else t.contiguous()
 
 
+def _kernel_operand(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as the kernels' tensor maps can describe it: rows contiguous, and no dimension of several elements
+    with stride 0 (an expanded tensor is copied)."""
+    repeats = any(n > 1 and st == 0 for n, st in zip(t.shape[:3], t.stride()[:3]))
+    return t.contiguous() if repeats else _last_dim_contiguous(t)
+
+
+def _key_value_operands(k: torch.Tensor, v: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Key and value as the kernels read them; a value that is a view of the key's storage stays one."""
+    if k.stride(-1) == 1 and _kv_shared(k, v):
+        kc = _kernel_operand(k)
+        return kc, v if kc is k else kc[..., :v.shape[-1]]
+    return _kernel_operand(k), _kernel_operand(v)
+
+
 def _strides(t: torch.Tensor):
     return _lib.I64x3(t.stride(0), t.stride(1), t.stride(2))
 
@@ -211,7 +226,7 @@ def _flash_attn_fwd(q, k, v, startend_row_indices=None, softmax_scale=None, caus
         raise RuntimeError("flashmask_b200 runs on CUDA (sm_100a) tensors only; there is no CPU path")
     idx = startend_row_indices
     _check_shapes(q, k, v, idx, causal)
-    q, k, v = _last_dim_contiguous(q), _last_dim_contiguous(k), _last_dim_contiguous(v)
+    q, (k, v) = _kernel_operand(q), _key_value_operands(k, v)
     B, Sq, Hq, d = q.shape
     Sk, dv = k.shape[1], v.shape[3]
     if softmax_scale is None:
@@ -271,8 +286,8 @@ def _flash_attn_bwd(q, k, v, out, dout, lse, startend_row_indices=None, softmax_
     Reference: _flash_attn_bwd, flashmask/cute/ops/bwd.py:56-1261."""
     idx = startend_row_indices
     _check_shapes(q, k, v, idx, causal)
-    q, k, v = _last_dim_contiguous(q), _last_dim_contiguous(k), _last_dim_contiguous(v)
-    out, dout = _last_dim_contiguous(out), _last_dim_contiguous(dout)
+    q, (k, v) = _kernel_operand(q), _key_value_operands(k, v)
+    out, dout = _last_dim_contiguous(out), _kernel_operand(dout)
     B, Sq, Hq, d = q.shape
     Sk, Hkv, dv = k.shape[1], k.shape[2], v.shape[3]
     if softmax_scale is None:

@@ -69,6 +69,43 @@ def run_product(q, k, v, do, idx, causal, sink, deterministic=None):
                 dsink=grads[3] if s is not None else None)
 
 
+def run_c_abi(q, k, v, do, idx, causal, sink=None, scale=None, workspace=None, static_scratch=False,
+              deterministic=True):
+    """Forward and backward through the C ABI on the tensors as they are: nothing is copied or laid out first.
+    ``workspace``: bytes handed to fm_bwd (default: what fm_bwd_workspace_bytes asks for)."""
+    import ctypes as C
+    from flashmask_b200 import _lib, ops
+    lib = _lib.load()
+    stream = torch.cuda.current_stream().cuda_stream
+    B, Sq, Hq, d = q.shape
+    Sk, Hkv, dv = k.shape[1], k.shape[2], v.shape[3]
+    scale = 1.0 / math.sqrt(d) if scale is None else scale
+    out = torch.empty(B, Sq, Hq, dv, dtype=q.dtype, device=q.device)
+    lse = torch.empty(B, Hq, Sq, device=q.device)
+    sink = None if sink is None else sink.to(q.device).float().contiguous()
+    info = None if idx is None else fm.prepare_mask(idx, Sq, causal, *fm.fwd_tile_shape(d, dv))
+    a = ops._base_args(q, k, v, out, lse, idx, info, causal, scale, sink)
+    _lib.check(lib.fm_fwd(C.byref(a), stream), "fm_fwd")
+    info = None if idx is None else fm.prepare_mask(idx, Sq, causal, *fm.bwd_tile_shape(d, dv))
+    a = ops._base_args(q, k, v, out, lse, idx, info, causal, scale, sink)
+    dq = torch.empty(B, Sq, Hq, d, dtype=q.dtype, device=q.device)
+    dk = torch.empty(B, Sk, Hkv, d, dtype=q.dtype, device=q.device)
+    dvv = torch.empty(B, Sk, Hkv, dv, dtype=q.dtype, device=q.device)
+    dsink = None if sink is None else torch.empty(Hq, device=q.device)
+    a.d_o, a.dq, a.dk, a.dv_out = do.data_ptr(), dq.data_ptr(), dk.data_ptr(), dvv.data_ptr()
+    a.do_stride, a.dq_stride, a.dk_stride, a.dv_stride = (ops._strides(t) for t in (do, dq, dk, dvv))
+    a.dsink = None if dsink is None else dsink.data_ptr()
+    a.deterministic = int(deterministic)
+    if static_scratch:
+        _lib.check(lib.fm_bwd_static_scratch(C.byref(a), stream), "fm_bwd_static_scratch")
+    else:
+        n = lib.fm_bwd_workspace_bytes(C.byref(a)) if workspace is None else workspace
+        ws = torch.empty(n, dtype=torch.uint8, device=q.device)
+        a.workspace, a.workspace_bytes = ws.data_ptr(), n
+        _lib.check(lib.fm_bwd(C.byref(a), stream), "fm_bwd")
+    return dict(out=out, lse=lse, dq=dq, dk=dk, dv=dvv, dsink=dsink)
+
+
 def run_oracle(q, k, v, do, idx, causal, sink):
     return oracle.attention_forward_backward(
         q.cpu(), k.cpu(), v.cpu(), do.cpu(), None if idx is None else idx.cpu().numpy(), causal,

@@ -11,7 +11,7 @@ import torch
 from flashmask_b200 import workloads as W
 import flashmask_b200 as fm
 from flashmask_b200 import _lib
-from _util import (assert_lse, assert_parity, make_inputs, naive_lowp, run_oracle, run_product)
+from _util import (assert_lse, assert_parity, make_inputs, naive_lowp, run_c_abi, run_oracle, run_product)
 
 pytestmark = pytest.mark.gpu
 
@@ -378,6 +378,60 @@ def test_layout_invariance(fwd_variant):
     b = run_product(bhsd(q), bhsd(k), bhsd(v), bhsd(do), idx, causal, None, deterministic=True)
     for n in ("out", "dq", "dk", "dv"):
         assert torch.equal(a[n], b[n]), n
+
+
+@pytest.mark.parametrize("what", ["kv batch", "kv heads", "q batch", "do batch", "k rows"])
+@pytest.mark.parametrize("d,dv", [(64, 64), (128, 128), (192, 128), (256, 256), (512, 512), (576, 512)])
+def test_expanded_tensors(d, dv, what):
+    """Tensors that repeat along a dimension (stride 0).  Through the operator they are copied: bitwise the call on
+    dense copies.  Through the C ABI the warp-MMA kernels take them as they are, with mask reductions over the wider
+    tiles of the kernels that would have run."""
+    B, S, Hq, Hkv = 2, 200, 4, 2
+    idx_np, causal = _mask("causal_doc", B, S, S, 71)
+    idx = torch.from_numpy(np.ascontiguousarray(idx_np).copy()).cuda()
+    q, k, v, do, s = make_inputs(B, S, S, Hq, Hkv, d, dv, 71, sink=True)
+    q, k, v, do = q.cuda(), k.cuda(), v.cuda(), do.cuda()
+    if what == "kv batch":
+        k, v = k[:1].expand_as(k), v[:1].expand_as(v)
+    elif what == "kv heads":
+        k, v = k[:, :, :1].expand_as(k), v[:, :, :1].expand_as(v)
+    elif what == "q batch":
+        q = q[:1].expand_as(q)
+    elif what == "do batch":
+        do = do[:1].expand_as(do)
+    else:
+        k = k[:, :1].expand_as(k)
+    dense = [t.contiguous() for t in (q, k, v, do)]
+    assert any(0 in t.stride() for t in (q, k, v, do)) and not any(0 in t.stride() for t in dense)
+    leaves = [t.detach().requires_grad_(True) for t in (q, k, v)]
+    out, lse = fm.flashmask_attention(*leaves, idx, causal=causal, sink=s.cuda(), return_lse=True, deterministic=True)
+    got = [out.detach(), lse, *torch.autograd.grad(out, leaves, do)]
+    ref = run_product(*dense, idx, causal, s, deterministic=True)
+    for g_, n in zip(got, ("out", "lse", "dq", "dk", "dv")):
+        assert torch.equal(g_, ref[n]), n
+    raw = run_c_abi(q, k, v, do, idx, causal, s)
+    cpu = [t.cpu() for t in dense]
+    oracle_ = run_oracle(*cpu, idx, causal, s)
+    assert_parity(raw, oracle_, naive_lowp(*dense, idx, causal, s))
+    assert_lse(raw, oracle_)
+    assert _kernel_status() == 0
+
+
+def test_expanded_shared_key_value():
+    """One latent shown to every batch entry, the value a view of it: gradients as on a dense copy (dV folded into
+    dK, the value's own gradient zero)."""
+    B, S, d, dv = 2, 160, 576, 512
+    q, k, _, do, _ = make_inputs(B, S, S, 2, 1, d, dv, 72)
+    q, do, lat = q.cuda(), do.cuda(), k[:1].cuda()
+    res = []
+    for kk in (lat.expand(B, S, 1, d), lat.expand(B, S, 1, d).contiguous()):
+        kk = kk.detach().requires_grad_(True)
+        vv = kk[..., :dv].detach().requires_grad_(True)
+        out = fm.flashmask_attention(q, kk, vv, causal=True, deterministic=True)
+        res.append([out.detach(), *torch.autograd.grad(out, [kk, vv], do)])
+    assert float(res[0][2].abs().max()) == 0.0 and float(res[0][1].abs().max()) > 0.0
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
 
 
 def test_window_size_kwarg():

@@ -75,6 +75,37 @@ def test_kernel_variant_routing_needs_no_gpu():
         assert got == has, (d, dv, got)
 
 
+def test_repeated_operands_take_no_tensor_map():
+    """A dimension of several elements with stride 0 cannot be described to the kernels' tensor maps: the hosts copy
+    such a tensor (and keep a value that is a view of the key), and the C ABI routes the call to the kernels that
+    compute addresses."""
+    from flashmask_b200.ops import _kernel_operand, _key_value_operands
+    k = torch.randn(1, 6, 1, 576)
+    for t in (k.expand(3, 6, 1, 576), k.expand(1, 6, 4, 576), k[:, :1].expand(1, 6, 1, 576)):
+        got = _kernel_operand(t)
+        assert got.is_contiguous() and torch.equal(got, t)
+    one = torch.empty_strided((1, 6, 1, 8), (0, 8, 0, 1))        # one element: any stride will do
+    assert _kernel_operand(one) is one and _kernel_operand(k) is k
+    ke = k.expand(3, 6, 1, 576)
+    kc, vc = _key_value_operands(ke, ke[..., :512])
+    assert kc.data_ptr() == vc.data_ptr() and kc.stride() == vc.stride() and vc.shape[-1] == 512
+    assert min(kc.stride()) > 0 and torch.equal(kc, ke)
+    lib = _lib.load()
+    a = _lib.AttnArgs()
+    a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.Hm, a.mask_B, a.d, a.dv, a.softmax_scale = 2, 64, 64, 4, 2, 1, 1, 128, 128, 0.1
+
+    def accumulates(**strides):
+        for name, H in (("q", 4), ("k", 2), ("v", 2), ("do", 4)):
+            setattr(a, name + "_stride", _lib.I64x3(*strides.get(name, (64 * H * 128, H * 128, 128))))
+        return lib.fm_bwd_accumulates(ctypes.byref(a))
+    assert accumulates() == 1
+    for name, H in (("q", 4), ("k", 2), ("v", 2), ("do", 4)):
+        for s in ((0, H * 128, 128), (64 * H * 128, 0, 128), (64 * H * 128, H * 128, 0)):
+            assert accumulates(**{name: s}) == 0, (name, s)
+    a.B = a.mask_B = 1
+    assert accumulates(k=(0, 256, 128)) == 1
+
+
 def test_pair_backward_workspace_is_bounded():
     """The CTA-pair backward keeps P and dS of at least 256 rows of a kv group: up to 8 GiB, and none at all (the
     kernels without a workspace serve the call) where that would not do."""
