@@ -368,7 +368,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (SPLIT && n_parts > 1) {
         // partial result of this share of the tiles, in fp32: 4 * DV contiguous bytes per row
         const int64_t at = (((int64_t)b * p.Hq + head) * p.Sq + row) * n_parts + part_of(s);
-        if (prow < n_rows) p.part_lse[at] = l_tot > 0.f ? m_fin + log2f(l_tot) : neg_inf();
+        // (-inf marks a part without a visible key; the sum of a part with a NaN or infinite score is NaN and stays one)
+        if (prow < n_rows) p.part_lse[at] = l_tot == 0.f ? neg_inf() : m_fin + log2f(l_tot);
 #pragma unroll
         for (int c = 0; c < DV / 32; ++c) {
           uint32_t orr[32];
@@ -593,7 +594,7 @@ __global__ void __launch_bounds__(256) fwd_combine_kernel(const AttnKParams p) {
   const float mine = lane < n_parts ? lse[lane] : neg_inf();
   float m = mine;
 #pragma unroll
-  for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));   // (drops NaN; the weights keep it)
   if (m == neg_inf()) m = 0.f;
   const float w_mine = exp2f(mine - m);
   float l = w_mine;
@@ -605,7 +606,7 @@ __global__ void __launch_bounds__(256) fwd_combine_kernel(const AttnKParams p) {
   const float* src = p.part_o + row * n_parts * DV + lane * PER;
   for (int s = 0; s < n_parts; ++s) {
     const float w = __shfl_sync(0xffffffffu, w_mine, s);
-    if (w == 0.f) continue;                                               // (an empty part's O is not written)
+    if (__shfl_sync(0xffffffffu, mine, s) == neg_inf()) continue;         // (an empty part's O is not written)
     if constexpr (PER == 4) {
       const float4 v = *reinterpret_cast<const float4*>(src + s * DV);
       acc[0] += w * v.x; acc[1] += w * v.y; acc[2] += w * v.z; acc[3] += w * v.w;

@@ -219,6 +219,38 @@ def test_rows_of_one_sub_tile(B, Sq, Sk, Hq, Hkv, d, dv):
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("what", ["k nan", "k inf", "q nan", "v nan", "v inf"])
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,d", [(1, 1, 8192, 4, 1, 128),       # split and alternating
+                                              (1, 1, 300, 2, 2, 64),         # alternating only
+                                              (1, 256, 8192, 2, 2, 128)])    # split only
+def test_non_finite_inputs_of_a_split_forward(B, Sq, Sk, Hq, Hkv, d, what):
+    """A NaN or an infinity that a query sees reaches its output whatever share of the keys holds it: the elements
+    that are NaN or infinite are those of the dense softmax, the others are finite and right."""
+    q, k, v, _, _ = (t if t is None else t.cuda() for t in make_inputs(B, Sq, Sk, Hq, Hkv, d, d, 95))
+    q[0, 0, 0, 5] = q[0, 0, 0, 5].abs() + 1          # (the first query's score of an infinite key is +inf)
+    dict(q=q, k=k, v=v)[what[0]][0, 0, 0, 5] = float(what[2:])
+    with torch.no_grad():
+        out, lse = fm.flashmask_attention(q, k, v, causal=True, return_lse=True)
+    rep = lambda t: t.double().repeat_interleave(Hq // Hkv, dim=2).permute(0, 2, 1, 3)
+    s = rep(q) if Hq == Hkv else q.double().permute(0, 2, 1, 3)
+    s = s @ rep(k).transpose(-1, -2) / math.sqrt(d)
+    hidden = torch.arange(Sk, device="cuda")[None] > torch.arange(Sq, device="cuda")[:, None] + Sk - Sq
+    att = torch.softmax(s.masked_fill(hidden, -math.inf), -1)
+    want = (att @ rep(v)).permute(0, 2, 1, 3)
+    if what == "v inf":      # the weight of the infinite element is positive in both
+        assert torch.isinf(want).any()
+    else:
+        assert torch.isnan(want).any()
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
+    fin = torch.isfinite(want)
+    # P and the result are rounded to 8 bits of mantissa each (half a unit: 2^-9 relative)
+    bound = 2 ** -8 * (att @ rep(v).abs()).permute(0, 2, 1, 3)
+    assert ((out.double() - want)[fin].abs() <= bound[fin]).all()
+    bad = torch.isnan(want).all(-1)                  # rows whose softmax sum is NaN: LSE -inf, as in an unsplit call
+    assert torch.equal(torch.isneginf(lse), bad.permute(0, 2, 1))
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("kind", MASKS)
 def test_masks_d64(kind, fwd_variant):
     """Every mask family through the 64-column variants: GQA, rows long enough to wrap the K/V ring."""
