@@ -100,15 +100,18 @@ static bool fwd_uses_sm100(int d, int dv) {
 
 static bool stride_ok(const int64_t* s) { return s[0] % 8 == 0 && s[1] % 8 == 0 && s[2] % 8 == 0; }
 
-// The tcgen05 kernels read q, k, v and d_o through tensor maps, which have no stride 0: a tensor that repeats along
-// a dimension (an expanded batch, one key head shown as several) is served by the warp-MMA kernels, which compute
-// their addresses.  (The torch hosts copy such a tensor instead and keep the faster kernels.)
+// What the tcgen05 kernels ask of a call; the warp-MMA kernels serve the others.
+// They read q, k, v and d_o through tensor maps, which have no stride 0: a tensor that repeats along a dimension (an
+// expanded batch, one key head shown as several) needs computed addresses.  (The torch hosts copy such a tensor
+// instead and keep the faster kernels.)
+// They mask a score with -inf and take the row maximum before the scale is applied, which needs a positive scale.
 static bool mappable(const int64_t* s, int B, int S, int H) {
   return (B == 1 || s[0] > 0) && (S == 1 || s[1] > 0) && (H == 1 || s[2] > 0);
 }
-static bool operands_mappable(const fm_attn_args* a, bool backward) {
-  return mappable(a->q_stride, a->B, a->Sq, a->Hq) && mappable(a->k_stride, a->B, a->Sk, a->Hkv) &&
-         mappable(a->v_stride, a->B, a->Sk, a->Hkv) && (!backward || mappable(a->do_stride, a->B, a->Sq, a->Hq));
+static bool fits_tcgen05(const fm_attn_args* a, bool backward) {
+  return a->softmax_scale > 0.f && mappable(a->q_stride, a->B, a->Sq, a->Hq) &&
+         mappable(a->k_stride, a->B, a->Sk, a->Hkv) && mappable(a->v_stride, a->B, a->Sk, a->Hkv) &&
+         (!backward || mappable(a->do_stride, a->B, a->Sq, a->Hq));
 }
 
 static int validate_common(const fm_attn_args* a, const char* who) {
@@ -208,7 +211,7 @@ static BwdKernels bwd_kernels_by_geometry(const fm_attn_args* a) {
   return pair_dims(a->d, a->dv) && !g_opt.bwd_mma && bwd_pair_supported(a) ? BWD_PAIR : BWD_WARP_MMA;
 }
 static BwdKernels bwd_kernels(const fm_attn_args* a) {
-  return operands_mappable(a, true) ? bwd_kernels_by_geometry(a) : BWD_WARP_MMA;
+  return fits_tcgen05(a, true) ? bwd_kernels_by_geometry(a) : BWD_WARP_MMA;
 }
 
 // preprocess -> main kernels of the selected variant -> dsink, on one stream
@@ -287,7 +290,7 @@ static int fwd_impl(const fm_attn_args* a, const BlockScore& bs, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   FM_REQUIRE((((uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v) & 15) == 0, FM_ERR_INVALID_ARGUMENT,
              "forward: q/k/v must be 16-byte aligned");
-  if (!fwd_uses_sm100(a->d, a->dv) || !operands_mappable(a, false)) return fwd_mma_launch(p, a->dtype, s);
+  if (!fwd_uses_sm100(a->d, a->dv) || !fits_tcgen05(a, false)) return fwd_mma_launch(p, a->dtype, s);
   // Past the CTA-pair kernels' key limit, and for block scores at 512 and 576, the warp-MMA kernels serve.
   if (pair_dims(a->d, a->dv))
     return fwd_pair_supported(a) && !(bs.block_logit && a->d > 256) ? fwd_pair_launch(p, a, s) : fwd_mma_launch(p, a->dtype, s);

@@ -10,6 +10,7 @@ import torch
 
 from flashmask_b200 import workloads as W
 import flashmask_b200 as fm
+import oracle
 from flashmask_b200 import _lib
 from _util import (assert_lse, assert_parity, make_inputs, naive_lowp, run_c_abi, run_oracle, run_product)
 
@@ -446,6 +447,27 @@ def test_expanded_tensors(d, dv, what):
     oracle_ = run_oracle(*cpu, idx, causal, s)
     assert_parity(raw, oracle_, naive_lowp(*dense, idx, causal, s))
     assert_lse(raw, oracle_)
+    assert _kernel_status() == 0
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.07])
+@pytest.mark.parametrize("d,dv", [(64, 64), (128, 128), (192, 128), (256, 256), (512, 512), (576, 512)])
+def test_scale_that_is_not_positive(d, dv, scale):
+    """A masked score stays masked whatever the sign of the scale (0: every visible key has the same weight)."""
+    S = 200
+    idx_np, causal = _mask("causal_doc", 1, S, S, 73)
+    idx = torch.from_numpy(np.ascontiguousarray(idx_np).copy()).cuda()
+    q, k, v, do, _ = (t if t is None else t.cuda() for t in make_inputs(1, S, S, 2, 2, d, dv, 73))
+    x = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    out, lse = fm.flashmask_attention(*x, idx, causal=causal, softmax_scale=scale, return_lse=True)
+    got = [out.detach(), *torch.autograd.grad(out, x, do)]
+    y = [t.double().requires_grad_(True) for t in (q, k, v)]
+    s = torch.einsum("bihd,bjhd->bhij", y[0], y[1]) * scale + torch.from_numpy(oracle.dense_bias(idx_np, S, S, causal)).cuda()
+    ref = torch.einsum("bhij,bjhd->bihd", torch.softmax(s, -1), y[2])
+    assert (lse.double() - torch.logsumexp(s, -1)).abs().max() < 1e-4
+    for g_, r, n in zip(got, [ref.detach(), *torch.autograd.grad(ref, y, do.double())], ("out", "dq", "dk", "dv")):
+        # P, dS and the results are rounded to 16 bits: a few units of 2^-9 in the 2-norm
+        assert (g_.double() - r).norm() <= 1e-2 * r.norm(), n
     assert _kernel_status() == 0
 
 

@@ -104,6 +104,9 @@ def test_repeated_operands_take_no_tensor_map():
             assert accumulates(**{name: s}) == 0, (name, s)
     a.B = a.mask_B = 1
     assert accumulates(k=(0, 256, 128)) == 1
+    for scale in (0.0, -0.1, float("nan")):
+        a.softmax_scale = scale
+        assert accumulates() == 0, scale
 
 
 def test_pair_backward_workspace_is_bounded():
