@@ -430,7 +430,7 @@ static size_t bwd_workspace_bytes(const fm_attn_args* a, BwdKernels kernels) {
 
 // (by geometry: a host may ask before it knows its tensors)
 extern "C" size_t fm_bwd_workspace_bytes(const fm_attn_args* a) {
-  if (!a || a->B <= 0 || a->Hq <= 0 || a->Sq <= 0 || a->Sk <= 0 || a->Hkv <= 0) return 0;
+  if (!a || a->B <= 0 || a->Hq <= 0 || a->Sq <= 0) return 0;
   return bwd_workspace_bytes(a, bwd_kernels_by_geometry(a));
 }
 

@@ -730,10 +730,12 @@ static BwdPairPlan bwd_pair_plan(const fm_attn_args* a) {
 
 bool bwd_pair_supported(const fm_attn_args* a) {
   const bool dims = (a->d == 256 && a->dv == 256) || ((a->d == 512 || a->d == 576) && a->dv == 512);
+  // (a size query comes before the arguments are validated)
+  if (!dims || a->Sq <= 0 || a->Sk <= 0 || a->Hkv <= 0 || a->Hq <= 0 || a->Hq % a->Hkv) return false;
   // a chunk is at least 256 rows of every head of one group; past four budgets the warp-MMA kernels, which need no
   // workspace, keep the call
   const size_t least = (size_t)(a->Hq / a->Hkv) * (((size_t)a->Sk + 255) / 256 * 256) * 4 * 256;
-  return dims && (a->Sk + 127) / 128 <= kPairListMax && (a->Sq + 127) / 128 <= kPairListMax && least <= 4 * kBudget;
+  return (a->Sk + 127) / 128 <= kPairListMax && (a->Sq + 127) / 128 <= kPairListMax && least <= 4 * kBudget;
 }
 
 size_t bwd_pair_workspace_bytes(const fm_attn_args* a) {

@@ -109,6 +109,21 @@ def test_repeated_operands_take_no_tensor_map():
         assert accumulates() == 0, scale
 
 
+@pytest.mark.parametrize("d,dv", [(64, 64), (256, 256), (576, 512)])
+def test_size_queries_survive_arguments_that_a_call_would_refuse(d, dv):
+    """Hosts ask for sizes before anything is validated: heads that do not divide or are missing, lengths of 0."""
+    lib = _lib.load()
+    for Sq, Sk, Hq, Hkv in ((512, 512, 4, 8), (512, 512, 6, 4), (512, 512, 4, 0), (512, 512, 0, 4), (512, 0, 4, 4),
+                            (0, 512, 4, 4), (512, 512, 4, -1), (-1, -1, -1, -1)):
+        a = _lib.AttnArgs()
+        a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.Hm, a.mask_B, a.d, a.dv = 1, Sq, Sk, Hq, Hkv, 1, 1, d, dv
+        # without a usable geometry no variant with a large workspace is meant
+        assert lib.fm_bwd_workspace_bytes(ctypes.byref(a)) <= 4 << 20, (Sq, Sk, Hq, Hkv)
+        assert lib.fm_bwd_accumulates(ctypes.byref(a)) == 0
+        assert lib.fm_fwd_workspace_bytes(ctypes.byref(a)) == 0 or Hq % max(Hkv, 1) == 0
+        assert [lib.fm_launch_order_ints(ctypes.byref(a), w) for w in range(3)] == [0, 0, 0]
+
+
 def test_pair_backward_workspace_is_bounded():
     """The CTA-pair backward keeps P and dS of at least 256 rows of a kv group: up to 8 GiB, and none at all (the
     kernels without a workspace serve the call) where that would not do."""
