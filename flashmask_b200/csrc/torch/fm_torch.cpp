@@ -243,13 +243,15 @@ std::pair<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Tens
                                     const std::optional<Tensor>& sink, std::optional<double> scale, bool causal,
                                     int deterministic) {
   TORCH_CHECK(q.is_cuda(), "flashmask_b200 runs on CUDA (sm_100a) tensors only; there is no CPU path");
+  require(k.device() == q.device() && v.device() == q.device(), "q/k/v must be on one device");
   require(q.dim() == 4 && k.dim() == 4 && v.dim() == 4, "q/k/v must be [B, S, H, D]");
   const int64_t B = q.size(0), Hq = q.size(2), d = q.size(3), Sk = k.size(1), Hkv = k.size(2);
   require(k.size(0) == B && k.size(3) == d && v.size(0) == B && v.size(1) == Sk && v.size(2) == Hkv, "k/v shapes do not match q");
   require(Hkv > 0 && Hq % Hkv == 0, "num q heads must be a multiple of num kv heads");
   require(q.scalar_type() == k.scalar_type() && q.scalar_type() == v.scalar_type(), "q/k/v must share a dtype");
   if (idx) {
-    require(idx->is_cuda() && idx->scalar_type() == at::kInt, "startend_row_indices must be int32");
+    require(idx->device() == q.device(), "startend_row_indices must be on the device of q");
+    require(idx->scalar_type() == at::kInt, "startend_row_indices must be int32");
     require(idx->dim() == 4, "startend_row_indices must be [B, Hm, Sk, n]");
     require(idx->size(0) == B || idx->size(0) == 1, "startend_row_indices batch must match q");
     require(idx->size(2) == Sk, "startend_row_indices seqlen must match k");

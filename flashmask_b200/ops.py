@@ -174,7 +174,9 @@ def _check_shapes(q, k, v, idx, causal):
     assert (Bk, dk) == (B, d) and v.shape[:3] == k.shape[:3], "k/v shapes do not match q"
     assert Hq % Hkv == 0, "num q heads must be a multiple of num kv heads"
     assert q.dtype == k.dtype == v.dtype, "q/k/v must share a dtype"
+    assert q.device == k.device == v.device, "q/k/v must be on one device"
     if idx is not None:
+        assert idx.device == q.device, "startend_row_indices must be on the device of q"
         assert idx.dtype == torch.int32, "startend_row_indices must be int32"
         assert idx.dim() == 4, "startend_row_indices must be [B, Hm, Sk, n]"
         assert idx.shape[0] in (B, 1), "startend_row_indices batch must match q"
@@ -286,6 +288,7 @@ def _flash_attn_bwd(q, k, v, out, dout, lse, startend_row_indices=None, softmax_
     Reference: _flash_attn_bwd, flashmask/cute/ops/bwd.py:56-1261."""
     idx = startend_row_indices
     _check_shapes(q, k, v, idx, causal)
+    assert out.device == dout.device == lse.device == q.device, "out, dout and lse must be on the device of q"
     q, (k, v) = _kernel_operand(q), _key_value_operands(k, v)
     out, dout = _last_dim_contiguous(out), _kernel_operand(dout)
     B, Sq, Hq, d = q.shape

@@ -509,6 +509,20 @@ def test_errors():
                                v.cuda()[..., :40].contiguous().repeat(1, 1, 1, 8))
 
 
+def test_operands_elsewhere_are_refused_before_any_launch():
+    """A key, value or mask that is not on the query's device never reaches a kernel as a raw pointer."""
+    q, k, v, do, _ = make_inputs(1, 64, 64, 2, 2, 64, 64, 1)
+    c = [t.cuda() for t in (q, k, v)]
+    idx = torch.full((1, 1, 64, 1), 64, dtype=torch.int32)
+    before = _lib.load().fm_launch_count()
+    for args in ((c[0], k, c[2], None), (c[0], c[1], v, None), (*c, idx)):
+        with pytest.raises(AssertionError, match="device"):
+            fm.flashmask_attention(*args, causal=True)
+        with pytest.raises(AssertionError, match="device"):
+            fm._flash_attn_fwd(*args, causal=True)
+    assert _lib.load().fm_launch_count() == before
+
+
 def test_bounded_wait_reports_timeout_without_fault():
     """A wait on a barrier nothing arrives on gives up after its budget, the kernel
     returns, the status word says FM_ERR_TIMEOUT and the context keeps working."""

@@ -165,6 +165,17 @@ def test_workload_shapes():
         assert 0.0 <= wl.sparsity() < 1.0
 
 
+def test_operands_on_several_devices_are_refused():
+    from flashmask_b200.ops import _check_shapes
+    x = torch.zeros(1, 8, 1, 64, dtype=torch.bfloat16)
+    idx = torch.zeros(1, 1, 8, 1, dtype=torch.int32)
+    _check_shapes(x, x, x, idx, True)
+    m = x.to("meta")
+    for args in ((x, m, x, None), (x, x, m, None), (m, x, x, None), (m, m, m, idx)):
+        with pytest.raises(AssertionError, match="device"):
+            _check_shapes(*args, True)
+
+
 def test_sliding_window_kwarg_bounds():
     idx = fm.sliding_window_indices(16, 16, 4, True, 2, "cpu")
     ref, _ = W.sliding_window(2, 16, 16, 4)
