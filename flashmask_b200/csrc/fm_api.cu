@@ -1,5 +1,6 @@
 // extern "C" entry points: argument validation, kernel-variant selection,
 // workspace carving.  No allocation, no host synchronisation.
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdlib>
@@ -263,6 +264,43 @@ extern "C" int fm_bwd_tile_shape(int d, int dv, int* tile_m, int* tile_n) {
   return rc;
 }
 
+// Kernel family of a forward at 256, 512 or 576 / 512.
+//
+// The CTA-pair kernel works on blocks of 256 rows, one block on two SMs: it is the fastest wherever blocks are full,
+// and up to four times slower than smaller blocks on batches of short sequences.  There the one-CTA kernel (256, blocks
+// of 128 rows) or the warp-MMA kernel (512 and 576, blocks of 64) serves.  The family follows from an estimate of both
+// launches in microseconds, the longer of the longest block and waves x the average block, fitted to 976 calls of 1 to
+// 64 sequences of 32 to 1024 rows, and of 1 to 128 rows against up to 8192 keys (16 heads, causal and full):
+//   64 x 64 rows, 576 / 512 causal    pair 276 us, warp-MMA 105    64 x 128 rows, 256 full    pair 131 us, one CTA 65
+//   64 x 128 rows, 576 / 512 full     pair 293 us, warp-MMA 312    32 x 512 rows, 256 full    pair 188 us, one CTA 258
+//   8 x 16 rows of 1024 keys, 256, 16 / 4 heads  pair 35, one CTA 27;  8 x 1 row of 8192 keys  pair 173, one CTA 202
+// Within 3 %, and past 2048 rows, the pair kernel is kept.
+enum FwdWide { FWD_PAIR, FWD_ONE_CTA, FWD_WARP_MMA };
+static double fwd_launch_us(const fm_attn_args* a, int rows, int keys, int units, int slots, double fixed, double per_tile) {
+  const int n_blocks = (a->Sq + rows - 1) / rows, n_tiles = (a->Sk + keys - 1) / keys;
+  int64_t sum = 0;
+  int most = 0;
+  for (int i = 0; i < n_blocks; ++i) {
+    const int last = std::min((i + 1) * rows, a->Sq) + a->Sk - a->Sq;      // keys the block's last row sees
+    const int n = a->causal ? std::max(0, std::min(n_tiles, (last + keys - 1) / keys)) : n_tiles;
+    sum += n;
+    most = std::max(most, n);
+  }
+  const int64_t waves = ((int64_t)units * n_blocks + slots - 1) / slots;
+  return std::max(fixed + per_tile * most, waves * (fixed + per_tile * sum / n_blocks));
+}
+static FwdWide fwd_wide_kernels(const fm_attn_args* a) {
+  if (!fwd_pair_supported(a)) return FWD_WARP_MMA;
+  if (a->Sq > 2048) return FWD_PAIR;
+  const int n_sm = sm_count(), units = a->B * a->Hq;
+  if (a->d == 256) {
+    const double pair = fwd_launch_us(a, 256, 128, units, n_sm / 2, a->causal ? 11.8 : 10.5, 0.95);
+    return fwd_launch_us(a, 128, 128, units, n_sm, 6.4, 3.2) < 0.97 * pair ? FWD_ONE_CTA : FWD_PAIR;
+  }
+  const double pair = fwd_launch_us(a, 256, 128, 2 * units, n_sm / 2, a->causal ? 9.2 : 7.8, 2.1);   // (two slices of V)
+  return fwd_launch_us(a, 64, 32, units, n_sm, 3.3, 6.2) < 0.97 * pair ? FWD_WARP_MMA : FWD_PAIR;
+}
+
 // Side output of the forward (fm_fwd_block_score); block_logit == nullptr: none.
 struct BlockScore { float* block_logit; const int32_t* block_bos; int block_size, block_ld; };
 
@@ -291,9 +329,12 @@ static int fwd_impl(const fm_attn_args* a, const BlockScore& bs, void* stream) {
   FM_REQUIRE((((uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v) & 15) == 0, FM_ERR_INVALID_ARGUMENT,
              "forward: q/k/v must be 16-byte aligned");
   if (!fwd_uses_sm100(a->d, a->dv) || !fits_tcgen05(a, false)) return fwd_mma_launch(p, a->dtype, s);
-  // Past the CTA-pair kernels' key limit, and for block scores at 512 and 576, the warp-MMA kernels serve.
-  if (pair_dims(a->d, a->dv))
-    return fwd_pair_supported(a) && !(bs.block_logit && a->d > 256) ? fwd_pair_launch(p, a, s) : fwd_mma_launch(p, a->dtype, s);
+  if (pair_dims(a->d, a->dv)) {
+    const FwdWide kernels = fwd_wide_kernels(a);
+    // (block scores at 512 and 576: the warp-MMA kernel alone has them)
+    if (kernels == FWD_WARP_MMA || (bs.block_logit && a->d > 256)) return fwd_mma_launch(p, a->dtype, s);
+    if (kernels == FWD_PAIR) return fwd_pair_launch(p, a, s);
+  }
   return fwd_sm100_launch(p, a, s);
 }
 
@@ -318,8 +359,8 @@ static bool order_geometry_any(const fm_attn_args* a, int which, OrderGeom* g) {
   if (!a || a->ncols == 0 || a->Sq <= 0 || a->Sk <= 0 || a->B <= 0 || a->Hq <= 0 || a->Hkv <= 0) return false;
   if (!(a->Hm == 1 || a->Hm == a->Hkv) || !(a->mask_B == 1 || a->mask_B == a->B) || a->Hq % a->Hkv) return false;
   const int nk = (a->Sk + 127) / 128;
-  // (the 256-column forward owns 128 rows per CTA and takes no table; the 192-column backward runs the
-  // one-unit kernels, which take none either)
+  // (the forward takes no table at 256 and above; the 192-column backward runs the one-unit kernels, which take
+  // none either)
   if (which == FM_ORDER_FWD) {
     if (!fwd_uses_sm100(a->d, a->dv) || a->d > 192) return false;
     *g = OrderGeom{0, 256, (a->Sq + 255) / 256, nk, a->Hq};

@@ -1,8 +1,9 @@
 // Forward attention on the 5th-generation tensor cores (tcgen05 / UMMA) for
 // head dims up to 128: a 64-column and a 128-column variant; smaller head dims
 // (multiples of 8) run in the next variant up, the TMA loads filling the
-// columns past the end of a head with zeros.  A third variant serves d = 192 /
-// dv = 128 (same plan, 48 KB K tiles, two ring slots).
+// columns past the end of a head with zeros.  Two more variants serve d = 192 /
+// dv = 128 (same plan, 48 KB K tiles, two ring slots) and short calls at
+// d = dv = 256 (below).
 //
 // One CTA owns 256 query rows of one (batch, q head) as two 128-row sub-tiles
 // that share every K/V tile.  Warp roles:
@@ -20,6 +21,15 @@
 // maximum grew by more than 2^8 (the rescale is done by the softmax warps
 // themselves).  Every mbarrier wait is bounded: on expiry the CTA raises an
 // abort flag, all roles unwind, TMEM is freed and a status word is set.
+//
+// d = dv = 256: the O accumulator of 128 rows alone needs 256 TMEM columns, so a CTA owns 128 query
+// rows and its two "sub-tiles" are the two 128-column halves of V / O for the SAME rows: both
+// warpgroups run the softmax of the same scores (S is computed once per warpgroup, in its own
+// buffer), warpgroup s accumulates O[:, 128 s : 128 s + 128) = P V[:, 128 s : ...).  One 64 KB Q tile
+// and a two-slot ring of 64 KB K / V tiles.  The score GEMM runs twice per tile (6 MMA units for the
+// 4 the mathematics needs), so the CTA-pair kernel is the faster one wherever its blocks of 256 rows
+// are full; where they are not, this variant wastes half as many rows and puts twice as many blocks
+// on the chip at a time (fwd_wide_kernels in fm_api.cu has the line and the figures).
 #include <type_traits>
 
 #include "fm_attn_params.cuh"
@@ -44,10 +54,12 @@ __device__ long long g_fprof[64 * 16];
 #define FPROF_VAL(slot, v)
 #endif
 
-// D: width q / k are computed at (64, 128 or 192), DV: width of v / o (64 or 128).
+// D: width q / k are computed at (64, 128, 192 or 256), DV: width of v / o (64, 128 or 256).
 template <int D, int DV = D>
 struct FwdSm100Cfg {
-  static constexpr int ROWS = 256;                      // query rows per CTA
+  static constexpr bool SPLITV = D == 256;              // sub-tiles are halves of V / O, not of the rows
+  static constexpr int ROWS = SPLITV ? 128 : 256;       // query rows per CTA
+  static constexpr int DVS = SPLITV ? DV / 2 : DV;      // O columns per warpgroup
   // the 64-column variant doubles the ring depth: its slots are half as large; the 192-column one has room
   // for two slots (one K tile and one V tile in flight) beside its two 48 KB Q sub-tiles
   static constexpr int BM = 128, BN = 128, NSTAGE = (D == 64 ? 8 : (D > 128 ? 2 : 4)), NBND = 2, LIST_MAX = 2048;
@@ -58,7 +70,7 @@ struct FwdSm100Cfg {
   static constexpr int SLOT_BYTES = K_BYTES > V_BYTES ? K_BYTES : V_BYTES;
   static constexpr int BND_BYTES = 128 * 4 * 4;
   static constexpr int OFF_Q = 0;
-  static constexpr int OFF_KV = OFF_Q + 2 * Q_BYTES;
+  static constexpr int OFF_KV = OFF_Q + (SPLITV ? 1 : 2) * Q_BYTES;
   // Causal masks: the K and V tiles of the diagonal (the first tile of the list, right to left) are requested at
   // kernel entry into slots 0 and 1, before the list exists, where the ring is deep enough to keep the list
   // build's staging area (64 KB) clear of those two slots.
@@ -77,7 +89,8 @@ struct FwdSm100Cfg {
   static constexpr int B_QFULL = 0, B_KVFULL = 2, B_KVEMPTY = 2 + NSTAGE, B_SFULL = 2 + 2 * NSTAGE,
                        B_PFULL = B_SFULL + 2, B_ODONE = B_PFULL + 2, B_BNDFULL = B_ODONE + 2,
                        B_BNDEMPTY = B_BNDFULL + NBND, B_COUNT = B_BNDEMPTY + NBND;
-  static_assert((D == 64 && DV == 64) || (D == 128 && DV == 128) || (D == 192 && DV == 128), "head-dim variants");
+  static_assert((D == 64 && DV == 64) || (D == 128 && DV == 128) || (D == 192 && DV == 128) ||
+                    (D == 256 && DV == 256), "head-dim variants");
   static_assert(SMEM_BS <= 227 * 1024 && SMEM <= 227 * 1024, "shared memory");
   static_assert(B_COUNT <= 32, "barrier storage");
   static_assert(OFF_STAGE + LIST_MAX * 8 * 4 <= OFF_BND, "the ring stages the reductions of the list build");
@@ -100,7 +113,9 @@ __global__ void __launch_bounds__(384, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const AttnKParams p) {
   using Cfg = FwdSm100Cfg<D, DV>;
-  constexpr int ROWS = Cfg::ROWS;
+  constexpr bool SPLITV = Cfg::SPLITV;
+  constexpr int ROWS = Cfg::ROWS, DVS = Cfg::DVS;
+  static_assert(!(SPLITV && SPLIT), "split calls have head dims up to 128");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
@@ -121,7 +136,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int n_rows = p.Sq << lg;             // row x of the launch: query x >> lg, head hq + (x & (2^lg - 1))
   const int n_tiles = (n_rows + ROWS - 1) / ROWS;
   int t = n_tiles - 1 - (SPLIT ? blockIdx.x / p.n_split : blockIdx.x), hq = blockIdx.y << lg, b = blockIdx.z;
-  if (!SPLIT && p.fwd_order) {
+  if (!SPLIT && !SPLITV && p.fwd_order) {
     const OrderedCta c = ordered_cta(p.fwd_order, p.Hq);
     t = c.unit; hq = c.head; b = c.b;
   }
@@ -132,7 +147,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int ms = t * ROWS;
   const int off = p.Sk - p.Sq;
   const bool alt = SPLIT && p.alternate;
-  const int sub_rows = alt ? 0 : 128;        // first row of sub-tile 1 against that of sub-tile 0
+  const int sub_rows = alt || SPLITV ? 0 : 128;        // first row of sub-tile 1 against that of sub-tile 0
   // queries [q_lo(s), q_hi(s)) of sub-tile s
   auto q_lo = [&](int s) { return (ms + sub_rows * s) >> lg; };
   auto q_hi = [&](int s) { return min(((ms + sub_rows * s + 127) >> lg) + 1, p.Sq); };
@@ -155,7 +170,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     fence_mbar_init();
     // both Q sub-tiles are requested right away: the loads overlap with the
     // list build (rows past the end of the sequence arrive as zeros)
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < (SPLITV ? 1 : 2); ++s) {
       mbar_arrive_expect_tx(bar(Cfg::B_QFULL + s), Cfg::Q_BYTES);
       for (int dc = 0; dc < D / 64; ++dc)
         tma_load_4d(sQ + s * Cfg::Q_BYTES + dc * Cfg::SUB, &tm_q, bar(Cfg::B_QFULL + s), dc * 64, hq,
@@ -188,7 +203,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       uint32_t f0 = 0, f1 = 0;
       if (n >= 0) {
         f0 = tile_flags(mst, 0, n, q_lo(0), q_hi(0), 128);
-        if (ms + 128 < n_rows) f1 = tile_flags(mst, 0, n, q_lo(1), q_hi(1), 128);
+        if (SPLITV) f1 = f0;
+        else if (ms + 128 < n_rows) f1 = tile_flags(mst, 0, n, q_lo(1), q_hi(1), 128);
         if (spec && n == n_hi - 1 && (f0 | f1) == 0) {
           // the diagonal tile is already on its way into slots 0 / 1, so it is the first list entry whatever its
           // class: an invisible one is computed with the element mask (every score masked, P = 0)
@@ -227,7 +243,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // tensor memory is returned before leaving
     if (warp == 8 && lane == 0) {
       mbar_wait(bar(Cfg::B_QFULL + 0), 0u, wc);
-      mbar_wait(bar(Cfg::B_QFULL + 1), 0u, wc);
+      if (!SPLITV) mbar_wait(bar(Cfg::B_QFULL + 1), 0u, wc);
     }
     if (warp == 9) tmem_dealloc(tmem, 512);
     if constexpr (SPLIT) {
@@ -283,7 +299,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     int bs_bos = 0, bs_pend_lo = INT_MAX, bs_pend_hi = -1;    // pending groups [lo, hi]; lo > hi: none
     bool bs_vec = false;
     if constexpr (BLOCK_SCORE != 0) {
-      if (row < p.Sq)
+      // (d = 256: both warpgroups see the same scores; warpgroup 0 writes them)
+      if (row < p.Sq && !(SPLITV && s == 1))
         bs_dst = p.block_logit + (((int64_t)b * p.Hq + hq) * p.Sq + row) * p.block_ld;
       if constexpr (BLOCK_BOS) {
         bs_acc = reinterpret_cast<float*>(smem + Cfg::OFF_BS) + tid;
@@ -386,9 +403,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           }
         }
       } else {
-      uint8_t* stage = smem + Cfg::OFF_Q + s * Cfg::Q_BYTES;   // Q is no longer needed
+      uint8_t* stage = smem + Cfg::OFF_Q + (SPLITV ? 0 : s * Cfg::Q_BYTES);   // Q is no longer needed
+      constexpr int CH0 = SPLITV ? DVS / 8 : 0;          // d = 256: warpgroup s stages chunks [16 s, 16 s + 16)
 #pragma unroll
-      for (int c = 0; c < DV / 32; ++c) {
+      for (int c = 0; c < DVS / 32; ++c) {
         uint32_t orr[32];
         if (n_done > 0) {
           tmem_ld32(tO + 32 * c, orr);
@@ -404,20 +422,20 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           v.y = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 2]) * inv, __uint_as_float(orr[8 * q4 + 3]) * inv);
           v.z = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 4]) * inv, __uint_as_float(orr[8 * q4 + 5]) * inv);
           v.w = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 6]) * inv, __uint_as_float(orr[8 * q4 + 7]) * inv);
-          const int chunk = 4 * c + q4;                 // 16-byte chunk inside the row
+          const int chunk = CH0 * s + 4 * c + q4;       // 16-byte chunk inside the row
           *reinterpret_cast<uint4*>(stage + r * (DV * 2) + ((chunk ^ (r & (DV / 8 - 1))) << 4)) = v;
         }
       }
-      if (prow < n_rows)
+      if (prow < n_rows && !(SPLITV && s == 1))
         p.lse[((int64_t)b * p.Hq + head) * p.Sq + row] = l_tot > 0.f ? (m_fin + log2f(l_tot)) * kLn2 : neg_inf();
       __syncwarp();   // each warp stores the 32 rows it staged itself: no cross-warp dependency
-      const int rbase = ms + 128 * s;
+      const int rbase = ms + (SPLITV ? 0 : 128 * s);
       uint16_t* go = reinterpret_cast<uint16_t*>(p.o) + b * p.o_b + hq * p.o_h;
-      constexpr int CH = DV / 8;                         // chunks per row
+      constexpr int CH = DV / 8, CHW = DVS / 8;          // chunks per row, chunks this warpgroup staged
       const int wrow = (warp & 3) * 32;
 #pragma unroll 4
-      for (int idx = lane; idx < 32 * CH; idx += 32) {
-        const int rr = wrow + idx / CH, cc = idx % CH;
+      for (int idx = lane; idx < 32 * CHW; idx += 32) {
+        const int rr = wrow + idx / CHW, cc = CH0 * s + idx % CHW;
         const int x = rbase + rr;
         if (x < n_rows && cc * 8 < p.dv_dim) {
           const uint4 v = *reinterpret_cast<const uint4*>(stage + rr * (DV * 2) + ((cc ^ (rr & (CH - 1))) << 4));
@@ -463,12 +481,12 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
       }
       // a sub-tile without work never consumed its Q load: make sure it has landed
-      if (ok && lane == 0) { mbar_wait(bar(Cfg::B_QFULL + 0), 0u, wc); mbar_wait(bar(Cfg::B_QFULL + 1), 0u, wc); }
+      if (ok && lane == 0) { mbar_wait(bar(Cfg::B_QFULL + 0), 0u, wc); if (!SPLITV) mbar_wait(bar(Cfg::B_QFULL + 1), 0u, wc); }
     } else if (warp == 9) {
       // =========================== UMMA issuer ===========================
       if (elect_one()) {
         constexpr uint32_t idesc_qk = make_idesc(IS_BF16, 128, 128, 0, 0);
-        constexpr uint32_t idesc_pv = make_idesc(IS_BF16, 128, DV, 0, 1);
+        constexpr uint32_t idesc_pv = make_idesc(IS_BF16, 128, DVS, 0, 1);
         int npv[2] = {0, 0};
         bool q_ready[2] = {false, false};
         bool ok = true;
@@ -481,10 +499,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             constexpr int s = decltype(sub)::value;   // compile-time: the per-sub-tile counters stay in registers
           const int k = 2 * i, slot = k % Cfg::NSTAGE;
           ok = ok && mbar_wait(bar(Cfg::B_KVFULL + slot), (uint32_t)(k / Cfg::NSTAGE) & 1u, wc);
-          if (ok && !q_ready[s]) { ok = mbar_wait(bar(Cfg::B_QFULL + s), 0u, wc); q_ready[s] = true; }
+          if (ok && !q_ready[s]) { ok = mbar_wait(bar(Cfg::B_QFULL + (SPLITV ? 0 : s)), 0u, wc); q_ready[s] = true; }
           if (!ok) return;
           tc_fence_after();
-          const uint64_t da = dq0 + (uint64_t)(s * (Cfg::Q_BYTES >> 4));
+          const uint64_t da = dq0 + (uint64_t)(SPLITV ? 0 : s * (Cfg::Q_BYTES >> 4));
           const uint64_t db = dk0 + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4));
           const uint32_t dst = tmem + 128u * s;
           if constexpr (D == 128) umma_ss_x8<(Cfg::SUB >> 4), (Cfg::SUB >> 4)>(dst, da, db, idesc_qk, 0u);
@@ -492,6 +510,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             // three 64-column sub-tiles of q / k: eight k-steps, then four more on top
             umma_ss_x8<(Cfg::SUB >> 4), (Cfg::SUB >> 4)>(dst, da, db, idesc_qk, 0u);
             umma_ss_x4(dst, da + (uint64_t)(2 * (Cfg::SUB >> 4)), db + (uint64_t)(2 * (Cfg::SUB >> 4)), idesc_qk, 1u);
+          } else if constexpr (D == 256) {
+            // four 64-column sub-tiles: eight k-steps over the first two, eight over the last two
+            umma_ss_x8<(Cfg::SUB >> 4), (Cfg::SUB >> 4)>(dst, da, db, idesc_qk, 0u);
+            umma_ss_x8<(Cfg::SUB >> 4), (Cfg::SUB >> 4)>(dst, da + (uint64_t)(2 * (Cfg::SUB >> 4)),
+                                                         db + (uint64_t)(2 * (Cfg::SUB >> 4)), idesc_qk, 1u);
           } else umma_ss_x4(dst, da, db, idesc_qk, 0u);
           tc_commit(bar(Cfg::B_SFULL + s));
         };
@@ -502,7 +525,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           ok = ok && mbar_wait(bar(Cfg::B_PFULL + s), (uint32_t)npv[s] & 1u, wc);
           if (!ok) return;
           tc_fence_after();
-          const uint64_t db = dv0 + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4));
+          // (d = 256: warpgroup s owns V columns [128 s, 128 s + 128): sub-tiles 2 s and 2 s + 1 of the V tile)
+          const uint64_t db = dv0 + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4) + (SPLITV ? s * 2 * (Cfg::SUB >> 4) : 0));
           const uint32_t dst = tmem + 256u + 128u * s, src = tmem + 128u * s + 64u;
           const uint32_t acc0 = npv[s] > 0 ? 1u : 0u;
           umma_ts_xn<8>(dst, src, db, idesc_pv, acc0);
@@ -783,6 +807,8 @@ int fwd_sm100_launch(const AttnKParams& p_in, const fm_attn_args* a, cudaStream_
   }
 #define FM_FWD_DISPATCH(BSZ, BOS)                                                                         \
   do {                                                                                                    \
+    if (a->d == 256)                                                                                      \
+      return bf ? launch_fwd_sm100<256, 256, true, BSZ, BOS>(p, a, s) : launch_fwd_sm100<256, 256, false, BSZ, BOS>(p, a, s); \
     if (a->d == 192)                                                                                      \
       return bf ? launch_fwd_sm100<192, 128, true, BSZ, BOS>(p, a, s) : launch_fwd_sm100<192, 128, false, BSZ, BOS>(p, a, s); \
     if (small)                                                                                            \

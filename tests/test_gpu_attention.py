@@ -167,6 +167,25 @@ def test_ragged_shapes_big_head_dims(kind, d, dv):
 
 
 @pytest.mark.parametrize("kind", MASKS)
+def test_masks_d256_short_sequences(kind):
+    """Batches of short sequences at 256 / 256: the forward of blocks of 128 rows (one CTA, its two warpgroups own the
+    two halves of V / O).  One partial block, a full and a nearly empty one, three blocks with several key tiles."""
+    for S in (40, 129, 300):
+        _run(kind, 10, S, S, 8, 4, 256, 256, sink=True, seed=53)
+    assert _kernel_status() == 0
+
+
+@pytest.mark.parametrize("d,dv", [(512, 512), (576, 512)])
+@pytest.mark.parametrize("kind", ["causal_doc", "none_full", "four_column"])
+def test_short_sequences_of_the_widest_heads(kind, d, dv):
+    """Batches of short sequences at 512 and 576 / 512: the warp-MMA forward, here with mask reductions over tiles
+    wider than its own."""
+    for S in (33, 64, 100):
+        _run(kind, 16, S, S, 8, 1, d, dv, sink=True, seed=54)
+    assert _kernel_status() == 0
+
+
+@pytest.mark.parametrize("kind", MASKS)
 def test_masks_d256(kind):
     """Every mask family through the 256 / 256 forward variant of the tcgen05 kernel (128 query rows per CTA, the
     two warpgroups own the two 128-column halves of V / O); the backward of this head dim is the warp-MMA one."""

@@ -69,7 +69,8 @@ def test_block_logit_shapes(b, s, sk, h, d, causal, variant):
 
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("b,s,sk,h,d,dv", [(1, 512, 512, 8, 256, 256), (1, 1024, 1024, 2, 256, 256),
-                                           (1, 511, 513, 2, 256, 256), (1, 320, 320, 4, 192, 128)])
+                                           (1, 511, 513, 2, 256, 256), (1, 320, 320, 4, 192, 128),
+                                           (10, 130, 130, 8, 256, 256)])
 def test_block_logit_head_dims_above_128(b, s, sk, h, d, dv, causal):
     """Both head dims run the tcgen05 forward (d = 256 is the reference's HySparse full-attention configuration):
     the plain forward and the block-score variant must agree bitwise on O and LSE."""
