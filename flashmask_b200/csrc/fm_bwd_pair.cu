@@ -10,8 +10,8 @@
 // 8 GEMM units instead of 5 at 256, 2.6 times the work at 576 / 512.  Written once and read twice, P and dS cost
 // 4 bytes and 10 bytes of traffic per visible pair and head against 5 x 512 (5 x 1100) flops: the HBM time stays
 // below the tensor time at these head dims (it would not at 128).  The workspace is bounded (kBudget): a chunk is
-// as many kv groups, or failing that as many query rows of one group, as fit; dK / dV of a group that needs
-// several row chunks are summed in fp32 accumulators in chunk order.  Every sum has one owner and a fixed order.
+// as many kv groups (of all batch entries), or failing that as many query rows of one group, as fit; dK / dV of a group
+// that needs several row chunks are summed in fp32 accumulators in chunk order.  Every sum has one owner and a fixed order.
 //
 // Workspace format.  128 query rows x 64 keys are one 16 KB block [8-key piece][row][8 keys]: a warp (32 rows)
 // stores 512 contiguous bytes, the block is at the same time a K-major operand (dQ: M = rows) and an MN-major one
@@ -37,15 +37,20 @@ using namespace sm100;
 
 __device__ int g_bwd_pair_status = 0;
 
-// One chunk: q heads [head0, head0 + heads) of batch b, query rows [row0, row0 + 128 * row_blocks).
+// One chunk: q heads [head0, head0 + heads), counted through all batch entries, query rows
+// [row0, row0 + 128 * row_blocks).
 struct BwdPairChunk {
   uint4* ws_p; uint4* ws_ds;     // [heads][row_blocks][key_blocks] blocks of 16 KB
   float* acc_dk; float* acc_dv;  // fp32 sums of earlier row chunks, [unit][CTA][column][128 rows]
-  int b, head0, heads, row0, row_blocks, key_blocks;
+  int head0, heads, row0, row_blocks, key_blocks;
   int first, last;               // first / last row chunk of its heads
   int n_units, n_seg;            // scores: units; parts a row block's key tiles are dealt into
   int n_dk, n_dv, n_dq;          // grads: units of each kind, in this order
 };
+
+// Batch entry and head of a head counted through all entries.
+struct BatchHead { int b, h; };
+__device__ __forceinline__ BatchHead batch_head(int flat, int heads) { return {flat / heads, flat % heads}; }
 
 constexpr int kPairListMax = 2048;
 
@@ -145,13 +150,13 @@ bwd_pair_scores_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       const ScoreUnit un = score_unit(ck, u);
       const int cnt = infos[j & 1];
       const uint32_t* list = lists + (j & 1) * Cfg::LIST_MAX;
-      const int hq = ck.head0 + un.h;
+      const BatchHead bh = batch_head(ck.head0 + un.h, p.Hq);
       const int rb = 2 * un.rp + rank;
       const int row = ck.row0 + 128 * rb + r;
-      const int bh_mask = md.ncols ? ((md.mask_B == 1 ? 0 : ck.b) * md.Hm + hq / (p.Hq / md.Hm)) : 0;
+      const int bh_mask = md.ncols ? ((md.mask_B == 1 ? 0 : bh.b) * md.Hm + bh.h / (p.Hq / md.Hm)) : 0;
       float lse2 = 0.f, dps = 0.f;
       if (row < p.Sq_r) {
-        const int64_t at = ((int64_t)ck.b * p.Hq + hq) * p.Sq_r + row;
+        const int64_t at = (int64_t)(ck.head0 + un.h) * p.Sq_r + row;
         lse2 = p.lse_log2[at];
         dps = p.dpsum[at];
       }
@@ -246,8 +251,8 @@ bwd_pair_scores_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         if (j >= 2) ok = __all_sync(0xffffffffu, mbar_wait_idle(bar(PairInfoBars::FREE + (j & 1)), (uint32_t)((j >> 1) - 1) & 1u, wc));
         if (!ok) break;
         const ScoreUnit un = score_unit(ck, u);
-        const int hq = ck.head0 + un.h;
-        const int bh_mask = md.ncols ? ((md.mask_B == 1 ? 0 : ck.b) * md.Hm + hq / (p.Hq / md.Hm)) : 0;
+        const BatchHead bh = batch_head(ck.head0 + un.h, p.Hq);
+        const int bh_mask = md.ncols ? ((md.mask_B == 1 ? 0 : bh.b) * md.Hm + bh.h / (p.Hq / md.Hm)) : 0;
         const int ms = ck.row0 + 256 * un.rp;
         const int nb = (p.Sk + 127) / 128;
         const int n_hi = ms >= p.Sq ? 0 : (md.causal ? max(0, min(nb, (min(ms + 256, p.Sq) + off + 127) / 128)) : nb);
@@ -287,7 +292,8 @@ bwd_pair_scores_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           const ScoreUnit un = score_unit(ck, u);
           const int cnt = infos[j & 1];
           const uint32_t* list = lists + (j & 1) * Cfg::LIST_MAX;
-          const int hq = ck.head0 + un.h, hk = hq / (p.Hq / p.Hkv);
+          const BatchHead bh = batch_head(ck.head0 + un.h, p.Hq);
+          const int hk = bh.h / (p.Hq / p.Hkv);
           const int row = ck.row0 + 128 * (2 * un.rp + rank);
           for (int i = 0; i < cnt && ok; ++i) {
             const int key = (int)(list[i] & 0xFFFFu) * 256 + 128 * rank;
@@ -298,8 +304,8 @@ bwd_pair_scores_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
               const uint32_t dst = sRing + slot * Cfg::SLOT_BYTES, fb = full + 8u * (uint32_t)slot;
               const bool first = c < D / 64;
               const int col = 64 * (first ? c : c - D / 64);
-              tma2_load_4d(dst, first ? &tm_q : &tm_do, fb, col, hq, row, ck.b);
-              tma2_load_4d(dst + Cfg::SUB128, first ? &tm_k : &tm_v, fb, col, hk, key, ck.b);
+              tma2_load_4d(dst, first ? &tm_q : &tm_do, fb, col, bh.h, row, bh.b);
+              tma2_load_4d(dst + Cfg::SUB128, first ? &tm_k : &tm_v, fb, col, hk, key, bh.b);
               if (++slot == Cfg::NSTAGE) { slot = 0; phase ^= 1u; }
             }
           }
@@ -489,9 +495,10 @@ bwd_pair_grads_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_con
       const int n_rows = g.kind == GRAD_DQ ? p.Sq : p.Sk;
       // where the result goes: the output, or (dK / dV of a group in several row chunks) the fp32 sums
       uint16_t* out;
-      if (g.kind == GRAD_DQ) out = reinterpret_cast<uint16_t*>(p.dq) + ck.b * p.dq_b + (int64_t)row * p.dq_s + (ck.head0 + g.h) * p.dq_h;
-      else if (g.kind == GRAD_DK) out = reinterpret_cast<uint16_t*>(p.dk) + ck.b * p.dk_b + (int64_t)row * p.dk_s + (ck.head0 / G + g.h) * p.dk_h;
-      else out = reinterpret_cast<uint16_t*>(p.dv) + ck.b * p.dv_b + (int64_t)row * p.dv_s + (ck.head0 / G + g.h) * p.dv_h;
+      const BatchHead bh = g.kind == GRAD_DQ ? batch_head(ck.head0 + g.h, p.Hq) : batch_head(ck.head0 / G + g.h, p.Hkv);
+      if (g.kind == GRAD_DQ) out = reinterpret_cast<uint16_t*>(p.dq) + bh.b * p.dq_b + (int64_t)row * p.dq_s + bh.h * p.dq_h;
+      else if (g.kind == GRAD_DK) out = reinterpret_cast<uint16_t*>(p.dk) + bh.b * p.dk_b + (int64_t)row * p.dk_s + bh.h * p.dk_h;
+      else out = reinterpret_cast<uint16_t*>(p.dv) + bh.b * p.dv_b + (int64_t)row * p.dv_s + bh.h * p.dv_h;
       out += 256 * g.slice;
       const bool sums_in = g.kind != GRAD_DQ && !ck.first, sums_out = g.kind != GRAD_DQ && !ck.last;
       float* acc = nullptr;
@@ -560,8 +567,8 @@ bwd_pair_grads_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_con
         if (j >= 2) ok = __all_sync(0xffffffffu, mbar_wait_idle(bar(PairInfoBars::FREE + (j & 1)), (uint32_t)((j >> 1) - 1) & 1u, wc));
         if (!ok) break;
         const GradUnit g = grad_unit<D, DV>(ck, u, groups);
-        const int hq = ck.head0 + (g.kind == GRAD_DQ ? g.h : g.h * G);
-        const int bh_mask = md.ncols ? ((md.mask_B == 1 ? 0 : ck.b) * md.Hm + hq / (p.Hq / md.Hm)) : 0;
+        const BatchHead bh = batch_head(ck.head0 + (g.kind == GRAD_DQ ? g.h : g.h * G), p.Hq);
+        const int bh_mask = md.ncols ? ((md.mask_B == 1 ? 0 : bh.b) * md.Hm + bh.h / (p.Hq / md.Hm)) : 0;
         uint16_t* list = lists + (j & 1) * Cfg::LIST_MAX;
         int cnt = 0;
         // dQ: key tiles that either half of the 256 rows sees; dK / dV: 128-row blocks that see either half of the keys
@@ -610,7 +617,7 @@ bwd_pair_grads_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_con
           const int n_heads = is_dq ? 1 : G;
           for (int hh = 0; hh < n_heads && ok; ++hh) {
             const int h = is_dq ? g.h : g.h * G + hh;                  // q head inside the chunk
-            const int hB = is_dq ? (ck.head0 + g.h) / G : ck.head0 + h;   // head of the B operand
+            const BatchHead bB = is_dq ? batch_head((ck.head0 + g.h) / G, p.Hkv) : batch_head(ck.head0 + h, p.Hq);   // of the B operand
             for (int i = 0; i < cnt && ok; ++i) {
               const int x = list[i];
               const int rb = is_dq ? 2 * g.blk + rank : x;
@@ -625,9 +632,9 @@ bwd_pair_grads_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_con
               tma2_load_2d(dst, tA, fb, 0, blk * 128, stream_policy);
               tma2_load_2d(dst + Cfg::SUB128, tA, fb, 0, blk * 128 + 128, stream_policy);
               const int col = 256 * g.slice + 128 * rank;
-              tma2_load_4d(dst + Cfg::A_BYTES, tB, fb, col, hB, rowB, ck.b);
-              tma2_load_4d(dst + Cfg::A_BYTES + Cfg::SUB128, tB, fb, col + 64, hB, rowB, ck.b);
-              if (tail) tma2_load_4d(dst + Cfg::A_BYTES + Cfg::B_BYTES, tT, fb, 256 * Cfg::NS_D + 32 * rank, hB, rowB, ck.b);
+              tma2_load_4d(dst + Cfg::A_BYTES, tB, fb, col, bB.h, rowB, bB.b);
+              tma2_load_4d(dst + Cfg::A_BYTES + Cfg::SUB128, tB, fb, col + 64, bB.h, rowB, bB.b);
+              if (tail) tma2_load_4d(dst + Cfg::A_BYTES + Cfg::B_BYTES, tT, fb, 256 * Cfg::NS_D + 32 * rank, bB.h, rowB, bB.b);
               if (++slot == Cfg::NSTAGE) { slot = 0; phase ^= 1u; }
             }
           }
@@ -719,7 +726,7 @@ static BwdPairPlan bwd_pair_plan(const fm_attn_args* a) {
   const size_t sq = ((size_t)a->Sq + 255) / 256 * 256, sk = ((size_t)a->Sk + 255) / 256 * 256;
   const size_t row = (size_t)G * sk * 4;              // P and dS of one query row of every head of a group
   pl.key_blocks = (int)(sk / 64);
-  pl.groups = (int)std::min<size_t>(a->Hkv, std::max<size_t>(1, kBudget / (row * sq)));
+  pl.groups = (int)std::min<size_t>((size_t)a->B * a->Hkv, std::max<size_t>(1, kBudget / (row * sq)));
   pl.rows = (int)std::min(sq, std::max<size_t>(256, kBudget / row / 256 * 256));
   pl.sums = (size_t)pl.rows < sq;
   pl.block_bytes = (size_t)pl.groups * pl.rows * row / 2;
@@ -732,6 +739,10 @@ bool bwd_pair_supported(const fm_attn_args* a) {
   const bool dims = (a->d == 256 && a->dv == 256) || ((a->d == 512 || a->d == 576) && a->dv == 512);
   // (a size query comes before the arguments are validated)
   if (!dims || a->Sq <= 0 || a->Sk <= 0 || a->Hkv <= 0 || a->Hq <= 0 || a->Hq % a->Hkv) return false;
+  // Sequences of one 64-row tile: a 256 x 256 tile of the score kernel is mostly padding.  64 x 64 rows with 16 heads,
+  // backward: 256 / 256 warp-MMA 162 us against 230, 576 / 512 266 against 322; 64 x 100 rows at 256 351 against 264.
+  // With few kv heads the warp-MMA kernels leave the chip idle (8 x 64 rows, 16 / 4 heads: 40 us, pair 36).
+  if (a->Sq <= 64 && a->Sk <= 64 && a->B * a->Hkv >= 16 * std::min(a->Hq / a->Hkv, 4)) return false;
   // a chunk is at least 256 rows of every head of one group; past four budgets the warp-MMA kernels, which need no
   // workspace, keep the call
   const size_t least = (size_t)(a->Hq / a->Hkv) * (((size_t)a->Sk + 255) / 256 * 256) * 4 * 256;
@@ -789,26 +800,26 @@ static int launch_bwd_pair(const AttnKParams& p, const fm_attn_args* a, uint8_t*
   c.acc_dk = reinterpret_cast<float*>(ws + 2 * pl.block_bytes);
   c.acc_dv = reinterpret_cast<float*>(ws + 2 * pl.block_bytes + pl.acc_dk_bytes);
   c.key_blocks = pl.key_blocks;
-  for (int b = 0; b < a->B; ++b)
-    for (int g0 = 0; g0 < a->Hkv; g0 += pl.groups)
-      for (int row0 = 0; row0 < a->Sq; row0 += pl.rows) {
-        const int groups = std::min(pl.groups, a->Hkv - g0);
-        const int rows = (std::min(pl.rows, a->Sq - row0) + 255) / 256 * 256;
-        c.b = b; c.head0 = g0 * G; c.heads = groups * G; c.row0 = row0; c.row_blocks = rows / 128;
-        c.first = row0 == 0; c.last = row0 + pl.rows >= a->Sq;
-        // about eight units per pair: the last round of units is then a small part of the launch
-        const int blocks = c.heads * c.row_blocks / 2;
-        c.n_seg = std::max(1, std::min(n_tiles256, (8 * pairs + blocks / 2) / blocks));
-        c.n_units = blocks * c.n_seg;
-        c.n_dk = groups * n_tiles256 * GC::NS_D;
-        c.n_dv = groups * n_tiles256 * GC::NS_V;
-        c.n_dq = blocks * GC::NS_D;
-        k1<<<2 * std::min(pairs, c.n_units), 384, PairScoreCfg::SMEM, s>>>(q, dO, k, v, p, c);
-        FM_CUDA_TRY(cudaGetLastError());
-        k2<<<2 * std::min(pairs, c.n_dk + c.n_dv + c.n_dq), 384, GC::SMEM, s>>>(tp, tds, q, dO, k, qt, kt, p, c);
-        FM_CUDA_TRY(cudaGetLastError());
-        count_launches(2);
-      }
+  const int all_groups = a->B * a->Hkv;
+  for (int g0 = 0; g0 < all_groups; g0 += pl.groups)
+    for (int row0 = 0; row0 < a->Sq; row0 += pl.rows) {
+      const int groups = std::min(pl.groups, all_groups - g0);
+      const int rows = (std::min(pl.rows, a->Sq - row0) + 255) / 256 * 256;
+      c.head0 = g0 * G; c.heads = groups * G; c.row0 = row0; c.row_blocks = rows / 128;
+      c.first = row0 == 0; c.last = row0 + pl.rows >= a->Sq;
+      // about eight units per pair: the last round of units is then a small part of the launch
+      const int blocks = c.heads * c.row_blocks / 2;
+      c.n_seg = std::max(1, std::min(n_tiles256, (8 * pairs + blocks / 2) / blocks));
+      c.n_units = blocks * c.n_seg;
+      c.n_dk = groups * n_tiles256 * GC::NS_D;
+      c.n_dv = groups * n_tiles256 * GC::NS_V;
+      c.n_dq = blocks * GC::NS_D;
+      k1<<<2 * std::min(pairs, c.n_units), 384, PairScoreCfg::SMEM, s>>>(q, dO, k, v, p, c);
+      FM_CUDA_TRY(cudaGetLastError());
+      k2<<<2 * std::min(pairs, c.n_dk + c.n_dv + c.n_dq), 384, GC::SMEM, s>>>(tp, tds, q, dO, k, qt, kt, p, c);
+      FM_CUDA_TRY(cudaGetLastError());
+      count_launches(2);
+    }
   return FM_OK;
 }
 

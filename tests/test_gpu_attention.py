@@ -175,6 +175,17 @@ def test_masks_d256_short_sequences(kind):
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("kind", ["causal_doc", "none_full", "sliding_window"])
+@pytest.mark.parametrize("B,S,Hq,Hkv,d,dv", [(3, 300, 4, 2, 256, 256), (5, 130, 2, 1, 576, 512), (4, 64, 4, 4, 256, 256),
+                                             (4, 65, 4, 4, 256, 256), (2, 257, 3, 3, 512, 512)])
+def test_batches_through_the_pair_backward(kind, B, S, Hq, Hkv, d, dv):
+    """Heads of several batch entries in one pair of launches, masks of their own, either side of the line to the
+    warp-MMA kernels."""
+    _run(kind, B, S, S, Hq, Hkv, d, dv, sink=True, seed=55)
+    _run(kind, B, S, S, Hq, Hkv, d, dv, seed=56, hm=Hkv if Hkv > 1 else 1)
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("d,dv", [(512, 512), (576, 512)])
 @pytest.mark.parametrize("kind", ["causal_doc", "none_full", "four_column"])
 def test_short_sequences_of_the_widest_heads(kind, d, dv):
