@@ -89,6 +89,51 @@ __device__ __forceinline__ ScoreUnit score_unit(const BwdPairChunk& c, int u) {
   return s;
 }
 
+// Masks the scores of 128 columns whose bounds start at src (`valid` of them exist).
+// Every lane reads the same bounds: broadcasts from the L1.  One loop per mask form, so that several columns' bounds
+// are in flight (with the form decided inside the loop a partial tile waited for 128 loads in turn: 16 x 1024 rows of
+// short documents, 16 heads, d = 256, took 1322 us against 733 us for the causal triangle that contains them).
+__device__ __forceinline__ void mask_columns(const MaskDesc& md, const int32_t* src, int valid, int row, uint32_t* sr) {
+  const uint32_t NEG = 0xff800000u;
+  if (md.ncols == 1) {
+    if (valid == 128 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const int4 v = __ldg(reinterpret_cast<const int4*>(src) + j);
+        if (row >= v.x) sr[4 * j] = NEG;
+        if (row >= v.y) sr[4 * j + 1] = NEG;
+        if (row >= v.z) sr[4 * j + 2] = NEG;
+        if (row >= v.w) sr[4 * j + 3] = NEG;
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < 128; ++c)
+        if (c < valid && row >= __ldg(src + c)) sr[c] = NEG;
+    }
+  } else if (md.ncols == 2 && md.causal) {
+#pragma unroll
+    for (int c = 0; c < 128; ++c)
+      if (c < valid) {
+        const int2 v = __ldg(reinterpret_cast<const int2*>(src) + c);
+        if (row >= v.x && row < v.y) sr[c] = NEG;
+      }
+  } else if (md.ncols == 2) {
+#pragma unroll
+    for (int c = 0; c < 128; ++c)
+      if (c < valid) {
+        const int2 v = __ldg(reinterpret_cast<const int2*>(src) + c);
+        if (row >= v.x || row < v.y) sr[c] = NEG;
+      }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 128; ++c)
+      if (c < valid) {
+        const int4 v = __ldg(reinterpret_cast<const int4*>(src) + c);
+        if ((row >= v.x && row < v.y) || (row >= v.z && row < v.w)) sr[c] = NEG;
+      }
+  }
+}
+
 template <int D, int DV, bool IS_BF16>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
 bwd_pair_scores_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
@@ -168,9 +213,6 @@ bwd_pair_scores_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         ok = __all_sync(0xffffffffu, mbar_wait(bar(Cfg::B_SFULL), it & 1u, wc));
         if (!ok) break;
         tc_fence_after();
-        const int64_t blk = blk0 + 4 * n2 + 2 * w;
-        uint4* gp = ck.ws_p + blk * 1024 + r;              // + 128 * (8-key piece)
-        uint4* gd = ck.ws_ds + blk * 1024 + r;
         uint32_t sr[128];
         tmem_ld32(tS, sr); tmem_ld32(tS + 32, sr + 32); tmem_ld32(tS + 64, sr + 64); tmem_ld32(tS + 96, sr + 96);
         tc_wait_ld();
@@ -181,13 +223,7 @@ bwd_pair_scores_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         if (flags & FM_TF_BOUNDS) {
           const int valid = min(128, p.Sk - j0);
           const int32_t* src = md.mask + ((size_t)bh_mask * p.Sk + j0) * md.ncols;
-#pragma unroll
-          for (int c = 0; c < 128; ++c) {
-            if (c < valid) {
-              const Bounds4 bd = load_bounds(md, src + (size_t)c * md.ncols);
-              if ((row >= bd.lts && row < bd.lte) || (row >= bd.uts && row < bd.ute)) sr[c] = NEG;
-            }
-          }
+          mask_columns(md, src, valid, row, sr);
         }
         if (flags & (FM_TF_CAUSAL | FM_TF_RAGGED)) {
           int jmax = p.Sk - 1 - j0;
@@ -200,6 +236,9 @@ bwd_pair_scores_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 #pragma unroll
           for (int c = 0; c < 128; ++c) sr[c] = NEG;
         }
+        const int64_t blk = blk0 + 4 * n2 + 2 * w;
+        uint4* gp = ck.ws_p + blk * 1024 + r;              // + 128 * (8-key piece)
+        uint4* gd = ck.ws_ds + blk * 1024 + r;
 #pragma unroll
         for (int c = 0; c < 128; c += 8) {
           uint32_t pk[4];

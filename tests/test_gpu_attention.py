@@ -186,6 +186,15 @@ def test_batches_through_the_pair_backward(kind, B, S, Hq, Hkv, d, dv):
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("kind", ["causal_doc", "random_eviction", "bidir_doc", "four_column"])
+@pytest.mark.parametrize("S", [512, 513, 515])
+def test_bounds_of_partial_tiles_in_the_pair_backward(kind, S):
+    """The mask forms of partial tiles (one, two and four bounds per column), whole and ragged tiles, and bounds whose
+    rows start on and off a 16-byte boundary (a second mask head after an odd number of columns)."""
+    _run(kind, 1, S, S, 2, 2, 256, 256, seed=59, hm=2)
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("d,dv", [(512, 512), (576, 512)])
 @pytest.mark.parametrize("kind", ["causal_doc", "none_full", "four_column"])
 def test_short_sequences_of_the_widest_heads(kind, d, dv):
