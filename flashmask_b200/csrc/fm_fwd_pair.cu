@@ -53,7 +53,7 @@ struct FwdPairCfg {
   static constexpr int SMEM_BS = OFF_BSA + 16 * 128 * 4 + 1024;
   static_assert(D != 256 || SMEM_BS <= 227 * 1024, "shared memory of the block-score variant");
   static constexpr int B_Q = 0, B_KVFULL = 1, B_KVEMPTY = B_KVFULL + NSTAGE, B_SFULL = B_KVEMPTY + NSTAGE,
-                       B_PFULL = B_SFULL + 2, B_ODONE = B_PFULL + 2, B_BNDFULL = B_ODONE + 1,
+                       B_PFULL = B_SFULL + 2, B_ODONE = B_PFULL + 2, B_BNDFULL = B_ODONE + 2,
                        B_BNDEMPTY = B_BNDFULL + NBND, B_COUNT = B_BNDEMPTY + NBND;
   static_assert(D == 256 || D == 512 || D == 576, "head-dim variants");
   static_assert(B_COUNT <= 32, "barrier storage");
@@ -123,7 +123,7 @@ fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     mbar_init(bar(Cfg::B_Q), 1);
     for (int i = 0; i < Cfg::NSTAGE; ++i) { mbar_init(bar(Cfg::B_KVFULL + i), 1); mbar_init(bar(Cfg::B_KVEMPTY + i), 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(bar(Cfg::B_SFULL + s), 1); mbar_init(bar(Cfg::B_PFULL + s), 16); }
-    mbar_init(bar(Cfg::B_ODONE), 1);
+    for (int s = 0; s < 2; ++s) mbar_init(bar(Cfg::B_ODONE + s), 1);
     for (int i = 0; i < Cfg::NBND; ++i) { mbar_init(bar(Cfg::B_BNDFULL + i), 32); mbar_init(bar(Cfg::B_BNDEMPTY + i), 256); }
     fence_mbar_init();
   }
@@ -350,7 +350,7 @@ fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           l_run *= alpha;
         }
         if (__any_sync(0xffffffffu, need) && i > 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait(bar(Cfg::B_ODONE), (uint32_t)(i - 1) & 1u, wc));
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(Cfg::B_ODONE + ((i - 1) & 1)), (uint32_t)((i - 1) >> 1) & 1u, wc));
           tc_fence_after();
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -389,10 +389,11 @@ fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int g = bs_pend_hi; g >= bs_pend_lo; --g) block_flush<128>(bs_dst, bs_acc, g, bs_vec, p.block_cols);
     }
     // ---- epilogue: O / l -> 16 bit -> smem staging -> coalesced stores; LSE ----
-    // (the scores of the last tile only prove O of the last tile but two: its phases are awaited one by one)
-    if (ok && cnt > 1) ok = __all_sync(0xffffffffu, mbar_wait(bar(Cfg::B_ODONE), (uint32_t)(cnt - 2) & 1u, wc));
+    // O of tile i is signalled on the barrier of its parity.  The scores of the last tile prove O of the last tile but
+    // two, so the phase before the awaited one is over; and no later phase can pass by a warp that comes late (with one
+    // barrier for all tiles, awaited phase by phase, the last one could: the wait then ran out).
     if (ok) {
-      ok = __all_sync(0xffffffffu, mbar_wait(bar(Cfg::B_ODONE), (uint32_t)(cnt - 1) & 1u, wc));
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(Cfg::B_ODONE + ((cnt - 1) & 1)), (uint32_t)((cnt - 1) >> 1) & 1u, wc));
       tc_fence_after();
     }
     // (every warp has read the maxima of the last tile before it handed over P, and O is done only after that)
@@ -549,7 +550,7 @@ fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             release();
           }
           if (!ok) break;
-          tc2_commit_both(bar(Cfg::B_ODONE));
+          tc2_commit_both(bar(Cfg::B_ODONE + (i & 1)));
         }
       }
       __syncwarp();

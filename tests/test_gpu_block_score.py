@@ -6,6 +6,7 @@ rejection, the probe tests of which entries are written) and add what that file 
 column-bound masks and document-relative block ids.  Tolerance as there:
 ``0.06 * sqrt(d) * softmax_scale`` on the finite entries, identical -inf pattern.
 """
+import ctypes
 import math
 
 import numpy as np
@@ -180,6 +181,34 @@ def test_block_logit_with_column_bound_mask(block_size, with_bos, variant):
     _, _, bl = _run(q, k, v, True, block_size, idx=idx, bos=bos if with_bos else None)
     ref = oracle.block_logit_ref(q, k, idx.numpy(), True, None, block_size, block_bos=bos if with_bos else None)
     _check(bl, ref, 128)
+
+
+@pytest.mark.parametrize("block_size", [32, 64, 128])
+@pytest.mark.parametrize("with_bos", [False, True])
+@pytest.mark.parametrize("B,S,hq,d,dv", [(1, 1000, 2, 256, 256), (10, 300, 8, 256, 256), (2, 700, 4, 256, 256)])
+def test_block_logit_wide_heads_with_documents(B, S, hq, d, dv, block_size, with_bos):
+    """The variants above 192 with a document mask and document-relative ids, whose last scores are merged into the
+    output while the last tile's P V runs: no wait runs out.  Scores, and O and LSE bitwise those of the plain forward."""
+    status = lambda: (_lib.check(_lib.load().fm_kernel_status(ctypes.byref(st), 1), "fm_kernel_status"), st.value)[1]
+    st = ctypes.c_int(0)
+    status()
+    cuts = [[S // 7 + 3 * b, S // 2 - b, S // 2 + 1] for b in range(B)]
+    idx, bos, _ = _doc_mask(B, S, cuts)
+    q, k, v = _inputs(B, S, S, hq, max(1, hq // 2), d, dv, 12)
+    o0, l0 = fm._flash_attn_fwd(q.cuda(), k.cuda(), v.cuda(), idx.cuda(), causal=True)
+    ref = oracle.block_logit_ref(q, k, idx.numpy(), True, None, block_size, block_bos=bos if with_bos else None)
+    for _ in range(3):
+        o1, l1, bl = _run(q, k, v, True, block_size, idx=idx, bos=bos if with_bos else None)
+        assert status() == 0
+        assert torch.equal(o0, o1) and torch.equal(l0, l1)
+        _check(bl, ref, d)
+    # ids that change inside every warp, whatever the mask
+    bos = (torch.arange(S, dtype=torch.int32) // 13 * 13)[None].expand(B, S).contiguous()
+    o0, l0 = fm._flash_attn_fwd(q.cuda(), k.cuda(), v.cuda(), causal=True)
+    o1, l1, bl = _run(q, k, v, True, block_size, bos=bos if with_bos else None)
+    assert status() == 0
+    assert torch.equal(o0, o1) and torch.equal(l0, l1)
+    _check(bl, oracle.block_logit_ref(q, k, None, True, None, block_size, block_bos=bos if with_bos else None), d)
 
 
 def test_block_logit_packed_equals_alone():
