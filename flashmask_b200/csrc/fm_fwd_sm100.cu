@@ -30,6 +30,7 @@
 // 4 the mathematics needs), so the CTA-pair kernel is the faster one wherever its blocks of 256 rows
 // are full; where they are not, this variant wastes half as many rows and puts twice as many blocks
 // on the chip at a time (fwd_wide_kernels in fm_api.cu has the line and the figures).
+#include <algorithm>
 #include <type_traits>
 
 #include "fm_attn_params.cuh"
@@ -723,38 +724,49 @@ int bounded_wait_selftest_launch(uint64_t budget_ns, cudaStream_t s) {
 
 // Split plan of a call (SPLIT above): heads packed per query, parts, bytes of partial results.
 //
-// The plan is for calls without a mask tensor (the tiles a mask leaves are not known to the host) whose row blocks
-// do not fill the chip.  Packing is taken where it saves row blocks.  The number of parts minimises
-// waves x (tiles per part + 4): an unsplit tile step is 1 to 1.7 us and entry, list build and epilogue of a CTA cost
-// about four of them.  512 queries against 16384 keys (32 / 8 heads, d = 128): 64 CTAs of 128 tiles -> 128 of 64,
-// 231 -> 152 us; one query of 8 sequences against 8192 keys: 256 CTAs -> 128 packed ones, 220 -> 69 us.
-//
-// Where all rows of a block fit one sub-tile (packed decoding, up to 128 rows) both sub-tiles take its tiles in turn
-// // (p.alternate) from two tiles on: two chains of scores, softmax and P V instead of one, and a step is counted as 0.6
-// of an unalternated one.  8 sequences against 8192 keys (32 / 8 heads): 69 -> 54 us (5.0 TB/s of K / V); one
-// sequence against 32768 keys 39 us (3.4 TB/s).
+// The plan is for calls without a mask tensor (the tiles a mask leaves are not known to the host).  Packing the heads
+// of a group, dealing K tiles to several CTAs, and (where all rows of a block fit one sub-tile: p.alternate) letting
+// both sub-tiles take the tiles of a CTA in turn are each taken where an estimate of the launch says that it pays.
+// The estimate, in microseconds, is waves x (entry and exit + tiles per part + fp32 partial results of a part's rows)
+// + the merge, fitted to 2000 launches of 1 to 300 rows against 1 to 200 tiles on 1 to 1200 CTAs:
+//   alternating, d = 128, 148 CTAs of 64 tiles   1 row 113 -> 98 us, 128 rows 138 -> 117
+//                         1200 CTAs of 2 tiles   1 row  69 -> 63 us, 128 rows  85 -> 178: not taken
+//                         600 CTAs of 8 tiles   64 rows 98 -> 106 us: not taken
+//   keys in two parts, 64 packed CTAs of 128 tiles (512 queries against 16384 keys, 32 / 8 heads, d = 128): 231 -> 153 us
+//   packed heads, 3 x 700 queries (16 / 4 heads, 132 CTAs for 144, both one wave): 80 -> 85 us: not taken
 struct FwdSplitPlan { int pack_log2, n_split; bool alternate; size_t bytes; };
 static FwdSplitPlan fwd_split_plan(const fm_attn_args* a) {
   FwdSplitPlan pl{0, 1, false, 0};
   if (a->ncols != 0 || a->d > 128 || a->dv > 128) return pl;
-  const int G = a->Hq / a->Hkv, n_sm = sm_count();
+  const int G = a->Hq / a->Hkv, n_sm = sm_count(), tiles = (a->Sk + 127) / 128;
+  const bool small = a->d <= 64 && a->dv <= 64;
+  const double entry = small ? 4.9 : 5.7, in_turn = small ? 0.59 : 0.68, partial = small ? 4.5 : 10.0, merge = small ? 3.8 : 2.2;
+  auto tile = [&](int64_t rows) { return rows <= 128 ? (small ? 1.54 : 1.84) : (small ? 1.95 : 2.0); };   // one / both sub-tiles
   auto blocks = [&](int64_t rows) { return (rows + 255) / 256; };
-  int64_t units = blocks(a->Sq) * a->Hq * a->B;
-  if (units >= 4 * n_sm && blocks(a->Sq) > 1) return pl;
-  if ((G & (G - 1)) == 0 && G <= 128 && blocks((int64_t)a->Sq * G) < blocks(a->Sq) * G) {
-    while ((1 << pl.pack_log2) < G) ++pl.pack_log2;
-    units = blocks((int64_t)a->Sq * G) * a->Hkv * a->B;
-  }
-  const int tiles = (a->Sk + 127) / 128;
-  pl.alternate = ((int64_t)a->Sq << pl.pack_log2) <= 128 && tiles >= 2;
-  const double step = pl.alternate ? 0.6 : 1.0;
+  if (blocks(a->Sq) * a->Hq * a->B >= 4 * n_sm && blocks(a->Sq) > 1) return pl;
   double best = 1e30;
-  for (int s = 1; s <= (pl.alternate ? 16 : 32) && s <= tiles && (s == 1 || units < n_sm); ++s) {
-    const double cost = (double)((units * s + n_sm - 1) / n_sm) * (step * tiles / s + 4) + (s > 1 ? 3 : 0);
-    if (cost < best) { best = cost; pl.n_split = s; }
+  auto consider = [&](int pack_log2, double handicap) {
+    const int64_t rows = (int64_t)a->Sq << pack_log2, units = blocks(rows) * (a->Hq >> pack_log2) * a->B;
+    const double share = std::min<int64_t>(rows, 128) / 128.0;      // of a sub-tile's rows that have a partial result
+    for (int s = 1; s <= 32 && s <= tiles && (s == 1 || units < n_sm); ++s) {
+      const int n = (tiles + s - 1) / s;                            // tiles of a CTA
+      for (int alt = 0; alt <= (rows <= 128 && n >= 2 && s <= 16 ? 1 : 0); ++alt) {
+        const bool parts = alt || s > 1;
+        const double cost = handicap * (((units * s + n_sm - 1) / n_sm) * (entry + (alt ? in_turn : 1.0) * tile(rows) * n +
+                                        (parts ? partial * share : 0.0)) + (parts ? merge : 0.0));
+        if (cost < best) { best = cost; pl.pack_log2 = pack_log2; pl.n_split = s; pl.alternate = alt; }
+      }
+    }
+  };
+  consider(0, 1.0);
+  if (G > 1 && (G & (G - 1)) == 0 && G <= 128 && blocks((int64_t)a->Sq * G) < blocks(a->Sq) * G) {
+    int lg = 0;
+    while ((1 << lg) < G) ++lg;
+    // (few blocks saved: the packed kernel's own pace counts)
+    consider(lg, 4 * blocks((int64_t)a->Sq * G) > 3 * blocks(a->Sq) * G ? 1.05 : 1.0);
   }
   const size_t parts = (size_t)pl.n_split << pl.alternate;
-  if (parts > 1) pl.bytes = (size_t)a->B * a->Hq * a->Sq * parts * (((a->d <= 64 && a->dv <= 64) ? 64 : 128) + 1) * sizeof(float);
+  if (parts > 1) pl.bytes = (size_t)a->B * a->Hq * a->Sq * parts * ((small ? 64 : 128) + 1) * sizeof(float);
   return pl;
 }
 

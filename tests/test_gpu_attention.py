@@ -259,9 +259,27 @@ def test_rows_of_one_sub_tile(B, Sq, Sk, Hq, Hkv, d, dv):
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,d,dv,parts", [
+    (160, 1, 200, 4, 4, 128, 128, 2),     # two tiles: one per sub-tile
+    (150, 2, 330, 4, 4, 64, 64, 2),       # three
+    (8, 32, 3000, 16, 4, 128, 128, 8),    # 128 packed rows, a full sub-tile; four CTAs of six tiles
+    (3, 2, 9000, 16, 2, 96, 96, 24),      # a dozen CTAs, some of them with an odd share
+    (1, 33, 641, 4, 1, 128, 128, 6),      # 132 packed rows: one tile serves both sub-tiles
+    (300, 64, 140, 2, 2, 64, 64, 0)])     # a chip full of short calls: none
+def test_partial_results(B, Sq, Sk, Hq, Hkv, d, dv, parts):
+    """Either side of the rule that deals K tiles to several CTAs and to the two sub-tiles of a CTA."""
+    import ctypes as C
+    a = _lib.AttnArgs()
+    a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.Hm, a.mask_B, a.d, a.dv, a.causal = B, Sq, Sk, Hq, Hkv, 1, 1, d, dv, 1
+    assert _lib.load().fm_fwd_workspace_bytes(C.byref(a)) == B * Hq * Sq * parts * ((64 if d <= 64 else 128) + 1) * 4
+    for kind in ("none_causal", "none_full"):
+        _run(kind, B, Sq, Sk, Hq, Hkv, d, dv, sink=True, seed=94)
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("what", ["k nan", "k inf", "q nan", "v nan", "v inf"])
 @pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,d", [(1, 1, 8192, 4, 1, 128),       # split and alternating
-                                              (1, 1, 300, 2, 2, 64),         # alternating only
+                                              (160, 1, 200, 4, 4, 128),      # alternating only
                                               (1, 256, 8192, 2, 2, 128)])    # split only
 def test_non_finite_inputs_of_a_split_forward(B, Sq, Sk, Hq, Hkv, d, what):
     """A NaN or an infinity that a query sees reaches its output whatever share of the keys holds it: the elements

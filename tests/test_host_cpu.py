@@ -75,6 +75,27 @@ def test_kernel_variant_routing_needs_no_gpu():
         assert got == has, (d, dv, got)
 
 
+def test_partial_results_of_the_forward_are_asked_for_where_they_pay():
+    """The forward's workspace query says which calls are split: few rows against many keys, not a chip full of
+    short calls, where the fp32 partial results would cost several times the output."""
+    lib = _lib.load()
+
+    def nbytes(B, Sq, Sk, Hq, Hkv, d, ncols=0):
+        a = _lib.AttnArgs()
+        a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.Hm, a.mask_B, a.d, a.dv, a.causal = B, Sq, Sk, Hq, Hkv, 1, 1, d, d, 1
+        a.ncols = ncols
+        return lib.fm_fwd_workspace_bytes(ctypes.byref(a))
+    for d in (64, 128):
+        assert nbytes(8, 1, 8192, 32, 8, d) > 0 and nbytes(1, 1, 32768, 32, 8, d) > 0
+        assert nbytes(1, 512, 16384, 32, 8, d) > 0
+        assert nbytes(512, 128, 256, 16, 16, d) == 0 and nbytes(48, 128, 1024, 16, 16, d) == 0
+        assert nbytes(16, 128, 384, 16, 16, d) == 0 and nbytes(1, 4096, 4096, 32, 8, d) == 0
+        assert nbytes(8, 1, 8192, 32, 8, d, ncols=1) == 0        # (a mask's tiles are not known to the host)
+        # never more than 32 parts of a row
+        for args in ((1, 1, 262144, 1, 1, d), (1, 7, 100000, 4, 1, d), (3, 200, 65536, 2, 2, d)):
+            assert nbytes(*args) <= 32 * args[0] * args[1] * args[3] * (d + 1) * 4
+
+
 def test_repeated_operands_take_no_tensor_map():
     """A dimension of several elements with stride 0 cannot be described to the kernels' tensor maps: the hosts copy
     such a tensor (and keep a value that is a view of the key), and the C ABI routes the call to the kernels that
