@@ -59,7 +59,8 @@ int fwd_pair_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s)
 int fwd_pair_status(int* out, bool reset);
 bool bwd_pair_supported(const fm_attn_args* a);
 size_t bwd_pair_workspace_bytes(const fm_attn_args* a);
-int bwd_pair_launch(const AttnKParams& p, const fm_attn_args* a, void* ws, cudaStream_t s);
+bool bwd_pair_fits(const fm_attn_args* a, size_t bytes);
+int bwd_pair_launch(const AttnKParams& p, const fm_attn_args* a, void* ws, size_t bytes, cudaStream_t s);
 int bwd_pair_status(int* out, bool reset);
 
 int fwd_sm100_status(int* out, bool reset);
@@ -238,7 +239,7 @@ static int run_bwd_kernels(const fm_attn_args* a, BwdKernels kernels, const Attn
     const bool persist = p.dq_order && p.dkdv_order && g_opt.bwd_persist && a->d <= 128;   // 192 / 128: one-unit kernels only
     rc = persist ? bwd_sm100_persist_launch(p, a, s) : bwd_sm100_launch(p, a, s);
   } else if (p.pair_ws) {
-    rc = bwd_pair_launch(p, a, p.pair_ws, s);
+    rc = bwd_pair_launch(p, a, p.pair_ws, p.pair_ws_bytes, s);
   } else {
     rc = bwd_mma_launch(p, a->dtype, s);
   }
@@ -469,7 +470,17 @@ static size_t bwd_workspace_bytes(const fm_attn_args* a, BwdKernels kernels) {
   return n;
 }
 
+// What fm_bwd cannot do without: the CTA-pair backward works in smaller chunks when it gets less than it asks for, and
+// leaves the call to the warp-MMA kernels, which keep row statistics only, when not even the smallest chunk fits.
+static size_t bwd_min_workspace_bytes(const fm_attn_args* a, BwdKernels kernels) {
+  return bwd_workspace_bytes(a, kernels == BWD_PAIR ? BWD_WARP_MMA : kernels);
+}
+
 // (by geometry: a host may ask before it knows its tensors)
+extern "C" size_t fm_bwd_min_workspace_bytes(const fm_attn_args* a) {
+  if (!a || a->B <= 0 || a->Hq <= 0 || a->Sq <= 0) return 0;
+  return bwd_min_workspace_bytes(a, bwd_kernels_by_geometry(a));
+}
 extern "C" size_t fm_bwd_workspace_bytes(const fm_attn_args* a) {
   if (!a || a->B <= 0 || a->Hq <= 0 || a->Sq <= 0) return 0;
   return bwd_workspace_bytes(a, bwd_kernels_by_geometry(a));
@@ -494,7 +505,7 @@ extern "C" int fm_bwd(const fm_attn_args* a, void* stream) {
   FM_REQUIRE(a->ncols == 0 || a->tile_n == tn, FM_ERR_INVALID_ARGUMENT,
              "fm_bwd: minmax was prepared for tile_n=%d, this variant needs %d", a->tile_n, tn);
   const BwdKernels kernels = bwd_kernels(a);
-  const size_t need = bwd_workspace_bytes(a, kernels);
+  const size_t need = bwd_min_workspace_bytes(a, kernels);
   FM_REQUIRE(a->workspace && a->workspace_bytes >= need, FM_ERR_WORKSPACE,
              "fm_bwd: workspace too small (%zu bytes given, %zu needed)", a->workspace_bytes, need);
   FM_REQUIRE(((uintptr_t)a->workspace & 255) == 0, FM_ERR_WORKSPACE, "fm_bwd: workspace must be 256-byte aligned");
@@ -511,7 +522,11 @@ extern "C" int fm_bwd(const fm_attn_args* a, void* stream) {
     p.stat_dp = p.stat_s + (size_t)a->B * a->Hq * p.Sq_r * 8;
     p.bwd_flags = a->bwd_flags;
   }
-  if (kernels == BWD_PAIR) p.pair_ws = reinterpret_cast<uint8_t*>(a->workspace) + bwd_row_stat_bytes(a);
+  const size_t beyond_stats = a->workspace_bytes - bwd_row_stat_bytes(a);
+  if (kernels == BWD_PAIR && bwd_pair_fits(a, beyond_stats)) {
+    p.pair_ws = reinterpret_cast<uint8_t*>(a->workspace) + bwd_row_stat_bytes(a);
+    p.pair_ws_bytes = beyond_stats;
+  }
   cudaStream_t s = (cudaStream_t)stream;
   attach_bwd_tables(a, &p);
   return run_bwd_kernels(a, kernels, p, s);

@@ -15,6 +15,7 @@ struct AttnKParams {
   // (-c_hi, -c_lo, 0 x 6) with c = LSE*log2e / scale_log2, and (-d_hi, -d_lo, 0 x 6) with d = rowsum(O dO)
   uint16_t* stat_s; uint16_t* stat_dp;
   void* pair_ws;    // CTA-pair backward: workspace of P, dS and fp32 sums (nullptr: that variant is not used)
+  size_t pair_ws_bytes;
   int bwd_flags;    // FM_BWD_DQ_CARRY: the accumulator holds earlier sums; FM_BWD_DQ_LEAVE: dq is not written
   int64_t q_b, q_s, q_h, k_b, k_s, k_h, v_b, v_s, v_h, o_b, o_s, o_h;
   int64_t do_b, do_s, do_h, dq_b, dq_s, dq_h, dk_b, dk_s, dk_h, dv_b, dv_s, dv_h;

@@ -753,25 +753,40 @@ bwd_pair_grads_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_con
 // ---------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------
-// Bytes of P and dS a call may keep at a time.  At S = 16384 that is two heads, or 2048 rows of 16 heads: enough
+// Bytes of P and dS a call keeps at a time when the caller gives what it is asked for; with less it works in smaller
+// chunks (see bwd_pair_plan).  At S = 16384 that is two heads, or 2048 rows of 16 heads: enough
 // tiles for 74 pairs several times over, so a larger budget gains nothing, and each chunk still reads dK / dV
 // sums (if any) for 2048 rows of work.
 constexpr size_t kBudget = (size_t)2 << 30;
 
 struct BwdPairPlan { int groups, rows, key_blocks; bool sums; size_t block_bytes, acc_dk_bytes, acc_dv_bytes; };
-static BwdPairPlan bwd_pair_plan(const fm_attn_args* a) {
+// The plan with up to `budget` bytes of P and dS (at least 256 rows of a group).
+static BwdPairPlan bwd_pair_plan_for(const fm_attn_args* a, size_t budget) {
   BwdPairPlan pl;
   const int G = a->Hq / a->Hkv;
   const size_t sq = ((size_t)a->Sq + 255) / 256 * 256, sk = ((size_t)a->Sk + 255) / 256 * 256;
   const size_t row = (size_t)G * sk * 4;              // P and dS of one query row of every head of a group
   pl.key_blocks = (int)(sk / 64);
-  pl.groups = (int)std::min<size_t>((size_t)a->B * a->Hkv, std::max<size_t>(1, kBudget / (row * sq)));
-  pl.rows = (int)std::min(sq, std::max<size_t>(256, kBudget / row / 256 * 256));
+  pl.groups = (int)std::min<size_t>((size_t)a->B * a->Hkv, std::max<size_t>(1, budget / (row * sq)));
+  pl.rows = (int)std::min(sq, std::max<size_t>(256, budget / row / 256 * 256));
   pl.sums = (size_t)pl.rows < sq;
   pl.block_bytes = (size_t)pl.groups * pl.rows * row / 2;
   pl.acc_dk_bytes = pl.sums ? sk * a->d * 4 : 0;
   pl.acc_dv_bytes = pl.sums ? sk * a->dv * 4 : 0;
   return pl;
+}
+static size_t plan_bytes(const BwdPairPlan& pl) { return 2 * pl.block_bytes + pl.acc_dk_bytes + pl.acc_dv_bytes; }
+
+// The largest plan that fits `bytes` of workspace; false: not even 256 rows of one group do.
+static bool bwd_pair_plan(const fm_attn_args* a, size_t bytes, BwdPairPlan* pl) {
+  *pl = bwd_pair_plan_for(a, kBudget);
+  if (plan_bytes(*pl) <= bytes) return true;
+  *pl = bwd_pair_plan_for(a, bytes);                  // whole groups
+  if (plan_bytes(*pl) <= bytes) return true;
+  const size_t sums = (((size_t)a->Sk + 255) / 256 * 256) * (a->d + a->dv) * 4;
+  if (bytes <= sums) return false;
+  *pl = bwd_pair_plan_for(a, bytes - sums);           // rows of one group beside its sums
+  return plan_bytes(*pl) <= bytes;
 }
 
 bool bwd_pair_supported(const fm_attn_args* a) {
@@ -788,10 +803,8 @@ bool bwd_pair_supported(const fm_attn_args* a) {
   return (a->Sk + 127) / 128 <= kPairListMax && (a->Sq + 127) / 128 <= kPairListMax && least <= 4 * kBudget;
 }
 
-size_t bwd_pair_workspace_bytes(const fm_attn_args* a) {
-  const BwdPairPlan pl = bwd_pair_plan(a);
-  return 2 * pl.block_bytes + pl.acc_dk_bytes + pl.acc_dv_bytes;
-}
+size_t bwd_pair_workspace_bytes(const fm_attn_args* a) { return plan_bytes(bwd_pair_plan_for(a, kBudget)); }
+bool bwd_pair_fits(const fm_attn_args* a, size_t bytes) { BwdPairPlan pl; return bwd_pair_plan(a, bytes, &pl); }
 
 static int make_block_tmap(CUtensorMap* out, void* base, size_t bytes) {
   EncodeTiledFn enc = get_encode_tiled();
@@ -807,9 +820,8 @@ static int make_block_tmap(CUtensorMap* out, void* base, size_t bytes) {
 }
 
 template <int D, int DV, bool IS_BF16>
-static int launch_bwd_pair(const AttnKParams& p, const fm_attn_args* a, uint8_t* ws, cudaStream_t s) {
+static int launch_bwd_pair(const AttnKParams& p, const fm_attn_args* a, uint8_t* ws, const BwdPairPlan& pl, cudaStream_t s) {
   using GC = PairGradCfg<D, DV>;
-  const BwdPairPlan pl = bwd_pair_plan(a);
   const int G = a->Hq / a->Hkv;
   CUtensorMap q, dO, k, v, qt, kt, tp, tds;
   int rc;
@@ -862,12 +874,14 @@ static int launch_bwd_pair(const AttnKParams& p, const fm_attn_args* a, uint8_t*
   return FM_OK;
 }
 
-int bwd_pair_launch(const AttnKParams& p, const fm_attn_args* a, void* ws, cudaStream_t s) {
+int bwd_pair_launch(const AttnKParams& p, const fm_attn_args* a, void* ws, size_t bytes, cudaStream_t s) {
+  BwdPairPlan pl;
+  FM_REQUIRE(bwd_pair_plan(a, bytes, &pl), FM_ERR_WORKSPACE, "backward: %zu bytes hold no chunk of P and dS", bytes);
   const bool bf = a->dtype == FM_DTYPE_BF16;
   uint8_t* w = reinterpret_cast<uint8_t*>(ws);
-  if (a->d == 256) return bf ? launch_bwd_pair<256, 256, true>(p, a, w, s) : launch_bwd_pair<256, 256, false>(p, a, w, s);
-  if (a->d == 512) return bf ? launch_bwd_pair<512, 512, true>(p, a, w, s) : launch_bwd_pair<512, 512, false>(p, a, w, s);
-  return bf ? launch_bwd_pair<576, 512, true>(p, a, w, s) : launch_bwd_pair<576, 512, false>(p, a, w, s);
+  if (a->d == 256) return bf ? launch_bwd_pair<256, 256, true>(p, a, w, pl, s) : launch_bwd_pair<256, 256, false>(p, a, w, pl, s);
+  if (a->d == 512) return bf ? launch_bwd_pair<512, 512, true>(p, a, w, pl, s) : launch_bwd_pair<512, 512, false>(p, a, w, pl, s);
+  return bf ? launch_bwd_pair<576, 512, true>(p, a, w, pl, s) : launch_bwd_pair<576, 512, false>(p, a, w, pl, s);
 }
 
 int bwd_pair_status(int* out, bool reset) {

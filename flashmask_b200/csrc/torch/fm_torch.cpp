@@ -9,6 +9,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -138,6 +139,22 @@ std::pair<Tensor, Tensor> kv_rows(const Tensor& k, const Tensor& v) {
   return {rows(k), rows(v)};
 }
 
+// Workspace of a backward call.  When the device has no room for what the call asks for (2 GiB and more at the head dims
+// 256, 512 and 576) it gets less, down to what it cannot do without.
+Tensor bwd_workspace(fm_attn_args* a, const Tensor& like) {
+  const size_t least = fm_bwd_min_workspace_bytes(a);
+  for (size_t n = fm_bwd_workspace_bytes(a);; n = std::max(least, n / 4)) {
+    try {
+      Tensor ws = at::empty({(int64_t)std::max<size_t>(n, 256)}, like.options().dtype(at::kByte));
+      a->workspace = ws.data_ptr();
+      a->workspace_bytes = n;
+      return ws;
+    } catch (const c10::OutOfMemoryError&) {
+      if (n <= least) throw;
+    }
+  }
+}
+
 class FlashMask : public torch::autograd::Function<FlashMask> {
  public:
   static variable_list forward(AutogradContext* ctx, const Variable& q_in, const Variable& k_in, const Variable& v_in,
@@ -216,10 +233,7 @@ class FlashMask : public torch::autograd::Function<FlashMask> {
     }
     if (tables.defined() && dq_at >= 0) a.dq_order = tables.data_ptr<int>() + dq_at;
     if (tables.defined() && dkdv_at >= 0) a.dkdv_order = tables.data_ptr<int>() + dkdv_at;
-    const size_t nbytes = fm_bwd_workspace_bytes(&a);
-    const Tensor ws = at::empty({(int64_t)std::max<size_t>(nbytes, 256)}, q.options().dtype(at::kByte));
-    a.workspace = ws.data_ptr();
-    a.workspace_bytes = nbytes;
+    const Tensor ws = bwd_workspace(&a, q);
     check(fm_bwd(&a, stream), "fm_bwd");
     if (kv_shared(k, v)) {
       // value is a view of key's leading dv columns at these head dims: one gradient for the storage

@@ -274,6 +274,23 @@ def _flash_attn_fwd(q, k, v, startend_row_indices=None, softmax_scale=None, caus
     return out, lse
 
 
+def _bwd_workspace(a: "_lib.AttnArgs", device) -> torch.Tensor:
+    """Workspace of a backward call, set in ``a``.  When the device has no room for what the call asks for (2 GiB and
+    more at the head dims 256, 512 and 576) it gets less, down to what it cannot do without."""
+    lib = _lib.load()
+    n, least = lib.fm_bwd_workspace_bytes(C.byref(a)), lib.fm_bwd_min_workspace_bytes(C.byref(a))
+    while True:
+        try:
+            ws = torch.empty(max(n, 256), dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            if n <= least:
+                raise
+            n = max(least, n // 4)
+            continue
+        a.workspace, a.workspace_bytes = ws.data_ptr(), n
+        return ws
+
+
 def _flash_attn_bwd(q, k, v, out, dout, lse, startend_row_indices=None, softmax_scale=None,
                     causal=False, learnable_sink=None, deterministic=False,
                     mask_info: Optional[FlashMaskInfo] = None, dq_chain: Optional[dict] = None):
@@ -315,23 +332,21 @@ def _flash_attn_bwd(q, k, v, out, dout, lse, startend_row_indices=None, softmax_
     if info is not None:
         a.dq_order = _launch_order(a, info, _lib.FM_ORDER_BWD_DQ, q)
         a.dkdv_order = _launch_order(a, info, _lib.FM_ORDER_BWD_DKDV, q)
-    nbytes = lib.fm_bwd_workspace_bytes(C.byref(a))
     chained = dq_chain is not None and bool(lib.fm_bwd_accumulates(C.byref(a)))
-    if chained:
+    if chained and "ws" in dq_chain:
         # one workspace for the whole chain: the accumulator carries the sums from call to call
-        if "ws" in dq_chain:
-            a.bwd_flags |= _lib.FM_BWD_DQ_CARRY
-        else:
-            dq_chain["ws"] = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=q.device)
-        if not dq_chain.get("last", False):
-            a.bwd_flags |= _lib.FM_BWD_DQ_LEAVE
-        ws = dq_chain["ws"]
+        a.bwd_flags |= _lib.FM_BWD_DQ_CARRY
+        ws, nbytes = dq_chain["ws"], lib.fm_bwd_workspace_bytes(C.byref(a))
         assert ws.numel() >= nbytes, "the backward calls of a chain must share one problem geometry"
+        a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
     else:
-        ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=q.device)
+        ws = _bwd_workspace(a, q.device)
+        if chained:
+            dq_chain["ws"] = ws
+    if chained and not dq_chain.get("last", False):
+        a.bwd_flags |= _lib.FM_BWD_DQ_LEAVE
     if dq_chain is not None:
         dq_chain["summed"] = chained
-    a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
     _lib.check(lib.fm_bwd(C.byref(a), _stream(q)), "fm_bwd")
     if chained and not dq_chain.get("last", False):
         dq = None

@@ -276,8 +276,9 @@ FM_API int fm_selftest_bounded_wait(int budget_us, void* stream);
  * Replaces _flash_attn_bwd (flashmask/cute/ops/bwd.py:56-1261): preprocess
  * (flash_bwd_preprocess.py:184-342), main (flash_bwd_sm100.py:1435-),
  * postprocess (flash_bwd_postprocess.py:309-) and dsink
- * (flash_bwd_sink.py:67-114).  `workspace` must hold
- * fm_bwd_workspace_bytes(args) bytes; its contents need no initialisation.
+ * (flash_bwd_sink.py:67-114).  `workspace` should hold
+ * fm_bwd_workspace_bytes(args) bytes (and has to hold
+ * fm_bwd_min_workspace_bytes); its contents need no initialisation.
  * The size depends on args->deterministic: the one-kernel backward
  * (flash_bwd_sm100.py:129-140: S, dP, dV, dK and dQ of a tile pair computed once)
  * adds an fp32 dQ accumulator [B, Hq, roundup(Sq,128), 64|128] behind the row
@@ -286,8 +287,16 @@ FM_API int fm_selftest_bounded_wait(int budget_us, void* stream);
  * postprocess, flash_bwd_postprocess.py).  Ask for the size with the same
  * args->deterministic the call will carry. */
 FM_API size_t fm_bwd_workspace_bytes(const fm_attn_args* args);
+/* The least workspace fm_bwd takes.  It is less than fm_bwd_workspace_bytes at
+ * the head dims 256, 512 and 576 only, where the fast kernels keep P and dS of a
+ * chunk of the problem (2 GiB, more where 256 rows of all heads of a kv group
+ * need more): with fewer bytes the chunks are smaller, and where not even the
+ * smallest fits, other kernels serve that keep row statistics only.  Results are
+ * bitwise reproducible for a given workspace size; another size sums dK and dV in
+ * another order. */
+FM_API size_t fm_bwd_min_workspace_bytes(const fm_attn_args* args);
 /* 1 when fm_bwd(args) would run the one-kernel variant (and so honours
- * args->bwd_flags), else 0. */
+ * args->bwd_flags), else 0.  Reads the strides and softmax_scale too. */
 FM_API int fm_bwd_accumulates(const fm_attn_args* args);
 FM_API int fm_bwd(const fm_attn_args* args, void* stream);
 

@@ -70,9 +70,10 @@ def run_product(q, k, v, do, idx, causal, sink, deterministic=None):
 
 
 def run_c_abi(q, k, v, do, idx, causal, sink=None, scale=None, workspace=None, static_scratch=False,
-              deterministic=True):
+              deterministic=True, count=None):
     """Forward and backward through the C ABI on the tensors as they are: nothing is copied or laid out first.
-    ``workspace``: bytes handed to fm_bwd (default: what fm_bwd_workspace_bytes asks for)."""
+    ``workspace``: bytes handed to fm_bwd (default: what fm_bwd_workspace_bytes asks for); ``count``: a list that
+    receives the number of kernels of the backward."""
     import ctypes as C
     from flashmask_b200 import _lib, ops
     lib = _lib.load()
@@ -96,6 +97,7 @@ def run_c_abi(q, k, v, do, idx, causal, sink=None, scale=None, workspace=None, s
     a.do_stride, a.dq_stride, a.dk_stride, a.dv_stride = (ops._strides(t) for t in (do, dq, dk, dvv))
     a.dsink = None if dsink is None else dsink.data_ptr()
     a.deterministic = int(deterministic)
+    launched = lib.fm_launch_count()
     if static_scratch:
         _lib.check(lib.fm_bwd_static_scratch(C.byref(a), stream), "fm_bwd_static_scratch")
     else:
@@ -103,6 +105,8 @@ def run_c_abi(q, k, v, do, idx, causal, sink=None, scale=None, workspace=None, s
         ws = torch.empty(n, dtype=torch.uint8, device=q.device)
         a.workspace, a.workspace_bytes = ws.data_ptr(), n
         _lib.check(lib.fm_bwd(C.byref(a), stream), "fm_bwd")
+    if count is not None:
+        count.append(lib.fm_launch_count() - launched)
     return dict(out=out, lse=lse, dq=dq, dk=dk, dv=dvv, dsink=dsink)
 
 

@@ -195,6 +195,78 @@ def test_bounds_of_partial_tiles_in_the_pair_backward(kind, S):
     assert _kernel_status() == 0
 
 
+def _pair_row_bytes(Sk, G):
+    return G * -(-Sk // 256) * 256 * 4          # P and dS of one query row of every head of a group
+
+
+@pytest.mark.parametrize("kind", ["causal_doc", "none_causal", "four_column"])
+@pytest.mark.parametrize("d,dv", [(256, 256), (512, 512), (576, 512)])
+def test_pair_backward_in_smaller_workspaces(d, dv, kind):
+    """The chunks of the CTA-pair backward: whole groups, one group, row chunks whose dK / dV are summed in fp32 (the
+    last one short, some without visible work for a key block), and none at all (the warp-MMA kernels, on mask
+    reductions over wider tiles than their own)."""
+    B, S, Hq, Hkv = 2, 700, 8, 1
+    G = Hq // Hkv
+    idx_np, causal = _mask(kind, B, S, S, 57)
+    idx = None if idx_np is None else torch.from_numpy(np.ascontiguousarray(idx_np).copy()).cuda()
+    q, k, v, do, s = make_inputs(B, S, S, Hq, Hkv, d, dv, 57, sink=True)
+    dev = [t.cuda() for t in (q, k, v, do)]
+    ref = run_oracle(q, k, v, do, idx, causal, s)
+    lowp = naive_lowp(*dev, idx, causal, s)
+    stats = 2 * 4 * B * Hq * 768
+    row, sums = _pair_row_bytes(S, G), 768 * (d + dv) * 4
+    # (workspace, launches of the score and gradient kernels: two per chunk)
+    sizes = [(stats + 2 * 768 * row, 2), (stats + 768 * row, 4), (stats + 768 * row - 1, 8),
+             (stats + 512 * row + sums, 8), (stats + 256 * row + sums, 12), (stats + 256 * row + sums - 1, 2), (stats, 2)]
+    full = None
+    for nbytes, launches in sizes:
+        got = run_c_abi(*dev, idx, causal, s, workspace=nbytes, count=(before := []))
+        assert before[0] == launches + 2, (nbytes, before)          # + row statistics and sink gradient
+        assert_parity(got, ref, lowp, label=f"{nbytes}: ")
+        again = run_c_abi(*dev, idx, causal, s, workspace=nbytes)
+        for n in ("dq", "dk", "dv", "dsink"):
+            assert torch.equal(got[n], again[n]), n
+        full = full or got
+        if nbytes >= stats + 256 * row + sums:
+            assert torch.equal(got["dq"], full["dq"])               # only dK and dV are summed in another order
+    with pytest.raises(RuntimeError, match="workspace too small"):
+        run_c_abi(*dev, idx, causal, s, workspace=stats - 1)
+    # without a workspace: the warp-MMA kernels
+    got = run_c_abi(*dev, idx, causal, s, static_scratch=True)
+    least = run_c_abi(*dev, idx, causal, s, workspace=stats)
+    for n in ("dq", "dk", "dv", "dsink"):
+        assert torch.equal(got[n], least[n]), n
+    assert _kernel_status() == 0
+
+
+def test_backward_when_memory_is_short():
+    """A backward that gets no room for the workspace it asks for works in smaller chunks (an allocator limit of this
+    process stands in for a full device)."""
+    B, S, H, d = 1, 4096, 8, 256                                    # asks for 512 MiB
+    q, k, v, do, _ = (t if t is None else t.cuda() for t in make_inputs(B, S, S, H, H, d, d, 58))
+    x = [t.requires_grad_(True) for t in (q, k, v)]
+    grads = lambda: torch.autograd.grad(fm.flashmask_attention(*x, causal=True), x, do)
+    py = lambda: fm._flash_attn_bwd(q.detach(), k.detach(), v.detach(), *fwd, lse=lse, causal=True)[:3]
+    with torch.no_grad():
+        out, lse = fm._flash_attn_fwd(q, k, v, causal=True)
+    fwd = (out, do)
+    want = [t.clone() for t in grads()]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (256 << 20)) / total)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            torch.empty(512 << 20, dtype=torch.uint8, device="cuda")
+        for call in (grads, py):
+            for g_, w_ in zip(call(), want):
+                # the sums of dK and dV are rounded to bf16 once, from another order of fp32 additions
+                assert (g_.float() - w_.float()).norm() <= 2 ** -8 * w_.float().norm()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("d,dv", [(512, 512), (576, 512)])
 @pytest.mark.parametrize("kind", ["causal_doc", "none_full", "four_column"])
 def test_short_sequences_of_the_widest_heads(kind, d, dv):

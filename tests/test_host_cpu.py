@@ -161,6 +161,18 @@ def test_pair_backward_workspace_is_bounded():
     assert sizes[128, 131072] == 0 and sizes[128, 65536] > 8 << 30
 
 
+def test_least_workspace_of_the_backward():
+    """What fm_bwd cannot do without: everything it asks for, but at the head dims of the CTA-pair backward the row
+    statistics alone."""
+    lib = _lib.load()
+    for d, dv in ((64, 64), (128, 128), (192, 128), (256, 256), (512, 512), (576, 512)):
+        a = _lib.AttnArgs()
+        a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.Hm, a.mask_B, a.d, a.dv = 2, 4096, 4096, 8, 2, 1, 1, d, dv
+        n, least = lib.fm_bwd_workspace_bytes(ctypes.byref(a)), lib.fm_bwd_min_workspace_bytes(ctypes.byref(a))
+        assert least == (n if d < 256 else 2 * 4 * 2 * 8 * 4096)
+        assert n - least == (0 if d < 256 else 4 << 28)         # (P and dS of four groups, 256 MiB each)
+
+
 def test_struct_layout_matches_header():
     # 18 int32/float + 15 pointers/size_t + 24 int64
     assert ctypes.sizeof(_lib.AttnArgs) == 18 * 4 + 15 * 8 + 24 * 8 + 3 * 8
