@@ -332,8 +332,7 @@ static int fwd_impl(const fm_attn_args* a, const BlockScore& bs, void* stream) {
   if (!fwd_uses_sm100(a->d, a->dv) || !fits_tcgen05(a, false)) return fwd_mma_launch(p, a->dtype, s);
   if (pair_dims(a->d, a->dv)) {
     const FwdWide kernels = fwd_wide_kernels(a);
-    // (block scores at 512 and 576: the warp-MMA kernel alone has them)
-    if (kernels == FWD_WARP_MMA || (bs.block_logit && a->d > 256)) return fwd_mma_launch(p, a->dtype, s);
+    if (kernels == FWD_WARP_MMA) return fwd_mma_launch(p, a->dtype, s);
     if (kernels == FWD_PAIR) return fwd_pair_launch(p, a, s);
   }
   return fwd_sm100_launch(p, a, s);

@@ -30,14 +30,15 @@ using namespace sm100;
 
 __device__ int g_fwd_pair_status = 0;
 
-template <int D>
+// BS: the block-score variants, which keep their accumulators where the others have one more ring slot (512, 576).
+template <int D, bool BS = false>
 struct FwdPairCfg {
   static constexpr int SLICES = D == 256 ? 1 : 2;       // 256-column slices of V / O
   static constexpr int NTHREADS = 384, LIST_MAX = 2048, NBND = 2;
   static constexpr int SUB128 = 128 * 128, SUB64 = 64 * 128;   // 128- / 64-row x 64-column sub-tiles (bytes)
   static constexpr int Q_BYTES = 128 * D * 2;
   static constexpr int SLOT_BYTES = 2 * SUB64;          // 64 keys x 128 columns of K, or 64 keys x 128 columns of V
-  static constexpr int NSTAGE = D == 256 ? 8 : (D == 512 ? 5 : 4);
+  static constexpr int NSTAGE = D == 256 ? 8 : (D == 512 ? 5 : 4) - (BS ? 1 : 0);
   static constexpr int KSLOTS = (D + 127) / 128;        // ring slots of a K tile (the last one half full at D = 576)
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_KV = OFF_Q + Q_BYTES;
@@ -51,7 +52,7 @@ struct FwdPairCfg {
   // block-score variant only: maxima handed over per tile parity, 16 block accumulators per row
   static constexpr int OFF_BSX = OFF_MISC + 64, OFF_BSA = OFF_BSX + 2 * 3 * 128 * 4;
   static constexpr int SMEM_BS = OFF_BSA + 16 * 128 * 4 + 1024;
-  static_assert(D != 256 || SMEM_BS <= 227 * 1024, "shared memory of the block-score variant");
+  static_assert(!BS || SMEM_BS <= 227 * 1024, "shared memory of the block-score variant");
   static constexpr int B_Q = 0, B_KVFULL = 1, B_KVEMPTY = B_KVFULL + NSTAGE, B_SFULL = B_KVEMPTY + NSTAGE,
                        B_PFULL = B_SFULL + 2, B_ODONE = B_PFULL + 2, B_BNDFULL = B_ODONE + 2,
                        B_BNDEMPTY = B_BNDFULL + NBND, B_COUNT = B_BNDEMPTY + NBND;
@@ -59,7 +60,7 @@ struct FwdPairCfg {
   static_assert(B_COUNT <= 32, "barrier storage");
   static_assert(SMEM > 120 * 1024 && SMEM <= 227 * 1024, "one CTA per SM (512 TMEM columns)");
   static_assert(OFF_KV % 1024 == 0 && 128 * 512 <= Q_BYTES, "aligned tiles; the Q tile stages the output");
-  static_assert(LIST_MAX * 8 * 4 <= NSTAGE * SLOT_BYTES, "the ring stages the reductions of the list build");
+  static_assert(LIST_MAX * 8 * 4 <= Q_BYTES, "the Q tile's place stages the reductions of the list build");
 };
 
 // Maxima over the blocks (of BS key columns) that 64 masked scores of a row touch: column j of the 64 lies in
@@ -84,14 +85,14 @@ __device__ __forceinline__ float half_block_scores(const uint32_t* sr, int rel, 
   return all;
 }
 
-// BLOCK_SCORE: 0, or the block size of the block-score side output (d = 256 only); BLOCK_BOS: document starts are
-// given, so a block may straddle two tiles.  The threads of warpgroup 0 own the output rows; warpgroup 1 hands
-// them the maxima of its 64 columns through shared memory together with the row maximum.
+// BLOCK_SCORE: 0, or the block size of the block-score side output; BLOCK_BOS: document starts are given, so a block
+// may straddle two tiles.  The threads of warpgroup 0 (of the first slice's pair) own the output rows; warpgroup 1
+// hands them the maxima of its 64 columns through shared memory together with the row maximum.
 template <int D, bool IS_BF16, int BLOCK_SCORE = 0, bool BLOCK_BOS = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
 fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const AttnKParams p) {
-  using Cfg = FwdPairCfg<D>;
+  using Cfg = FwdPairCfg<D, BLOCK_SCORE != 0>;
   extern __shared__ uint8_t smem_raw[];
   // (the dynamic shared memory starts at the same address in both CTAs, so the aligned base is the same too)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -130,7 +131,7 @@ fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (warp == 10) {
     // surviving K tiles, right to left: those that either CTA's rows see, with the flags of both
     int cnt = 0;
-    const MaskDesc mst = stage_minmax(md, bh_mask, 0, n_hi, reinterpret_cast<int32_t*>(smem + Cfg::OFF_KV),
+    const MaskDesc mst = stage_minmax(md, bh_mask, 0, n_hi, reinterpret_cast<int32_t*>(smem + Cfg::OFF_Q),
                                       Cfg::LIST_MAX, lane);
     for (int base = n_hi - 1; base >= 0; base -= 32) {
       const int n = base - lane;
@@ -146,7 +147,7 @@ fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       cnt += __popc(bal);
     }
     if (lane == 0) misc[1] = min(cnt, Cfg::LIST_MAX);
-    fence_proxy_async_smem();   // the staging area is handed back to the TMA loads of the ring
+    fence_proxy_async_smem();   // the staging area is handed to the TMA loads of Q
   }
   if (warp == 9) {
     tmem2_alloc(sbase + Cfg::OFF_MISC, 512);
@@ -202,7 +203,7 @@ fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     bool bs_vec = false;
     if constexpr (BLOCK_SCORE != 0) {
       if (row < p.Sq) {
-        if (w == 0) bs_dst = p.block_logit + (((int64_t)b * p.Hq + hq) * p.Sq + row) * p.block_ld;
+        if (w == 0 && slice == 0) bs_dst = p.block_logit + (((int64_t)b * p.Hq + hq) * p.Sq + row) * p.block_ld;
         if constexpr (BLOCK_BOS) bs_bos = p.block_bos[(int64_t)b * p.Sq + row];
       }
       if constexpr (BLOCK_BOS) {
@@ -577,7 +578,7 @@ fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // ---------------------------------------------------------------------------
 template <int D, bool IS_BF16, int BLOCK_SCORE = 0, bool BLOCK_BOS = false>
 static int launch_fwd_pair(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s) {
-  using Cfg = FwdPairCfg<D>;
+  using Cfg = FwdPairCfg<D, BLOCK_SCORE != 0>;
   CUtensorMap tq, tk, tv;
   int rc;
   if ((rc = make_bshd_tmap(&tq, a->q, a->dtype, a->B, a->Sq, a->Hq, a->d, a->q_stride[0], a->q_stride[1], a->q_stride[2], 128))) return rc;
@@ -599,24 +600,24 @@ bool fwd_pair_supported(const fm_attn_args* a) {
   return dims && (a->Sk + 127) / 128 <= FwdPairCfg<256>::LIST_MAX;
 }
 
-// (with p.block_logit: d = 256 only)
+template <int D, bool IS_BF16>
+static int launch_fwd_pair_any(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s) {
+  if (!p.block_logit) return launch_fwd_pair<D, IS_BF16>(p, a, s);
+  if (p.block_bos) {
+    if (p.block_log2 == 5) return launch_fwd_pair<D, IS_BF16, 32, true>(p, a, s);
+    if (p.block_log2 == 6) return launch_fwd_pair<D, IS_BF16, 64, true>(p, a, s);
+    return launch_fwd_pair<D, IS_BF16, 128, true>(p, a, s);
+  }
+  if (p.block_log2 == 5) return launch_fwd_pair<D, IS_BF16, 32>(p, a, s);
+  if (p.block_log2 == 6) return launch_fwd_pair<D, IS_BF16, 64>(p, a, s);
+  return launch_fwd_pair<D, IS_BF16, 128>(p, a, s);
+}
+
 int fwd_pair_launch(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s) {
   const bool bf = a->dtype == FM_DTYPE_BF16;
-#define FM_PAIR_BS(BSZ, BOS) return bf ? launch_fwd_pair<256, true, BSZ, BOS>(p, a, s) : launch_fwd_pair<256, false, BSZ, BOS>(p, a, s)
-  if (p.block_logit && p.block_bos) {
-    if (p.block_log2 == 5) FM_PAIR_BS(32, true);
-    if (p.block_log2 == 6) FM_PAIR_BS(64, true);
-    FM_PAIR_BS(128, true);
-  }
-  if (p.block_logit) {
-    if (p.block_log2 == 5) FM_PAIR_BS(32, false);
-    if (p.block_log2 == 6) FM_PAIR_BS(64, false);
-    FM_PAIR_BS(128, false);
-  }
-#undef FM_PAIR_BS
-  if (a->d == 256) return bf ? launch_fwd_pair<256, true>(p, a, s) : launch_fwd_pair<256, false>(p, a, s);
-  if (a->d == 512) return bf ? launch_fwd_pair<512, true>(p, a, s) : launch_fwd_pair<512, false>(p, a, s);
-  return bf ? launch_fwd_pair<576, true>(p, a, s) : launch_fwd_pair<576, false>(p, a, s);
+  if (a->d == 256) return bf ? launch_fwd_pair_any<256, true>(p, a, s) : launch_fwd_pair_any<256, false>(p, a, s);
+  if (a->d == 512) return bf ? launch_fwd_pair_any<512, true>(p, a, s) : launch_fwd_pair_any<512, false>(p, a, s);
+  return bf ? launch_fwd_pair_any<576, true>(p, a, s) : launch_fwd_pair_any<576, false>(p, a, s);
 }
 
 int fwd_pair_status(int* out, bool reset) {

@@ -71,7 +71,8 @@ def test_block_logit_shapes(b, s, sk, h, d, causal, variant):
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("b,s,sk,h,d,dv", [(1, 512, 512, 8, 256, 256), (1, 1024, 1024, 2, 256, 256),
                                            (1, 511, 513, 2, 256, 256), (1, 320, 320, 4, 192, 128),
-                                           (10, 130, 130, 8, 256, 256)])
+                                           (10, 130, 130, 8, 256, 256), (1, 511, 513, 2, 512, 512),
+                                           (2, 1100, 1100, 2, 576, 512), (16, 40, 40, 8, 576, 512)])
 def test_block_logit_head_dims_above_128(b, s, sk, h, d, dv, causal):
     """Both head dims run the tcgen05 forward (d = 256 is the reference's HySparse full-attention configuration):
     the plain forward and the block-score variant must agree bitwise on O and LSE."""
@@ -185,7 +186,8 @@ def test_block_logit_with_column_bound_mask(block_size, with_bos, variant):
 
 @pytest.mark.parametrize("block_size", [32, 64, 128])
 @pytest.mark.parametrize("with_bos", [False, True])
-@pytest.mark.parametrize("B,S,hq,d,dv", [(1, 1000, 2, 256, 256), (10, 300, 8, 256, 256), (2, 700, 4, 256, 256)])
+@pytest.mark.parametrize("B,S,hq,d,dv", [(1, 1000, 2, 256, 256), (10, 300, 8, 256, 256), (2, 700, 4, 256, 256),
+                                         (1, 1000, 2, 512, 512), (1, 700, 4, 576, 512)])
 def test_block_logit_wide_heads_with_documents(B, S, hq, d, dv, block_size, with_bos):
     """The variants above 192 with a document mask and document-relative ids, whose last scores are merged into the
     output while the last tile's P V runs: no wait runs out.  Scores, and O and LSE bitwise those of the plain forward."""
