@@ -89,9 +89,6 @@ static Options read_options() {
 static Options g_opt = read_options();
 int option_order_classes() { return g_opt.order_classes; }
 
-// Head dims of the CTA-pair kernels.
-static bool pair_dims(int d, int dv) { return (d == 256 && dv == 256) || ((d == 512 || d == 576) && dv == 512); }
-
 // Kernel variant of the forward for (d, dv): the tcgen05 kernels cover head dims up to 128 (multiples of 8),
 // 192 / 128 and, on CTA pairs, 256, 512 and 576 / 512; FLASHMASK_B200_FWD=mma forces the warp-MMA variant (A/B runs).
 static bool fwd_uses_sm100(int d, int dv) {

@@ -61,6 +61,8 @@ struct OrderJob { int axis, block_rows, n_units, n_other, rep_h, rep_b, heads, i
 struct OrderJobs { OrderJob job[3]; };
 // Builds up to three tables in one launch (one CTA each).
 int launch_order_build(const MaskDesc& md, int tile_n, const OrderJobs& jobs, int n_jobs, cudaStream_t s);
+// Head dims of the CTA-pair kernels.
+inline bool pair_dims(int d, int dv) { return (d == 256 && dv == 256) || ((d == 512 || d == 576) && dv == 512); }
 // Multiprocessors of the current device.
 int sm_count();
 // Work classes requested through the environment when the library was loaded (0: the default).

@@ -7,9 +7,10 @@
 //
 // Why a workspace.  The accumulators of dK and dV for 128 keys take 2 x 256 of the 512 tensor-memory columns at
 // d = 256 and 1088 at 576 / 512, so a kernel that keeps them recomputes S and dP for every slice of the outputs:
-// 8 GEMM units instead of 5 at 256, 2.6 times the work at 576 / 512.  Written once and read twice, P and dS cost
-// 4 bytes and 10 bytes of traffic per visible pair and head against 5 x 512 (5 x 1100) flops: the HBM time stays
-// below the tensor time at these head dims (it would not at 128).  The workspace is bounded (kBudget): a chunk is
+// 8 GEMM units instead of 5 at 256, 2.6 times the work at 576 / 512.  Per visible pair and head P and dS are 4 bytes
+// written and, for each 256-column slice of the gradients, 6 bytes read (dS for dQ and for dK, P for dV): 10 bytes
+// against 5 x 512 flops at 256, 16 against 5 x 1100 at 576 / 512.  That HBM time stays below the tensor time at these
+// head dims (it would not at 128).  The workspace is bounded (kBudget): a chunk is
 // as many kv groups (of all batch entries), or failing that as many query rows of one group, as fit; dK / dV of a group
 // that needs several row chunks are summed in fp32 accumulators in chunk order.  Every sum has one owner and a fixed order.
 //
@@ -790,9 +791,8 @@ static bool bwd_pair_plan(const fm_attn_args* a, size_t bytes, BwdPairPlan* pl) 
 }
 
 bool bwd_pair_supported(const fm_attn_args* a) {
-  const bool dims = (a->d == 256 && a->dv == 256) || ((a->d == 512 || a->d == 576) && a->dv == 512);
   // (a size query comes before the arguments are validated)
-  if (!dims || a->Sq <= 0 || a->Sk <= 0 || a->Hkv <= 0 || a->Hq <= 0 || a->Hq % a->Hkv) return false;
+  if (!pair_dims(a->d, a->dv) || a->Sq <= 0 || a->Sk <= 0 || a->Hkv <= 0 || a->Hq <= 0 || a->Hq % a->Hkv) return false;
   // Sequences of one 64-row tile: a 256 x 256 tile of the score kernel is mostly padding.  64 x 64 rows with 16 heads,
   // backward: 256 / 256 warp-MMA 162 us against 230, 576 / 512 266 against 322; 64 x 100 rows at 256 351 against 264.
   // With few kv heads the warp-MMA kernels leave the chip idle (8 x 64 rows, 16 / 4 heads: 40 us, pair 36).

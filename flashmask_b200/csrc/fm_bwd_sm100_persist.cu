@@ -340,7 +340,7 @@ bwd_sm100_persist_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __g
       } else {
         const int i = row0 + r;
         if (i < p.Sq) {
-          // from the L2: this kernel does not wait for the one that wrote them (the dK / dV kernel before it did)
+          // (no wait here: the dK / dV kernel waited for the row statistics before its trigger, see grid_dep_wait)
           lse2_row = __ldcg(p.lse_log2 + ((int64_t)b * p.Hq + hq0) * p.Sq_r + i);
           dps_row = __ldcg(p.dpsum + ((int64_t)b * p.Hq + hq0) * p.Sq_r + i);
         }

@@ -31,6 +31,11 @@ int cuda_fail(cudaError_t e, const char* what);
 // grid_dep_trigger() (only kernels that the same call always follows with another of its own do), B is launched with
 // launch_dependent() and calls grid_dep_wait() before it touches what A writes, or before it ends when it needs
 // nothing of A; either way B is complete only after A is.
+// A kernel C launched the same way behind B may read what A wrote without a wait of its own if every block of B calls
+// grid_dep_wait() before grid_dep_trigger(): C starts when all of B's blocks have triggered or left, so A is complete
+// and flushed by then.  (The deterministic backward: row statistics, dK / dV, dQ.  A kernel put between them, or a
+// trigger moved ahead of B's wait, takes that away; and since B may have started on an SM before A's results were
+// flushed, C reads them past the L1.)
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>

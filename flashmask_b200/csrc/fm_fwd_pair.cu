@@ -602,8 +602,7 @@ static int launch_fwd_pair(const AttnKParams& p, const fm_attn_args* a, cudaStre
 
 // d = dv = 256, 512, and 576 / 512, up to 2048 K tiles.
 bool fwd_pair_supported(const fm_attn_args* a) {
-  const bool dims = (a->d == 256 && a->dv == 256) || ((a->d == 512 || a->d == 576) && a->dv == 512);
-  return dims && (a->Sk + 127) / 128 <= FwdPairCfg<256>::LIST_MAX;
+  return pair_dims(a->d, a->dv) && (a->Sk + 127) / 128 <= FwdPairCfg<256>::LIST_MAX;
 }
 
 template <int D, bool IS_BF16>

@@ -124,7 +124,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint32_t* list = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_LIST);
   const uint32_t bars = sbase + Cfg::OFF_BAR;
   volatile int* misc = reinterpret_cast<volatile int*>(smem + Cfg::OFF_MISC);
-  // misc[0] tmem base, [1] cnt, [2] cnt_s0, [3] cnt_s1, [4] abort
+  // misc[0] tmem base, [1] cnt, [4] abort
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
 
   const int tid = threadIdx.x;
@@ -194,7 +194,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   }
   if (warp == 10) {
     // surviving K tiles, right to left, with the flags of both sub-tiles
-    int cnt = 0, c0 = 0, c1 = 0;
+    int cnt = 0;
     // the reductions the classification needs are staged in the (still idle) K/V ring
     const MaskDesc mst = stage_minmax(md, bh_mask, 0, n_hi, reinterpret_cast<int32_t*>(smem + Cfg::OFF_STAGE),
                                       Cfg::LIST_MAX, lane);
@@ -218,10 +218,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int pos = cnt + __popc(bal & ((1u << lane) - 1u));
       if (keep && pos < Cfg::LIST_MAX) list[pos] = (uint32_t)n | (f0 << 16) | (f1 << 20);
       cnt += __popc(bal);
-      c0 += __popc(__ballot_sync(0xffffffffu, f0 != 0));
-      c1 += __popc(__ballot_sync(0xffffffffu, f1 != 0));
     }
-    if (lane == 0) { misc[1] = min(cnt, Cfg::LIST_MAX); misc[2] = c0; misc[3] = c1; FPROF(10); }
+    if (lane == 0) { misc[1] = min(cnt, Cfg::LIST_MAX); FPROF(10); }
     fence_proxy_async_smem();   // the staging area is handed back to the TMA loads of the ring
   }
   tc_fence_before();
@@ -268,7 +266,6 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     return;
   }
-  const int cnt_s[2] = {misc[2], misc[3]};
 
   if (warp < 8) {
     // =========================== softmax warpgroups ===========================
@@ -404,45 +401,45 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           }
         }
       } else {
-      uint8_t* stage = smem + Cfg::OFF_Q + (SPLITV ? 0 : s * Cfg::Q_BYTES);   // Q is no longer needed
-      constexpr int CH0 = SPLITV ? DVS / 8 : 0;          // d = 256: warpgroup s stages chunks [16 s, 16 s + 16)
+        uint8_t* stage = smem + Cfg::OFF_Q + (SPLITV ? 0 : s * Cfg::Q_BYTES);   // Q is no longer needed
+        constexpr int CH0 = SPLITV ? DVS / 8 : 0;          // d = 256: warpgroup s stages chunks [16 s, 16 s + 16)
 #pragma unroll
-      for (int c = 0; c < DVS / 32; ++c) {
-        uint32_t orr[32];
-        if (n_done > 0) {
-          tmem_ld32(tO + 32 * c, orr);
-          tc_wait_ld();
-        } else {
+        for (int c = 0; c < DVS / 32; ++c) {
+          uint32_t orr[32];
+          if (n_done > 0) {
+            tmem_ld32(tO + 32 * c, orr);
+            tc_wait_ld();
+          } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) orr[j] = 0u;
+            for (int j = 0; j < 32; ++j) orr[j] = 0u;
+          }
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) {
+            uint4 v;
+            v.x = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 0]) * inv, __uint_as_float(orr[8 * q4 + 1]) * inv);
+            v.y = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 2]) * inv, __uint_as_float(orr[8 * q4 + 3]) * inv);
+            v.z = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 4]) * inv, __uint_as_float(orr[8 * q4 + 5]) * inv);
+            v.w = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 6]) * inv, __uint_as_float(orr[8 * q4 + 7]) * inv);
+            const int chunk = CH0 * s + 4 * c + q4;       // 16-byte chunk inside the row
+            *reinterpret_cast<uint4*>(stage + r * (DV * 2) + ((chunk ^ (r & (DV / 8 - 1))) << 4)) = v;
+          }
         }
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          uint4 v;
-          v.x = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 0]) * inv, __uint_as_float(orr[8 * q4 + 1]) * inv);
-          v.y = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 2]) * inv, __uint_as_float(orr[8 * q4 + 3]) * inv);
-          v.z = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 4]) * inv, __uint_as_float(orr[8 * q4 + 5]) * inv);
-          v.w = pack2<IS_BF16>(__uint_as_float(orr[8 * q4 + 6]) * inv, __uint_as_float(orr[8 * q4 + 7]) * inv);
-          const int chunk = CH0 * s + 4 * c + q4;       // 16-byte chunk inside the row
-          *reinterpret_cast<uint4*>(stage + r * (DV * 2) + ((chunk ^ (r & (DV / 8 - 1))) << 4)) = v;
-        }
-      }
-      if (prow < n_rows && !(SPLITV && s == 1))
-        p.lse[((int64_t)b * p.Hq + head) * p.Sq + row] = l_tot > 0.f ? (m_fin + log2f(l_tot)) * kLn2 : neg_inf();
-      __syncwarp();   // each warp stores the 32 rows it staged itself: no cross-warp dependency
-      const int rbase = ms + (SPLITV ? 0 : 128 * s);
-      uint16_t* go = reinterpret_cast<uint16_t*>(p.o) + b * p.o_b + hq * p.o_h;
-      constexpr int CH = DV / 8, CHW = DVS / 8;          // chunks per row, chunks this warpgroup staged
-      const int wrow = (warp & 3) * 32;
+        if (prow < n_rows && !(SPLITV && s == 1))
+          p.lse[((int64_t)b * p.Hq + head) * p.Sq + row] = l_tot > 0.f ? (m_fin + log2f(l_tot)) * kLn2 : neg_inf();
+        __syncwarp();   // each warp stores the 32 rows it staged itself: no cross-warp dependency
+        const int rbase = ms + (SPLITV ? 0 : 128 * s);
+        uint16_t* go = reinterpret_cast<uint16_t*>(p.o) + b * p.o_b + hq * p.o_h;
+        constexpr int CH = DV / 8, CHW = DVS / 8;          // chunks per row, chunks this warpgroup staged
+        const int wrow = (warp & 3) * 32;
 #pragma unroll 4
-      for (int idx = lane; idx < 32 * CHW; idx += 32) {
-        const int rr = wrow + idx / CHW, cc = CH0 * s + idx % CHW;
-        const int x = rbase + rr;
-        if (x < n_rows && cc * 8 < p.dv_dim) {
-          const uint4 v = *reinterpret_cast<const uint4*>(stage + rr * (DV * 2) + ((cc ^ (rr & (CH - 1))) << 4));
-          *reinterpret_cast<uint4*>(go + (int64_t)(x >> lg) * p.o_s + (x & ((1 << lg) - 1)) * p.o_h + cc * 8) = v;
+        for (int idx = lane; idx < 32 * CHW; idx += 32) {
+          const int rr = wrow + idx / CHW, cc = CH0 * s + idx % CHW;
+          const int x = rbase + rr;
+          if (x < n_rows && cc * 8 < p.dv_dim) {
+            const uint4 v = *reinterpret_cast<const uint4*>(stage + rr * (DV * 2) + ((cc ^ (rr & (CH - 1))) << 4));
+            *reinterpret_cast<uint4*>(go + (int64_t)(x >> lg) * p.o_s + (x & ((1 << lg) - 1)) * p.o_h + cc * 8) = v;
+          }
         }
-      }
       }
     }
     if (tid == 0) FPROF(5);

@@ -37,8 +37,8 @@ def _native_host():
 
 
 class FlashMaskFunc(torch.autograd.Function):
-    """The operator as a Python autograd function over ops.py; ``flashmask_attention`` runs the same calls
-    natively."""
+    """The operator as a Python autograd function over ops.py, for hosts that subclass it or need a Python node in
+    the graph; ``flashmask_attention`` makes the same calls natively, with bitwise the same results."""
 
     @staticmethod
     def forward(ctx, q, k, v, startend_row_indices, softmax_scale, causal, learnable_sink,

@@ -217,13 +217,14 @@ def _flash_attn_fwd(q, k, v, startend_row_indices=None, softmax_scale=None, caus
     With ``block_logit`` (fp32 ``[B, Hq, Sq, >= ceil(Sk / block_size)]``, filled with -inf by the
     caller) the kernel also merges into it, with fmax, the maximum of the masked, scaled scores of
     every (query row, block of ``block_size`` key columns); ``block_bos`` (int32 ``[B, Sq]``, first
-    key of the row's document) makes the block ids document-relative.  Queries are never packed
-    over the heads of a GQA group here, so ``pack_gqa`` must be False (or left at its default);
-    the reference defaults it to True under GQA and rejects that combination.
+    key of the row's document) makes the block ids document-relative.  With ``block_logit`` queries
+    are not packed over the heads of a GQA group, so ``pack_gqa`` must be False (or left at its default);
+    the reference defaults it to True under GQA and rejects that combination.  Without it the library decides
+    by itself whether a call with few queries packs heads and splits the keys.
 
     Reference: _flash_attn_fwd, flashmask/cute/ops/fwd.py:52-882 (same argument
-    meaning; block-score arguments :75-77,605-658; split-KV and pack-GQA are not part of
-    this operator surface)."""
+    meaning; block-score arguments :75-77,605-658; its split-KV and pack-GQA switches are not
+    part of this operator surface)."""
     if not q.is_cuda:
         raise RuntimeError("flashmask_b200 runs on CUDA (sm_100a) tensors only; there is no CPU path")
     idx = startend_row_indices

@@ -279,8 +279,7 @@ def test_short_sequences_of_the_widest_heads(kind, d, dv):
 
 @pytest.mark.parametrize("kind", MASKS)
 def test_masks_d256(kind):
-    """Every mask family through the 256 / 256 forward variant of the tcgen05 kernel (128 query rows per CTA, the
-    two warpgroups own the two 128-column halves of V / O); the backward of this head dim is the warp-MMA one."""
+    """Every mask family through the CTA-pair kernels at 256 / 256, forward and backward."""
     _run(kind, 2, 384, 384, 4, 2, 256, 256, seed=51)
     _run(kind, 1, 1411, 1411, 2, 1, 256, 256, sink=True, seed=52)
     assert _kernel_status() == 0

@@ -56,8 +56,8 @@ def test_argument_errors_need_no_gpu():
 
 def test_kernel_variant_routing_needs_no_gpu():
     """Tile shapes and launch tables by head dim: the tcgen05 variants (128-column K tiles; 64-query items in the
-    backward) serve every head dim up to 128, 192 / 128 in both directions and the 256 / 256 forward; a launch
-    table exists only where the variant walks one (not for the 256 forward, not for the 192 backward)."""
+    backward up to 192) serve every head dim up to 128, 192 / 128, 256 / 256, 512 / 512 and 576 / 512 in both directions;
+    a launch table exists only where the variant walks one (not at 256 and above, not for the 192 backward)."""
     for d, dv in [(8, 8), (64, 64), (96, 80), (128, 128), (192, 128), (256, 256)]:
         assert fm.fwd_tile_shape(d, dv) == (128, 128), (d, dv)
     for d, dv in [(64, 64), (128, 64), (128, 128), (192, 128)]:
