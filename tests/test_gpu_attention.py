@@ -616,6 +616,45 @@ def test_expanded_shared_key_value():
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("kind,d,dv,B,Hq,Hkv,hm,dtype,sink", [
+    ("causal_doc", 64, 64, 2, 4, 2, 1, torch.bfloat16, torch.float32),      # launch tables
+    ("four_column", 128, 128, 1, 4, 2, 2, torch.float16, torch.bfloat16),   # a mask per kv head
+    ("bidir_doc", 96, 80, 2, 3, 3, 1, torch.bfloat16, None),                # padded head dims
+    ("none_causal", 128, 128, 3, 4, 1, 1, torch.bfloat16, torch.float32),
+    ("sliding_window", 192, 128, 1, 4, 2, 1, torch.bfloat16, torch.float32),  # two tile shapes
+    ("share_question", 256, 256, 2, 2, 2, 1, torch.float16, torch.float32),
+    ("causal_doc", 576, 512, 1, 4, 1, 1, torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("layout", ["dense", "transposed", "shared kv"])
+def test_native_host_and_python_autograd_function_agree(kind, d, dv, B, Hq, Hkv, hm, dtype, sink, layout):
+    """flashmask_attention (native checks, allocations, autograd node) against FlashMaskFunc (the same over ops.py):
+    output, LSE and every gradient bitwise."""
+    S = 330
+    idx_np, causal = _mask(kind, B, S, S, 101)
+    if hm > 1:
+        idx_np = np.concatenate([_mask(kind, B, S, S, 101 + h)[0] for h in range(hm)], axis=1)
+    idx = None if idx_np is None else torch.from_numpy(np.ascontiguousarray(idx_np).copy()).cuda()
+    q, k, v, do, s = make_inputs(B, S, S, Hq, Hkv, d, dv, 101, dtype=dtype, sink=True)
+    q, k, v, do = q.cuda(), k.cuda(), v.cuda(), do.cuda()
+    if layout == "transposed":
+        q, k, v, do = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (q, k, v, do))
+    elif layout == "shared kv":
+        v = k[..., :dv]
+    s = None if sink is None else s.cuda().to(sink).reshape(1, Hq, 1, 1)
+    res = []
+    for call in (lambda *a: fm.flashmask_attention(*a[:4], causal=causal, sink=a[4], softmax_scale=0.11, return_lse=True,
+                                                   deterministic=True),
+                 lambda *a: fm.FlashMaskFunc.apply(*a[:4], 0.11, causal, a[4], True)):
+        leaves = [t.detach().requires_grad_(True) for t in (q, k, v)]
+        sk = None if s is None else s.detach().requires_grad_(True)
+        out, lse = call(*leaves, idx, sk)
+        assert out.requires_grad and not lse.requires_grad
+        res.append([out.detach(), lse, *torch.autograd.grad(out, leaves + ([] if sk is None else [sk]), do)])
+    assert len(res[0]) == (5 if sink is None else 6)
+    for a, b in zip(*res):
+        assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
+    assert _kernel_status() == 0
+
+
 def test_window_size_kwarg():
     q, k, v, do, _ = make_inputs(1, 256, 256, 2, 2, 64, 64, 1)
     out = fm.flashmask_attention(q.cuda(), k.cuda(), v.cuda(), causal=True, window_size=32)
