@@ -738,8 +738,12 @@ static FwdSplitPlan fwd_split_plan(const fm_attn_args* a) {
   const int G = a->Hq / a->Hkv, n_sm = sm_count(), tiles = (a->Sk + 127) / 128;
   const bool small = a->d <= 64 && a->dv <= 64;
   const double entry = small ? 4.9 : 5.7, in_turn = small ? 0.59 : 0.68, partial = small ? 4.5 : 10.0, merge = small ? 3.8 : 2.2;
-  auto tile = [&](int64_t rows) { return rows <= 128 ? (small ? 1.54 : 1.84) : (small ? 1.95 : 2.0); };   // one / both sub-tiles
   auto blocks = [&](int64_t rows) { return (rows + 255) / 256; };
+  auto tile = [&](int64_t rows) {                                   // one sub-tile of a CTA's two, or both
+    const double one = small ? 1.54 : 1.84, both = small ? 1.95 : 2.0;
+    const int64_t nb = blocks(rows);
+    return ((nb - 1) * both + (rows - 256 * (nb - 1) <= 128 ? one : both)) / nb;
+  };
   if (blocks(a->Sq) * a->Hq * a->B >= 4 * n_sm && blocks(a->Sq) > 1) return pl;
   double best = 1e30;
   auto consider = [&](int pack_log2, double handicap) {
