@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(256) count_visible_kernel(MaskDesc md, int64_t
 //      batches sharing a broadcast mask) of the class's units, repeat-major: CTAs next to
 //      each other in dispatch order work on neighbouring tiles of the same head, as in the
 //      index order, so operands shared between neighbouring tiles still meet in L2.
-// smem: work[E], order[E], hist/start[FM_ORDER_BUCKETS + 1], red[32], class[E] bytes.
+// smem: work[E], order[E], start[FM_ORDER_BUCKETS + 1], red[32], class and rank[E] bytes, counts of 32 units each.
 constexpr int FM_ORDER_BUCKETS = 8;
 constexpr int FM_PERSIST_MAX_ITEMS = 96;
 
@@ -124,11 +124,15 @@ __global__ void __launch_bounds__(1024) launch_order_kernel(MaskDesc md_in, int 
   if (stage_ints) {
     const int row4 = (md.BHm * md.nblk_pad) >> 2;                      // int4 per reduction
     const uint32_t which = md.ncols == 1 ? 0x03u : (md.ncols == 4 ? 0xFFu : (md.causal ? 0x0Fu : 0xC3u));
-    for (int w = 0; w < 8; ++w) {
-      if (!(which >> w & 1u)) continue;
-      const int4* src = reinterpret_cast<const int4*>(md_in.minmax) + (size_t)w * row4;
-      int4* dst = reinterpret_cast<int4*>(sm_all) + (size_t)w * row4;
-      for (int i = threadIdx.x; i < row4; i += 1024) dst[i] = __ldg(src + i);
+    // (all reductions' loads of a round are in flight together)
+    for (int i = threadIdx.x; i < row4; i += 1024) {
+      int4 v[8];
+#pragma unroll
+      for (int w = 0; w < 8; ++w)
+        if (which >> w & 1u) v[w] = __ldg(reinterpret_cast<const int4*>(md_in.minmax) + (size_t)w * row4 + i);
+#pragma unroll
+      for (int w = 0; w < 8; ++w)
+        if (which >> w & 1u) reinterpret_cast<int4*>(sm_all)[(size_t)w * row4 + i] = v[w];
     }
     md.minmax = sm_all;
     __syncthreads();
@@ -139,7 +143,8 @@ __global__ void __launch_bounds__(1024) launch_order_kernel(MaskDesc md_in, int 
   int32_t* sorder = sm + E;
   int32_t* sstart = sm + 2 * E;           // [FM_ORDER_BUCKETS + 1]
   int32_t* sred = sstart + FM_ORDER_BUCKETS + 1;  // [32]
-  uint8_t* sclass = reinterpret_cast<uint8_t*>(sred + 32);  // [E]
+  uint8_t* sclass = reinterpret_cast<uint8_t*>(sred + 32);  // [E] class | rank inside its 32 units << 3
+  uint16_t* scnt = reinterpret_cast<uint16_t*>(sclass + ((E + 3) & ~3));  // [ceil(E / 32)][FM_ORDER_BUCKETS]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n_cta = E * rep_h * rep_b;
   int2* table = reinterpret_cast<int2*>(out);
@@ -163,7 +168,6 @@ __global__ void __launch_bounds__(1024) launch_order_kernel(MaskDesc md_in, int 
     for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0) { swork[e] = cnt; gwork[e] = cnt; }
   }
-  if (tid <= FM_ORDER_BUCKETS) sstart[tid] = 0;
   __syncthreads();
 
   int mx = 0;
@@ -177,27 +181,63 @@ __global__ void __launch_bounds__(1024) launch_order_kernel(MaskDesc md_in, int 
   __shared__ long long stot[32];
   if (lane == 0) { sred[warp] = mx; stot[warp] = total; }
   __syncthreads();
-  mx = 0;
-  total = 0;
-  for (int w = 0; w < 32; ++w) { mx = max(mx, sred[w]); total += stot[w]; }
+  mx = sred[lane];
+#pragma unroll
+  for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   // [E+2]: 1 while a unit averages at most FM_PERSIST_MAX_ITEMS work items, the range in which the
   // persistent backward variant (which hides the per-unit prologue and epilogue at a slightly slower
   // main loop) was measured faster; information for the host, the kernels do not read it
-  if (tid == 0) gorder[E + 2] = total * item_mult <= (long long)FM_PERSIST_MAX_ITEMS * E ? 1 : 0;
-  for (int e = tid; e < E; e += 1024) {
-    const int k = (int)(((long long)(mx - swork[e]) * n_classes) / (mx + 1));  // 0 = heaviest class
-    sclass[e] = (uint8_t)k;
-    atomicAdd(&sstart[k + 1], 1);
+  if (warp == 0) {
+    total = stot[lane];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    if (lane == 0) gorder[E + 2] = total * item_mult <= (long long)FM_PERSIST_MAX_ITEMS * E ? 1 : 0;
+  }
+  // Stable counting sort by class.  A warp ranks 32 consecutive units with one ballot per class; scnt[chunk][class] counts
+  // them, and a scan over the chunks turns the counts into places.
+  const int n_chunks = (E + 31) >> 5;
+  for (int ch = warp; ch < n_chunks; ch += 32) {
+    const int e = 32 * ch + lane;
+    // class 0 is the heaviest (work * classes fits 32 bits: a unit has fewer than 2^26 tiles)
+    const int k = e < E ? (int)(((unsigned)(mx - swork[e]) * (unsigned)n_classes) / (unsigned)(mx + 1)) : -1;
+    int rank = 0, count = 0;
+#pragma unroll
+    for (int c = 0; c < FM_ORDER_BUCKETS; ++c) {
+      const uint32_t bal = __ballot_sync(0xffffffffu, k == c);
+      if (k == c) rank = __popc(bal & ((1u << lane) - 1u));
+      if (lane == c) count = __popc(bal);
+    }
+    if (e < E) sclass[e] = (uint8_t)(k | rank << 3);
+    if (lane < FM_ORDER_BUCKETS) scnt[ch * FM_ORDER_BUCKETS + lane] = (uint16_t)count;
   }
   __syncthreads();
-  if (tid == 0)
-    for (int k = 0; k < FM_ORDER_BUCKETS; ++k) sstart[k + 1] += sstart[k];
+  if (warp < FM_ORDER_BUCKETS) {
+    // warp c: units of class c in the chunks before each chunk
+    int before = 0;
+    for (int base = 0; base < n_chunks; base += 32) {
+      const int ch = base + lane;
+      const int mine = ch < n_chunks ? scnt[ch * FM_ORDER_BUCKETS + warp] : 0;
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      if (ch < n_chunks) scnt[ch * FM_ORDER_BUCKETS + warp] = (uint16_t)(before + incl - mine);
+      before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) sred[warp] = before;                  // units of the class
+  }
+  __syncthreads();
+  if (tid <= FM_ORDER_BUCKETS) {
+    int at = 0;
+    for (int k = 0; k < tid; ++k) at += sred[k];
+    sstart[tid] = at;
+  }
   __syncthreads();
   for (int e = tid; e < E; e += 1024) {
-    const int k = sclass[e];
-    int before = 0;
-    for (int j = 0; j < e; ++j) before += sclass[j] == k;
-    const int r = sstart[k] + before;
+    const int k = sclass[e] & 7;
+    const int r = sstart[k] + scnt[(e >> 5) * FM_ORDER_BUCKETS + k] + (sclass[e] >> 3);
     sorder[r] = e;
     gorder[r] = e;
   }
@@ -226,7 +266,8 @@ int fm::launch_order_build(const MaskDesc& md, int tile_n, const OrderJobs& jobs
   size_t smem = 0;
   for (int i = 0; i < n_jobs; ++i) {
     const size_t E = (size_t)md.BHm * jobs.job[i].n_units;
-    smem = std::max(smem, sizeof(int32_t) * (2 * E + FM_ORDER_BUCKETS + 1 + 32) + E);
+    smem = std::max(smem, sizeof(int32_t) * (2 * E + FM_ORDER_BUCKETS + 1 + 32) + ((E + 3) & ~(size_t)3) +
+                              (E + 31) / 32 * FM_ORDER_BUCKETS * sizeof(uint16_t));
   }
   int n_classes = FM_ORDER_BUCKETS;
   if (const int e = option_order_classes()) n_classes = std::min(FM_ORDER_BUCKETS, std::max(1, e));
