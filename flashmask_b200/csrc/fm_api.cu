@@ -392,6 +392,18 @@ extern "C" int64_t fm_launch_order_ints(const fm_attn_args* a, int which) {
   return 2 * g.n_cta + 2 * g.E + 4;
 }
 
+// An order only matters where CTAs queue: when every CTA of a launch starts at once the table costs its launch
+// (9 us, on the critical path of the forward) and changes nothing.  The two backward tables go together, since the
+// persistent two-kernel backward walks both.  1024 rows, 2 heads, d = 64, forward + backward: 96 -> 91 us.
+extern "C" int fm_launch_order_useful(const fm_attn_args* a, int which) {
+  OrderGeom g;
+  if (!order_geometry(a, which, &g)) return 0;
+  int64_t n = g.n_cta;
+  if (which != FM_ORDER_FWD && order_geometry(a, which == FM_ORDER_BWD_DQ ? FM_ORDER_BWD_DKDV : FM_ORDER_BWD_DQ, &g))
+    n = std::max(n, g.n_cta);
+  return n > sm_count();
+}
+
 // The counters of the persistent kernels live behind the table and the two unit arrays.
 static void attach_bwd_tables(const fm_attn_args* a, AttnKParams* p) {
   OrderGeom g;

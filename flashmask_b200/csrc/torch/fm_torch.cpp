@@ -109,8 +109,10 @@ Tables build_tables(const fm_attn_args& a, const Tensor& like, void* stream) {
   Tables t{Tensor(), {-1, -1, -1}};
   if (a.ncols == 0 || a.tile_n != 128) return t;      // only the kernels with 128-column tiles read tables
   const unsigned want = wanted_orders();
+  const bool asked_for = std::getenv("FLASHMASK_B200_ORDER") != nullptr;   // tables for every size (A/B runs)
   int64_t total = 0;
   for (int w = 0; w < 3; ++w) {
+    if (!asked_for && !fm_launch_order_useful(&a, w)) continue;
     const int64_t n = (want >> w & 1u) ? fm_launch_order_ints(&a, w) : 0;
     if (n <= 0) continue;
     t.at[w] = total;

@@ -251,6 +251,9 @@ FM_API int fm_fwd_block_score(const fm_attn_args* args, float* block_logit, int 
 #define FM_ORDER_BWD_DQ 1
 #define FM_ORDER_BWD_DKDV 2
 FM_API int64_t fm_launch_order_ints(const fm_attn_args* args, int which);
+/* 1 when the launch has more CTAs than the device has multiprocessors, so that their order matters (0: also when the
+ * kernel takes none).  A host that skips a useless table passes NULL for it; results do not depend on tables. */
+FM_API int fm_launch_order_useful(const fm_attn_args* args, int which);
 FM_API int fm_launch_order(const fm_attn_args* args, int which, int32_t* out, void* stream);
 /* The same for up to three kernels in ONE launch (a NULL pointer skips that kernel's table). */
 FM_API int fm_launch_orders(const fm_attn_args* args, int32_t* out_fwd, int32_t* out_dq, int32_t* out_dkdv,
