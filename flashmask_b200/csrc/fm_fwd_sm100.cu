@@ -88,7 +88,7 @@ struct FwdSm100Cfg {
   static_assert(SMEM_BS <= 227 * 1024, "shared memory of the block-score variant");
   // barrier indices
   static constexpr int B_QFULL = 0, B_KVFULL = 2, B_KVEMPTY = 2 + NSTAGE, B_SFULL = 2 + 2 * NSTAGE,
-                       B_PFULL = B_SFULL + 2, B_ODONE = B_PFULL + 2, B_BNDFULL = B_ODONE + 2,
+                       B_PFULL = B_SFULL + 2, B_PPART = B_PFULL + 2, B_ODONE = B_PPART + 2, B_BNDFULL = B_ODONE + 2,
                        B_BNDEMPTY = B_BNDFULL + NBND, B_COUNT = B_BNDEMPTY + NBND;
   static_assert((D == 64 && DV == 64) || (D == 128 && DV == 128) || (D == 192 && DV == 128) ||
                     (D == 256 && DV == 256), "head-dim variants");
@@ -165,7 +165,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     mbar_init(bar(Cfg::B_QFULL + 0), 1); mbar_init(bar(Cfg::B_QFULL + 1), 1);
     for (int i = 0; i < Cfg::NSTAGE; ++i) { mbar_init(bar(Cfg::B_KVFULL + i), 1); mbar_init(bar(Cfg::B_KVEMPTY + i), 1); }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(bar(Cfg::B_SFULL + s), 1); mbar_init(bar(Cfg::B_PFULL + s), 128); mbar_init(bar(Cfg::B_ODONE + s), 1);
+      mbar_init(bar(Cfg::B_SFULL + s), 1); mbar_init(bar(Cfg::B_PFULL + s), 4); mbar_init(bar(Cfg::B_PPART + s), 4); mbar_init(bar(Cfg::B_ODONE + s), 1);
     }
     for (int i = 0; i < Cfg::NBND; ++i) { mbar_init(bar(Cfg::B_BNDFULL + i), 32); mbar_init(bar(Cfg::B_BNDEMPTY + i), 256); }
     fence_mbar_init();
@@ -356,7 +356,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           tc_wait_st();
         }
         tc_fence_before();
-        mbar_arrive(bar(Cfg::B_PFULL + s));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(Cfg::B_PFULL + s));
         ++n_done;
       }
       if (any_bounds) {
@@ -485,6 +486,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (elect_one()) {
         constexpr uint32_t idesc_qk = make_idesc(IS_BF16, 128, 128, 0, 0);
         constexpr uint32_t idesc_pv = make_idesc(IS_BF16, 128, DVS, 0, 1);
+        // P V starts on the first 96 keys of a tile while the softmax still computes the last 32 (B_PPART): the wait for a
+        // tile's P, P V and the next scores is one dependent chain per sub-tile, and this takes up to 384 of its cycles out.
+        // Dense 8192 x 2, 32 / 8 heads, d = 64: 1694 -> 1604 us; 32768 share-question, d = 128: 975 -> 930 us.  The split
+        // variant, whose sub-tiles mostly take turns, lost 2 % by it and waits for the whole tile.
+        constexpr int B_PFIRST = SPLIT ? Cfg::B_PFULL : Cfg::B_PPART;
         int npv[2] = {0, 0};
         bool q_ready[2] = {false, false};
         bool ok = true;
@@ -520,14 +526,23 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             constexpr int s = decltype(sub)::value;
           const int k = 2 * i + 1, slot = k % Cfg::NSTAGE;
           ok = ok && mbar_wait(bar(Cfg::B_KVFULL + slot), (uint32_t)(k / Cfg::NSTAGE) & 1u, wc);
-          ok = ok && mbar_wait(bar(Cfg::B_PFULL + s), (uint32_t)npv[s] & 1u, wc);
+          ok = ok && mbar_wait(bar(B_PFIRST + s), (uint32_t)npv[s] & 1u, wc);
           if (!ok) return;
           tc_fence_after();
           // (d = 256: warpgroup s owns V columns [128 s, 128 s + 128): sub-tiles 2 s and 2 s + 1 of the V tile)
           const uint64_t db = dv0 + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4) + (SPLITV ? s * 2 * (Cfg::SUB >> 4) : 0));
           const uint32_t dst = tmem + 256u + 128u * s, src = tmem + 128u * s + 64u;
           const uint32_t acc0 = npv[s] > 0 ? 1u : 0u;
-          umma_ts_xn<8>(dst, src, db, idesc_pv, acc0);
+          if constexpr (SPLIT) {
+            umma_ts_xn<8>(dst, src, db, idesc_pv, acc0);
+          } else {
+            umma_ts_xn<4>(dst, src, db, idesc_pv, acc0);
+            umma_ts_x2(dst, src + 32u, db + (uint64_t)(4 * 128), idesc_pv);
+            ok = mbar_wait(bar(Cfg::B_PFULL + s), (uint32_t)npv[s] & 1u, wc);
+            if (!ok) return;
+            tc_fence_after();
+            umma_ts_x2(dst, src + 48u, db + (uint64_t)(6 * 128), idesc_pv);
+          }
           tc_commit(bar(Cfg::B_ODONE + s));
           ++npv[s];
         };
@@ -563,8 +578,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           // the sub-tile whose P is ready first goes first (sub-tile 0 when both or neither are)
           bool one_first = false;
           if (((e >> 16) & 0xFu) && ((e >> 20) & 0xFu))
-            one_first = !mbar_try_wait(bar(Cfg::B_PFULL + 0), (uint32_t)npv[0] & 1u) &&
-                        mbar_try_wait(bar(Cfg::B_PFULL + 1), (uint32_t)npv[1] & 1u);
+            one_first = !mbar_try_wait(bar(B_PFIRST + 0), (uint32_t)npv[0] & 1u) &&
+                        mbar_try_wait(bar(B_PFIRST + 1), (uint32_t)npv[1] & 1u);
           if (one_first) {
             issue_pv(std::integral_constant<int, 1>{}, i);
             if (ok && ((en >> 20) & 0xFu)) issue_qk(std::integral_constant<int, 1>{}, i + 1);

@@ -340,6 +340,18 @@ __device__ __forceinline__ uint64_t make_sdesc_noswz(uint32_t smem_addr, uint32_
          ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
+// Two more k-steps of the same GEMM (always accumulating).
+__device__ __forceinline__ void umma_ts_x2(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred pt;\n\t.reg .b64 tb;\n\t.reg .b32 ta;\n\t"
+      "setp.eq.b32 pt, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, pt;\n\t"
+      "add.u32 ta, %1, 8;  add.s64 tb, %2, 128;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], tb, %3, pt;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b), "r"(idesc)
+      : "memory");
+}
+
 // Block maxima of one row of a 128-column tile (reference: the fused block-score epilogue,
 // flashmask/cute/flash_fwd_sm100.py:4256-4371).  `sr` holds the masked raw scores (masked =
 // -inf), `rel0` is the first column of the tile relative to the start of the row's document.
