@@ -198,15 +198,23 @@ static bool bwd_uses_sm100(int d, int dv) {
 // The one-kernel backward (five GEMMs per tile pair, dQ summed into an fp32 accumulator in an order
 // that is not fixed) serves the tcgen05 head dims whenever the call does not ask for deterministic
 // gradients; the two-kernel variant gives every output element one owner and a fixed order.
-// Measured on 8K-128K masks it is 5-22 % faster at d = dv = 64 and d = dv = 128; head dims that only
-// partly fill a 64-column box measured slower (d = 96: +25 %), so they keep the two-kernel variant.
+// Measured on 8K-128K masks it is 5-22 % faster at d = dv = 64 and d = dv = 128.  Head dims between them run it too (the
+// GEMMs stop at the end of a head) where the key tiles fill the chip twice: a dK / dV unit walks every q head of its group,
+// while the two kernels spread dQ over them.  Forward + backward, two kernels -> one: 2 x 8192 documents, 32 / 8 heads
+// (1024 units) d = 96 1470 -> 1258 us, d = 72 1565 -> 1335; 16384 full, 16 heads (2048) d = 80 8266 -> 6620; 4 x 2048, 16
+// heads (1024) d = 96 313 -> 277.  Not taken: 2 x 3001, 16 / 4 heads (192) d = 96 270 -> 267; 3 x 1600, 16 / 4 heads (156)
+// d = 80 196 -> 228; 9500, 32 / 2 heads (150) d = 96 905 -> 1094; 4096, 32 / 2 heads (64) d = 80 1300 -> 1439.
 // The CTA-pair backward (256, 512, 576 / 512) keeps P and dS of a chunk of query rows in the caller's workspace;
 // without one (fm_bwd_static_scratch) and past its index range the warp-MMA kernels serve these head dims.
 enum BwdKernels { BWD_ONE_KERNEL, BWD_TWO_KERNELS, BWD_PAIR, BWD_WARP_MMA };
+// Head dims that the one-kernel backward serves whatever the sizes: calls over the same queries may share its accumulator.
+static bool bwd_fills_boxes(const fm_attn_args* a) { return a->d == a->dv && (a->d == 64 || a->d == 128); }
 // By geometry and options alone: what the workspace is sized for.
 static BwdKernels bwd_kernels_by_geometry(const fm_attn_args* a) {
-  const bool exact = a->d == a->dv && (a->d == 64 || a->d == 128);
-  if (bwd_uses_sm100(a->d, a->dv)) return exact && !a->deterministic && !g_opt.bwd_split ? BWD_ONE_KERNEL : BWD_TWO_KERNELS;
+  if (bwd_uses_sm100(a->d, a->dv)) {
+    const bool one = bwd_fills_boxes(a) || (a->d == a->dv && a->d > 64 && (int64_t)((a->Sk + 127) / 128) * a->Hkv * a->B >= 2 * sm_count());
+    return one && !a->deterministic && !g_opt.bwd_split ? BWD_ONE_KERNEL : BWD_TWO_KERNELS;
+  }
   return pair_dims(a->d, a->dv) && !g_opt.bwd_mma && bwd_pair_supported(a) ? BWD_PAIR : BWD_WARP_MMA;
 }
 static BwdKernels bwd_kernels(const fm_attn_args* a) {
@@ -479,8 +487,10 @@ static size_t bwd_workspace_bytes(const fm_attn_args* a, BwdKernels kernels) {
 }
 
 // What fm_bwd cannot do without: the CTA-pair backward works in smaller chunks when it gets less than it asks for, and
-// leaves the call to the warp-MMA kernels, which keep row statistics only, when not even the smallest chunk fits.
+// leaves the call to the warp-MMA kernels, which keep row statistics only, when not even the smallest chunk fits; between the
+// head dims 64 and 128 the two-kernel backward takes a call without room for the accumulator.
 static size_t bwd_min_workspace_bytes(const fm_attn_args* a, BwdKernels kernels) {
+  if (kernels == BWD_ONE_KERNEL && !bwd_fills_boxes(a)) kernels = BWD_TWO_KERNELS;
   return bwd_workspace_bytes(a, kernels == BWD_PAIR ? BWD_WARP_MMA : kernels);
 }
 
@@ -495,7 +505,7 @@ extern "C" size_t fm_bwd_workspace_bytes(const fm_attn_args* a) {
 }
 
 extern "C" int fm_bwd_accumulates(const fm_attn_args* a) {
-  return (a && a->d > 0 && a->dv > 0 && bwd_kernels(a) == BWD_ONE_KERNEL) ? 1 : 0;
+  return (a && a->d > 0 && a->dv > 0 && bwd_fills_boxes(a) && bwd_kernels(a) == BWD_ONE_KERNEL) ? 1 : 0;
 }
 
 extern "C" int fm_bwd(const fm_attn_args* a, void* stream) {
@@ -512,7 +522,7 @@ extern "C" int fm_bwd(const fm_attn_args* a, void* stream) {
   if (rc != FM_OK) return rc;
   FM_REQUIRE(a->ncols == 0 || a->tile_n == tn, FM_ERR_INVALID_ARGUMENT,
              "fm_bwd: minmax was prepared for tile_n=%d, this variant needs %d", a->tile_n, tn);
-  const BwdKernels kernels = bwd_kernels(a);
+  BwdKernels kernels = bwd_kernels(a);
   const size_t need = bwd_min_workspace_bytes(a, kernels);
   FM_REQUIRE(a->workspace && a->workspace_bytes >= need, FM_ERR_WORKSPACE,
              "fm_bwd: workspace too small (%zu bytes given, %zu needed)", a->workspace_bytes, need);
@@ -523,12 +533,13 @@ extern "C" int fm_bwd(const fm_attn_args* a, void* stream) {
   const size_t rows = (size_t)a->B * a->Hq * p.Sq_r;
   p.dpsum = reinterpret_cast<float*>(a->workspace);
   p.lse_log2 = p.dpsum + rows;
+  if (kernels == BWD_ONE_KERNEL && a->workspace_bytes < bwd_workspace_bytes(a, kernels)) kernels = BWD_TWO_KERNELS;
   if (kernels == BWD_ONE_KERNEL) {
     uint8_t* w = reinterpret_cast<uint8_t*>(a->workspace) + bwd_row_stat_bytes(a);
     p.dq_accum = reinterpret_cast<float*>(w);
     p.stat_s = reinterpret_cast<uint16_t*>(w + bwd_sm100_fused_accum_bytes(a));
     p.stat_dp = p.stat_s + (size_t)a->B * a->Hq * p.Sq_r * 8;
-    p.bwd_flags = a->bwd_flags;
+    p.bwd_flags = bwd_fills_boxes(a) ? a->bwd_flags : 0;      // (see fm_bwd_accumulates)
   }
   const size_t beyond_stats = a->workspace_bytes - bwd_row_stat_bytes(a);
   if (kernels == BWD_PAIR && bwd_pair_fits(a, beyond_stats)) {

@@ -1,4 +1,4 @@
-// Backward attention as ONE tcgen05 kernel for head dims up to 128: S, dP, dV, dK and dQ of
+// Backward attention as ONE tcgen05 kernel for equal head dims from 64 to 128: S, dP, dV, dK and dQ of
 // a (query block, key tile) pair are each computed once (five GEMMs per pair).
 //
 // A CTA owns a sequence of UNITS, one 128-key tile of one kv head each (from the dK/dV launch
@@ -552,9 +552,9 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           const uint64_t dSs = make_sdesc_noswz(sAux, sbase + Cfg::OFF_ZEROS - sAux, 128);
           const uint64_t dSd = make_sdesc_noswz(sAux + 1024, sbase + Cfg::OFF_ZEROS - (sAux + 1024), 128);
           if constexpr (D == 128) {
-            umma_ss_x8<(Cfg::SUB128 >> 4), (Cfg::SUB64 >> 4)>(tmem + C_S, dKk, dq_, idesc_g, 0u);
+            umma_ss_width<(Cfg::SUB128 >> 4), (Cfg::SUB64 >> 4)>(tmem + C_S, dKk, dq_, idesc_g, p.d);
             umma_ss(tmem + C_S, dOnes, dSs, idesc_g, 1u);
-            umma_ss_x8<(Cfg::SUB128 >> 4), (Cfg::SUB64 >> 4)>(tmem + C_DP, dVk, do_, idesc_g, 0u);
+            umma_ss_width<(Cfg::SUB128 >> 4), (Cfg::SUB64 >> 4)>(tmem + C_DP, dVk, do_, idesc_g, p.dv_dim);
             umma_ss(tmem + C_DP, dOnes, dSd, idesc_g, 1u);
           } else {
             umma_ss_x4(tmem + C_S, dKk, dq_, idesc_g, 0u);
@@ -572,7 +572,8 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   } else if (warp == 11) {
     // =========================== UMMA issuer 2: dV, dK, dQ^T ===========================
     if (elect_one()) {
-      constexpr uint32_t idesc_acc = make_idesc(IS_BF16, 128, D, 0, 1);     // dV, dK
+      // dV, dK: as many columns as the heads have (rounded up to 16; d == dv in this kernel)
+      const uint32_t idesc_acc = make_idesc(IS_BF16, 128, D == 64 ? 64 : (p.d + 15) & ~15, 0, 1);
       constexpr uint32_t idesc_dq = make_idesc(IS_BF16, 128, 64, 1, 1);     // dQ^T
       const uint64_t dKm = make_sdesc(sStat, Cfg::SUB128, 1024);            // K tile, MN-major (A of dQ^T)
       const uint64_t dRm = make_sdesc(sRing, Cfg::SUB64, 1024);             // MN-major view of a ring slot
@@ -665,7 +666,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(Cfg::B_DQFREE));
-        if (32 * ew < D) {
+        if (32 * ew < p.d) {
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             uint8_t* sb = wst + (rnd & 1u) * Cfg::RBUF_BYTES;

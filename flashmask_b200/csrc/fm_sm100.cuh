@@ -340,6 +340,20 @@ __device__ __forceinline__ uint64_t make_sdesc_noswz(uint32_t smem_addr, uint32_
          ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
+// D[tmem] = A[smem] * B[smem] over the first `width` of 128 columns of K, both operands K-major in two 64-column
+// sub-tiles (A_SUB and B_SUB: distance of the second one, in 16-byte units): the k-steps that lie wholly past the end of a head
+// read zeros and are left out.
+template <int A_SUB, int B_SUB>
+__device__ __forceinline__ void umma_ss_width(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, int width) {
+  if (width > 112) {
+    umma_ss_x8<A_SUB, B_SUB>(d_tmem, a, b, idesc, 0u);
+  } else {
+    umma_ss_x4(d_tmem, a, b, idesc, 0u);
+    for (int s = 0; s < (width - 49) / 16; ++s)
+      umma_ss(d_tmem, a + (uint64_t)(A_SUB + 2 * s), b + (uint64_t)(B_SUB + 2 * s), idesc, 1u);
+  }
+}
+
 // Two more k-steps of the same GEMM (always accumulating).
 __device__ __forceinline__ void umma_ts_x2(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc) {
   asm volatile(

@@ -290,16 +290,19 @@ FM_API int fm_selftest_bounded_wait(int budget_us, void* stream);
  * postprocess, flash_bwd_postprocess.py).  Ask for the size with the same
  * args->deterministic the call will carry. */
 FM_API size_t fm_bwd_workspace_bytes(const fm_attn_args* args);
-/* The least workspace fm_bwd takes.  It is less than fm_bwd_workspace_bytes at
- * the head dims 256, 512 and 576 only, where the fast kernels keep P and dS of a
+/* The least workspace fm_bwd takes.  It is less than fm_bwd_workspace_bytes for
+ * equal head dims between 64 and 128, where calls with many key tiles run the
+ * one-kernel variant and, without room for its accumulator, the two-kernel one;
+ * and at the head dims 256, 512 and 576, where the fast kernels keep P and dS of a
  * chunk of the problem (2 GiB, more where 256 rows of all heads of a kv group
  * need more): with fewer bytes the chunks are smaller, and where not even the
  * smallest fits, other kernels serve that keep row statistics only.  Results are
  * bitwise reproducible for a given workspace size; another size sums dK and dV in
  * another order. */
 FM_API size_t fm_bwd_min_workspace_bytes(const fm_attn_args* args);
-/* 1 when fm_bwd(args) would run the one-kernel variant (and so honours
- * args->bwd_flags), else 0.  Reads the strides and softmax_scale too. */
+/* 1 when fm_bwd(args) would run the one-kernel variant and honours
+ * args->bwd_flags (head dims 64 and 128, whatever the sizes), else 0.  Reads the
+ * strides and softmax_scale too. */
 FM_API int fm_bwd_accumulates(const fm_attn_args* args);
 FM_API int fm_bwd(const fm_attn_args* args, void* stream);
 

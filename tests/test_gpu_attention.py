@@ -396,6 +396,28 @@ def test_padded_head_dims(d, dv, fwd_variant):
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("kind", ["causal_doc", "bidir_doc", "none_full"])
+@pytest.mark.parametrize("d", [72, 80, 96, 104, 120])
+def test_one_kernel_backward_between_64_and_128(d, kind):
+    """320 key tiles fill the chip twice, so the one-kernel backward serves head dims that do not fill their second 64-column
+    box: GEMMs that stop at 5, 6, 7 and 8 k-steps, ragged last tiles, and nothing past the end of a head.  With room for the
+    row statistics only the two-kernel backward takes the call."""
+    B, S, Hq, Hkv = 8, 517, 16, 8
+    idx_np, causal = _mask(kind, B, S, S, 61)
+    idx = None if idx_np is None else torch.from_numpy(np.ascontiguousarray(idx_np).copy()).cuda()
+    q, k, v, do, s = make_inputs(B, S, S, Hq, Hkv, d, d, 61, sink=True)
+    dev = [t.cuda() for t in (q, k, v, do)]
+    stats = 2 * 4 * B * Hq * 640
+    got = run_c_abi(*dev, idx, causal, s, deterministic=False)
+    assert_parity(got, run_oracle(q, k, v, do, idx, causal, s), naive_lowp(*dev, idx, causal, s))
+    least = run_c_abi(*dev, idx, causal, s, deterministic=False, workspace=stats)
+    fixed = run_c_abi(*dev, idx, causal, s, deterministic=True)
+    for n in ("dq", "dk", "dv", "dsink"):
+        assert torch.equal(least[n], fixed[n]), n
+    assert not torch.equal(got["dq"], fixed["dq"])              # sums over the key tiles in another order
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("kind", ["none_causal", "causal_doc", "random_eviction"])
 def test_sink(kind, fwd_variant):
     _run(kind, 2, 256, 256, 4, 2, 128, 128, sink=True, seed=7)
