@@ -165,7 +165,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     mbar_init(bar(Cfg::B_QFULL + 0), 1); mbar_init(bar(Cfg::B_QFULL + 1), 1);
     for (int i = 0; i < Cfg::NSTAGE; ++i) { mbar_init(bar(Cfg::B_KVFULL + i), 1); mbar_init(bar(Cfg::B_KVEMPTY + i), 1); }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(bar(Cfg::B_SFULL + s), 1); mbar_init(bar(Cfg::B_PFULL + s), 4); mbar_init(bar(Cfg::B_PPART + s), 4); mbar_init(bar(Cfg::B_ODONE + s), 1);
+      mbar_init(bar(Cfg::B_SFULL + s), 1); mbar_init(bar(Cfg::B_PFULL + s), SPLIT ? 128 : 4); mbar_init(bar(Cfg::B_PPART + s), 4); mbar_init(bar(Cfg::B_ODONE + s), 1);
     }
     for (int i = 0; i < Cfg::NBND; ++i) { mbar_init(bar(Cfg::B_BNDFULL + i), 32); mbar_init(bar(Cfg::B_BNDEMPTY + i), 256); }
     fence_mbar_init();
@@ -356,8 +356,12 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           tc_wait_st();
         }
         tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(Cfg::B_PFULL + s));
+        if constexpr (SPLIT) {
+          mbar_arrive(bar(Cfg::B_PFULL + s));
+        } else {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(Cfg::B_PFULL + s));
+        }
         ++n_done;
       }
       if (any_bounds) {
