@@ -218,7 +218,9 @@ static BwdKernels bwd_kernels_by_geometry(const fm_attn_args* a) {
   return pair_dims(a->d, a->dv) && !g_opt.bwd_mma && bwd_pair_supported(a) ? BWD_PAIR : BWD_WARP_MMA;
 }
 static BwdKernels bwd_kernels(const fm_attn_args* a) {
-  return fits_tcgen05(a, true) ? bwd_kernels_by_geometry(a) : BWD_WARP_MMA;
+  const BwdKernels k = fits_tcgen05(a, true) ? bwd_kernels_by_geometry(a) : BWD_WARP_MMA;
+  // the one-kernel backward divides LSE by the scale: both stay far inside fp32
+  return k == BWD_ONE_KERNEL && a->softmax_scale < 0x1p-100f ? BWD_TWO_KERNELS : k;
 }
 
 // preprocess -> main kernels of the selected variant -> dsink, on one stream
@@ -474,7 +476,7 @@ static size_t bwd_row_stat_bytes(const fm_attn_args* a) {
   return (2 * rows * sizeof(float) + 255) & ~(size_t)255;
 }
 
-// One-kernel backward: the statistics once more as 16-bit GEMM operands, 2 x 16 bytes per row.
+// One-kernel backward: the statistics once more as GEMM operands (three bf16 parts each), 2 x 16 bytes per row.
 static size_t bwd_stat_operand_bytes(const fm_attn_args* a) {
   return (size_t)a->B * a->Hq * round_up(a->Sq, 128) * 32;
 }

@@ -386,6 +386,15 @@ __global__ void __launch_bounds__(256) bwd_dq_mma_kernel(const AttnKParams p) {
 // ---------------------------------------------------------------------------
 // preprocess + dsink
 // ---------------------------------------------------------------------------
+// An fp32 value as three bf16 numbers whose sum it is, in the first columns of a 16-byte operand row.  Each part takes the
+// next 8 bits of the significand and bf16 has the exponents of fp32, so range and precision are those of fp32 (but for the
+// last 2^-8 below FLT_MAX, which round up to infinity); two parts hold 16 bits, and fp16 ones end at 65504.
+__device__ __forceinline__ uint4 stat_operand(float x) {
+  const float hi = __bfloat162float(__float2bfloat16_rn(x));
+  const float mid = __bfloat162float(__float2bfloat16_rn(x - hi));
+  return make_uint4(pack2<true>(hi, mid), pack2<true>(x - hi - mid, 0.f), 0u, 0u);
+}
+
 // dPsum[b,h,i] = sum_c O[b,i,h,c] * dO[b,i,h,c]; lse_log2 = LSE * log2(e) (-inf -> 0).
 // LPR lanes share one row (each lane owns 8-element chunks), so a warp covers
 // 32 / LPR rows per pass and every lane has a 16-byte load in flight.
@@ -436,18 +445,9 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const AttnKParams p
     p.dpsum[at] = acc;
     p.lse_log2[at] = lse2;
     if (p.stat_s) {
-      // the same two values as 16-bit GEMM operands (hi + lo parts, negated): see the one-kernel backward
-      const float c = lse2 / p.scale_log2;
-      float c_hi, c_lo, d_hi, d_lo;
-      if constexpr (IS_BF16) {
-        c_hi = __bfloat162float(__float2bfloat16_rn(c)); c_lo = c - c_hi;
-        d_hi = __bfloat162float(__float2bfloat16_rn(acc)); d_lo = acc - d_hi;
-      } else {
-        c_hi = __half2float(__float2half_rn(c)); c_lo = c - c_hi;
-        d_hi = __half2float(__float2half_rn(acc)); d_lo = acc - d_hi;
-      }
-      *reinterpret_cast<uint4*>(p.stat_s + at * 8) = make_uint4(pack2<IS_BF16>(-c_hi, -c_lo), 0u, 0u, 0u);
-      *reinterpret_cast<uint4*>(p.stat_dp + at * 8) = make_uint4(pack2<IS_BF16>(-d_hi, -d_lo), 0u, 0u, 0u);
+      // the same two values as GEMM operands of the one-kernel backward (negated)
+      *reinterpret_cast<uint4*>(p.stat_s + at * 8) = stat_operand(-lse2 / p.scale_log2);
+      *reinterpret_cast<uint4*>(p.stat_dp + at * 8) = stat_operand(-acc);
     }
   }
 }

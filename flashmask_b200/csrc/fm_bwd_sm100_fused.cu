@@ -50,11 +50,12 @@ struct BwdFusedCfg {
   static constexpr int OFF_RING = OFF_STAT + 2 * TILE_BYTES;
   static constexpr int OFF_DS = OFF_RING + NSLOT * SLOT_BYTES;          // one buffer per item parity
   // STAT: the per-query statistics enter through the GEMMs.  S^T = K Q^T gets one more k-step whose A is a
-  // tile of ones and whose B holds, per query, (-c_hi, -c_lo, 0, ...) with c = LSE*log2e / scale_log2 split
-  // into two 16-bit parts: the accumulator then already holds S - c, and P = exp2(scale_log2 * (S - c)) needs
-  // no per-column value in the compute warps.  dP^T = V dO^T likewise gets (-d_hi, -d_lo) with d = rowsum(O dO).
-  // Both operands are K-major without swizzle: 8-row x 16-byte core matrices; the second half of K (columns
-  // 8..15) of A reads the ones again, that of B a block of zeros.
+  // tile of ones and whose B holds, per query, the three parts of -c (0 in the other columns), c = LSE*log2e / scale_log2:
+  // the accumulator then already holds S - c, and P = exp2(scale_log2 * (S - c)) needs no per-column value in the
+  // compute warps.  dP^T = V dO^T likewise gets -d, d = rowsum(O dO).  The parts are bf16 whatever the type of the call
+  // (A and B of one MMA share a type, MMAs into one accumulator need not): three of them carry the 24 bits and the range
+  // of the fp32 value.  Both operands are K-major without swizzle: 8-row x 16-byte core matrices; the second half of K
+  // (columns 8..15) of A reads the ones again, that of B a block of zeros.
   static constexpr int OFF_AUX = OFF_DS + 2 * DS_BYTES;                 // per ring slot: S statistics, dP statistics
   static constexpr int OFF_ONES = OFF_AUX + NSLOT * AUX_BYTES;          // 17 core matrices of ones (2176 bytes)
   static constexpr int OFF_ZEROS = OFF_ONES + 2176;                     // 8 core matrices of zeros (1 KB)
@@ -210,9 +211,8 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
 
   if (tid == 0) misc[4] = 0;
   {
-    // constant operands of the statistics k-step: ones (1.0 in the kernel's 16-bit type) and zeros
-    const uint32_t one2 = IS_BF16 ? 0x3F803F80u : 0x3C003C00u;
-    for (int x = tid; x < 2176 / 4; x += Cfg::NTHREADS) reinterpret_cast<uint32_t*>(smem + Cfg::OFF_ONES)[x] = one2;
+    // constant operands of the statistics k-step: ones (bf16) and zeros
+    for (int x = tid; x < 2176 / 4; x += Cfg::NTHREADS) reinterpret_cast<uint32_t*>(smem + Cfg::OFF_ONES)[x] = 0x3F803F80u;
     for (int x = tid; x < 1024 / 4; x += Cfg::NTHREADS) reinterpret_cast<uint32_t*>(smem + Cfg::OFF_ZEROS)[x] = 0u;
     fence_proxy_async_smem();
   }
@@ -515,6 +515,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     // the operands of item kk have landed; nothing here waits for the compute warpgroups' results.
     if (elect_one()) {
       constexpr uint32_t idesc_g = make_idesc(IS_BF16, 128, 64, 0, 0);      // S^T, dP^T
+      constexpr uint32_t idesc_stat = make_idesc(true, 128, 64, 0, 0);      // their statistics k-step
       const uint64_t dKk = make_sdesc(sStat, 16, 1024);                     // K tile, K-major (A of S^T)
       const uint64_t dVk = make_sdesc(sStat + Cfg::TILE_BYTES, 16, 1024);   // V tile, K-major (A of dP^T)
       const uint64_t dRk = make_sdesc(sRing, 16, 1024);                     // K-major view of a ring slot
@@ -553,14 +554,14 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           const uint64_t dSd = make_sdesc_noswz(sAux + 1024, sbase + Cfg::OFF_ZEROS - (sAux + 1024), 128);
           if constexpr (D == 128) {
             umma_ss_width<(Cfg::SUB128 >> 4), (Cfg::SUB64 >> 4)>(tmem + C_S, dKk, dq_, idesc_g, p.d);
-            umma_ss(tmem + C_S, dOnes, dSs, idesc_g, 1u);
+            umma_ss(tmem + C_S, dOnes, dSs, idesc_stat, 1u);
             umma_ss_width<(Cfg::SUB128 >> 4), (Cfg::SUB64 >> 4)>(tmem + C_DP, dVk, do_, idesc_g, p.dv_dim);
-            umma_ss(tmem + C_DP, dOnes, dSd, idesc_g, 1u);
+            umma_ss(tmem + C_DP, dOnes, dSd, idesc_stat, 1u);
           } else {
             umma_ss_x4(tmem + C_S, dKk, dq_, idesc_g, 0u);
-            umma_ss(tmem + C_S, dOnes, dSs, idesc_g, 1u);
+            umma_ss(tmem + C_S, dOnes, dSs, idesc_stat, 1u);
             umma_ss_x4(tmem + C_DP, dVk, do_, idesc_g, 0u);
-            umma_ss(tmem + C_DP, dOnes, dSd, idesc_g, 1u);
+            umma_ss(tmem + C_DP, dOnes, dSd, idesc_stat, 1u);
           }
           tc_commit(bar(Cfg::B_GFULL + pz));
           if (k == K_items - 1) tc_commit(bar(Cfg::B_VFREE));   // that was the unit's last read of V

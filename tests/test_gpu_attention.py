@@ -418,6 +418,59 @@ def test_one_kernel_backward_between_64_and_128(d, kind):
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("what", ["row sums", "scores", "small scale"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("d", [64, 96, 128])
+def test_row_statistics_beyond_16_bits(d, dtype, what):
+    """rowsum(O dO) of a million, LSE of thousands, LSE / scale of a hundred thousand: the backward subtracts both with the
+    range and precision of fp32, whatever the type of the call and whichever kernels serve it (320 key tiles: the
+    one-kernel backward, with launch tables).  Against 64 bits, on the O and LSE that the backward reads."""
+    B, S, Hq, Hkv = 8, 517, 16, 8
+    G, scale = Hq // Hkv, 5e-5 if what == "small scale" else 1 / math.sqrt(d)
+    idx_np, causal = _mask("causal_doc", B, S, S, 61)
+    idx = torch.from_numpy(np.ascontiguousarray(idx_np).copy()).cuda()
+    q, k, v, do, _ = (t if t is None else t.cuda().float() for t in make_inputs(B, S, S, Hq, Hkv, d, d, 62))
+    if what == "row sums":
+        v, do = v + 128, do + 100
+    elif what == "scores":
+        q, k, do = 20 + q / 8, 20 + k / 8, do.abs()
+    q, k, v, do = (t.to(dtype) for t in (q, k, v, do))
+    visible = torch.from_numpy(oracle.dense_bias(idx_np, S, S, causal)).cuda() == 0
+    heads = lambda t: t.double().permute(0, 2, 1, 3)
+    q64, do64 = heads(q), heads(do)
+    k64, v64 = (heads(t).repeat_interleave(G, dim=1) for t in (k, v))
+    by_key = lambda t: t.reshape(B, Hkv, G, S, -1).sum(2)              # the q heads of a group share dK and dV
+    u, tiny = (2 ** -8, 0.0) if dtype == torch.bfloat16 else (2 ** -11, 2 ** -25)
+    for deterministic in (False, True):
+        x = [t.detach().requires_grad_(True) for t in (q, k, v)]
+        out, lse = fm.flashmask_attention(*x, idx, causal=causal, softmax_scale=scale, return_lse=True,
+                                          deterministic=deterministic)
+        got = torch.autograd.grad(out, x, do)
+        dsum = (heads(out.detach()) * do64).sum(-1, keepdim=True)
+        lse = lse.detach().double()[..., None]
+        if what == "row sums":
+            assert dsum.abs().min() > 65504
+        else:
+            assert (lse / scale).abs().median() > 2e4
+        # exponent and dP - rowsum(O dO): fp32 sums of head-dim products, a few units of 2^-24 of their largest terms;
+        # the exponent is then a relative error of P (and exp2 itself has one of 2^-22)
+        p = torch.exp(q64 @ k64.transpose(-1, -2) * scale - lse) * visible
+        e_p = 2 ** -21 * (scale * q64.norm(dim=-1, keepdim=True) * k64.norm(dim=-1)[:, :, None] + lse.abs() + 1)
+        dp = do64 @ v64.transpose(-1, -2) - dsum
+        e_dp = 2 ** -21 * (do64.norm(dim=-1, keepdim=True) * v64.norm(dim=-1)[:, :, None] + dsum.abs())
+        ds = p * dp
+        # P and dS are rounded to the 16-bit type, the results once more; the sums are fp32
+        d_p = p * (e_p + u + 2 ** -18) + tiny
+        d_ds = ds.abs() * (e_p + u + 2 ** -18) + p * e_dp + tiny
+        ref = [(scale * ds) @ k64, by_key((scale * ds).transpose(-1, -2) @ q64), by_key(p.transpose(-1, -2) @ do64)]
+        bound = [scale * (d_ds @ k64.abs()), by_key(scale * (d_ds.transpose(-1, -2) @ q64.abs())),
+                 by_key(d_p.transpose(-1, -2) @ do64.abs())]
+        for g_, r, b, n in zip(got, ref, bound, ("dq", "dk", "dv")):
+            err = (heads(g_) - r).abs()
+            assert (err <= b + u * (r.abs() + b) + tiny).all(), (n, deterministic, (err - b).max().item())
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("kind", ["none_causal", "causal_doc", "random_eviction"])
 def test_sink(kind, fwd_variant):
     _run(kind, 2, 256, 256, 4, 2, 128, 128, sink=True, seed=7)
