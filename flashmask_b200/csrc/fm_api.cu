@@ -198,21 +198,43 @@ static bool bwd_uses_sm100(int d, int dv) {
 // The one-kernel backward (five GEMMs per tile pair, dQ summed into an fp32 accumulator in an order
 // that is not fixed) serves the tcgen05 head dims whenever the call does not ask for deterministic
 // gradients; the two-kernel variant gives every output element one owner and a fixed order.
-// Measured on 8K-128K masks it is 5-22 % faster at d = dv = 64 and d = dv = 128.  Head dims between them run it too (the
-// GEMMs stop at the end of a head) where the key tiles fill the chip twice: a dK / dV unit walks every q head of its group,
-// while the two kernels spread dQ over them.  Forward + backward, two kernels -> one: 2 x 8192 documents, 32 / 8 heads
-// (1024 units) d = 96 1470 -> 1258 us, d = 72 1565 -> 1335; 16384 full, 16 heads (2048) d = 80 8266 -> 6620; 4 x 2048, 16
-// heads (1024) d = 96 313 -> 277.  Not taken: 2 x 3001, 16 / 4 heads (192) d = 96 270 -> 267; 3 x 1600, 16 / 4 heads (156)
-// d = 80 196 -> 228; 9500, 32 / 2 heads (150) d = 96 905 -> 1094; 4096, 32 / 2 heads (64) d = 80 1300 -> 1439.
+// Measured on 8K-128K masks it is 5-22 % faster at d = dv = 64 and d = dv = 128.  Head dims between them run it too where
+// one_kernel_pays (the GEMMs stop at the end of a head).
 // The CTA-pair backward (256, 512, 576 / 512) keeps P and dS of a chunk of query rows in the caller's workspace;
 // without one (fm_bwd_static_scratch) and past its index range the warp-MMA kernels serve these head dims.
 enum BwdKernels { BWD_ONE_KERNEL, BWD_TWO_KERNELS, BWD_PAIR, BWD_WARP_MMA };
 // Head dims that the one-kernel backward serves whatever the sizes: calls over the same queries may share its accumulator.
 static bool bwd_fills_boxes(const fm_attn_args* a) { return a->d == a->dv && (a->d == 64 || a->d == 128); }
+// Head dims between 64 and 128.  A unit of the one kernel is a key tile of a kv head with every q head of its group (G), and
+// does five GEMMs an item; the two kernels do seven, but spread three of them over the q heads.  So the one kernel needs
+// units that fill the chip evenly and rows enough in each to pay for its accumulator (512 bytes a query row, cleared, added
+// to and rounded).  Forward + backward in us, two kernels -> one, d = 96, (units);
+// Hkv * B copies of a key tile share the mask's heaviest columns:
+//   masks, 4 copies and more, units >= 2 an SM: 4800 documents 32 / 8 heads (304) 417 -> 369, 9500, 32 / 4 (300) 872 -> 768,
+//     2 x 8192, 32 / 8 (1024) 1470 -> 1246; 9563, 4 / 4 (300) 136 -> 139
+//   2 and 3 copies, >= 3 an SM: 28763, 8 / 2 (450) 576 -> 501, 19163, 6 / 3 (450) 303 -> 267; but 19163, 8 / 2 (300)
+//     547 -> 632, 32 / 2 2050 -> 2483, share-question, 12763, 12 / 3 (300) 1242 -> 1274
+//   1 copy, >= 4 an SM: 76763, 4 / 1 (600) 1493 -> 1221; but 57563, 4 / 1 (450) 797 -> 881
+//   rows of a unit: 8 x 900 documents, 8 / 8 (512) 145 -> 136; but 16 x 640, 16 / 16 (1280) 264 -> 262, 64 x 256, 16 / 16 304 -> 320,
+//     64 x 200, 16 / 4 250 -> 261
+//   accumulator in L2, or rows that reuse it: 12 x 520, 32 / 8 (126 MB) 317 -> 304; but 64 x 512, 16 / 4 (268 MB) 591 -> 614
+// Without a mask units are even, and the two kernels walk no tables:
+//   G >= 4, any length: 64 x 100, 32 / 8 causal 238 -> 225, 40 x 64, 64 / 8 211 -> 185; 4800, 32 / 8 949 -> 865
+//   G < 4: 8 x 1280, 16 / 16 causal (1280) 370 -> 349; but 64 x 256, 16 / 16 330 -> 337
+//   G = 1 in less than three waves, where the last is nearly empty: 2432, 16 / 16 (304) 173 -> 171; but 5 x 1000, 8 / 8 (320)
+//     104 -> 114, 4 x 1280, 8 / 8 (320) 117 -> 125
+static bool one_kernel_pays(const fm_attn_args* a) {
+  if (a->Hkv <= 0 || a->Sk <= 0 || a->Hq < a->Hkv) return false;
+  const int64_t copies = (int64_t)a->Hkv * a->B, units = copies * ((a->Sk + 127) / 128), sms = sm_count();
+  const int64_t G = a->Hq / a->Hkv, rows = G * a->Sq;
+  if (a->ncols == 0) return units >= 2 * sms && (G >= 4 || (rows >= 896 && (G >= 2 || a->Sq >= 2048 || units >= 3 * sms)));
+  return units >= (copies >= 4 ? 2 : copies >= 2 ? 3 : 4) * sms && rows >= 896 &&
+         (a->Sq >= 896 || bwd_sm100_fused_accum_bytes(a) <= (size_t)126000000);
+}
 // By geometry and options alone: what the workspace is sized for.
 static BwdKernels bwd_kernels_by_geometry(const fm_attn_args* a) {
   if (bwd_uses_sm100(a->d, a->dv)) {
-    const bool one = bwd_fills_boxes(a) || (a->d == a->dv && a->d > 64 && (int64_t)((a->Sk + 127) / 128) * a->Hkv * a->B >= 2 * sm_count());
+    const bool one = bwd_fills_boxes(a) || (a->d == a->dv && a->d > 64 && one_kernel_pays(a));
     return one && !a->deterministic && !g_opt.bwd_split ? BWD_ONE_KERNEL : BWD_TWO_KERNELS;
   }
   return pair_dims(a->d, a->dv) && !g_opt.bwd_mma && bwd_pair_supported(a) ? BWD_PAIR : BWD_WARP_MMA;

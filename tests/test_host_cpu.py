@@ -173,6 +173,39 @@ def test_least_workspace_of_the_backward():
         assert n - least == (0 if d < 256 else 4 << 28)         # (P and dS of four groups, 256 MiB each)
 
 
+@pytest.mark.parametrize("one,B,S,Hq,Hkv,ncols", [
+    # (without a GPU the library counts 148 multiprocessors)
+    (1, 2, 8192, 32, 8, 1), (1, 1, 4800, 32, 8, 1), (1, 8, 517, 16, 8, 2), (0, 1, 4600, 32, 8, 1),   # two units each
+    (0, 1, 19163, 32, 2, 1), (1, 1, 28763, 32, 2, 2), (0, 1, 12763, 12, 3, 1), (1, 1, 19163, 6, 3, 1),    # few copies
+    (0, 1, 57563, 4, 1, 4), (1, 1, 76763, 4, 1, 1),
+    (0, 16, 640, 16, 16, 1), (1, 8, 900, 8, 8, 1), (0, 64, 200, 16, 4, 1),                              # short units
+    (0, 64, 512, 16, 4, 1), (1, 12, 520, 32, 8, 1), (1, 20, 900, 16, 16, 1),                            # accumulator in L2
+    (1, 64, 100, 32, 8, 0), (0, 64, 256, 16, 16, 0), (1, 1, 19000, 32, 2, 0), (0, 1, 18800, 32, 2, 0),  # no mask
+    (0, 5, 1000, 8, 8, 0), (1, 8, 1280, 16, 16, 0), (1, 1, 2432, 16, 16, 0), (1, 8, 517, 16, 8, 0)])
+@pytest.mark.parametrize("d", [72, 96, 120])
+def test_which_backward_serves_head_dims_between_64_and_128(d, one, B, S, Hq, Hkv, ncols):
+    """Either side of every line of the rule: only the one-kernel backward asks for an accumulator."""
+    lib = _lib.load()
+    a = _lib.AttnArgs()
+    a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.Hm, a.mask_B, a.ncols, a.d, a.dv = B, S, S, Hq, Hkv, 1, B, ncols, d, d
+    rows = B * Hq * -(-S // 128) * 128
+    sizes = lambda: (lib.fm_bwd_workspace_bytes(ctypes.byref(a)), lib.fm_bwd_min_workspace_bytes(ctypes.byref(a)))
+    assert sizes() == (rows * (552 if one else 8), rows * 8)
+    assert lib.fm_bwd_accumulates(ctypes.byref(a)) == 0
+    a.deterministic = 1
+    assert sizes() == (rows * 8, rows * 8)
+    a.deterministic, a.dv = 0, d - 8                              # unequal head dims: two kernels
+    assert sizes() == (rows * 8, rows * 8)
+
+
+@pytest.mark.parametrize("d", [96, 128])
+def test_size_queries_of_impossible_heads(d):
+    for Hq, Hkv, Sk in ((4, 0, 512), (0, 4, 512), (4, -1, 512), (4, 4, 0)):
+        a = _lib.AttnArgs()
+        a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.Hm, a.mask_B, a.d, a.dv = 1, 4096, Sk, Hq, Hkv, 1, 1, d, d
+        assert _lib.load().fm_bwd_workspace_bytes(ctypes.byref(a)) <= (8 + 32 + 512) * 4 * 4096
+
+
 def test_struct_layout_matches_header():
     # 18 int32/float + 15 pointers/size_t + 24 int64
     assert ctypes.sizeof(_lib.AttnArgs) == 18 * 4 + 15 * 8 + 24 * 8 + 3 * 8
