@@ -498,7 +498,7 @@ static size_t bwd_row_stat_bytes(const fm_attn_args* a) {
   return (2 * rows * sizeof(float) + 255) & ~(size_t)255;
 }
 
-// One-kernel backward: the statistics once more as GEMM operands (three bf16 parts each), 2 x 16 bytes per row.
+// One-kernel backward: the statistics once more as GEMM operands (bf16 parts), 2 x 16 bytes per row.
 static size_t bwd_stat_operand_bytes(const fm_attn_args* a) {
   return (size_t)a->B * a->Hq * round_up(a->Sq, 128) * 32;
 }

@@ -11,8 +11,8 @@ struct AttnKParams {
   float* dpsum;     // [B,Hq,Sq_r] fp32 workspace: rowsum(O * dO)
   float* lse_log2;  // [B,Hq,Sq_r] fp32 workspace: LSE * log2(e), -inf -> 0
   float* dq_accum;  // [B,Hq,Sq_r,64|128] fp32 workspace (one-kernel backward: dQ summed by reductions)
-  // one-kernel backward only: the row statistics as bf16 GEMM operands, [B,Hq,Sq_r,8] each: three parts that sum to
-  // -c, c = LSE*log2e / scale_log2, and to -d, d = rowsum(O dO), then five zeros
+  // one-kernel backward only: the row statistics as bf16 GEMM operands, [B,Hq,Sq_r,8] each: parts that sum to
+  // -c, c = LSE*log2e / scale_log2 (four), and to -d, d = rowsum(O dO) (three), then zeros
   uint16_t* stat_s; uint16_t* stat_dp;
   void* pair_ws;    // CTA-pair backward: workspace of P, dS and fp32 sums (nullptr: that variant is not used)
   size_t pair_ws_bytes;

@@ -50,11 +50,11 @@ struct BwdFusedCfg {
   static constexpr int OFF_RING = OFF_STAT + 2 * TILE_BYTES;
   static constexpr int OFF_DS = OFF_RING + NSLOT * SLOT_BYTES;          // one buffer per item parity
   // STAT: the per-query statistics enter through the GEMMs.  S^T = K Q^T gets one more k-step whose A is a
-  // tile of ones and whose B holds, per query, the three parts of -c (0 in the other columns), c = LSE*log2e / scale_log2:
-  // the accumulator then already holds S - c, and P = exp2(scale_log2 * (S - c)) needs no per-column value in the
+  // tile of ones and whose B holds, per query, -c in parts (0 in the other columns), c = LSE*log2e / scale_log2: the
+  // accumulator then already holds S - c, and P = exp2(scale_log2 * (S - c)) needs no per-column value in the
   // compute warps.  dP^T = V dO^T likewise gets -d, d = rowsum(O dO).  The parts are bf16 whatever the type of the call
   // (A and B of one MMA share a type, MMAs into one accumulator need not): three of them carry the 24 bits and the range
-  // of the fp32 value.  Both operands are K-major without swizzle: 8-row x 16-byte core matrices; the second half of K
+  // of an fp32 value, a fourth the remainder of c's division.  Both operands are K-major without swizzle: 8-row x 16-byte core matrices; the second half of K
   // (columns 8..15) of A reads the ones again, that of B a block of zeros.
   static constexpr int OFF_AUX = OFF_DS + 2 * DS_BYTES;                 // per ring slot: S statistics, dP statistics
   static constexpr int OFF_ONES = OFF_AUX + NSLOT * AUX_BYTES;          // 17 core matrices of ones (2176 bytes)
