@@ -141,11 +141,11 @@ std::pair<Tensor, Tensor> kv_rows(const Tensor& k, const Tensor& v) {
   return {rows(k), rows(v)};
 }
 
-// Workspace of a backward call.  When the device has no room for what the call asks for (2 GiB and more at the head dims
-// 256, 512 and 576) it gets less, down to what it cannot do without.
+// Workspace of a backward call.  When the device has no room for what the call asks for it gets less: by quarters at the
+// head dims 256, 512 and 576 (2 GiB and more, used in chunks of any size), else what it cannot do without at once.
 Tensor bwd_workspace(fm_attn_args* a, const Tensor& like) {
   const size_t least = fm_bwd_min_workspace_bytes(a);
-  for (size_t n = fm_bwd_workspace_bytes(a);; n = std::max(least, n / 4)) {
+  for (size_t n = fm_bwd_workspace_bytes(a);; n = a->d >= 256 ? std::max(least, n / 4) : least) {
     try {
       Tensor ws = at::empty({(int64_t)std::max<size_t>(n, 256)}, like.options().dtype(at::kByte));
       a->workspace = ws.data_ptr();

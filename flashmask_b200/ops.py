@@ -276,8 +276,9 @@ def _flash_attn_fwd(q, k, v, startend_row_indices=None, softmax_scale=None, caus
 
 
 def _bwd_workspace(a: "_lib.AttnArgs", device) -> torch.Tensor:
-    """Workspace of a backward call, set in ``a``.  When the device has no room for what the call asks for (2 GiB and
-    more at the head dims 256, 512 and 576) it gets less, down to what it cannot do without."""
+    """Workspace of a backward call, set in ``a``.  When the device has no room for what the call asks for it gets less: by
+    quarters at the head dims 256, 512 and 576 (2 GiB and more, used in chunks of any size), else what it cannot do
+    without at once."""
     lib = _lib.load()
     n, least = lib.fm_bwd_workspace_bytes(C.byref(a)), lib.fm_bwd_min_workspace_bytes(C.byref(a))
     while True:
@@ -286,7 +287,7 @@ def _bwd_workspace(a: "_lib.AttnArgs", device) -> torch.Tensor:
         except torch.OutOfMemoryError:
             if n <= least:
                 raise
-            n = max(least, n // 4)
+            n = max(least, n // 4) if a.d >= 256 else least
             continue
         a.workspace, a.workspace_bytes = ws.data_ptr(), n
         return ws

@@ -267,6 +267,35 @@ def test_backward_when_memory_is_short():
     assert _kernel_status() == 0
 
 
+def test_backward_without_room_for_its_accumulator():
+    """Between the head dims 64 and 128 a backward that gets no room for the accumulator runs the two kernels, and holds
+    no more memory than they use."""
+    B, S, Hq, Hkv, d = 2, 8192, 16, 8, 96
+    q, k, v, do, _ = (t if t is None else t.cuda() for t in make_inputs(B, S, S, Hq, Hkv, d, d, 58))
+    x = [t.requires_grad_(True) for t in (q, k, v)]
+    want = torch.autograd.grad(fm.flashmask_attention(*x, causal=True, deterministic=True), x, do)
+    out, lse = fm.flashmask_attention(*x, causal=True, return_lse=True, deterministic=False)
+    native = lambda: torch.autograd.grad(out, x, do, retain_graph=True)
+    py = lambda: fm._flash_attn_bwd(q.detach(), k.detach(), v.detach(), out.detach(), do, lse, causal=True)[:3]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    rows, results = B * Hq * S, sum(t.numel() * 2 for t in x)
+    assert rows * 552 > 128 << 20
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + results + (100 << 20)) / total)
+    try:
+        for call in (native, py):
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            got = call()
+            assert torch.cuda.max_memory_allocated() - before <= results + 8 * rows + (1 << 20)
+            assert all(torch.equal(g_, w_) for g_, w_ in zip(got, want))
+            del got
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("d,dv", [(512, 512), (576, 512)])
 @pytest.mark.parametrize("kind", ["causal_doc", "none_full", "four_column"])
 def test_short_sequences_of_the_widest_heads(kind, d, dv):
