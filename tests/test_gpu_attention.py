@@ -447,6 +447,44 @@ def test_one_kernel_backward_between_64_and_128(d, kind):
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Sq,Sk,Hq,Hkv", [(517, 517, 16, 8), (330, 645, 32, 8)])
+@pytest.mark.parametrize("d", [72, 88, 96, 112, 120])
+def test_one_kernel_backward_between_64_and_128_walks_units(d, Sq, Sk, Hq, Hkv, dtype, monkeypatch):
+    """The same with launch tables, as masked calls of both hosts run it: a CTA takes several of 320 or 384 units, some of
+    them empty, over accumulators as wide as the head.  dK and dV are bitwise those of one unit per CTA; nothing of the
+    workspace reaches a result that the call has not written."""
+    B = 8
+    idx_np, causal = _mask("causal_doc", B, Sq, Sk, 63)
+    idx_np = idx_np.copy()
+    idx_np[1::2, :, 128:256, 0] = np.clip(np.arange(128, 256) - (Sk - Sq), 0, Sq)    # a key tile that no query sees
+    idx = torch.from_numpy(np.ascontiguousarray(idx_np)).cuda()
+    q, k, v, do, s = make_inputs(B, Sq, Sk, Hq, Hkv, d, d, 63, dtype=dtype, sink=True)
+    dev = [t.cuda() for t in (q, k, v, do)]
+    sizes, plain = [], fm.ops._bwd_workspace
+
+    def workspace_of_nans(a, device):
+        ws = plain(a, device).fill_(255)
+        sizes.append(ws.numel())
+        return ws
+    got = run_product(*dev, idx, causal, s, deterministic=False)
+    assert_parity(got, run_oracle(q, k, v, do, idx, causal, s), naive_lowp(*dev, idx, causal, s))
+    monkeypatch.setattr(fm.ops, "_bwd_workspace", workspace_of_nans)
+    info = fm.prepare_mask(idx, Sq, causal, 128, 128)
+    py = fm._flash_attn_bwd(*dev[:3], got["out"], dev[3], got["lse"], idx, causal=causal, learnable_sink=s, mask_info=info)
+    assert sizes == [B * Hq * -(-Sq // 128) * 128 * 552]               # with the accumulator: the one kernel
+    assert any(t is not None for key, t in info.orders.items() if key[0] == _lib.FM_ORDER_BWD_DKDV)
+    alone = run_c_abi(*dev, idx, causal, s, deterministic=False)
+    for n, t in zip(("dq", "dk", "dv", "dsink"), py):
+        assert torch.isfinite(t).all()
+        if n != "dq":
+            assert torch.equal(t, got[n]) and torch.equal(t, alone[n]), n
+    # dQ: fp32 sums over six key tiles in any order, rounded to 16 bits once
+    u = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+    assert ((py[0].double() - got["dq"].double()).norm() <= u * got["dq"].double().norm())
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("what", ["row sums", "scores", "small scale"])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("d", [64, 96, 128])
@@ -756,6 +794,35 @@ def test_native_host_and_python_autograd_function_agree(kind, d, dv, B, Hq, Hkv,
     assert len(res[0]) == (5 if sink is None else 6)
     for a, b in zip(*res):
         assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
+    assert _kernel_status() == 0
+
+
+@pytest.mark.parametrize("kind,d,dv,B,S,Hq,Hkv,hm,tables", [
+    ("causal_doc", 64, 64, 2, 330, 4, 2, 1, 0),           # every CTA of every launch starts at once
+    ("causal_doc", 128, 128, 3, 1025, 8, 8, 1, 1),        # the backward's two tables
+    ("four_column", 96, 80, 2, 1100, 16, 2, 2, 1),        # all three, the launch of dK / dV is the short one
+    ("bidir_doc", 192, 128, 2, 1300, 16, 4, 1, 1)])       # the forward's
+def test_launch_tables_of_the_native_host(kind, d, dv, B, S, Hq, Hkv, hm, tables, monkeypatch):
+    """The tables that the native host builds on its own (FLASHMASK_B200_ORDER unset), either side of its rule: bitwise
+    the Python host, which always builds them."""
+    monkeypatch.delenv("FLASHMASK_B200_ORDER", raising=False)
+    idx_np, causal = _mask(kind, B, S, S, 102)
+    if hm > 1:
+        idx_np = np.concatenate([_mask(kind, B, S, S, 102 + h)[0] for h in range(hm)], axis=1)
+    idx = torch.from_numpy(np.ascontiguousarray(idx_np).copy()).cuda()
+    q, k, v, do, s = make_inputs(B, S, S, Hq, Hkv, d, dv, 102, sink=True)
+    dev = [t.cuda() for t in (q, k, v, do)]
+    lib = _lib.load()
+    with torch.no_grad():
+        before = lib.fm_launch_count()
+        fm.flashmask_attention(*dev[:3], idx, causal=causal)
+        assert lib.fm_launch_count() - before == 2 + tables      # scan of the mask, tables, forward
+    got = run_product(*dev, idx, causal, s, deterministic=True)
+    x = [t.detach().requires_grad_(True) for t in dev[:3]]
+    sk = s.cuda().requires_grad_(True)
+    out, lse = fm.FlashMaskFunc.apply(*x, idx, 1 / math.sqrt(d), causal, sk, True)
+    for t, n in zip((out, lse, *torch.autograd.grad(out, [*x, sk], dev[3])), ("out", "lse", "dq", "dk", "dv", "dsink")):
+        assert torch.equal(t.detach(), got[n]), n
     assert _kernel_status() == 0
 
 

@@ -159,3 +159,12 @@ def test_launch_order_bit_exact(Sq, Sk, mask_b, hm, monkeypatch):
     a.d = a.dv = 128
     a.ncols = 0
     assert lib.fm_launch_order_ints(C.byref(a), _lib.FM_ORDER_BWD_DKDV) == 0
+
+
+@pytest.mark.parametrize("Sq,Sk", [(33001, 16500), (66000, 66000), (131072, 131072)])
+def test_launch_order_of_many_units(Sq, Sk, monkeypatch):
+    """516 to 4096 units (the most a table takes): the ranks of more than 32 groups of 32 units, partial groups."""
+    all_masks = _masks
+    few = lambda *a: [m for m in all_masks(*a) if m[0] in ("causal_doc", "sliding_window", "share_question")]
+    monkeypatch.setitem(test_launch_order_bit_exact.__globals__, "_masks", few)
+    test_launch_order_bit_exact(Sq, Sk, 2, 2, monkeypatch)

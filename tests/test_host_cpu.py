@@ -206,6 +206,24 @@ def test_size_queries_of_impossible_heads(d):
         assert _lib.load().fm_bwd_workspace_bytes(ctypes.byref(a)) <= (8 + 32 + 512) * 4 * 4096
 
 
+@pytest.mark.parametrize("d,B,S,Hq,Hkv,ncols,want", [
+    # (without a GPU the library counts 148 multiprocessors; CTAs of the forward, dQ and dK / dV launch behind each call)
+    (64, 1, 1024, 2, 2, 1, (0, 0, 0)),       # 8, 16, 16
+    (128, 1, 1024, 37, 1, 1, (0, 1, 1)),     # 148, 296, 8
+    (128, 1, 1025, 37, 1, 2, (1, 1, 1)),     # 185
+    (96, 2, 1100, 8, 8, 1, (0, 0, 0)),       # 80, 144, 144
+    (96, 3, 1100, 8, 8, 1, (0, 1, 1)),       # 120, 216, 216
+    (128, 4, 8192, 32, 8, 0, (0, 0, 0)),     # no mask, no table
+    (192, 1, 8192, 32, 8, 1, (1, 0, 0)),     # the backward takes none
+    (256, 1, 8192, 32, 8, 1, (0, 0, 0))])
+def test_launch_tables_are_useful_where_ctas_queue(d, B, S, Hq, Hkv, ncols, want):
+    lib = _lib.load()
+    a = _lib.AttnArgs()
+    a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.Hm, a.mask_B, a.ncols, a.d, a.dv = B, S, S, Hq, Hkv, 1, B, ncols, d, min(d, 128 if d < 256 else d)
+    assert tuple(lib.fm_launch_order_useful(ctypes.byref(a), w) for w in range(3)) == want
+    assert lib.fm_launch_order_useful(None, 0) == 0
+
+
 def test_struct_layout_matches_header():
     # 18 int32/float + 15 pointers/size_t + 24 int64
     assert ctypes.sizeof(_lib.AttnArgs) == 18 * 4 + 15 * 8 + 24 * 8 + 3 * 8
