@@ -165,7 +165,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     mbar_init(bar(Cfg::B_QFULL + 0), 1); mbar_init(bar(Cfg::B_QFULL + 1), 1);
     for (int i = 0; i < Cfg::NSTAGE; ++i) { mbar_init(bar(Cfg::B_KVFULL + i), 1); mbar_init(bar(Cfg::B_KVEMPTY + i), 1); }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(bar(Cfg::B_SFULL + s), 1); mbar_init(bar(Cfg::B_PFULL + s), SPLIT ? 128 : 4); mbar_init(bar(Cfg::B_PPART + s), 4); mbar_init(bar(Cfg::B_ODONE + s), 1);
+      mbar_init(bar(Cfg::B_SFULL + s), 1); mbar_init(bar(Cfg::B_PFULL + s), 4); mbar_init(bar(Cfg::B_PPART + s), 4); mbar_init(bar(Cfg::B_ODONE + s), 1);
     }
     for (int i = 0; i < Cfg::NBND; ++i) { mbar_init(bar(Cfg::B_BNDFULL + i), 32); mbar_init(bar(Cfg::B_BNDEMPTY + i), 256); }
     fence_mbar_init();
@@ -356,12 +356,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           tc_wait_st();
         }
         tc_fence_before();
-        if constexpr (SPLIT) {
-          mbar_arrive(bar(Cfg::B_PFULL + s));
-        } else {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(Cfg::B_PFULL + s));
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(Cfg::B_PFULL + s));   // (an arrival per thread instead of per warp measured the same)
         ++n_done;
       }
       if (any_bounds) {
@@ -492,7 +488,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         constexpr uint32_t idesc_pv = make_idesc(IS_BF16, 128, DVS, 0, 1);
         // P V starts on the first 96 keys of a tile while the softmax still computes the last 32 (B_PPART): the wait for a
         // tile's P, P V and the next scores is one dependent chain per sub-tile, and this takes up to 384 of its cycles out.
-        // Dense 8192 x 2, 32 / 8 heads, d = 64: 1694 -> 1604 us; 32768 share-question, d = 128: 975 -> 930 us.  The split
+        // Dense 8192 x 2, 32 / 8 heads, d = 64: 1665 -> 1559 us; 32768 share-question, d = 128: 921 -> 907 us.  The split
         // variant, whose sub-tiles mostly take turns, lost 2 % by it and waits for the whole tile.
         constexpr int B_PFIRST = SPLIT ? Cfg::B_PFULL : Cfg::B_PPART;
         int npv[2] = {0, 0};
