@@ -208,27 +208,27 @@ static bool bwd_fills_boxes(const fm_attn_args* a) { return a->d == a->dv && (a-
 // Head dims between 64 and 128.  A unit of the one kernel is a key tile of a kv head with every q head of its group (G), and
 // does five GEMMs an item; the two kernels do seven, but spread three of them over the q heads.  So the one kernel needs
 // units that fill the chip evenly and rows enough in each to pay for its accumulator (512 bytes a query row, cleared, added
-// to and rounded).  Forward + backward in us, two kernels -> one, d = 96, (units);
-// Hkv * B copies of a key tile share the mask's heaviest columns:
-//   masks, 4 copies and more, units >= 2 an SM: 4800 documents 32 / 8 heads (304) 417 -> 369, 9500, 32 / 4 (300) 872 -> 768,
-//     2 x 8192, 32 / 8 (1024) 1470 -> 1246; 9563, 4 / 4 (300) 136 -> 139
-//   2 and 3 copies, >= 3 an SM: 28763, 8 / 2 (450) 576 -> 501, 19163, 6 / 3 (450) 303 -> 267; but 19163, 8 / 2 (300)
-//     547 -> 632, 32 / 2 2050 -> 2483, share-question, 12763, 12 / 3 (300) 1242 -> 1274
-//   1 copy, >= 4 an SM: 76763, 4 / 1 (600) 1493 -> 1221; but 57563, 4 / 1 (450) 797 -> 881
-//   rows of a unit: 8 x 900 documents, 8 / 8 (512) 145 -> 136; but 16 x 640, 16 / 16 (1280) 264 -> 262, 64 x 256, 16 / 16 304 -> 320,
-//     64 x 200, 16 / 4 250 -> 261
-//   accumulator in L2, or rows that reuse it: 12 x 520, 32 / 8 (126 MB) 317 -> 304; but 64 x 512, 16 / 4 (268 MB) 591 -> 614
+// to and rounded).  Forward + backward in us, two kernels -> one, d = 96 unless said, (units), inputs changing from pass to pass:
+//   masks.  A long document is a run of long units in every kv head that shares the mask ("copies"); with few copies and
+//   few units the chip waits for them, the more the wider the head:
+//     6 copies and more, 2 units an SM: 4800 documents, 32 / 8 heads 1.11x, 6363, 24 / 6 1.09x, 2432, 16 / 16 1.07x
+//     3 to 5, 2.5: 12763, 24 / 3 (372) 1.07x, d = 120, 48 / 3 (402) 1.01x; but 9563, 16 / 4 (300) d = 96 1.06x, 80 0.96x, 120 0.85x
+//     2, 3: 28763, 8 / 2 (450) 1.16x, d = 120 (500) 1.00x; but 25563 (400) d = 120 0.91x, 19163 (300) 543 -> 635, 32 / 2 2059 -> 2513
+//     1, 4: 76763, 4 / 1 (600) 1.23x; but 57563, 4 / 1 (450) 805 -> 928, 4 x 10000, 4 / 1 (316) 647 -> 773
+//   short rows: 5 x 1000, 8 / 8 1.07x; but 16 x 640, 16 / 16 264 -> 266, 64 x 256, 16 / 16 304 -> 319, 64 x 200, 16 / 4 250 -> 261
+//   and an accumulator past L2: 12 x 520, 32 / 8 (126 MB) 1.05x; but 64 x 512, 16 / 4 (268 MB) 614 -> 631
 // Without a mask units are even, and the two kernels walk no tables:
 //   G >= 4, any length: 64 x 100, 32 / 8 causal 238 -> 225, 40 x 64, 64 / 8 211 -> 185; 4800, 32 / 8 949 -> 865
-//   G < 4: 8 x 1280, 16 / 16 causal (1280) 370 -> 349; but 64 x 256, 16 / 16 330 -> 337
+//   G < 4: 8 x 1280, 16 / 16 causal (1280) 370 -> 349; but 64 x 256, 16 / 16 331 -> 336
 //   G = 1 in less than three waves, where the last is nearly empty: 2432, 16 / 16 (304) 173 -> 171; but 5 x 1000, 8 / 8 (320)
-//     104 -> 114, 4 x 1280, 8 / 8 (320) 117 -> 125
+//   114 -> 116, 4 x 1280, 8 / 8 (320) d = 120 135 -> 142
 static bool one_kernel_pays(const fm_attn_args* a) {
   if (a->Hkv <= 0 || a->Sk <= 0 || a->Hq < a->Hkv) return false;
-  const int64_t copies = (int64_t)a->Hkv * a->B, units = copies * ((a->Sk + 127) / 128), sms = sm_count();
+  const int64_t units = (int64_t)a->Hkv * a->B * ((a->Sk + 127) / 128), sms = sm_count();
   const int64_t G = a->Hq / a->Hkv, rows = G * a->Sq;
   if (a->ncols == 0) return units >= 2 * sms && (G >= 4 || (rows >= 896 && (G >= 2 || a->Sq >= 2048 || units >= 3 * sms)));
-  return units >= (copies >= 4 ? 2 : copies >= 2 ? 3 : 4) * sms && rows >= 896 &&
+  const int64_t copies = (int64_t)(a->Hm > 1 ? 1 : a->Hkv) * (a->mask_B == 1 ? a->B : 1);
+  return 2 * units >= (copies >= 6 ? 4 : copies >= 3 ? 5 : copies == 2 ? 6 : 8) * sms && rows >= 896 &&
          (a->Sq >= 896 || bwd_sm100_fused_accum_bytes(a) <= (size_t)126000000);
 }
 // By geometry and options alone: what the workspace is sized for.

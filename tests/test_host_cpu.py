@@ -177,7 +177,8 @@ def test_least_workspace_of_the_backward():
     # (without a GPU the library counts 148 multiprocessors)
     (1, 2, 8192, 32, 8, 1), (1, 1, 4800, 32, 8, 1), (1, 8, 517, 16, 8, 2), (0, 1, 4600, 32, 8, 1),   # two units each
     (0, 1, 19163, 32, 2, 1), (1, 1, 28763, 32, 2, 2), (0, 1, 12763, 12, 3, 1), (1, 1, 19163, 6, 3, 1),    # few copies
-    (0, 1, 57563, 4, 1, 4), (1, 1, 76763, 4, 1, 1),
+    (0, 1, 57563, 4, 1, 4), (1, 1, 76763, 4, 1, 1), (0, 1, 9563, 16, 4, 1), (1, 1, 11900, 16, 4, 1),
+    (0, 4, 10000, 4, 1, 1), (0, 4, 5000, 8, 2, 2),
     (0, 16, 640, 16, 16, 1), (1, 8, 900, 8, 8, 1), (0, 64, 200, 16, 4, 1),                              # short units
     (0, 64, 512, 16, 4, 1), (1, 12, 520, 32, 8, 1), (1, 20, 900, 16, 16, 1),                            # accumulator in L2
     (1, 64, 100, 32, 8, 0), (0, 64, 256, 16, 16, 0), (1, 1, 19000, 32, 2, 0), (0, 1, 18800, 32, 2, 0),  # no mask
@@ -196,6 +197,16 @@ def test_which_backward_serves_head_dims_between_64_and_128(d, one, B, S, Hq, Hk
     assert sizes() == (rows * 8, rows * 8)
     a.deterministic, a.dv = 0, d - 8                              # unequal head dims: two kernels
     assert sizes() == (rows * 8, rows * 8)
+
+
+def test_heads_and_batch_entries_that_share_a_mask_are_copies():
+    lib = _lib.load()
+    for one, Hm, mask_B in ((0, 1, 4), (1, 1, 1), (0, 2, 4), (0, 2, 1)):      # copies: 2, 8, 1, 4
+        a = _lib.AttnArgs()
+        a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.d, a.dv, a.ncols = 4, 5000, 5000, 8, 2, 96, 96, 2
+        a.Hm, a.mask_B = Hm, mask_B
+        n, least = lib.fm_bwd_workspace_bytes(ctypes.byref(a)), lib.fm_bwd_min_workspace_bytes(ctypes.byref(a))
+        assert (n > least) == bool(one), (Hm, mask_B)
 
 
 @pytest.mark.parametrize("d", [96, 128])
