@@ -86,7 +86,8 @@ def _launch_order(a: "_lib.AttnArgs", info: FlashMaskInfo, which: int, ref: torc
     variant, or None when the variant takes none.  The tables of all three kernels are built
     together on first use, once per FlashMaskInfo (ONE small launch on the current stream).
     FLASHMASK_B200_ORDER=0 turns all tables off, a comma list out of fwd,dq,dkdv keeps only
-    those (A/B runs)."""
+    those (A/B runs).  This host builds a table whatever the number of CTAs: a FlashMaskInfo is meant to serve many
+    calls."""
     sel = os.environ.get("FLASHMASK_B200_ORDER", "1")
     names = ("fwd", "dq", "dkdv")
     wanted = [w for w in range(3) if sel == "1" or names[w] in sel.split(",")]

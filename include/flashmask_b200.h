@@ -129,9 +129,10 @@ typedef struct fm_attn_args {
   int32_t deterministic;  /* backward only: 1 = fixed summation order, bitwise
                              reproducible gradients (two tcgen05 kernels, one
                              owner per output element); 0 = the one-kernel
-                             backward may be used (d = dv = 64 or 128), whose dQ
-                             is summed by reductions in an order that is not
-                             fixed                                            */
+                             backward may be used (d = dv from 64 to 128; between
+                             them where B, the heads, the lengths and ncols make
+                             it the faster one), whose dQ is summed by reductions
+                             in an order that is not fixed                    */
   int32_t bwd_flags;      /* backward only, one-kernel variant: FM_BWD_* bits below, 0 = a
                              self-contained call                               */
   float softmax_scale;
@@ -252,7 +253,8 @@ FM_API int fm_fwd_block_score(const fm_attn_args* args, float* block_logit, int 
 #define FM_ORDER_BWD_DKDV 2
 FM_API int64_t fm_launch_order_ints(const fm_attn_args* args, int which);
 /* 1 when the launch has more CTAs than the device has multiprocessors, so that their order matters (0: also when the
- * kernel takes none).  A host that skips a useless table passes NULL for it; results do not depend on tables. */
+ * kernel takes none).  The backward's two tables go together: 1 for both when either launch has more.  A host that skips
+ * a useless table passes NULL for it; results do not depend on tables. */
 FM_API int fm_launch_order_useful(const fm_attn_args* args, int which);
 FM_API int fm_launch_order(const fm_attn_args* args, int which, int32_t* out, void* stream);
 /* The same for up to three kernels in ONE launch (a NULL pointer skips that kernel's table). */
@@ -291,14 +293,16 @@ FM_API int fm_selftest_bounded_wait(int budget_us, void* stream);
  * args->deterministic the call will carry. */
 FM_API size_t fm_bwd_workspace_bytes(const fm_attn_args* args);
 /* The least workspace fm_bwd takes.  It is less than fm_bwd_workspace_bytes for
- * equal head dims between 64 and 128, where calls with many key tiles run the
- * one-kernel variant and, without room for its accumulator, the two-kernel one;
+ * equal head dims between 64 and 128, where some calls run the one-kernel variant
+ * (552 bytes per (batch, q head, query padded to 128)) and, without room for its
+ * accumulator, the two-kernel one (8 bytes);
  * and at the head dims 256, 512 and 576, where the fast kernels keep P and dS of a
  * chunk of the problem (2 GiB, more where 256 rows of all heads of a kv group
  * need more): with fewer bytes the chunks are smaller, and where not even the
- * smallest fits, other kernels serve that keep row statistics only.  Results are
- * bitwise reproducible for a given workspace size; another size sums dK and dV in
- * another order. */
+ * smallest fits, other kernels serve that keep row statistics only.  There results
+ * are bitwise reproducible for a given workspace size, and another size sums dK
+ * and dV in another order; at the smaller head dims what args->deterministic says
+ * holds, and less than the full size is the two-kernel variant. */
 FM_API size_t fm_bwd_min_workspace_bytes(const fm_attn_args* args);
 /* 1 when fm_bwd(args) would run the one-kernel variant and honours
  * args->bwd_flags (head dims 64 and 128, whatever the sizes), else 0.  Reads the
