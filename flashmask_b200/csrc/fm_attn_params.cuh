@@ -10,7 +10,7 @@ struct AttnKParams {
   const void* d_o; void* dq; void* dk; void* dv; float* dsink;
   float* dpsum;     // [B,Hq,Sq_r] fp32 workspace: rowsum(O * dO)
   float* lse_log2;  // [B,Hq,Sq_r] fp32 workspace: LSE * log2(e), -inf -> 0
-  float* dq_accum;  // [B,Hq,Sq_r,64|128] fp32 workspace (one-kernel backward: dQ summed by reductions)
+  float* dq_accum;  // [B,Hq,Sq_r/64,64 x (64|128)] fp32 workspace (one-kernel backward: dQ summed by reductions, in the order that bwd_dq_round_kernel names)
   // one-kernel backward only: the row statistics as bf16 GEMM operands, [B,Hq,Sq_r,8] each: parts that sum to
   // -c, c = LSE*log2e / scale_log2 (four), and to -d, d = rowsum(O dO) (three), then zeros
   uint16_t* stat_s; uint16_t* stat_dp;

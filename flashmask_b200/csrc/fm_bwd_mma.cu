@@ -435,10 +435,10 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const AttnKParams p
 #pragma unroll
   for (int o2 = LPR / 2; o2; o2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o2);
   if (p.dq_accum && !(p.bwd_flags & FM_BWD_DQ_CARRY) && row < p.Sq_r) {
-    // one-kernel backward: this row of the fp32 dQ accumulator starts at zero (the lanes of the row share it), up to the
-    // last box of 32 columns that the kernel adds to
+    // one-kernel backward: the fp32 dQ accumulator starts at zero.  The columns in use of a block of 64 rows, in groups of 32
+    // as the kernel adds to them, are the first 64 * used floats of the block; a row (its lanes together) clears a 64th of them.
     const int dacc = (p.d <= 64 && p.dv_dim <= 64) ? 64 : 128, used = (p.d + 31) & ~31;
-    float4* z = reinterpret_cast<float4*>(p.dq_accum + (((int64_t)b * p.Hq + hq) * p.Sq_r + row) * dacc);
+    float4* z = reinterpret_cast<float4*>(p.dq_accum + (((int64_t)b * p.Hq + hq) * p.Sq_r + (row & ~63)) * dacc + (row & 63) * used);
     for (int c = ln; c < used / 4; c += LPR) z[c] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (ln == 0 && row < p.Sq_r) {

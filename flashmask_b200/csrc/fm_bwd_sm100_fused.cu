@@ -9,22 +9,27 @@
 //     dP^T = V dO^T             M=128, N=64
 //     P^T  = exp2(S^T scale - LSE), dS^T = P^T (dP^T - rowsum(O dO))   (compute warpgroups)
 //     dV  += P^T dO             A = P^T from TMEM (bf16)
-//     dK  += dS^T Q             A = dS^T from shared memory (K-major)
+//     dK  += dS^T Q             A = dS^T from TMEM
 //     dQ^T = K^T dS^T           M=128 head-dim columns, N=64 queries; A = the K tile read
-//                               MN-major, B = the same dS^T buffer read MN-major
+//                               MN-major, B = dS^T once more, from shared memory, read MN-major
 // dK / dV stay in TMEM for the whole unit and are written once.  dQ^T of an item is drained
-// by a fourth warpgroup and added to an fp32 accumulator in global memory with coalesced
-// reductions (a warp covers 32 consecutive floats of one query row); a small kernel rounds
-// the accumulator to the output type afterwards.  The order of those additions is not
-// fixed, so this kernel serves calls that did not ask for deterministic gradients; the
-// two-kernel variant (fm_bwd_sm100_persist.cu) has one owner per output element.
+// by a fourth warpgroup and added to an fp32 accumulator in global memory by bulk
+// reductions; a small kernel rounds the accumulator to the output type afterwards.  The
+// order of those additions is not fixed, so this kernel serves calls that did not ask for
+// deterministic gradients; the two-kernel variant (fm_bwd_sm100_persist.cu) has one owner per
+// output element.
 //
-// TMEM columns: S^T [0,64), dP^T [64,128) (one pair: an item's scores are in registers
-// before the next item's score GEMMs are issued), P^T of item parity p [128+32p, +32),
-// dQ^T [192,256), dV [256,384), dK [384,512).
+// TMEM columns.  S^T has a buffer per item parity p at [64p, +64); once an item's scores are in
+// registers its P^T and dS^T (16 bits) lie over it at +0 and +32 and are the A operands of dV and dK.
+//   128-column variant: dP^T [128,192) (one buffer), dQ^T [192,256), dV [256,384), dK [384,512).
+//   64-column variant: dP^T [128+64p, +64), dQ^T [256,320), dV [320,384), dK [384,448), and K and V
+//   of the unit, copied there once, at [448,480) and [480,512): A operands of S^T and dP^T.  An MMA of N = 64
+//   with A in shared memory reads 192 bytes per clock of a pipe that has 128, with A in TMEM 64.
+// 2 x 8192 documents, 32 / 8 heads, this kernel alone: d = 64 622 -> 536 us, d = 128 815 -> 776, d = 96 731 -> 690, against one
+// buffer each for S^T and dP^T, P^T in columns of its own and dS^T read from shared memory.
 //
 // Warp roles: 0-3 / 4-7 compute warpgroups (items alternate), 8 TMA producer, 9 UMMA issuer
-// (owns TMEM), 10 scheduler + list builder, 11 idle, 12-15 dQ reduction + dK/dV epilogue.
+// (owns TMEM), 10 scheduler + list builder, 11 second UMMA issuer (128 columns), 12-15 dQ reduction + dK/dV epilogue.
 // All waits are bounded.
 #include <algorithm>
 
@@ -37,12 +42,15 @@ using namespace sm100;
 
 __device__ int g_bwd_fused_status = 0;
 
+template <int D>
 struct BwdFusedCfg {
-  static constexpr int NSLOT = 3, LIST_MAX = 2048, NTHREADS = 512;
-  static constexpr int TILE_BYTES = 128 * 128 * 2;     // 128 rows x 128 cols bf16
+  // (a slot is taken for about 6000 cycles, a load's 1000 to 2000 among them: with three the 64-column variant waited for Q and
+  // dO, 603 instead of 554 us on 2 x 8192 documents, 32 / 8 heads; the 128-column one has no room for a fourth)
+  static constexpr int NSLOT = D == 64 ? 6 : 3, LIST_MAX = 2048, NTHREADS = 512;
+  static constexpr int TILE_BYTES = 128 * D * 2;       // 128 rows x D cols bf16
   static constexpr int SUB128 = 128 * 128;             // 128-row x 64-col sub-tile (bytes)
   static constexpr int SUB64 = 64 * 128;               // 64-row x 64-col sub-tile (bytes)
-  static constexpr int HALF_BYTES = 2 * SUB64;         // one operand of a half tile
+  static constexpr int HALF_BYTES = D / 64 * SUB64;    // one operand of a half tile
   static constexpr int SLOT_BYTES = 2 * HALF_BYTES;    // Q half + dO half
   static constexpr int DS_BYTES = 128 * 128;           // dS^T: 128 keys x 64 queries bf16
   static constexpr int AUX_BYTES = 2048;               // two 64-row x 16-byte statistics operands (see STAT below)
@@ -62,23 +70,25 @@ struct BwdFusedCfg {
   static constexpr int OFF_LIST = OFF_ZEROS + 1024;                     // two lists of 16-bit entries: units alternate
   static constexpr int OFF_STAGE = OFF_LIST + 2 * LIST_MAX * 2;         // reductions of the unit's K tile (8 x 4 ints)
   static constexpr int EPI_BYTES = 32 * 64;                             // per epilogue warp: 32 rows x 32 bf16 columns
-  static constexpr int RROWS = 16;                                      // dQ staging: 16 query rows x 32 floats per buffer,
-  static constexpr int RBUF_BYTES = RROWS * 32 * 4;                     // two buffers per warp of the reduction warpgroup
-  static constexpr int OFF_EPI = OFF_STAGE + 128;                       // dQ staging; the dK/dV epilogue reuses it
-  static constexpr int OFF_INFO = OFF_EPI + 4 * 2 * RBUF_BYTES;         // two unit records of 8 ints
+  static constexpr int RROWS = D == 64 ? 64 : 32;                       // dQ staging: query rows x 32 columns per buffer,
+  static constexpr int RBUF_BYTES = RROWS * 32 * 4, RBUFS = D == 64 ? 2 : 1;   // and buffers per warp that has dQ columns
+  static constexpr int OFF_EPI = OFF_STAGE + 128;                       // dQ staging; at 128 the dK/dV epilogue reuses it
+  static constexpr int OFF_EPI2 = D == 64 ? OFF_EPI + 2 * RBUFS * RBUF_BYTES : OFF_EPI;
+  static constexpr int EPI_STEP = D == 64 ? EPI_BYTES : RBUFS * RBUF_BYTES;
+  static constexpr int OFF_INFO = OFF_EPI2 + 4 * EPI_STEP;              // two unit records of 8 ints
   static constexpr int OFF_BAR = OFF_INFO + 2 * 8 * 4;
-  static constexpr int OFF_MISC = OFF_BAR + 32 * 8;
+  static constexpr int OFF_MISC = OFF_BAR + 40 * 8;
   static constexpr int SMEM = OFF_MISC + 64 + 1024;
   // item-level barriers (phases follow the CTA-wide item counter) ...
   static constexpr int B_RFULL = 0, B_REMPTY = NSLOT, B_GFULL = 2 * NSLOT, B_TFULL = B_GFULL + 2,
-                       B_DSFREE = B_TFULL + 2, B_SREAD = B_DSFREE + 2, B_DQFULL = B_SREAD + 1,
+                       B_DSFREE = B_TFULL + 2, B_SREAD = B_DSFREE + 2, B_PFREE = B_SREAD + 2, B_DQFULL = B_PFREE + 2,
                        B_DQFREE = B_DQFULL + 1;
   // ... and unit-level ones (phases follow the unit counter of the CTA)
   static constexpr int B_STAT = B_DQFREE + 1, B_VFREE = B_STAT + 1, B_KFREE = B_VFREE + 1, B_ACC = B_KFREE + 1,
                        B_ACCFREE = B_ACC + 1, B_INFOREADY = B_ACCFREE + 1, B_INFOFREE = B_INFOREADY + 2,
-                       B_COORD = B_INFOFREE + 2, B_FETCHGO = B_COORD + 2, B_COUNT = B_FETCHGO + 1;
+                       B_COORD = B_INFOFREE + 2, B_FETCHGO = B_COORD + 2, B_KVT = B_FETCHGO + 1, B_COUNT = B_KVT + 1;
   static constexpr int FETCH_AHEAD = 16;   // items left in a unit when the next one is claimed
-  static_assert(B_COUNT <= 32, "barrier storage");
+  static_assert(B_COUNT <= 40, "barrier storage");
   static_assert(RBUF_BYTES >= EPI_BYTES && OFF_EPI % 128 == 0, "epilogue staging fits the dQ staging");
   static_assert(OFF_RING % 1024 == 0 && OFF_DS % 1024 == 0 && SLOT_BYTES % 1024 == 0, "swizzled tiles are 1 KB aligned");
   static_assert(SMEM > 120 * 1024 && SMEM <= 227 * 1024, "one CTA per SM (512 TMEM columns)");
@@ -119,36 +129,17 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
-// Tiled reduction shared -> global through a 2-D tensor map: the box at (x, y) of the fp32 tensor gets
-// the staged box added to it by the copy engine; completion is tracked by this thread's bulk groups.
-__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* tmap, uint32_t src_smem, int x, int y) {
-  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(src_smem), "r"(x), "r"(y)
+// Reduction shared -> global: `bytes` of fp32 values at dst get the staged ones added to them by the copy engine; completion
+// is tracked by this thread's bulk groups.
+__device__ __forceinline__ void bulk_reduce_add(float* dst, uint32_t src_smem, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
+               ::"l"(dst), "r"(src_smem), "r"(bytes)
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
-// Four k-steps (K = 64) of D[tmem] (+)= A[smem] * B[smem]: A K-major (advances 32 bytes per
-// step inside its 128-byte rows), B MN-major (advances 16 rows = 2048 bytes per step).
-__device__ __forceinline__ void umma_ss_k_mn_x4(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                                uint32_t acc_first) {
-  asm volatile(
-      "{\n\t.reg .pred p, pt;\n\t.reg .b64 ta, tb;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.eq.b32 pt, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "add.s64 ta, %1, 2;  add.s64 tb, %2, 128;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], ta, tb, %3, pt;\n\t"
-      "add.s64 ta, %1, 4;  add.s64 tb, %2, 256;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], ta, tb, %3, pt;\n\t"
-      "add.s64 ta, %1, 6;  add.s64 tb, %2, 384;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], ta, tb, %3, pt;\n\t}"
-      ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc_first)
-      : "memory");
-}
 
 // Eight k-steps (K = 128) of D[tmem] = A[smem] * B[smem], both operands MN-major: each step
 // advances both by 16 rows (2048 bytes).
@@ -176,15 +167,15 @@ __device__ __forceinline__ void umma_ss_mn_mn_x8(uint32_t d_tmem, uint64_t a, ui
       : "memory");
 }
 
-// D: width the head dims are computed at (64 when both fit, else 128); the 64-column variant
-// keeps the shared-memory layout and leaves the second 64-column sub-tile of every operand
-// unloaded (the dQ^T GEMM then fills TMEM lanes 64..127 from unloaded memory; nothing reads them).
+// D: width the head dims are computed at (64 when both fit, else 128).  In the 64-column variant the A operand of
+// dQ^T (M = 128 head-dim columns) goes on into the V tile behind K; TMEM lanes 64..127 of dQ^T hold products nobody reads.
 template <bool IS_BF16, int D>
 __global__ void __launch_bounds__(512, 1)
 bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                        const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
-                       const __grid_constant__ CUtensorMap tm_dq, const AttnKParams p) {
-  using Cfg = BwdFusedCfg;
+                       const AttnKParams p) {
+  using Cfg = BwdFusedCfg<D>;
+  constexpr bool KV_T = D == 64;               // K and V are copied to tensor memory, and one thread issues all GEMMs
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
@@ -200,7 +191,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   const int lane = tid & 31;
   if (warp == 8 && lane == 0) {
     tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v);
-    tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_do); tma_prefetch_desc(&tm_dq);
+    tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_do);
   }
   const MaskDesc& md = p.md;
   const int off = p.Sk - p.Sq;
@@ -220,10 +211,11 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     for (int i = 0; i < Cfg::NSLOT; ++i) { mbar_init(bar(Cfg::B_RFULL + i), 1); mbar_init(bar(Cfg::B_REMPTY + i), 1); }
     for (int h = 0; h < 2; ++h) {
       mbar_init(bar(Cfg::B_GFULL + h), 1); mbar_init(bar(Cfg::B_TFULL + h), 4); mbar_init(bar(Cfg::B_DSFREE + h), 1);
-      mbar_init(bar(Cfg::B_INFOREADY + h), 1); mbar_init(bar(Cfg::B_INFOFREE + h), 15);
+      mbar_init(bar(Cfg::B_INFOREADY + h), 1); mbar_init(bar(Cfg::B_INFOFREE + h), KV_T ? 14 : 15);
       mbar_init(bar(Cfg::B_COORD + h), 1);
+      mbar_init(bar(Cfg::B_SREAD + h), 4); mbar_init(bar(Cfg::B_PFREE + h), 1);
     }
-    mbar_init(bar(Cfg::B_SREAD), 4); mbar_init(bar(Cfg::B_DQFULL), 1); mbar_init(bar(Cfg::B_DQFREE), 4);
+    mbar_init(bar(Cfg::B_KVT), 8); mbar_init(bar(Cfg::B_DQFULL), 1); mbar_init(bar(Cfg::B_DQFREE), 4);
     mbar_init(bar(Cfg::B_FETCHGO), 1);
     mbar_init(bar(Cfg::B_STAT), 1); mbar_init(bar(Cfg::B_VFREE), 1); mbar_init(bar(Cfg::B_KFREE), 1);
     mbar_init(bar(Cfg::B_ACC), 1); mbar_init(bar(Cfg::B_ACCFREE), 4);
@@ -238,11 +230,13 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   tc_fence_after();
   const uint32_t tmem = (uint32_t)misc[0];
   WaitCtx wc{misc + 4, global_timer_ns() + 2000000000ull};
-  constexpr uint32_t C_S = 0, C_DP = 64, C_P = 128, C_DQ = 192, C_DV = 256, C_DK = 384;
+  // S^T of item parity p at C_S + 64 p, its P^T and dS^T over it at +0 and +32; dP^T at C_DP (D = 64: + 64 p)
+  constexpr uint32_t C_S = 0, C_DP = 128, DP_STEP = KV_T ? 64 : 0, C_DQ = KV_T ? 256 : 192, C_DV = KV_T ? 320 : 256,
+                     C_DK = 384, C_K = 448, C_V = 480;
 
-  // 512 threads start with 128 registers each; the compute warpgroups take what the others give up
-  if (warp < 8) setmaxnreg_inc<168>();
-  else if (warp < 12) setmaxnreg_dec<80>();
+  // 512 threads start with 128 registers each; the compute warpgroups take what the others give up.  (168 / 80 / 96 left
+  // the 128-column variant with spills: 806 instead of 776 us.)
+  if (warp < 8) setmaxnreg_inc<160>();
   else setmaxnreg_dec<96>();
 
   if (warp == 10) {
@@ -328,8 +322,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     const int wg = warp >> 2;
     const int r = tid & 127;                     // TMEM lane = key row0 + r
     const uint32_t lane_field = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tS = tmem + lane_field + C_S, tDP = tmem + lane_field + C_DP;
-    const uint32_t tP = tmem + lane_field + C_P + 32u * (uint32_t)wg;
+    const uint32_t tS = tmem + lane_field + C_S + 64u * (uint32_t)wg, tDP = tmem + lane_field + C_DP + DP_STEP * (uint32_t)wg;
     uint8_t* dsrow = smem + Cfg::OFF_DS + wg * Cfg::DS_BYTES + r * 128;
     const float scale_log2 = p.scale_log2;
     bool ok = true;
@@ -356,7 +349,29 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(Cfg::B_INFOFREE + s));
+        if constexpr (KV_T) {
+          // (every phase of the barrier is waited for, or the next wait would take this one for its own)
+          ok = __all_sync(0xffffffffu, mbar_wait_parked(bar(Cfg::B_STAT), (uint32_t)j & 1u, wc));
+        }
         continue;
+      }
+      if constexpr (KV_T) {
+        // K (warpgroup 0) and V (warpgroup 1) of the unit: row r of the tile to lane r of the tensor memory.  The score GEMMs of the
+        // previous unit are done with theirs: the tiles that have landed were only requested after its last dQ^T GEMM.
+        ok = __all_sync(0xffffffffu, mbar_wait_parked(bar(Cfg::B_STAT), (uint32_t)j & 1u, wc));
+        if (!ok) break;
+        const uint8_t* src = smem + Cfg::OFF_STAT + wg * Cfg::TILE_BYTES + r * 128;
+        uint32_t kv[32];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint4 v = *reinterpret_cast<const uint4*>(src + ((c ^ (r & 7)) << 4));
+          kv[4 * c] = v.x; kv[4 * c + 1] = v.y; kv[4 * c + 2] = v.z; kv[4 * c + 3] = v.w;
+        }
+        tmem_st32(tmem + lane_field + (wg == 0 ? C_K : C_V), kv);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(Cfg::B_KVT));
       }
       // bounds of this lane's key for the whole unit
       int lts = INT_MAX, lte = INT_MAX, uts = 0, ute = 0;
@@ -374,26 +389,27 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         const uint32_t e = list[k % cnt];
         const int idx = (int)(e & 0xFFFu);
         const uint32_t flags = e >> 12;
+        // dS^T of this parity in shared memory is free once the dQ^T GEMM of item kk-2 has completed.  (Waited for here, where
+        // the scores are awaited anyway: under the operand reads of the GEMMs even a wait that is over costs 500 cycles.)
+        if (kk >= 2) {
+          ok = __all_sync(0xffffffffu, mbar_wait_parked(bar(Cfg::B_DSFREE + wg), (uint32_t)((kk >> 1) - 1) & 1u, wc));
+          if (!ok) break;
+        }
         ok = __all_sync(0xffffffffu, mbar_wait_parked(bar(Cfg::B_GFULL + wg), (uint32_t)(kk >> 1) & 1u, wc));
         if (!ok) break;
         tc_fence_after();
         const uint32_t NEG = 0xff800000u;
-        // 64 score columns; once they are in registers the score buffers belong to the next item
+        // 64 score columns; once they are in registers P^T and dS^T may overwrite S^T, and the next item's dP^T this one
         uint32_t sr[2][32], dr[2][32];
         tmem_ld32(tS, sr[0]); tmem_ld32(tDP, dr[0]);
         tmem_ld32(tS + 32, sr[1]); tmem_ld32(tDP + 32, dr[1]);
         tc_wait_ld();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(Cfg::B_SREAD));
-        // P^T / dS^T of this parity are free once the GEMMs of item kk-2 have completed
-        if (kk >= 2) {
-          ok = __all_sync(0xffffffffu, mbar_wait_parked(bar(Cfg::B_DSFREE + wg), (uint32_t)((kk >> 1) - 1) & 1u, wc));
-          if (!ok) break;
-        }
+        if (lane == 0) mbar_arrive(bar(Cfg::B_SREAD + wg));
         // 16 columns (queries) at a time, as passes over independent elements (exp2, then dS, then
         // the packs) so that no instruction waits on its predecessor; each quarter's P^T goes to TMEM
-        // and its dS^T to shared memory as soon as it is packed, which keeps few values live
+        // and its dS^T to TMEM and shared memory as soon as it is packed, which keeps few values live
 #pragma unroll
         for (int qd = 0; qd < 4; ++qd) {
           const int hc = qd >> 1, c0 = 16 * (qd & 1);
@@ -425,7 +441,8 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
             pk1[c] = pack2<IS_BF16>(pe[2 * c], pe[2 * c + 1]);
             pk2[c] = pack2<IS_BF16>(de[2 * c], de[2 * c + 1]);
           }
-          tmem_st8(tP + 8 * qd, pk1);
+          tmem_st8(tS + 8 * qd, pk1);
+          tmem_st8(tS + 32 + 8 * qd, pk2);
           // dS^T row of this key, queries [16 qd, 16 qd + 16): two 16-byte chunks, 128-byte swizzle
           *reinterpret_cast<uint4*>(dsrow + (((2 * qd) ^ (r & 7)) << 4)) = make_uint4(pk2[0], pk2[1], pk2[2], pk2[3]);
           *reinterpret_cast<uint4*>(dsrow + (((2 * qd + 1) ^ (r & 7)) << 4)) = make_uint4(pk2[4], pk2[5], pk2[6], pk2[7]);
@@ -459,7 +476,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         if (!ok) break;
       }
       if (elect_one()) {
-        mbar_arrive_expect_tx(bar(Cfg::B_STAT), 2 * Cfg::TILE_BYTES * D / 128);
+        mbar_arrive_expect_tx(bar(Cfg::B_STAT), 2 * Cfg::TILE_BYTES);
         for (int dc = 0; dc < D / 64; ++dc)
           tma_load_4d(sStat + Cfg::TILE_BYTES + dc * Cfg::SUB128, &tm_v, bar(Cfg::B_STAT), dc * 64, hk, row0, b);
       }
@@ -492,7 +509,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         if (elect_one()) {
           const uint32_t dst = sRing + slot * Cfg::SLOT_BYTES;
           const uint32_t fb = bar(Cfg::B_RFULL + slot);
-          mbar_arrive_expect_tx(fb, Cfg::SLOT_BYTES * D / 128 + Cfg::AUX_BYTES);
+          mbar_arrive_expect_tx(fb, Cfg::SLOT_BYTES + Cfg::AUX_BYTES);
           for (int dc = 0; dc < D / 64; ++dc) {
             tma_load_4d(dst + dc * Cfg::SUB64, &tm_q, fb, dc * 64, hstr, idx * 64, b);
             tma_load_4d(dst + Cfg::HALF_BYTES + dc * Cfg::SUB64, &tm_do, fb, dc * 64, hstr, idx * 64, b);
@@ -509,10 +526,103 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       if (lane == 0) mbar_arrive(bar(Cfg::B_INFOFREE + s));
       kb += K_items;
     }
-  } else if (warp == 9) {
+  } else if (KV_T && warp == 9) {
+    // =========================== UMMA issuer (D = 64) ===========================
+    // One thread issues all five GEMMs: what runs in the order of issue needs no barrier.  S^T of item k+2 follows the dV and dK
+    // GEMMs of item k, which read the P^T and dS^T that it overwrites; dP^T of item k+3 is issued behind item k's dQ^T, when
+    // the warpgroup of item k+1 has read its own.  The chain of an item (T -> dV, dK, S^T -> scores -> T) is what bounds this
+    // variant: with a second thread and a barrier between dK and S^T it was 200 cycles longer.
+    if (elect_one()) {
+      constexpr uint32_t idesc_g = make_idesc(IS_BF16, 128, 64, 0, 0), idesc_stat = make_idesc(true, 128, 64, 0, 0);
+      constexpr uint32_t idesc_acc = make_idesc(IS_BF16, 128, 64, 0, 1), idesc_dq = make_idesc(IS_BF16, 128, 64, 1, 1);
+      const uint64_t dRk = make_sdesc(sRing, 16, 1024), dRm = make_sdesc(sRing, Cfg::SUB64, 1024);   // ring slot, K- / MN-major
+      const uint64_t dKm = make_sdesc(sStat, Cfg::SUB128, 1024);            // K tile, MN-major (A of dQ^T)
+      const uint64_t dDm = make_sdesc(sDS, Cfg::DS_BYTES, 1024);            // dS^T, MN-major (B of dQ^T)
+      const uint64_t dOnes = make_sdesc_noswz(sbase + Cfg::OFF_ONES, 128, 128);
+      bool ok = true;
+      int kb = 0, ju = 0;
+      auto issue_dp = [&](int kk) {
+        const int slot = kk % Cfg::NSLOT;
+        ok = ok && mbar_wait_parked(bar(Cfg::B_RFULL + slot), (uint32_t)(kk / Cfg::NSLOT) & 1u, wc);
+        if (!ok) return;
+        tc_fence_after();
+        const uint32_t tDP = tmem + C_DP + 64u * (uint32_t)(kk & 1), sAux = sbase + Cfg::OFF_AUX + slot * Cfg::AUX_BYTES + 1024;
+        umma_ts_k_x4(tDP, tmem + C_V, dRk + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4) + (Cfg::HALF_BYTES >> 4)), idesc_g);
+        umma_ss(tDP, dOnes, make_sdesc_noswz(sAux, sbase + Cfg::OFF_ZEROS - sAux, 128), idesc_stat, 1u);
+      };
+      auto issue_s = [&](int kk) {
+        const int slot = kk % Cfg::NSLOT;
+        const uint32_t tS = tmem + C_S + 64u * (uint32_t)(kk & 1), sAux = sbase + Cfg::OFF_AUX + slot * Cfg::AUX_BYTES;
+        umma_ts_k_x4(tS, tmem + C_K, dRk + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4)), idesc_g);
+        umma_ss(tS, dOnes, make_sdesc_noswz(sAux, sbase + Cfg::OFF_ZEROS - sAux, 128), idesc_stat, 1u);
+        tc_commit(bar(Cfg::B_GFULL + (kk & 1)));
+      };
+      for (int j = 0; ok; ++j) {
+        const int s = j & 1;
+        ok = mbar_wait_parked(bar(Cfg::B_INFOREADY + s), (uint32_t)(j >> 1) & 1u, wc);
+        if (!ok) break;
+        const int cnt = infos[s * 8 + 3];
+        if (cnt < 0) break;
+        const int K_items = cnt * G;
+        mbar_arrive(bar(Cfg::B_INFOFREE + s));     // only the item count is needed here
+        if (K_items == 0) {
+          // the stationary tiles of an empty unit are not used
+          ok = mbar_wait_parked(bar(Cfg::B_STAT), (uint32_t)j & 1u, wc);
+          mbar_arrive(bar(Cfg::B_VFREE)); mbar_arrive(bar(Cfg::B_KFREE));
+          continue;
+        }
+        ok = mbar_wait_parked(bar(Cfg::B_KVT), (uint32_t)ju & 1u, wc);       // K and V have landed and are in tensor memory
+        if (!ok) break;
+        mbar_arrive(bar(Cfg::B_VFREE));            // (V is not read from shared memory again)
+        for (int k = 0; k < 2 && k < K_items && ok; ++k) {
+          issue_dp(kb + k);
+          if (ok) issue_s(kb + k);
+        }
+        for (int k = 0; k < K_items && ok; ++k) {
+          const int kk = kb + k, slot = kk % Cfg::NSLOT, pz = kk & 1;
+          ok = mbar_wait_parked(bar(Cfg::B_TFULL + pz), (uint32_t)(kk >> 1) & 1u, wc);
+          if (!ok) break;
+          if (k == 0 && ju > 0) {
+            // the accumulators still hold the previous unit until its epilogue has read them
+            ok = mbar_wait_parked(bar(Cfg::B_ACCFREE), (uint32_t)(ju - 1) & 1u, wc);
+            if (!ok) break;
+          }
+          tc_fence_after();
+          const uint64_t dm_q = dRm + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4));
+          const uint32_t tP = tmem + C_S + 64u * (uint32_t)pz;
+          umma_ts_xn<4>(tmem + C_DV, tP, dm_q + (uint64_t)(Cfg::HALF_BYTES >> 4), idesc_acc, k > 0 ? 1u : 0u);
+          umma_ts_xn<4>(tmem + C_DK, tP + 32u, dm_q, idesc_acc, k > 0 ? 1u : 0u);
+          tc_commit(bar(Cfg::B_REMPTY + slot));
+          if (k + 2 < K_items) {
+            if (k == 0) issue_dp(kk + 2);          // (T of item k: its dP^T has been read)
+            if (!ok) break;
+            issue_s(kk + 2);
+          }
+          // dQ^T = K^T dS^T: its buffer is free once the reduction warpgroup has read item kk-1
+          if (kk >= 1) {
+            ok = mbar_wait_parked(bar(Cfg::B_DQFREE), (uint32_t)(kk - 1) & 1u, wc);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          umma_ss_mn_mn_x8(tmem + C_DQ, dKm, dDm + (uint64_t)(pz * (Cfg::DS_BYTES >> 4)), idesc_dq);
+          tc_commit(bar(Cfg::B_DQFULL));
+          tc_commit(bar(Cfg::B_DSFREE + pz));
+          if (k == K_items - 1) { tc_commit(bar(Cfg::B_KFREE)); tc_commit(bar(Cfg::B_ACC)); }
+          if (k + 3 < K_items) {
+            ok = mbar_wait_parked(bar(Cfg::B_SREAD + (pz ^ 1)), (uint32_t)((kk + 1) >> 1) & 1u, wc);
+            if (!ok) break;
+            issue_dp(kk + 3);
+          }
+        }
+        ++ju;
+        kb += K_items;
+      }
+    }
+    __syncwarp();
+  } else if (!KV_T && warp == 9) {
     // =========================== UMMA issuer 1: the score GEMMs ===========================
-    // S^T and dP^T of item kk are issued as soon as the scores of item kk-1 are in registers and
-    // the operands of item kk have landed; nothing here waits for the compute warpgroups' results.
+    // dP^T of item kk is issued as soon as that of item kk-1 has been read out of its buffer, S^T as soon as the dV and dK
+    // GEMMs of item kk-2 are through with the P^T and dS^T that lie over it.
     if (elect_one()) {
       constexpr uint32_t idesc_g = make_idesc(IS_BF16, 128, 64, 0, 0);      // S^T, dP^T
       constexpr uint32_t idesc_stat = make_idesc(true, 128, 64, 0, 0);      // their statistics k-step
@@ -541,7 +651,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         for (int k = 0; k < K_items && ok; ++k) {
           const int kk = kb + k;
           const int slot = kk % Cfg::NSLOT, pz = kk & 1;
-          if (kk >= 1) ok = mbar_wait_parked(bar(Cfg::B_SREAD), (uint32_t)(kk - 1) & 1u, wc);
+          if (kk >= 1) ok = mbar_wait_parked(bar(Cfg::B_SREAD + (pz ^ 1)), (uint32_t)((kk - 1) >> 1) & 1u, wc);
           ok = ok && mbar_wait_parked(bar(Cfg::B_RFULL + slot), (uint32_t)(kk / Cfg::NSLOT) & 1u, wc);
           if (!ok) break;
           tc_fence_after();
@@ -552,17 +662,16 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           const uint32_t sAux = sbase + Cfg::OFF_AUX + slot * Cfg::AUX_BYTES;
           const uint64_t dSs = make_sdesc_noswz(sAux, sbase + Cfg::OFF_ZEROS - sAux, 128);
           const uint64_t dSd = make_sdesc_noswz(sAux + 1024, sbase + Cfg::OFF_ZEROS - (sAux + 1024), 128);
-          if constexpr (D == 128) {
-            umma_ss_width<(Cfg::SUB128 >> 4), (Cfg::SUB64 >> 4)>(tmem + C_S, dKk, dq_, idesc_g, p.d);
-            umma_ss(tmem + C_S, dOnes, dSs, idesc_stat, 1u);
-            umma_ss_width<(Cfg::SUB128 >> 4), (Cfg::SUB64 >> 4)>(tmem + C_DP, dVk, do_, idesc_g, p.dv_dim);
-            umma_ss(tmem + C_DP, dOnes, dSd, idesc_stat, 1u);
-          } else {
-            umma_ss_x4(tmem + C_S, dKk, dq_, idesc_g, 0u);
-            umma_ss(tmem + C_S, dOnes, dSs, idesc_stat, 1u);
-            umma_ss_x4(tmem + C_DP, dVk, do_, idesc_g, 0u);
-            umma_ss(tmem + C_DP, dOnes, dSd, idesc_stat, 1u);
+          const uint32_t tS = tmem + C_S + 64u * (uint32_t)pz, tDP = tmem + C_DP;
+          umma_ss_width<(Cfg::SUB128 >> 4), (Cfg::SUB64 >> 4)>(tDP, dVk, do_, idesc_g, p.dv_dim);
+          umma_ss(tDP, dOnes, dSd, idesc_stat, 1u);
+          if (kk >= 2) {
+            ok = mbar_wait_parked(bar(Cfg::B_PFREE + pz), (uint32_t)((kk >> 1) - 1) & 1u, wc);
+            if (!ok) break;
+            tc_fence_after();
           }
+          umma_ss_width<(Cfg::SUB128 >> 4), (Cfg::SUB64 >> 4)>(tS, dKk, dq_, idesc_g, p.d);
+          umma_ss(tS, dOnes, dSs, idesc_stat, 1u);
           tc_commit(bar(Cfg::B_GFULL + pz));
           if (k == K_items - 1) tc_commit(bar(Cfg::B_VFREE));   // that was the unit's last read of V
         }
@@ -570,15 +679,14 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       }
     }
     __syncwarp();
-  } else if (warp == 11) {
+  } else if (!KV_T && warp == 11) {
     // =========================== UMMA issuer 2: dV, dK, dQ^T ===========================
     if (elect_one()) {
       // dV, dK: as many columns as the heads have (rounded up to 16; d == dv in this kernel)
-      const uint32_t idesc_acc = make_idesc(IS_BF16, 128, D == 64 ? 64 : (p.d + 15) & ~15, 0, 1);
+      const uint32_t idesc_acc = make_idesc(IS_BF16, 128, (p.d + 15) & ~15, 0, 1);
       constexpr uint32_t idesc_dq = make_idesc(IS_BF16, 128, 64, 1, 1);     // dQ^T
       const uint64_t dKm = make_sdesc(sStat, Cfg::SUB128, 1024);            // K tile, MN-major (A of dQ^T)
       const uint64_t dRm = make_sdesc(sRing, Cfg::SUB64, 1024);             // MN-major view of a ring slot
-      const uint64_t dDk = make_sdesc(sDS, 16, 1024);                       // dS^T, K-major (A of dK)
       const uint64_t dDm = make_sdesc(sDS, Cfg::DS_BYTES, 1024);            // dS^T, MN-major (B of dQ^T)
       bool ok = true;
       int kb = 0, ju = 0;
@@ -606,9 +714,11 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           const uint64_t dm_do = dm_q + (uint64_t)(Cfg::HALF_BYTES >> 4);           // dO half, MN-major
           const uint32_t acc_on = k > 0 ? 1u : 0u;
           // dV += P^T dO, dK += dS^T Q; that was the last read of the ring slot
-          umma_ts_xn<4>(tmem + C_DV, tmem + C_P + 32u * (uint32_t)pz, dm_do, idesc_acc, acc_on);
-          umma_ss_k_mn_x4(tmem + C_DK, dDk + (uint64_t)(pz * (Cfg::DS_BYTES >> 4)), dm_q, idesc_acc, acc_on);
+          const uint32_t tP = tmem + C_S + 64u * (uint32_t)pz;
+          umma_ts_xn<4>(tmem + C_DV, tP, dm_do, idesc_acc, acc_on);
+          umma_ts_xn<4>(tmem + C_DK, tP + 32u, dm_q, idesc_acc, acc_on);
           tc_commit(bar(Cfg::B_REMPTY + slot));
+          tc_commit(bar(Cfg::B_PFREE + pz));
           // dQ^T = K^T dS^T: its buffer is free once the reduction warpgroup has read item kk-1
           if (kk >= 1) {
             ok = mbar_wait_parked(bar(Cfg::B_DQFREE), (uint32_t)(kk - 1) & 1u, wc);
@@ -633,9 +743,9 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     // bytes, 16-byte pieces XOR-swizzled by row) so that one store writes 8 rows x 64 contiguous bytes.
     const int ew = warp - 12;
     const uint32_t lane_field = (uint32_t)(ew * 32) << 16;
-    uint8_t* wst = smem + Cfg::OFF_EPI + ew * 2 * Cfg::RBUF_BYTES;   // this warp's two staging buffers
-    uint8_t* stg = wst;                                              // ... the first also stages dK / dV
-    uint32_t rnd = 0;                            // staging rounds of this warp so far (buffer = rnd & 1)
+    uint8_t* wst = smem + Cfg::OFF_EPI + ew * Cfg::RBUFS * Cfg::RBUF_BYTES;   // this warp's staging
+    uint8_t* stg = smem + Cfg::OFF_EPI2 + ew * Cfg::EPI_STEP;        // (at 128 the same bytes stage dK / dV)
+    uint32_t rnd = 0;                            // staging rounds of this warp so far
     bool ok = true;
     int ju = 0, kb = 0;
     for (int j = 0; ok; ++j) {
@@ -647,11 +757,13 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       const int b = infos[s * 8 + 0], head = infos[s * 8 + 1], row0 = infos[s * 8 + 2];
       const uint16_t* list = lists + s * Cfg::LIST_MAX;
       const int K_items = cnt * G;
-      // dQ^T of an item: this warp's lanes are 32 head-dim columns, the 64 TMEM columns the item's
-      // queries.  16 queries at a time the lane writes its column transposed into a staging buffer
-      // ([query][32 columns], conflict-free) and lane 0 hands the buffer to the copy engine, which adds
-      // the 16 x 32 box to the fp32 accumulator.  Two buffers per warp: before a buffer is rewritten lane 0
-      // waits until every reduction but the latest has read its source.
+      // dQ^T of an item: this warp's lanes are 32 head-dim columns, the 64 TMEM columns the item's queries.  The lane puts its
+      // column into the staging buffer four queries (16 bytes) at a time, [4 queries][32 columns][4 queries], and lane 0 hands
+      // the buffer to the copy engine, which adds it to the block of the fp32 accumulator that has the same order.  (Rows
+      // of 32 columns, four times as many stores: the kernel 806 -> 814 us on 2 x 8192 documents, 32 / 8 heads, d = 128, and
+      // 547 -> 557 at 64; through a tensor map, 16 x 32 boxes, 815 and 554.)  The reductions bound the 128-column variant: the L2
+      // takes 20 bytes per clock and SM of them (bulk or red.v4, measured alone), 1640 cycles for the 32 KB of an item
+      // that takes 2100.
       for (int k = 0; k < K_items && ok; ++k) {
         const int kk = kb + k;
         ok = group_all(mbar_wait_parked(bar(Cfg::B_DQFULL), (uint32_t)kk & 1u, wc), 2, 128);
@@ -659,7 +771,8 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         tc_fence_after();
         const int q0 = (int)(list[k % cnt] & 0xFFFu) * 64;
         const int hq = head * G + k / cnt;
-        const int row_base = (b * p.Hq + hq) * p.Sq_r + q0;   // rows past Sq (inside the padding) receive zeros
+        // this warp's 64 x 32 values of the accumulator (rows past Sq, inside the padding, receive zeros)
+        float* acc = p.dq_accum + (((int64_t)b * p.Hq + hq) * p.Sq_r + q0) * D + ew * 64 * 32;
         uint32_t v[4][16];
 #pragma unroll
         for (int r = 0; r < 4; ++r) tmem_ld16(tmem + lane_field + C_DQ + 16 * r, v[r]);
@@ -669,16 +782,19 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         if (lane == 0) mbar_arrive(bar(Cfg::B_DQFREE));
         if (32 * ew < p.d) {
 #pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            uint8_t* sb = wst + (rnd & 1u) * Cfg::RBUF_BYTES;
-            if (lane == 0) bulk_wait_read<1>();
+          for (int h = 0; h < 64 / Cfg::RROWS; ++h) {
+            // D = 64: the item in one piece, two buffers in turn; 128: in halves through one buffer
+            uint8_t* sb = wst + (Cfg::RBUFS == 2 ? (rnd & 1u) * Cfg::RBUF_BYTES : 0u);
+            if (lane == 0) bulk_wait_read<Cfg::RBUFS - 1>();
             __syncwarp();
 #pragma unroll
-            for (int c = 0; c < 16; ++c) reinterpret_cast<uint32_t*>(sb)[c * 32 + lane] = v[r][c];
+            for (int c = h * Cfg::RROWS; c < (h + 1) * Cfg::RROWS; c += 4)
+              reinterpret_cast<uint4*>(sb)[(c - h * Cfg::RROWS) / 4 * 32 + lane] =
+                  make_uint4(v[c / 16][c % 16], v[c / 16][c % 16 + 1], v[c / 16][c % 16 + 2], v[c / 16][c % 16 + 3]);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              tma_reduce_add_2d(&tm_dq, smem_u32(sb), 32 * ew, row_base + 16 * r);
+              bulk_reduce_add(acc + h * Cfg::RROWS * 32, smem_u32(sb), Cfg::RBUF_BYTES);
               bulk_commit();
             }
             ++rnd;
@@ -690,8 +806,8 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(Cfg::B_INFOFREE + s));
       if (cnt == 0) continue;                    // the compute warpgroups write the zeros of an empty unit
-      // the epilogue stages through this warp's first buffer: its reductions must have read it
-      if (lane == 0) bulk_wait_read<0>();
+      // at 128 the epilogue stages through the same buffer: its reductions must have read it
+      if (D != 64 && lane == 0) bulk_wait_read<0>();
       ok = group_all(mbar_wait_parked(bar(Cfg::B_ACC), (uint32_t)ju & 1u, wc), 2, 128);
       if (!ok) break;
       ++ju;
@@ -760,25 +876,55 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   }
 }
 
-// dq = round(scale * dq_accum): [B, Hq, Sq_r, D] fp32 -> [B, Sq, Hq, d] in the output type.
+// dq = round(scale * dq_accum).  The accumulator holds, per (batch, q head) and block of 64 query rows, groups of 32 columns,
+// each as [4 rows: 16][32 columns][4 rows] (what a lane of the reduction warps has of a column beside its neighbours'
+// columns).  A warp takes 16 rows of a group, 2 KB read as they lie (lane = column), and turns them through shuffles into
+// rows: at each step a lane gives half of what it has to the lane whose columns lie beside its own.
 template <bool IS_BF16, int D>
 __global__ void __launch_bounds__(256) bwd_dq_round_kernel(const AttnKParams p) {
-  constexpr int CPR = D / 8;                    // 16-byte output chunks per row
-  const int64_t n = (int64_t)p.B * p.Hq * p.Sq * CPR;
-  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(x % CPR);
-    const int64_t row = x / CPR;                // (b * Hq + h) * Sq + i
-    const int i = (int)(row % p.Sq);
-    const int64_t bh = row / p.Sq;
+  const int lane = threadIdx.x & 31;
+  const int n_grp = (p.d + 31) / 32, n16 = (p.Sq + 15) / 16;
+  const int64_t n = (int64_t)p.B * p.Hq * n16 * n_grp;
+  for (int64_t x = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); x < n; x += (int64_t)gridDim.x * 8) {
+    const int g = (int)(x % n_grp);
+    const int64_t r16 = x / n_grp;              // (b * Hq + h) * n16 + i / 16
+    const int i0 = (int)(r16 % n16) * 16;
+    const int64_t bh = r16 / n16;
     const int h = (int)(bh % p.Hq), b = (int)(bh / p.Hq);
-    if (c * 8 >= p.d) continue;
-    const float4* src = reinterpret_cast<const float4*>(p.dq_accum + ((bh * p.Sq_r + i) * D + c * 8));
-    const float4 a = src[0], g = src[1];
-    uint4 v;
-    v.x = pack2<IS_BF16>(a.x * p.scale, a.y * p.scale); v.y = pack2<IS_BF16>(a.z * p.scale, a.w * p.scale);
-    v.z = pack2<IS_BF16>(g.x * p.scale, g.y * p.scale); v.w = pack2<IS_BF16>(g.z * p.scale, g.w * p.scale);
-    uint16_t* dst = reinterpret_cast<uint16_t*>(p.dq) + b * p.dq_b + (int64_t)i * p.dq_s + h * p.dq_h + c * 8;
-    *reinterpret_cast<uint4*>(dst) = v;
+    const float4* src = reinterpret_cast<const float4*>(p.dq_accum + (bh * p.Sq_r + (i0 & ~63)) * D) + g * 512 + (i0 & 63) / 4 * 32 + lane;
+    uint32_t w[8];                              // rows 2 k and 2 k + 1 of this lane's column
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 v = __ldcs(src + 32 * e);
+      w[2 * e] = pack2<IS_BF16>(v.x * p.scale, v.y * p.scale);
+      w[2 * e + 1] = pack2<IS_BF16>(v.z * p.scale, v.w * p.scale);
+    }
+    // two columns: even lanes keep row 2 k, odd ones row 2 k + 1
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t o = __shfl_xor_sync(0xffffffffu, w[k], 1);
+      w[k] = (lane & 1) ? __byte_perm(o, w[k], 0x7632) : __byte_perm(w[k], o, 0x5410);
+    }
+    // four columns: lanes with bit 1 clear keep the even k
+    uint32_t y[4][2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t o = __shfl_xor_sync(0xffffffffu, (lane & 2) ? w[2 * k] : w[2 * k + 1], 2);
+      y[k][0] = (lane & 2) ? o : w[2 * k];
+      y[k][1] = (lane & 2) ? w[2 * k + 1] : o;
+    }
+    // eight columns: lanes with bit 2 clear keep the even ones of those
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const uint32_t o0 = __shfl_xor_sync(0xffffffffu, (lane & 4) ? y[2 * k][0] : y[2 * k + 1][0], 4);
+      const uint32_t o1 = __shfl_xor_sync(0xffffffffu, (lane & 4) ? y[2 * k][1] : y[2 * k + 1][1], 4);
+      const uint4 v = (lane & 4) ? make_uint4(o0, o1, y[2 * k + 1][0], y[2 * k + 1][1]) : make_uint4(y[2 * k][0], y[2 * k][1], o0, o1);
+      // k-th of this lane: its index among the eight row pairs has bit 0 from lane bit 1, bit 1 from lane bit 2, bit 2 from k
+      const int i = i0 + 2 * (4 * k + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1)) + (lane & 1);
+      const int c = g * 32 + (lane >> 3) * 8;
+      if (i < p.Sq && c < p.d)
+        *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.dq) + b * p.dq_b + (int64_t)i * p.dq_s + h * p.dq_h + c) = v;
+    }
   }
 }
 
@@ -793,7 +939,7 @@ size_t bwd_sm100_fused_accum_bytes(const fm_attn_args* a) {
 
 template <bool IS_BF16, int D>
 static int launch_bwd_sm100_fused(const AttnKParams& p, const fm_attn_args* a, cudaStream_t s) {
-  using Cfg = BwdFusedCfg;
+  using Cfg = BwdFusedCfg<D>;
   FM_REQUIRE((a->Sq + 63) / 64 <= Cfg::LIST_MAX, FM_ERR_UNSUPPORTED,
              "backward: Sq=%d exceeds the %d rows this kernel variant indexes", a->Sq, Cfg::LIST_MAX * 64);
   CUtensorMap k128, v128, q64, do64;
@@ -805,20 +951,6 @@ static int launch_bwd_sm100_fused(const AttnKParams& p, const fm_attn_args* a, c
   FM_TMAP(q64, a->q, a->Sq, a->Hq, a->d, a->q_stride, 64)
   FM_TMAP(do64, a->d_o, a->Sq, a->Hq, a->dv, a->do_stride, 64)
 #undef FM_TMAP
-  // fp32 dQ accumulator as a 2-D tensor [B*Hq*Sq_r rows, D columns], boxes of 16 rows x 32 columns
-  CUtensorMap dqmap;
-  {
-    EncodeTiledFn enc = get_encode_tiled();
-    FM_REQUIRE(enc != nullptr, FM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)p.B * p.Hq * p.Sq_r};
-    const cuuint64_t strides[1] = {(cuuint64_t)D * 4};
-    const cuuint32_t box[2] = {32, (cuuint32_t)Cfg::RROWS};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(&dqmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.dq_accum, dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    FM_REQUIRE(r == CUDA_SUCCESS, FM_ERR_CUDA, "cuTensorMapEncodeTiled (dQ accumulator) failed with CUresult %d", (int)r);
-  }
   auto kern = bwd_sm100_fused_kernel<IS_BF16, D>;
   FM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
   // (the accumulator was cleared by the preprocess kernel, row by row, unless this call carries earlier sums)
@@ -827,10 +959,10 @@ static int launch_bwd_sm100_fused(const AttnKParams& p, const fm_attn_args* a, c
   FM_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
   // with a launch table: one persistent CTA per SM (fewer when the table is shorter)
   const dim3 grid = p.dkdv_order ? dim3(std::min(p.dkdv_ncta, n_sm)) : dim3((p.Sk + 127) / 128, p.Hkv, p.B);
-  kern<<<grid, Cfg::NTHREADS, Cfg::SMEM, s>>>(k128, v128, q64, do64, dqmap, p);
+  kern<<<grid, Cfg::NTHREADS, Cfg::SMEM, s>>>(k128, v128, q64, do64, p);
   FM_CUDA_TRY(cudaGetLastError());
-  const int64_t n = (int64_t)p.B * p.Hq * p.Sq * (D / 8);
-  const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)n_sm * 16);
+  const int64_t n = (int64_t)p.B * p.Hq * ((p.Sq + 15) / 16) * ((p.d + 31) / 32);
+  const unsigned blocks = (unsigned)std::min<int64_t>((n + 7) / 8, (int64_t)n_sm * 16);
   if (!(p.bwd_flags & FM_BWD_DQ_LEAVE)) {
     bwd_dq_round_kernel<IS_BF16, D><<<blocks, 256, 0, s>>>(p);
     FM_CUDA_TRY(cudaGetLastError());

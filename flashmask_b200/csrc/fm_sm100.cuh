@@ -354,6 +354,23 @@ __device__ __forceinline__ void umma_ss_width(uint32_t d_tmem, uint64_t a, uint6
   }
 }
 
+// Four k-steps (K = 64) of D[tmem] = A[tmem] * B[smem], B K-major with 128-byte swizzle: A advances 8 columns, B 32 bytes.
+__device__ __forceinline__ void umma_ts_k_x4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred pf, pt;\n\t.reg .b64 tb;\n\t.reg .b32 ta;\n\t"
+      "setp.ne.b32 pf, 0, 0;\n\t"
+      "setp.eq.b32 pt, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, pf;\n\t"
+      "add.u32 ta, %1, 8;  add.s64 tb, %2, 2;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], tb, %3, pt;\n\t"
+      "add.u32 ta, %1, 16; add.s64 tb, %2, 4;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], tb, %3, pt;\n\t"
+      "add.u32 ta, %1, 24; add.s64 tb, %2, 6;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], tb, %3, pt;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b), "r"(idesc)
+      : "memory");
+}
+
 // Two more k-steps of the same GEMM (always accumulating).
 __device__ __forceinline__ void umma_ts_x2(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc) {
   asm volatile(
