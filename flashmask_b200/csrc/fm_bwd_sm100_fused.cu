@@ -141,6 +141,24 @@ template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// Four k-steps (K = 64 queries) of D[tmem] (+)= A[tmem] * B[smem], B MN-major: A is 16 columns of each 32-column half of the
+// score buffer (two k-steps from one half, two from the other), B advances 16 rows (2048 bytes) per step.
+__device__ __forceinline__ void umma_ts_halves_x4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t acc_first) {
+  asm volatile(
+      "{\n\t.reg .pred p, pt;\n\t.reg .b64 tb;\n\t.reg .b32 ta;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.eq.b32 pt, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "add.u32 ta, %1, 8;  add.s64 tb, %2, 128;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], tb, %3, pt;\n\t"
+      "add.u32 ta, %1, 32; add.s64 tb, %2, 256;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], tb, %3, pt;\n\t"
+      "add.u32 ta, %1, 40; add.s64 tb, %2, 384;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], tb, %3, pt;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b), "r"(idesc), "r"(acc_first)
+      : "memory");
+}
+
 // Eight k-steps (K = 128) of D[tmem] = A[smem] * B[smem], both operands MN-major: each step
 // advances both by 16 rows (2048 bytes).
 __device__ __forceinline__ void umma_ss_mn_mn_x8(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc) {
@@ -175,7 +193,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
                        const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                        const AttnKParams p) {
   using Cfg = BwdFusedCfg<D>;
-  constexpr bool KV_T = D == 64;               // K and V are copied to tensor memory, and one thread issues all GEMMs
+  constexpr bool KV_T = D == 64;               // K and V are copied to tensor memory
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
@@ -210,10 +228,10 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   if (warp == 8 && lane == 0) {
     for (int i = 0; i < Cfg::NSLOT; ++i) { mbar_init(bar(Cfg::B_RFULL + i), 1); mbar_init(bar(Cfg::B_REMPTY + i), 1); }
     for (int h = 0; h < 2; ++h) {
-      mbar_init(bar(Cfg::B_GFULL + h), 1); mbar_init(bar(Cfg::B_TFULL + h), 4); mbar_init(bar(Cfg::B_DSFREE + h), 1);
-      mbar_init(bar(Cfg::B_INFOREADY + h), 1); mbar_init(bar(Cfg::B_INFOFREE + h), KV_T ? 14 : 15);
+      mbar_init(bar(Cfg::B_GFULL + h), KV_T ? 2 : 1); mbar_init(bar(Cfg::B_TFULL + h), 8); mbar_init(bar(Cfg::B_DSFREE + h), 1);
+      mbar_init(bar(Cfg::B_INFOREADY + h), 1); mbar_init(bar(Cfg::B_INFOFREE + h), 15);
       mbar_init(bar(Cfg::B_COORD + h), 1);
-      mbar_init(bar(Cfg::B_SREAD + h), 4); mbar_init(bar(Cfg::B_PFREE + h), 1);
+      mbar_init(bar(Cfg::B_SREAD + h), 8); mbar_init(bar(Cfg::B_PFREE + h), 1);
     }
     mbar_init(bar(Cfg::B_KVT), 8); mbar_init(bar(Cfg::B_DQFULL), 1); mbar_init(bar(Cfg::B_DQFREE), 4);
     mbar_init(bar(Cfg::B_FETCHGO), 1);
@@ -233,11 +251,6 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   // S^T of item parity p at C_S + 64 p, its P^T and dS^T over it at +0 and +32; dP^T at C_DP (D = 64: + 64 p)
   constexpr uint32_t C_S = 0, C_DP = 128, DP_STEP = KV_T ? 64 : 0, C_DQ = KV_T ? 256 : 192, C_DV = KV_T ? 320 : 256,
                      C_DK = 384, C_K = 448, C_V = 480;
-
-  // 512 threads start with 128 registers each; the compute warpgroups take what the others give up.  (168 / 80 / 96 left
-  // the 128-column variant with spills: 806 instead of 776 us.)
-  if (warp < 8) setmaxnreg_inc<160>();
-  else setmaxnreg_dec<96>();
 
   if (warp == 10) {
     // =========================== scheduler + list builder ===========================
@@ -322,8 +335,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     const int wg = warp >> 2;
     const int r = tid & 127;                     // TMEM lane = key row0 + r
     const uint32_t lane_field = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tS = tmem + lane_field + C_S + 64u * (uint32_t)wg, tDP = tmem + lane_field + C_DP + DP_STEP * (uint32_t)wg;
-    uint8_t* dsrow = smem + Cfg::OFF_DS + wg * Cfg::DS_BYTES + r * 128;
+    const uint32_t tHalf = tmem + lane_field + 32u * (uint32_t)wg;
     const float scale_log2 = p.scale_log2;
     bool ok = true;
     int kb = 0;                                  // items of earlier units
@@ -383,37 +395,38 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           lts = bd.lts; lte = bd.lte; uts = bd.uts; ute = bd.ute;
         }
       }
-      // this warpgroup serves the items whose CTA-wide index kk = kb + k has parity wg
-      for (int k = (wg - kb) & 1; k < K_items && ok; k += 2) {
+      // the two warpgroups share an item: warpgroup wg has its queries [32 wg, 32 wg + 32)
+      for (int k = 0, at = 0; k < K_items && ok; ++k) {
         const int kk = kb + k;
-        const uint32_t e = list[k % cnt];
-        const int idx = (int)(e & 0xFFFu);
+        const uint32_t pz = (uint32_t)kk & 1u;
+        const uint32_t e = list[at];
+        if (++at == cnt) at = 0;
+        const int q0 = (int)(e & 0xFFFu) * 64 + 32 * wg;
         const uint32_t flags = e >> 12;
+        const uint32_t tS = tHalf + C_S + 64u * pz, tDP = tHalf + C_DP + DP_STEP * pz;
+        uint8_t* dsrow = smem + Cfg::OFF_DS + pz * Cfg::DS_BYTES + r * 128;
         // dS^T of this parity in shared memory is free once the dQ^T GEMM of item kk-2 has completed.  (Waited for here, where
         // the scores are awaited anyway: under the operand reads of the GEMMs even a wait that is over costs 500 cycles.)
         if (kk >= 2) {
-          ok = __all_sync(0xffffffffu, mbar_wait_parked(bar(Cfg::B_DSFREE + wg), (uint32_t)((kk >> 1) - 1) & 1u, wc));
+          ok = __all_sync(0xffffffffu, mbar_wait_parked(bar(Cfg::B_DSFREE + pz), (uint32_t)((kk >> 1) - 1) & 1u, wc));
           if (!ok) break;
         }
-        ok = __all_sync(0xffffffffu, mbar_wait_parked(bar(Cfg::B_GFULL + wg), (uint32_t)(kk >> 1) & 1u, wc));
+        ok = __all_sync(0xffffffffu, mbar_wait_parked(bar(Cfg::B_GFULL + pz), (uint32_t)(kk >> 1) & 1u, wc));
         if (!ok) break;
         tc_fence_after();
         const uint32_t NEG = 0xff800000u;
-        // 64 score columns; once they are in registers P^T and dS^T may overwrite S^T, and the next item's dP^T this one
-        uint32_t sr[2][32], dr[2][32];
-        tmem_ld32(tS, sr[0]); tmem_ld32(tDP, dr[0]);
-        tmem_ld32(tS + 32, sr[1]); tmem_ld32(tDP + 32, dr[1]);
+        // 32 score columns; once they are in registers P^T and dS^T may overwrite S^T, and the next item's dP^T this one
+        uint32_t sr[32], dr[32];
+        tmem_ld32(tS, sr); tmem_ld32(tDP, dr);
         tc_wait_ld();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(Cfg::B_SREAD + wg));
+        if (!KV_T && lane == 0) mbar_arrive(bar(Cfg::B_SREAD + pz));
         // 16 columns (queries) at a time, as passes over independent elements (exp2, then dS, then
-        // the packs) so that no instruction waits on its predecessor; each quarter's P^T goes to TMEM
-        // and its dS^T to TMEM and shared memory as soon as it is packed, which keeps few values live
+        // the packs) so that no instruction waits on its predecessor
 #pragma unroll
-        for (int qd = 0; qd < 4; ++qd) {
-          const int hc = qd >> 1, c0 = 16 * (qd & 1);
-          const int i0 = idx * 64 + 16 * qd;            // first query of this quarter
+        for (int hf = 0; hf < 2; ++hf) {
+          const int c0 = 16 * hf, i0 = q0 + c0;         // first query of this half
           if (flags & ~FM_TF_ACTIVE) {
             // for this key the masked queries are intervals of the 16 columns: one mask word, one bit test per column
             const int a0 = lts - i0, a1 = lte - i0, b0 = uts - i0, b1 = ute - i0;
@@ -422,36 +435,37 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
                                    bits_below(cz);
 #pragma unroll
             for (int c = 0; c < 16; ++c)
-              if (mbits & (1u << c)) sr[hc][c0 + c] = NEG;
+              if (mbits & (1u << c)) sr[c0 + c] = NEG;
           }
           // the accumulators already hold S - LSE/scale and dP - rowsum(O dO) (statistics k-step)
           float pe[16], de[16];
 #pragma unroll
           for (int c = 0; c < 16; c += 2) {
             float x0, x1;
-            mul2(x0, x1, __uint_as_float(sr[hc][c0 + c]), __uint_as_float(sr[hc][c0 + c + 1]), scale_log2, scale_log2);
+            mul2(x0, x1, __uint_as_float(sr[c0 + c]), __uint_as_float(sr[c0 + c + 1]), scale_log2, scale_log2);
             pe[c] = fast_exp2(x0); pe[c + 1] = fast_exp2(x1);
           }
 #pragma unroll
           for (int c = 0; c < 16; c += 2)
-            mul2(de[c], de[c + 1], pe[c], pe[c + 1], __uint_as_float(dr[hc][c0 + c]), __uint_as_float(dr[hc][c0 + c + 1]));
+            mul2(de[c], de[c + 1], pe[c], pe[c + 1], __uint_as_float(dr[c0 + c]), __uint_as_float(dr[c0 + c + 1]));
           uint32_t pk1[8], pk2[8];
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             pk1[c] = pack2<IS_BF16>(pe[2 * c], pe[2 * c + 1]);
             pk2[c] = pack2<IS_BF16>(de[2 * c], de[2 * c + 1]);
           }
-          tmem_st8(tS + 8 * qd, pk1);
-          tmem_st8(tS + 32 + 8 * qd, pk2);
-          // dS^T row of this key, queries [16 qd, 16 qd + 16): two 16-byte chunks, 128-byte swizzle
-          *reinterpret_cast<uint4*>(dsrow + (((2 * qd) ^ (r & 7)) << 4)) = make_uint4(pk2[0], pk2[1], pk2[2], pk2[3]);
-          *reinterpret_cast<uint4*>(dsrow + (((2 * qd + 1) ^ (r & 7)) << 4)) = make_uint4(pk2[4], pk2[5], pk2[6], pk2[7]);
+          tmem_st8(tS + 8 * hf, pk1);
+          tmem_st8(tS + 16 + 8 * hf, pk2);
+          // dS^T row of this key, 16 queries: two 16-byte chunks, 128-byte swizzle
+          const int ch = 4 * wg + 2 * hf;
+          *reinterpret_cast<uint4*>(dsrow + ((ch ^ (r & 7)) << 4)) = make_uint4(pk2[0], pk2[1], pk2[2], pk2[3]);
+          *reinterpret_cast<uint4*>(dsrow + (((ch + 1) ^ (r & 7)) << 4)) = make_uint4(pk2[4], pk2[5], pk2[6], pk2[7]);
         }
         tc_wait_st();
         fence_proxy_async_smem();   // the dS^T stores become visible to the tensor core's reads
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(Cfg::B_TFULL + wg));
+        if (lane == 0) mbar_arrive(bar(Cfg::B_TFULL + pz));
       }
       if (!ok) break;
       if (lane == 0) mbar_arrive(bar(Cfg::B_INFOFREE + s));   // list and record of this unit are no longer read
@@ -527,35 +541,27 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       kb += K_items;
     }
   } else if (KV_T && warp == 9) {
-    // =========================== UMMA issuer (D = 64) ===========================
-    // One thread issues all five GEMMs: what runs in the order of issue needs no barrier.  S^T of item k+2 follows the dV and dK
-    // GEMMs of item k, which read the P^T and dS^T that it overwrites; dP^T of item k+3 is issued behind item k's dQ^T, when
-    // the warpgroup of item k+1 has read its own.  The chain of an item (T -> dV, dK, S^T -> scores -> T) is what bounds this
-    // variant: with a second thread and a barrier between dK and S^T it was 200 cycles longer.
+    // =========================== UMMA issuer 1 (D = 64): dV, dK, S^T ===========================
+    // What runs in the order of issue needs no barrier: S^T of item k+2 follows the dV and dK GEMMs of item k, which read the P^T
+    // and dS^T that it overwrites.  dP^T and dQ^T are issued by another thread: a thread that issues spends its time waiting for
+    // the queue of the tensor pipe and, some 150 cycles each, for barriers, and one for all five GEMMs was busy for all of an
+    // item's 1640 cycles.
     if (elect_one()) {
       constexpr uint32_t idesc_g = make_idesc(IS_BF16, 128, 64, 0, 0), idesc_stat = make_idesc(true, 128, 64, 0, 0);
-      constexpr uint32_t idesc_acc = make_idesc(IS_BF16, 128, 64, 0, 1), idesc_dq = make_idesc(IS_BF16, 128, 64, 1, 1);
+      constexpr uint32_t idesc_acc = make_idesc(IS_BF16, 128, 64, 0, 1);
       const uint64_t dRk = make_sdesc(sRing, 16, 1024), dRm = make_sdesc(sRing, Cfg::SUB64, 1024);   // ring slot, K- / MN-major
-      const uint64_t dKm = make_sdesc(sStat, Cfg::SUB128, 1024);            // K tile, MN-major (A of dQ^T)
-      const uint64_t dDm = make_sdesc(sDS, Cfg::DS_BYTES, 1024);            // dS^T, MN-major (B of dQ^T)
       const uint64_t dOnes = make_sdesc_noswz(sbase + Cfg::OFF_ONES, 128, 128);
       bool ok = true;
       int kb = 0, ju = 0;
-      auto issue_dp = [&](int kk) {
-        const int slot = kk % Cfg::NSLOT;
-        ok = ok && mbar_wait_parked(bar(Cfg::B_RFULL + slot), (uint32_t)(kk / Cfg::NSLOT) & 1u, wc);
-        if (!ok) return;
-        tc_fence_after();
-        const uint32_t tDP = tmem + C_DP + 64u * (uint32_t)(kk & 1), sAux = sbase + Cfg::OFF_AUX + slot * Cfg::AUX_BYTES + 1024;
-        umma_ts_k_x4(tDP, tmem + C_V, dRk + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4) + (Cfg::HALF_BYTES >> 4)), idesc_g);
-        umma_ss(tDP, dOnes, make_sdesc_noswz(sAux, sbase + Cfg::OFF_ZEROS - sAux, 128), idesc_stat, 1u);
-      };
       auto issue_s = [&](int kk) {
         const int slot = kk % Cfg::NSLOT;
         const uint32_t tS = tmem + C_S + 64u * (uint32_t)(kk & 1), sAux = sbase + Cfg::OFF_AUX + slot * Cfg::AUX_BYTES;
         umma_ts_k_x4(tS, tmem + C_K, dRk + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4)), idesc_g);
         umma_ss(tS, dOnes, make_sdesc_noswz(sAux, sbase + Cfg::OFF_ZEROS - sAux, 128), idesc_stat, 1u);
         tc_commit(bar(Cfg::B_GFULL + (kk & 1)));
+      };
+      auto wait_ring = [&](int kk) {
+        return mbar_wait_parked(bar(Cfg::B_RFULL + kk % Cfg::NSLOT), (uint32_t)(kk / Cfg::NSLOT) & 1u, wc);
       };
       for (int j = 0; ok; ++j) {
         const int s = j & 1;
@@ -575,12 +581,15 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         if (!ok) break;
         mbar_arrive(bar(Cfg::B_VFREE));            // (V is not read from shared memory again)
         for (int k = 0; k < 2 && k < K_items && ok; ++k) {
-          issue_dp(kb + k);
-          if (ok) issue_s(kb + k);
+          ok = wait_ring(kb + k);
+          if (!ok) break;
+          tc_fence_after();
+          issue_s(kb + k);
         }
         for (int k = 0; k < K_items && ok; ++k) {
           const int kk = kb + k, slot = kk % Cfg::NSLOT, pz = kk & 1;
-          ok = mbar_wait_parked(bar(Cfg::B_TFULL + pz), (uint32_t)(kk >> 1) & 1u, wc);
+          if (k + 2 < K_items) ok = wait_ring(kk + 2);
+          ok = ok && mbar_wait_parked(bar(Cfg::B_TFULL + pz), (uint32_t)(kk >> 1) & 1u, wc);
           if (!ok) break;
           if (k == 0 && ju > 0) {
             // the accumulators still hold the previous unit until its epilogue has read them
@@ -590,31 +599,66 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           tc_fence_after();
           const uint64_t dm_q = dRm + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4));
           const uint32_t tP = tmem + C_S + 64u * (uint32_t)pz;
-          umma_ts_xn<4>(tmem + C_DV, tP, dm_q + (uint64_t)(Cfg::HALF_BYTES >> 4), idesc_acc, k > 0 ? 1u : 0u);
-          umma_ts_xn<4>(tmem + C_DK, tP + 32u, dm_q, idesc_acc, k > 0 ? 1u : 0u);
-          tc_commit(bar(Cfg::B_REMPTY + slot));
-          if (k + 2 < K_items) {
-            if (k == 0) issue_dp(kk + 2);          // (T of item k: its dP^T has been read)
-            if (!ok) break;
-            issue_s(kk + 2);
-          }
-          // dQ^T = K^T dS^T: its buffer is free once the reduction warpgroup has read item kk-1
-          if (kk >= 1) {
-            ok = mbar_wait_parked(bar(Cfg::B_DQFREE), (uint32_t)(kk - 1) & 1u, wc);
-            if (!ok) break;
-            tc_fence_after();
-          }
+          umma_ts_halves_x4(tmem + C_DV, tP, dm_q + (uint64_t)(Cfg::HALF_BYTES >> 4), idesc_acc, k > 0 ? 1u : 0u);
+          umma_ts_halves_x4(tmem + C_DK, tP + 16u, dm_q, idesc_acc, k > 0 ? 1u : 0u);
+          tc_commit(bar(Cfg::B_REMPTY + slot));    // (T: the score GEMMs of item k have read the slot too)
+          if (k + 2 < K_items) issue_s(kk + 2);
+          else if (k == K_items - 1) tc_commit(bar(Cfg::B_ACC));
+        }
+        ++ju;
+        kb += K_items;
+      }
+    }
+    __syncwarp();
+  } else if (KV_T && warp == 11) {
+    // =========================== UMMA issuer 2 (D = 64): dP^T, dQ^T ===========================
+    // T of item k says that its dP^T has been read: dP^T of item k+2, then dQ^T of item k.
+    if (elect_one()) {
+      constexpr uint32_t idesc_g = make_idesc(IS_BF16, 128, 64, 0, 0), idesc_stat = make_idesc(true, 128, 64, 0, 0);
+      constexpr uint32_t idesc_dq = make_idesc(IS_BF16, 128, 64, 1, 1);
+      const uint64_t dDo = make_sdesc(sRing + Cfg::HALF_BYTES, 16, 1024);   // dO half of a ring slot, K-major
+      const uint64_t dKm = make_sdesc(sStat, Cfg::SUB128, 1024);            // K tile, MN-major (A of dQ^T)
+      const uint64_t dDm = make_sdesc(sDS, Cfg::DS_BYTES, 1024);            // dS^T, MN-major (B of dQ^T)
+      const uint64_t dOnes = make_sdesc_noswz(sbase + Cfg::OFF_ONES, 128, 128);
+      bool ok = true;
+      int kb = 0, ju = 0;
+      auto issue_dp = [&](int kk) {
+        const int slot = kk % Cfg::NSLOT;
+        ok = ok && mbar_wait_parked(bar(Cfg::B_RFULL + slot), (uint32_t)(kk / Cfg::NSLOT) & 1u, wc);
+        if (!ok) return;
+        tc_fence_after();
+        const uint32_t tDP = tmem + C_DP + 64u * (uint32_t)(kk & 1), sAux = sbase + Cfg::OFF_AUX + slot * Cfg::AUX_BYTES + 1024;
+        umma_ts_k_x4(tDP, tmem + C_V, dDo + (uint64_t)(slot * (Cfg::SLOT_BYTES >> 4)), idesc_g);
+        umma_ss(tDP, dOnes, make_sdesc_noswz(sAux, sbase + Cfg::OFF_ZEROS - sAux, 128), idesc_stat, 1u);
+        tc_commit(bar(Cfg::B_GFULL + (kk & 1)));
+      };
+      for (int j = 0; ok; ++j) {
+        const int s = j & 1;
+        ok = mbar_wait_parked(bar(Cfg::B_INFOREADY + s), (uint32_t)(j >> 1) & 1u, wc);
+        if (!ok) break;
+        const int cnt = infos[s * 8 + 3];
+        if (cnt < 0) break;
+        const int K_items = cnt * G;
+        mbar_arrive(bar(Cfg::B_INFOFREE + s));
+        if (K_items == 0) continue;                // issuer 1 releases the tiles of an empty unit
+        ok = mbar_wait_parked(bar(Cfg::B_KVT), (uint32_t)ju & 1u, wc);
+        if (!ok) break;
+        ++ju;
+        issue_dp(kb);
+        if (K_items > 1) issue_dp(kb + 1);
+        for (int k = 0; k < K_items && ok; ++k) {
+          const int kk = kb + k, pz = kk & 1;
+          ok = mbar_wait_parked(bar(Cfg::B_TFULL + pz), (uint32_t)(kk >> 1) & 1u, wc);
+          if (k + 2 < K_items) issue_dp(kk + 2);
+          // the buffer of dQ^T is free once the reduction warpgroup has read item kk-1
+          if (kk >= 1) ok = ok && mbar_wait_parked(bar(Cfg::B_DQFREE), (uint32_t)(kk - 1) & 1u, wc);
+          if (!ok) break;
+          tc_fence_after();
           umma_ss_mn_mn_x8(tmem + C_DQ, dKm, dDm + (uint64_t)(pz * (Cfg::DS_BYTES >> 4)), idesc_dq);
           tc_commit(bar(Cfg::B_DQFULL));
           tc_commit(bar(Cfg::B_DSFREE + pz));
-          if (k == K_items - 1) { tc_commit(bar(Cfg::B_KFREE)); tc_commit(bar(Cfg::B_ACC)); }
-          if (k + 3 < K_items) {
-            ok = mbar_wait_parked(bar(Cfg::B_SREAD + (pz ^ 1)), (uint32_t)((kk + 1) >> 1) & 1u, wc);
-            if (!ok) break;
-            issue_dp(kk + 3);
-          }
+          if (k == K_items - 1) tc_commit(bar(Cfg::B_KFREE));
         }
-        ++ju;
         kb += K_items;
       }
     }
@@ -715,8 +759,8 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           const uint32_t acc_on = k > 0 ? 1u : 0u;
           // dV += P^T dO, dK += dS^T Q; that was the last read of the ring slot
           const uint32_t tP = tmem + C_S + 64u * (uint32_t)pz;
-          umma_ts_xn<4>(tmem + C_DV, tP, dm_do, idesc_acc, acc_on);
-          umma_ts_xn<4>(tmem + C_DK, tP + 32u, dm_q, idesc_acc, acc_on);
+          umma_ts_halves_x4(tmem + C_DV, tP, dm_do, idesc_acc, acc_on);
+          umma_ts_halves_x4(tmem + C_DK, tP + 16u, dm_q, idesc_acc, acc_on);
           tc_commit(bar(Cfg::B_REMPTY + slot));
           tc_commit(bar(Cfg::B_PFREE + pz));
           // dQ^T = K^T dS^T: its buffer is free once the reduction warpgroup has read item kk-1
