@@ -10,7 +10,7 @@
 //     P^T  = exp2(S^T scale - LSE), dS^T = P^T (dP^T - rowsum(O dO))   (compute warpgroups)
 //     dV  += P^T dO             A = P^T from TMEM (bf16)
 //     dK  += dS^T Q             A = dS^T from TMEM
-//     dQ^T = K^T dS^T           M=128 head-dim columns, N=64 queries; A = the K tile read
+//     dQ^T = K^T dS^T           M=128 (64) head-dim columns, N=64 queries; A = the K tile read
 //                               MN-major, B = dS^T once more, from shared memory, read MN-major
 // dK / dV stay in TMEM for the whole unit and are written once.  dQ^T of an item is drained
 // by a fourth warpgroup and added to an fp32 accumulator in global memory by bulk
@@ -20,16 +20,22 @@
 // output element.
 //
 // TMEM columns.  S^T has a buffer per item parity p at [64p, +64); once an item's scores are in
-// registers its P^T and dS^T (16 bits) lie over it at +0 and +32 and are the A operands of dV and dK.
+// registers its P^T and dS^T (16 bits) lie over them and are the A operands of dV and dK.
 //   128-column variant: dP^T [128,192) (one buffer), dQ^T [192,256), dV [256,384), dK [384,512).
 //   64-column variant: dP^T [128+64p, +64), dQ^T [256,320), dV [320,384), dK [384,448), and K and V
-//   of the unit, copied there once, at [448,480) and [480,512): A operands of S^T and dP^T.  An MMA of N = 64
-//   with A in shared memory reads 192 bytes per clock of a pipe that has 128, with A in TMEM 64.
-// 2 x 8192 documents, 32 / 8 heads, this kernel alone: d = 64 622 -> 536 us, d = 128 815 -> 776, d = 96 731 -> 690, against one
+//   of the unit, copied there once, at [448,480) and [480,512): A operands of S^T and dP^T.
+//
+// What bounds it.  An MMA of N = 64 with A in shared memory reads 192 bytes per clock of a pipe that has 128 (48 cycles, measured
+// alone; 32 with A in TMEM).  128-column variant: S^T, dP^T and dQ^T 1250 cycles an item, dV and dK 512, and the L2 takes 20
+// bytes per clock and SM of fp32 reductions (bulk or red.v4, measured alone), 1640 cycles for an item's 32 KB of dQ; it takes 2100.
+// 64-column variant: 860 cycles of MMAs, 1120 of the shared-memory pipe; it takes 1490 on full tiles.  There the chain scores -> P, dS
+// -> dV, dK -> next scores decided: both warpgroups work on the same item (the chain has half the exponentials; in turn, 535 instead
+// of 512 us), and two threads issue.
+// 2 x 8192 documents, 32 / 8 heads, this kernel alone: d = 64 622 -> 493 us, d = 128 815 -> 776, d = 96 731 -> 690, against one
 // buffer each for S^T and dP^T, P^T in columns of its own and dS^T read from shared memory.
 //
-// Warp roles: 0-3 / 4-7 compute warpgroups (items alternate), 8 TMA producer, 9 UMMA issuer
-// (owns TMEM), 10 scheduler + list builder, 11 second UMMA issuer (128 columns), 12-15 dQ reduction + dK/dV epilogue.
+// Warp roles: 0-3 / 4-7 compute warpgroups, 8 TMA producer, 9 UMMA issuer
+// (owns TMEM), 10 scheduler + list builder, 11 second UMMA issuer, 12-15 dQ reduction + dK/dV epilogue.
 // All waits are bounded.
 #include <algorithm>
 
@@ -70,10 +76,11 @@ struct BwdFusedCfg {
   static constexpr int OFF_LIST = OFF_ZEROS + 1024;                     // two lists of 16-bit entries: units alternate
   static constexpr int OFF_STAGE = OFF_LIST + 2 * LIST_MAX * 2;         // reductions of the unit's K tile (8 x 4 ints)
   static constexpr int EPI_BYTES = 32 * 64;                             // per epilogue warp: 32 rows x 32 bf16 columns
-  static constexpr int RROWS = D == 64 ? 64 : 32;                       // dQ staging: query rows x 32 columns per buffer,
-  static constexpr int RBUF_BYTES = RROWS * 32 * 4, RBUFS = D == 64 ? 2 : 1;   // and buffers per warp that has dQ columns
+  static constexpr int RCOLS = D == 64 ? 16 : 32;                       // dQ^T: head-dim columns of a reduction warp (64: M = 64)
+  static constexpr int RROWS = D == 64 ? 64 : 32;                       // dQ staging: query rows x RCOLS columns per buffer,
+  static constexpr int RBUF_BYTES = RROWS * RCOLS * 4, RBUFS = D == 64 ? 2 : 1;   // and buffers per warp
   static constexpr int OFF_EPI = OFF_STAGE + 128;                       // dQ staging; at 128 the dK/dV epilogue reuses it
-  static constexpr int OFF_EPI2 = D == 64 ? OFF_EPI + 2 * RBUFS * RBUF_BYTES : OFF_EPI;
+  static constexpr int OFF_EPI2 = D == 64 ? OFF_EPI + 4 * RBUFS * RBUF_BYTES : OFF_EPI;
   static constexpr int EPI_STEP = D == 64 ? EPI_BYTES : RBUFS * RBUF_BYTES;
   static constexpr int OFF_INFO = OFF_EPI2 + 4 * EPI_STEP;              // two unit records of 8 ints
   static constexpr int OFF_BAR = OFF_INFO + 2 * 8 * 4;
@@ -185,8 +192,7 @@ __device__ __forceinline__ void umma_ss_mn_mn_x8(uint32_t d_tmem, uint64_t a, ui
       : "memory");
 }
 
-// D: width the head dims are computed at (64 when both fit, else 128).  In the 64-column variant the A operand of
-// dQ^T (M = 128 head-dim columns) goes on into the V tile behind K; TMEM lanes 64..127 of dQ^T hold products nobody reads.
+// D: width the head dims are computed at (64 when both fit, else 128).
 template <bool IS_BF16, int D>
 __global__ void __launch_bounds__(512, 1)
 bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -228,10 +234,10 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   if (warp == 8 && lane == 0) {
     for (int i = 0; i < Cfg::NSLOT; ++i) { mbar_init(bar(Cfg::B_RFULL + i), 1); mbar_init(bar(Cfg::B_REMPTY + i), 1); }
     for (int h = 0; h < 2; ++h) {
-      mbar_init(bar(Cfg::B_GFULL + h), KV_T ? 2 : 1); mbar_init(bar(Cfg::B_TFULL + h), 8); mbar_init(bar(Cfg::B_DSFREE + h), 1);
+      mbar_init(bar(Cfg::B_GFULL + h), KV_T ? 2 : 1); mbar_init(bar(Cfg::B_TFULL + h), KV_T ? 8 : 4); mbar_init(bar(Cfg::B_DSFREE + h), 1);
       mbar_init(bar(Cfg::B_INFOREADY + h), 1); mbar_init(bar(Cfg::B_INFOFREE + h), 15);
       mbar_init(bar(Cfg::B_COORD + h), 1);
-      mbar_init(bar(Cfg::B_SREAD + h), 8); mbar_init(bar(Cfg::B_PFREE + h), 1);
+      mbar_init(bar(Cfg::B_SREAD + h), 4); mbar_init(bar(Cfg::B_PFREE + h), 1);
     }
     mbar_init(bar(Cfg::B_KVT), 8); mbar_init(bar(Cfg::B_DQFULL), 1); mbar_init(bar(Cfg::B_DQFREE), 4);
     mbar_init(bar(Cfg::B_FETCHGO), 1);
@@ -251,6 +257,13 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   // S^T of item parity p at C_S + 64 p, its P^T and dS^T over it at +0 and +32; dP^T at C_DP (D = 64: + 64 p)
   constexpr uint32_t C_S = 0, C_DP = 128, DP_STEP = KV_T ? 64 : 0, C_DQ = KV_T ? 256 : 192, C_DV = KV_T ? 320 : 256,
                      C_DK = 384, C_K = 448, C_V = 480;
+
+  // 128: 512 threads start with 128 registers each; the compute warpgroups take what the others give up.  (168 / 80 / 96 left
+  // spills: 806 instead of 776 us.)  64: half the columns to a thread, 128 do.
+  if constexpr (!KV_T) {
+    if (warp < 8) setmaxnreg_inc<160>();
+    else setmaxnreg_dec<96>();
+  }
 
   if (warp == 10) {
     // =========================== scheduler + list builder ===========================
@@ -335,7 +348,8 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     const int wg = warp >> 2;
     const int r = tid & 127;                     // TMEM lane = key row0 + r
     const uint32_t lane_field = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tHalf = tmem + lane_field + 32u * (uint32_t)wg;
+    constexpr int NC = KV_T ? 32 : 64;           // queries of an item this warpgroup has
+    const uint32_t tHalf = tmem + lane_field + (KV_T ? 32u * (uint32_t)wg : 0u);
     const float scale_log2 = p.scale_log2;
     bool ok = true;
     int kb = 0;                                  // items of earlier units
@@ -395,13 +409,13 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           lts = bd.lts; lte = bd.lte; uts = bd.uts; ute = bd.ute;
         }
       }
-      // the two warpgroups share an item: warpgroup wg has its queries [32 wg, 32 wg + 32)
-      for (int k = 0, at = 0; k < K_items && ok; ++k) {
+      // D = 64: the two warpgroups share an item, warpgroup wg has its queries [32 wg, 32 wg + 32); 128: they take the items in turn
+      // (those whose CTA-wide index has parity wg)
+      for (int k = KV_T ? 0 : (wg - kb) & 1; k < K_items && ok; k += KV_T ? 1 : 2) {
         const int kk = kb + k;
         const uint32_t pz = (uint32_t)kk & 1u;
-        const uint32_t e = list[at];
-        if (++at == cnt) at = 0;
-        const int q0 = (int)(e & 0xFFFu) * 64 + 32 * wg;
+        const uint32_t e = list[k % cnt];
+        const int q0 = (int)(e & 0xFFFu) * 64 + (KV_T ? 32 * wg : 0);
         const uint32_t flags = e >> 12;
         const uint32_t tS = tHalf + C_S + 64u * pz, tDP = tHalf + C_DP + DP_STEP * pz;
         uint8_t* dsrow = smem + Cfg::OFF_DS + pz * Cfg::DS_BYTES + r * 128;
@@ -415,18 +429,19 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         if (!ok) break;
         tc_fence_after();
         const uint32_t NEG = 0xff800000u;
-        // 32 score columns; once they are in registers P^T and dS^T may overwrite S^T, and the next item's dP^T this one
-        uint32_t sr[32], dr[32];
-        tmem_ld32(tS, sr); tmem_ld32(tDP, dr);
+        // NC score columns; once they are in registers P^T and dS^T may overwrite S^T, and the next item's dP^T this one
+        uint32_t sr[NC], dr[NC];
+#pragma unroll
+        for (int c = 0; c < NC; c += 32) { tmem_ld32(tS + c, sr + c); tmem_ld32(tDP + c, dr + c); }
         tc_wait_ld();
         tc_fence_before();
         __syncwarp();
         if (!KV_T && lane == 0) mbar_arrive(bar(Cfg::B_SREAD + pz));
         // 16 columns (queries) at a time, as passes over independent elements (exp2, then dS, then
-        // the packs) so that no instruction waits on its predecessor
+        // the packs) so that no instruction waits on its predecessor; what is packed is stored at once, which keeps few values live
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          const int c0 = 16 * hf, i0 = q0 + c0;         // first query of this half
+        for (int qd = 0; qd < NC / 16; ++qd) {
+          const int c0 = 16 * qd, i0 = q0 + c0;         // first query of these
           if (flags & ~FM_TF_ACTIVE) {
             // for this key the masked queries are intervals of the 16 columns: one mask word, one bit test per column
             const int a0 = lts - i0, a1 = lte - i0, b0 = uts - i0, b1 = ute - i0;
@@ -454,10 +469,10 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
             pk1[c] = pack2<IS_BF16>(pe[2 * c], pe[2 * c + 1]);
             pk2[c] = pack2<IS_BF16>(de[2 * c], de[2 * c + 1]);
           }
-          tmem_st8(tS + 8 * hf, pk1);
-          tmem_st8(tS + 16 + 8 * hf, pk2);
+          tmem_st8(tS + 8 * qd, pk1);
+          tmem_st8(tS + NC / 2 + 8 * qd, pk2);
           // dS^T row of this key, 16 queries: two 16-byte chunks, 128-byte swizzle
-          const int ch = 4 * wg + 2 * hf;
+          const int ch = (KV_T ? 4 * wg : 0) + 2 * qd;
           *reinterpret_cast<uint4*>(dsrow + ((ch ^ (r & 7)) << 4)) = make_uint4(pk2[0], pk2[1], pk2[2], pk2[3]);
           *reinterpret_cast<uint4*>(dsrow + (((ch + 1) ^ (r & 7)) << 4)) = make_uint4(pk2[4], pk2[5], pk2[6], pk2[7]);
         }
@@ -615,7 +630,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     // T of item k says that its dP^T has been read: dP^T of item k+2, then dQ^T of item k.
     if (elect_one()) {
       constexpr uint32_t idesc_g = make_idesc(IS_BF16, 128, 64, 0, 0), idesc_stat = make_idesc(true, 128, 64, 0, 0);
-      constexpr uint32_t idesc_dq = make_idesc(IS_BF16, 128, 64, 1, 1);
+      constexpr uint32_t idesc_dq = make_idesc(IS_BF16, 64, 64, 1, 1);
       const uint64_t dDo = make_sdesc(sRing + Cfg::HALF_BYTES, 16, 1024);   // dO half of a ring slot, K-major
       const uint64_t dKm = make_sdesc(sStat, Cfg::SUB128, 1024);            // K tile, MN-major (A of dQ^T)
       const uint64_t dDm = make_sdesc(sDS, Cfg::DS_BYTES, 1024);            // dS^T, MN-major (B of dQ^T)
@@ -759,8 +774,8 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           const uint32_t acc_on = k > 0 ? 1u : 0u;
           // dV += P^T dO, dK += dS^T Q; that was the last read of the ring slot
           const uint32_t tP = tmem + C_S + 64u * (uint32_t)pz;
-          umma_ts_halves_x4(tmem + C_DV, tP, dm_do, idesc_acc, acc_on);
-          umma_ts_halves_x4(tmem + C_DK, tP + 16u, dm_q, idesc_acc, acc_on);
+          umma_ts_xn<4>(tmem + C_DV, tP, dm_do, idesc_acc, acc_on);
+          umma_ts_xn<4>(tmem + C_DK, tP + 32u, dm_q, idesc_acc, acc_on);
           tc_commit(bar(Cfg::B_REMPTY + slot));
           tc_commit(bar(Cfg::B_PFREE + pz));
           // dQ^T = K^T dS^T: its buffer is free once the reduction warpgroup has read item kk-1
@@ -781,8 +796,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     __syncwarp();
   } else if (warp >= 12) {
     // =========================== dQ reduction + dK/dV epilogue ===========================
-    // Warp 12+e owns TMEM lanes [32e, 32e+32).  dQ^T of an item: lane = head-dim column, 64 columns
-    // = the item's queries; a warp adds 32 consecutive floats of one query row per instruction.
+    // Warp 12+e owns TMEM lanes [32e, 32e+32).
     // dK / dV of a unit: 32 columns at a time through a 2 KB staging area of the warp (rows of 64
     // bytes, 16-byte pieces XOR-swizzled by row) so that one store writes 8 rows x 64 contiguous bytes.
     const int ew = warp - 12;
@@ -801,13 +815,12 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       const int b = infos[s * 8 + 0], head = infos[s * 8 + 1], row0 = infos[s * 8 + 2];
       const uint16_t* list = lists + s * Cfg::LIST_MAX;
       const int K_items = cnt * G;
-      // dQ^T of an item: this warp's lanes are 32 head-dim columns, the 64 TMEM columns the item's queries.  The lane puts its
-      // column into the staging buffer four queries (16 bytes) at a time, [4 queries][32 columns][4 queries], and lane 0 hands
-      // the buffer to the copy engine, which adds it to the block of the fp32 accumulator that has the same order.  (Rows
-      // of 32 columns, four times as many stores: the kernel 806 -> 814 us on 2 x 8192 documents, 32 / 8 heads, d = 128, and
-      // 547 -> 557 at 64; through a tensor map, 16 x 32 boxes, 815 and 554.)  The reductions bound the 128-column variant: the L2
-      // takes 20 bytes per clock and SM of them (bulk or red.v4, measured alone), 1640 cycles for the 32 KB of an item
-      // that takes 2100.
+      // dQ^T of an item: this warp's lanes are 32 head-dim columns (D = 64: 16; an MMA of M = 64 leaves its row i in lane
+      // 32 (i / 16) + i % 16), the 64 TMEM columns the item's queries.  A lane puts its column into the staging buffer four queries (16
+      // bytes) at a time, [4 queries][columns][4 queries], and lane 0 hands the buffer to the copy engine, which adds it to
+      // the block of the fp32 accumulator that has the same order.  (Rows of 32 columns, four times as many stores: 814 instead
+      // of 806 us on 2 x 8192 documents, 32 / 8 heads, d = 128, 557 instead of 547 at 64; through a tensor map, 16 x 32 boxes,
+      // 815 and 554.  M = 128 at D = 64, half of it products nobody reads: 502 instead of 493.)
       for (int k = 0; k < K_items && ok; ++k) {
         const int kk = kb + k;
         ok = group_all(mbar_wait_parked(bar(Cfg::B_DQFULL), (uint32_t)kk & 1u, wc), 2, 128);
@@ -816,7 +829,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         const int q0 = (int)(list[k % cnt] & 0xFFFu) * 64;
         const int hq = head * G + k / cnt;
         // this warp's 64 x 32 values of the accumulator (rows past Sq, inside the padding, receive zeros)
-        float* acc = p.dq_accum + (((int64_t)b * p.Hq + hq) * p.Sq_r + q0) * D + ew * 64 * 32;
+        float* acc = p.dq_accum + (((int64_t)b * p.Hq + hq) * p.Sq_r + q0) * D + ew * 64 * Cfg::RCOLS;
         uint32_t v[4][16];
 #pragma unroll
         for (int r = 0; r < 4; ++r) tmem_ld16(tmem + lane_field + C_DQ + 16 * r, v[r]);
@@ -824,7 +837,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(Cfg::B_DQFREE));
-        if (32 * ew < p.d) {
+        if (Cfg::RCOLS * ew < p.d) {
 #pragma unroll
           for (int h = 0; h < 64 / Cfg::RROWS; ++h) {
             // D = 64: the item in one piece, two buffers in turn; 128: in halves through one buffer
@@ -833,12 +846,13 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
             __syncwarp();
 #pragma unroll
             for (int c = h * Cfg::RROWS; c < (h + 1) * Cfg::RROWS; c += 4)
-              reinterpret_cast<uint4*>(sb)[(c - h * Cfg::RROWS) / 4 * 32 + lane] =
-                  make_uint4(v[c / 16][c % 16], v[c / 16][c % 16 + 1], v[c / 16][c % 16 + 2], v[c / 16][c % 16 + 3]);
+              if (Cfg::RCOLS == 32 || lane < Cfg::RCOLS)
+                reinterpret_cast<uint4*>(sb)[(c - h * Cfg::RROWS) / 4 * Cfg::RCOLS + lane] =
+                    make_uint4(v[c / 16][c % 16], v[c / 16][c % 16 + 1], v[c / 16][c % 16 + 2], v[c / 16][c % 16 + 3]);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              bulk_reduce_add(acc + h * Cfg::RROWS * 32, smem_u32(sb), Cfg::RBUF_BYTES);
+              bulk_reduce_add(acc + h * Cfg::RROWS * Cfg::RCOLS, smem_u32(sb), Cfg::RBUF_BYTES);
               bulk_commit();
             }
             ++rnd;
@@ -920,12 +934,13 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   }
 }
 
-// dq = round(scale * dq_accum).  The accumulator holds, per (batch, q head) and block of 64 query rows, groups of 32 columns,
-// each as [4 rows: 16][32 columns][4 rows] (what a lane of the reduction warps has of a column beside its neighbours'
-// columns).  A warp takes 16 rows of a group, 2 KB read as they lie (lane = column), and turns them through shuffles into
+// dq = round(scale * dq_accum).  The accumulator holds, per (batch, q head) and block of 64 query rows, groups of 32 (D = 64: 16)
+// columns, each as [4 rows: 16][columns][4 rows] (what a lane of the reduction warps has of a column beside its neighbours'
+// columns).  A warp takes 16 rows x 32 columns, 2 KB read as they lie (lane = column), and turns them through shuffles into
 // rows: at each step a lane gives half of what it has to the lane whose columns lie beside its own.
 template <bool IS_BF16, int D>
 __global__ void __launch_bounds__(256) bwd_dq_round_kernel(const AttnKParams p) {
+  constexpr int RC = BwdFusedCfg<D>::RCOLS;
   const int lane = threadIdx.x & 31;
   const int n_grp = (p.d + 31) / 32, n16 = (p.Sq + 15) / 16;
   const int64_t n = (int64_t)p.B * p.Hq * n16 * n_grp;
@@ -935,11 +950,12 @@ __global__ void __launch_bounds__(256) bwd_dq_round_kernel(const AttnKParams p) 
     const int i0 = (int)(r16 % n16) * 16;
     const int64_t bh = r16 / n16;
     const int h = (int)(bh % p.Hq), b = (int)(bh / p.Hq);
-    const float4* src = reinterpret_cast<const float4*>(p.dq_accum + (bh * p.Sq_r + (i0 & ~63)) * D) + g * 512 + (i0 & 63) / 4 * 32 + lane;
+    const int col = g * 32 + lane;
+    const float4* src = reinterpret_cast<const float4*>(p.dq_accum + (bh * p.Sq_r + (i0 & ~63)) * D) + col / RC * (16 * RC) + (i0 & 63) / 4 * RC + col % RC;
     uint32_t w[8];                              // rows 2 k and 2 k + 1 of this lane's column
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const float4 v = __ldcs(src + 32 * e);
+      const float4 v = __ldcs(src + RC * e);
       w[2 * e] = pack2<IS_BF16>(v.x * p.scale, v.y * p.scale);
       w[2 * e + 1] = pack2<IS_BF16>(v.z * p.scale, v.w * p.scale);
     }
