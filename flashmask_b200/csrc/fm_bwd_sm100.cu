@@ -122,6 +122,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
                  const AttnKParams p) {
   using Cfg = BwdSm100Cfg<D>;
   constexpr bool BIG = D > 128;
+  constexpr bool SHARE = BIG;                    // both compute warpgroups work on every item, 32 of its columns each
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
@@ -164,7 +165,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
       mbar_init(bar(Cfg::B_RFULL + i), MODE == MODE_DQ ? 33 : 1);
       mbar_init(bar(Cfg::B_REMPTY + i), 1);
     }
-    for (int h = 0; h < 2; ++h) { mbar_init(bar(Cfg::B_GFULL + h), 1); mbar_init(bar(Cfg::B_TFULL + h), 4); mbar_init(bar(Cfg::B_GREAD + h), 4); }
+    for (int h = 0; h < 2; ++h) { mbar_init(bar(Cfg::B_GFULL + h), 1); mbar_init(bar(Cfg::B_TFULL + h), SHARE ? 8 : 4); mbar_init(bar(Cfg::B_GREAD + h), SHARE ? 8 : 4); }
     mbar_init(bar(Cfg::B_ACC), 1);
     fence_mbar_init();
     // the stationary tiles are requested right away: the loads overlap with the list build
@@ -276,13 +277,17 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
   constexpr uint32_t C_ACC1 = BIG ? 192 : ((MODE == MODE_DKDV) ? 256 : 384), C_ACC2 = BIG ? 320 : 384;
   static_assert(!BIG || C_ACC2 + D <= 512, "tensor memory columns");
 
+  // four k-steps of an accumulation GEMM
+  auto acc_x4 = [](uint32_t d, uint32_t at, uint64_t bd, uint32_t idesc, uint32_t on) {
+    if constexpr (SHARE) umma_ts_halves_x4(d, at, bd, idesc, on);
+    else umma_ts_xn<4>(d, at, bd, idesc, on);
+  };
+
   if (warp < 8) {
     // =========================== compute warpgroups ===========================
-    const int pz = warp >> 2;                    // item parity this warpgroup serves
+    const int wg = warp >> 2;                    // SHARE: half of an item's columns; else the item parity this warpgroup serves
     const int r = tid & 127;                     // TMEM lane
     const uint32_t lane_field = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tG1 = tmem + lane_field + C_G1 + 64u * pz;
-    const uint32_t tG2 = tmem + lane_field + C_G2 + (BIG ? 0u : 64u * pz);
     const float scale_log2 = p.scale_log2;
     bool ok = true;
 
@@ -305,7 +310,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
       }
     }
 
-    for (int k = pz; k < K_items && ok; k += 2) {
+    for (int k = SHARE ? 0 : wg; k < K_items && ok; k += SHARE ? 1 : 2) {
+      const int pz = k & 1;
+      const uint32_t tG1 = tmem + lane_field + C_G1 + 64u * pz;
+      const uint32_t tG2 = tmem + lane_field + C_G2 + (BIG ? 0u : 64u * pz);
       const uint32_t e = list[k % cnt];
       const int idx = (int)(e & 0xFFFFu);
       const uint32_t flags = e >> 16;
@@ -322,9 +330,13 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
       const uint32_t NEG = 0xff800000u;
       // 64 score columns; once they are in registers the score buffers may be
       // overwritten by the next item of this parity (signalled through g_read)
-      uint32_t sr[2][32], dr[2][32];
-      tmem_ld32(tG1, sr[0]); tmem_ld32(tG2, dr[0]);
-      tmem_ld32(tG1 + 32, sr[1]); tmem_ld32(tG2 + 32, dr[1]);
+      uint32_t sr[SHARE ? 1 : 2][32], dr[SHARE ? 1 : 2][32];
+      if constexpr (SHARE) {
+        tmem_ld32(tG1 + 32 * wg, sr[0]); tmem_ld32(tG2 + 32 * wg, dr[0]);
+      } else {
+        tmem_ld32(tG1, sr[0]); tmem_ld32(tG2, dr[0]);
+        tmem_ld32(tG1 + 32, sr[1]); tmem_ld32(tG2 + 32, dr[1]);
+      }
       tc_wait_ld();
       tc_fence_before();
       __syncwarp();
@@ -341,6 +353,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
     }
 
     // ---- epilogue ----
+    const int pz = wg;
     if (ok && K_items > 0) {
       ok = __all_sync(0xffffffffu, mbar_wait(bar(Cfg::B_ACC), 0u, wc));
       tc_fence_after();
@@ -516,14 +529,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
           const uint32_t acc_on = k > 0 ? 1u : 0u;
           if (MODE == MODE_DKDV) {
             // dV += P^T dO (streamed operand 2), dK += dS^T Q (streamed operand 1)
-            const uint32_t t1 = tmem + (BIG ? C_G1 : C_G2) + 64u * pz, t2 = t1 + 32u;
-            umma_ts_xn<4>(tmem + C_ACC1, t1, dm2, idesc_acc2, acc_on);
-            umma_ts_xn<4>(tmem + C_ACC2, t2, dm1, idesc_acc1, acc_on);
+            const uint32_t t1 = tmem + (BIG ? C_G1 : C_G2) + 64u * pz, t2 = t1 + (SHARE ? 16u : 32u);
+            acc_x4(tmem + C_ACC1, t1, dm2, idesc_acc2, acc_on);
+            acc_x4(tmem + C_ACC2, t2, dm1, idesc_acc1, acc_on);
           } else {
             // dQ += dS K (streamed operand 1)
             const uint32_t t2 = BIG ? tmem + C_G1 + 64u * pz
                                     : tmem + C_T + 32u * (uint32_t)((((k >> 1) & 1) << 1) + pz);
-            umma_ts_xn<4>(tmem + C_ACC1, t2, dm1, idesc_acc1, acc_on);
+            acc_x4(tmem + C_ACC1, t2, dm1, idesc_acc1, acc_on);
           }
           tc_commit(bar(Cfg::B_REMPTY + slot));
           TRACE(1, 25, k);                    // ACC issued

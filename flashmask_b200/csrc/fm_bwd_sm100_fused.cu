@@ -148,24 +148,6 @@ template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-// Four k-steps (K = 64 queries) of D[tmem] (+)= A[tmem] * B[smem], B MN-major: A is 16 columns of each 32-column half of the
-// score buffer (two k-steps from one half, two from the other), B advances 16 rows (2048 bytes) per step.
-__device__ __forceinline__ void umma_ts_halves_x4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t acc_first) {
-  asm volatile(
-      "{\n\t.reg .pred p, pt;\n\t.reg .b64 tb;\n\t.reg .b32 ta;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.eq.b32 pt, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "add.u32 ta, %1, 8;  add.s64 tb, %2, 128;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], tb, %3, pt;\n\t"
-      "add.u32 ta, %1, 32; add.s64 tb, %2, 256;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], tb, %3, pt;\n\t"
-      "add.u32 ta, %1, 40; add.s64 tb, %2, 384;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], tb, %3, pt;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b), "r"(idesc), "r"(acc_first)
-      : "memory");
-}
-
 // Eight k-steps (K = 128) of D[tmem] = A[smem] * B[smem], both operands MN-major: each step
 // advances both by 16 rows (2048 bytes).
 __device__ __forceinline__ void umma_ss_mn_mn_x8(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc) {

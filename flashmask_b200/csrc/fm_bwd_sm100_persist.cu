@@ -363,6 +363,7 @@ bwd_sm100_persist_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __g
         if (!ok) break;
         if (r == 0) TRACE(2 + pz, 12, k);   // scores observed ready
         tc_fence_after();
+        constexpr bool SHARE = false;
         const uint8_t* aux = smem + Cfg::OFF_AUX + slot * Cfg::AUX_BYTES;
         const uint32_t NEG = 0xff800000u;
         // 64 score columns; once they are in registers the score buffers may be
