@@ -485,6 +485,53 @@ def test_one_kernel_backward_between_64_and_128_walks_units(d, Sq, Sk, Hq, Hkv, 
     assert _kernel_status() == 0
 
 
+@pytest.mark.parametrize("d,B,Sq,Sk,Hq,Hkv,kind", [
+    (64, 1, 1, 130, 2, 1, "none_causal"),             # one query: items, row groups and boxes of one row
+    (64, 1, 65, 65, 3, 1, "causal_doc"),              # odd numbers of items, a second item of one query
+    (64, 2, 200, 129, 4, 2, "bidir_doc"),             # more queries than keys, a key tile of one key
+    (64, 1, 449, 449, 2, 2, "sliding_window"),
+    (64, 24, 517, 517, 16, 8, "causal_doc"),          # CTAs walk several units; some are empty
+    (128, 1, 15, 257, 2, 1, "none_causal"),
+    (128, 2, 63, 64, 1, 1, "none_full"),
+    (128, 1, 333, 200, 6, 2, "bidir_doc"),
+    (128, 24, 517, 517, 16, 8, "causal_doc"),
+    (192, 1, 1, 65, 2, 1, "none_causal"),             # (two kernels, both warpgroups on an item)
+    (192, 2, 333, 200, 6, 2, "bidir_doc"),
+    (192, 1, 700, 700, 3, 1, "causal_doc")])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_backward_at_the_edges_of_items_units_and_accumulator(d, B, Sq, Sk, Hq, Hkv, kind, dtype):
+    """dQ, dK and dV against 64 bits where items, units and the blocks of the dQ accumulator are not whole."""
+    G, scale, dv = Hq // Hkv, 1 / math.sqrt(d), min(d, 128)
+    idx_np, causal = _mask(kind, B, Sq, Sk, 71)
+    if kind == "causal_doc" and B > 1:
+        idx_np = idx_np.copy()
+        idx_np[::2, :, 128:256] = 0                   # nobody sees the second key tile of every other sequence
+    idx = None if idx_np is None else torch.from_numpy(np.ascontiguousarray(idx_np).copy()).cuda()
+    q, k, v, do, _ = (t if t is None else t.cuda().to(dtype) for t in make_inputs(B, Sq, Sk, Hq, Hkv, d, dv, 72))
+    x = [t.detach().requires_grad_(True) for t in (q, k, v)]
+    out, lse = fm.flashmask_attention(*x, idx, causal=causal, return_lse=True)
+    got = torch.autograd.grad(out, x, do)
+    i, j = torch.arange(Sq, device="cuda")[:, None], torch.arange(Sk, device="cuda")
+    visible = (j <= i + Sk - Sq if causal else torch.ones(Sq, Sk, device="cuda", dtype=torch.bool))[None, None]
+    if idx_np is not None:
+        visible = torch.from_numpy(oracle.dense_bias(idx_np, Sq, Sk, causal)).cuda() == 0
+    heads = lambda t: t.double().permute(0, 2, 1, 3)
+    by_key = lambda t: t.reshape(B, Hkv, G, Sk, -1).sum(2)
+    u, tiny = (2 ** -8, 0.0) if dtype == torch.bfloat16 else (2 ** -11, 2 ** -25)
+    q64, do64, k64, v64 = heads(q), heads(do), *(heads(t).repeat_interleave(G, dim=1) for t in (k, v))
+    lse = torch.nan_to_num(lse.detach().double(), neginf=0.0)[..., None]
+    p = torch.exp((q64 @ k64.transpose(-1, -2) * scale - lse).masked_fill(~visible, -math.inf))
+    ds = p * (do64 @ v64.transpose(-1, -2) - (heads(out.detach()) * do64).sum(-1, keepdim=True))
+    ref = [scale * ds @ k64, by_key(scale * ds.transpose(-1, -2) @ q64), by_key(p.transpose(-1, -2) @ do64)]
+    # P and dS are rounded to the 16-bit type (and S, dP and the sums to fp32: some 2^-16 of the largest terms), the results once more
+    d_p, d_ds = p * (u + 2 ** -14) + tiny, ds.abs() * (u + 2 ** -14) + p * 2 ** -14 + tiny
+    bound = [scale * d_ds @ k64.abs(), by_key(scale * d_ds.transpose(-1, -2) @ q64.abs()), by_key(d_p.transpose(-1, -2) @ do64.abs())]
+    for g_, r, b, n in zip(got, ref, bound, ("dq", "dk", "dv")):
+        assert torch.isfinite(g_).all(), n
+        assert ((heads(g_) - r).abs() <= b + u * r.abs() + 2 * tiny + 1e-6).all(), n
+    assert _kernel_status() == 0
+
+
 @pytest.mark.parametrize("what", ["row sums", "scores", "small scale"])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("d", [64, 96, 128])
