@@ -15,7 +15,8 @@
 //
 // Work items are the 64-row half tiles that the mask classification keeps; item
 // k is computed by softmax warpgroup k%2 out of score buffers k%2, so the
-// tensor pipe works on one item while the other warpgroup does exp2 / dS.
+// tensor pipe works on one item while the other warpgroup does exp2 / dS.  (192 / 128: both
+// warpgroups compute every item, 32 of its columns each, see below.)
 // Every output element has exactly one owner CTA and a fixed summation order:
 // the gradients are bitwise reproducible and need neither atomics nor fp32
 // accumulators in global memory.
@@ -113,8 +114,11 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
 // (dP) has a single buffer, and the bf16 operands P^T / dS^T (dS) of an item are written over the
 // S^T buffer of that item, which is dead once its warpgroup holds the scores in registers.  The
 // issue order then is: accumulation MMAs of item k, S^T of item k+2 (after them in the pipe, so
-// the overlay is no longer read), dP^T of item k+2 as soon as the other warpgroup has read dP^T of
-// item k+1 out of the single buffer.
+// the overlay is no longer read), dP^T of item k+2 as soon as dP^T of item k+1 has been read out of
+// the single buffer.  So the scores of item k+2 wait for item k from its own scores on, and the
+// exponentials are the longest link: the warpgroups share them (SHARE).  8192 documents, 32 / 8 heads:
+// dK / dV 439 -> 418 us, dQ 469 -> 450; 2048 bidirectional documents 169 -> 160, 260 -> 250; 16384 causal,
+// bound by the tensor pipe and the power limit, 4.47 and 3.56 ms either way.
 template <int MODE, bool IS_BF16, int D, int DV>
 __global__ void __launch_bounds__(384, 1)
 bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_constant__ CUtensorMap tm_stat2,
