@@ -208,7 +208,8 @@ static bool bwd_fills_boxes(const fm_attn_args* a) { return a->d == a->dv && (a-
 // Head dims between 64 and 128.  A unit of the one kernel is a key tile of a kv head with every q head of its group (G), and
 // does five GEMMs an item; the two kernels do seven, but spread three of them over the q heads.  So the one kernel needs
 // units that fill the chip evenly and rows enough in each to pay for its accumulator (512 bytes a query row, cleared, added
-// to and rounded).  Forward + backward in us, two kernels -> one, d = 96 unless said, (units), inputs changing from pass to pass:
+// to and rounded).  (The figures are those of the kernel's form before P and dS lay over the scores; it is 5 to 6 % faster now, so
+// that the line is on the safe side.)  Forward + backward in us, two kernels -> one, d = 96 unless said, (units), inputs changing from pass to pass:
 //   masks.  A long document is a run of long units in every kv head that shares the mask ("copies"); with few copies and
 //   few units the chip waits for them, the more the wider the head:
 //     6 copies and more, 2 units an SM: 4800 documents, 32 / 8 heads 1.11x, 6363, 24 / 6 1.09x, 2432, 16 / 16 1.07x
