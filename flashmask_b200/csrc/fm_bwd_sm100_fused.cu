@@ -363,8 +363,12 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(Cfg::B_INFOFREE + s));
         if constexpr (KV_T) {
-          // (every phase of the barrier is waited for, or the next wait would take this one for its own)
+          // Every phase of the barrier is waited for, or the next wait would take this one for its own; and the tiles of the next
+          // unit are only requested once every warp has, or the phase after it could be over too, which looks like this one
+          // pending: the issuers release the tiles of an empty unit behind B_KVT, as those of any other.
           ok = __all_sync(0xffffffffu, mbar_wait_parked(bar(Cfg::B_STAT), (uint32_t)j & 1u, wc));
+          if (!ok) break;
+          if (lane == 0) mbar_arrive(bar(Cfg::B_KVT));
         }
         continue;
       }
@@ -574,15 +578,10 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         if (cnt < 0) break;
         const int K_items = cnt * G;
         mbar_arrive(bar(Cfg::B_INFOFREE + s));     // only the item count is needed here
-        if (K_items == 0) {
-          // the stationary tiles of an empty unit are not used
-          ok = mbar_wait_parked(bar(Cfg::B_STAT), (uint32_t)j & 1u, wc);
-          mbar_arrive(bar(Cfg::B_VFREE)); mbar_arrive(bar(Cfg::B_KFREE));
-          continue;
-        }
-        ok = mbar_wait_parked(bar(Cfg::B_KVT), (uint32_t)ju & 1u, wc);       // K and V have landed and are in tensor memory
+        ok = mbar_wait_parked(bar(Cfg::B_KVT), (uint32_t)j & 1u, wc);        // K and V have landed and are in tensor memory
         if (!ok) break;
         mbar_arrive(bar(Cfg::B_VFREE));            // (V is not read from shared memory again)
+        if (K_items == 0) continue;                // (the tiles of an empty unit are not used)
         for (int k = 0; k < 2 && k < K_items && ok; ++k) {
           ok = wait_ring(kb + k);
           if (!ok) break;
@@ -624,7 +623,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       const uint64_t dDm = make_sdesc(sDS, Cfg::DS_BYTES, 1024);            // dS^T, MN-major (B of dQ^T)
       const uint64_t dOnes = make_sdesc_noswz(sbase + Cfg::OFF_ONES, 128, 128);
       bool ok = true;
-      int kb = 0, ju = 0;
+      int kb = 0;
       auto issue_dp = [&](int kk) {
         const int slot = kk % Cfg::NSLOT;
         ok = ok && mbar_wait_parked(bar(Cfg::B_RFULL + slot), (uint32_t)(kk / Cfg::NSLOT) & 1u, wc);
@@ -643,10 +642,13 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         if (cnt < 0) break;
         const int K_items = cnt * G;
         mbar_arrive(bar(Cfg::B_INFOFREE + s));
-        if (K_items == 0) continue;                // issuer 1 releases the tiles of an empty unit
-        ok = mbar_wait_parked(bar(Cfg::B_KVT), (uint32_t)ju & 1u, wc);
+        ok = mbar_wait_parked(bar(Cfg::B_KVT), (uint32_t)j & 1u, wc);
         if (!ok) break;
-        ++ju;
+        if (K_items == 0) {
+          // issuer 1 releases V, this thread K: the next phase of B_KVT comes after both have waited for this one
+          mbar_arrive(bar(Cfg::B_KFREE));
+          continue;
+        }
         issue_dp(kb);
         if (K_items > 1) issue_dp(kb + 1);
         for (int k = 0; k < K_items && ok; ++k) {

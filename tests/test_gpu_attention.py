@@ -485,27 +485,8 @@ def test_one_kernel_backward_between_64_and_128_walks_units(d, Sq, Sk, Hq, Hkv, 
     assert _kernel_status() == 0
 
 
-@pytest.mark.parametrize("d,B,Sq,Sk,Hq,Hkv,kind", [
-    (64, 1, 1, 130, 2, 1, "none_causal"),             # one query: items, row groups and boxes of one row
-    (64, 1, 65, 65, 3, 1, "causal_doc"),              # odd numbers of items, a second item of one query
-    (64, 2, 200, 129, 4, 2, "bidir_doc"),             # more queries than keys, a key tile of one key
-    (64, 1, 449, 449, 2, 2, "sliding_window"),
-    (64, 24, 517, 517, 16, 8, "causal_doc"),          # CTAs walk several units; some are empty
-    (128, 1, 15, 257, 2, 1, "none_causal"),
-    (128, 2, 63, 64, 1, 1, "none_full"),
-    (128, 1, 333, 200, 6, 2, "bidir_doc"),
-    (128, 24, 517, 517, 16, 8, "causal_doc"),
-    (192, 1, 1, 65, 2, 1, "none_causal"),             # (two kernels, both warpgroups on an item)
-    (192, 2, 333, 200, 6, 2, "bidir_doc"),
-    (192, 1, 700, 700, 3, 1, "causal_doc")])
-@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_backward_at_the_edges_of_items_units_and_accumulator(d, B, Sq, Sk, Hq, Hkv, kind, dtype):
-    """dQ, dK and dV against 64 bits where items, units and the blocks of the dQ accumulator are not whole."""
+def _assert_gradients_as_in_64_bits(d, B, Sq, Sk, Hq, Hkv, idx_np, causal, dtype):
     G, scale, dv = Hq // Hkv, 1 / math.sqrt(d), min(d, 128)
-    idx_np, causal = _mask(kind, B, Sq, Sk, 71)
-    if kind == "causal_doc" and B > 1:
-        idx_np = idx_np.copy()
-        idx_np[::2, :, 128:256] = 0                   # nobody sees the second key tile of every other sequence
     idx = None if idx_np is None else torch.from_numpy(np.ascontiguousarray(idx_np).copy()).cuda()
     q, k, v, do, _ = (t if t is None else t.cuda().to(dtype) for t in make_inputs(B, Sq, Sk, Hq, Hkv, d, dv, 72))
     x = [t.detach().requires_grad_(True) for t in (q, k, v)]
@@ -530,6 +511,56 @@ def test_backward_at_the_edges_of_items_units_and_accumulator(d, B, Sq, Sk, Hq, 
         assert torch.isfinite(g_).all(), n
         assert ((heads(g_) - r).abs() <= b + u * r.abs() + 2 * tiny + 1e-6).all(), n
     assert _kernel_status() == 0
+
+
+@pytest.mark.parametrize("d,B,Sq,Sk,Hq,Hkv,kind", [
+    (64, 1, 1, 130, 2, 1, "none_causal"),             # one query: items, row groups and boxes of one row
+    (64, 1, 65, 65, 3, 1, "causal_doc"),              # odd numbers of items, a second item of one query
+    (64, 2, 200, 129, 4, 2, "bidir_doc"),             # more queries than keys, a key tile of one key
+    (64, 1, 449, 449, 2, 2, "sliding_window"),
+    (64, 24, 517, 517, 16, 8, "causal_doc"),          # CTAs walk several units; one in ten is empty, at the end of the table
+    (128, 1, 15, 257, 2, 1, "none_causal"),
+    (128, 2, 63, 64, 1, 1, "none_full"),
+    (128, 1, 333, 200, 6, 2, "bidir_doc"),
+    (128, 24, 517, 517, 16, 8, "causal_doc"),
+    (192, 1, 1, 65, 2, 1, "none_causal"),             # (two kernels, both warpgroups on an item)
+    (192, 2, 333, 200, 6, 2, "bidir_doc"),
+    (192, 1, 700, 700, 3, 1, "causal_doc")])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_backward_at_the_edges_of_items_units_and_accumulator(d, B, Sq, Sk, Hq, Hkv, kind, dtype):
+    """dQ, dK and dV against 64 bits where items, units and the blocks of the dQ accumulator are not whole."""
+    idx_np, causal = _mask(kind, B, Sq, Sk, 71)
+    if kind == "causal_doc" and B > 1:
+        idx_np = idx_np.copy()
+        idx_np[::2, :, 128:256] = 0                   # nobody sees the second key tile of every other sequence
+    _assert_gradients_as_in_64_bits(d, B, Sq, Sk, Hq, Hkv, idx_np, causal, dtype)
+
+
+@pytest.mark.parametrize("what", ["runs of empty units", "empty and light units"])
+@pytest.mark.parametrize("d,dtype", [(64, torch.bfloat16), (64, torch.float16), (40, torch.bfloat16), (128, torch.bfloat16)])
+def test_backward_walks_units_that_nobody_sees(d, dtype, what):
+    """Key tiles without a query among the units that a CTA of the one-kernel backward walks: runs of four and more of them
+    behind two others, and, where one document is much longer than the rest, in turn with tiles of one or two items."""
+    if what == "runs of empty units":
+        B, S, H = 37, 300, 8                          # 888 units, two of three empty
+        idx_np, causal = _mask("causal_doc", B, S, S, 73)
+        idx_np = idx_np.copy()
+        for b in range(B):
+            for n in range(3):
+                if n != b % 3:
+                    idx_np[b, :, 128 * n:128 * n + 128] = 0
+    else:
+        B, S, H = 6, 2100, 8                          # 816 units; the long document's reach 33 items
+        short = [[61] * (S // 61) + [S % 61] for _ in range(B - 1)]
+        idx_np = np.concatenate([W.causal_document(1, S, S, np.array(lens))[0] for lens in [[S]] + short])
+        causal = True
+        for b in range(1, B):
+            for n in range(17):
+                if (n * n + b) % 3 == 0:
+                    idx_np[b, :, 128 * n:128 * n + 128] = 0
+                elif (n + b) % 2:
+                    idx_np[b, :, 128 * n + 50:128 * n + 128] = 0     # fewer items still
+    _assert_gradients_as_in_64_bits(d, B, S, S, H, H, idx_np, causal, dtype)
 
 
 @pytest.mark.parametrize("what", ["row sums", "scores", "small scale"])
