@@ -437,9 +437,22 @@ extern "C" int fm_launch_order_useful(const fm_attn_args* a, int which) {
   return n > sm_count();
 }
 
+// A wait of a kernel is given up two seconds after its CTA started.  A CTA of the persistent backward kernels lives as long as
+// its launch and one of the others as long as its unit, so they get time for that too: every 64 x 128 item of the call at 20 us, some
+// fifteen times what one takes, shared by the SMs, and those of one unit (131072 queries, 262144 keys, 96 / 8 heads, 2.3 s
+// of items: 55 s).  The bound lies here and not in the kernels because their waits have no room: with an end for each
+// wait from its own first look at the clock (two forms), or a deadline renewed with every unit, forward + backward of 3001 prefix-LM
+// tokens, 16 / 4 heads, d = 96, takes 262 -> 272, 262 -> 283, 255 -> 262 us; in this form 264.5 -> 264.7.
+static uint64_t bwd_wait_ns(const fm_attn_args* a) {
+  const uint64_t halves = ((uint64_t)a->Sq + 63) / 64, tiles = ((uint64_t)a->Sk + 127) / 128;
+  const uint64_t of_call = (uint64_t)a->B * a->Hq * halves * tiles, of_key_tile = (uint64_t)(a->Hq / a->Hkv) * halves;
+  return 2000000000ull + (of_call / (uint64_t)sm_count() + of_key_tile + 2 * tiles) * 20000ull;
+}
+
 // The counters of the persistent kernels live behind the table and the two unit arrays.
 static void attach_bwd_tables(const fm_attn_args* a, AttnKParams* p) {
   OrderGeom g;
+  p->wait_ns = bwd_wait_ns(a);
   p->dq_sched = p->dkdv_sched = nullptr;
   p->dq_ncta = p->dkdv_ncta = 0;
   if (p->dq_order && order_geometry_any(a, FM_ORDER_BWD_DQ, &g)) {

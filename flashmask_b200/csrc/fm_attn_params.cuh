@@ -40,6 +40,7 @@ struct AttnKParams {
   int pack_log2, n_split, alternate;
   float* part_o; float* part_lse;
   int block_log2, block_cols, block_ld;   // log2(block size), ceil(Sk / block size), row stride
+  uint64_t wait_ns;   // backward up to head dim 192: life of a CTA after which its waits are given up
 };
 
 // CTA coordinates under a launch order: the CTAs of a launch are numbered in

@@ -242,7 +242,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __grid_cons
     grid_dep_wait();                    // row statistics of the preprocess kernel
     grid_dep_trigger();                 // the dQ kernel reads nothing of this one: it fills the SMs this one leaves
   }
-  WaitCtx wc{misc + 4, global_timer_ns() + 2000000000ull};
+  WaitCtx wc{misc + 4, global_timer_ns() + p.wait_ns};
   if (tid == 0) { PROF(1); PROF_VAL(10, (long long)cnt * ((MODE == MODE_DKDV) ? p.Hq / p.Hkv : 1)); }
   if (cnt == 0) {
     // this tile's gradients are all zero: store them; the stationary loads already

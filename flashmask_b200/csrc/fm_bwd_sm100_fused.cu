@@ -235,7 +235,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = (uint32_t)misc[0];
-  WaitCtx wc{misc + 4, global_timer_ns() + 2000000000ull};
+  WaitCtx wc{misc + 4, global_timer_ns() + p.wait_ns};
   // S^T of item parity p at C_S + 64 p, its P^T and dS^T over it at +0 and +32; dP^T at C_DP (D = 64: + 64 p)
   constexpr uint32_t C_S = 0, C_DP = 128, DP_STEP = KV_T ? 64 : 0, C_DQ = KV_T ? 256 : 192, C_DV = KV_T ? 320 : 256,
                      C_DK = 384, C_K = 448, C_V = 480;

@@ -164,7 +164,7 @@ bwd_sm100_persist_kernel(const __grid_constant__ CUtensorMap tm_stat1, const __g
     grid_dep_wait();                    // row statistics of the preprocess kernel
     grid_dep_trigger();                 // the dQ kernel reads nothing of this one: it fills the SMs this one leaves
   }
-  WaitCtx wc{misc + 4, global_timer_ns() + 2000000000ull};
+  WaitCtx wc{misc + 4, global_timer_ns() + p.wait_ns};
   if (tid == 0) PROF(1);
   // TMEM columns: score buffers G1_p at 64p, G2_p at 128+64p.
   //   DKDV: P^T_p / dS^T_p (bf16) overlay G2_p at +0 / +32; dV at 256, dK at 384.  G1_p is dead as soon as

@@ -262,7 +262,8 @@ FM_API int fm_launch_orders(const fm_attn_args* args, int32_t* out_fwd, int32_t*
                             void* stream);
 
 /* Device-side status of the kernels that wait on barriers (the tcgen05
- * variants): every wait is bounded, and a wait that ran out makes its CTA
+ * variants): every wait is bounded (by two seconds from the start of its CTA,
+ * plus, in the backward, time for the work of the call), and a wait that ran out makes its CTA
  * unwind and record FM_ERR_TIMEOUT here instead of hanging.  Synchronises the
  * device (debug / test use; not called on the hot path).  `reset` != 0 clears
  * the word.  The reference instead traps the GPU from its spin watchdog

@@ -954,6 +954,32 @@ def test_bounded_wait_reports_timeout_without_fault():
     _run("causal_doc", 1, 256, 256, 2, 2, 128, 128, seed=2)
 
 
+def test_one_kernel_backward_runs_longer_than_a_wait_is_given():
+    """A launch of more than the two seconds that a wait has (131072 queries, 262144 keys, 96 / 8 heads, nothing masked): no wait
+    is given up, and dK and dV of a kv head are those of a call of its own, an eighth as long."""
+    Sq, Sk, Hq, Hkv, d = 131072, 262144, 96, 8, 64
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, out, do = (torch.randn(1, Sq, Hq, d, generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    k, v = (torch.randn(1, Sk, Hkv, d, generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    lse = torch.full((1, Hq, Sq), 13.0, device="cuda")               # log(262144) = 12.5, + 0.5 for the scores' variance
+    idx = torch.zeros(1, 1, Sk, 2, dtype=torch.int32, device="cuda")
+    idx[..., 0] = Sq
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    info = fm.prepare_mask(idx, Sq, False, 128, 128)
+    start.record()
+    _, dk, dv, _ = fm._flash_attn_bwd(q, k, v, out, do, lse, idx, mask_info=info)
+    end.record()
+    torch.cuda.synchronize()
+    assert _kernel_status() == 0
+    assert start.elapsed_time(end) > 2000, "larger sizes are needed to outlast a wait's budget"
+    for h in (0, Hkv - 1):
+        r = slice(h * 12, h * 12 + 12)
+        _, dk1, dv1, _ = fm._flash_attn_bwd(q[:, :, r].contiguous(), k[:, :, h:h + 1].contiguous(), v[:, :, h:h + 1].contiguous(),
+                                            out[:, :, r].contiguous(), do[:, :, r].contiguous(), lse[:, r].contiguous(), idx)
+        assert torch.equal(dk[:, :, h:h + 1], dk1) and torch.equal(dv[:, :, h:h + 1], dv1)
+    assert torch.isfinite(dk).all() and torch.isfinite(dv).all() and _kernel_status() == 0
+
+
 def test_shared_kv_convention():
     """value = key[..., :dv] on the same storage (576/512): dv comes back zero and dk
     carries dK + dV (reference: flashmask/cute/ops/_common.py:52-88)."""
