@@ -279,3 +279,16 @@ def test_sliding_window_kwarg_bounds():
     vis = W.dense_visible(idx2.numpy(), 16, False)[0, 0]
     i, j = np.indices((16, 16))
     assert np.array_equal(vis, (j - i <= 2) & (i - j <= 3))
+
+
+def test_every_included_file_is_a_dependency_of_the_objects():
+    """An object is compiled again when anything that a source includes has changed, textually included sources too."""
+    from flashmask_b200 import build as b
+    known = {os.path.basename(h) for h in b.headers()}
+    csrc = os.path.join(ROOT, "flashmask_b200", "csrc")
+    own = set(os.listdir(csrc)) | set(os.listdir(os.path.join(ROOT, "include")))
+    seen = set()
+    for f in sorted(os.listdir(csrc)):
+        if f.endswith((".cu", ".cuh", ".cpp", ".inc")):
+            seen |= {os.path.basename(n) for n in re.findall(r'#include "([^"]+)"', open(os.path.join(csrc, f)).read())}
+    assert len(seen & own) >= 5 and (seen & own) <= known, sorted((seen & own) - known)
