@@ -198,7 +198,8 @@ static bool bwd_uses_sm100(int d, int dv) {
 // The one-kernel backward (five GEMMs per tile pair, dQ summed into an fp32 accumulator in an order
 // that is not fixed) serves the tcgen05 head dims whenever the call does not ask for deterministic
 // gradients; the two-kernel variant gives every output element one owner and a fixed order.
-// Measured on 8K-128K masks it is 5-22 % faster at d = dv = 64 and d = dv = 128.  Head dims between them run it too where
+// Forward + backward of 8192 to 131072 tokens, masks and full tiles, takes 1.15 to 1.33 times as long with the two kernels at d = dv = 64
+// and d = dv = 128 (backward alone 1.20 to 1.55).  Head dims between them run it too where
 // one_kernel_pays (the GEMMs stop at the end of a head).
 // The CTA-pair backward (256, 512, 576 / 512) keeps P and dS of a chunk of query rows in the caller's workspace;
 // without one (fm_bwd_static_scratch) and past its index range the warp-MMA kernels serve these head dims.
@@ -208,21 +209,26 @@ static bool bwd_fills_boxes(const fm_attn_args* a) { return a->d == a->dv && (a-
 // Head dims between 64 and 128.  A unit of the one kernel is a key tile of a kv head with every q head of its group (G), and
 // does five GEMMs an item; the two kernels do seven, but spread three of them over the q heads.  So the one kernel needs
 // units that fill the chip evenly and rows enough in each to pay for its accumulator (512 bytes a query row, cleared, added
-// to and rounded).  (The figures are those of the kernel's form before P and dS lay over the scores; it is 5 to 6 % faster now, so
-// that the line is on the safe side.)  Forward + backward in us, two kernels -> one, d = 96 unless said, (units), inputs changing from pass to pass:
+// to and rounded).  The lines were drawn for a form of the one kernel that took 5 to 6 % longer (one buffer of scores), each where it began to
+// lose; with the present form most of them lie on the safe side.  Forward + backward in us, two kernels -> one, present form, documents and d = 96
+// unless said, (units), inputs changing from pass to pass; after "below" calls that the rule leaves to the two kernels:
 //   masks.  A long document is a run of long units in every kv head that shares the mask ("copies"); with few copies and
 //   few units the chip waits for them, the more the wider the head:
-//     6 copies and more, 2 units an SM: 4800 documents, 32 / 8 heads 1.11x, 6363, 24 / 6 1.09x, 2432, 16 / 16 1.07x
-//     3 to 5, 2.5: 12763, 24 / 3 (372) 1.07x, d = 120, 48 / 3 (402) 1.01x; but 9563, 16 / 4 (300) d = 96 1.06x, 80 0.96x, 120 0.85x
-//     2, 3: 28763, 8 / 2 (450) 1.16x, d = 120 (500) 1.00x; but 25563 (400) d = 120 0.91x, 19163 (300) 543 -> 635, 32 / 2 2059 -> 2513
-//     1, 4: 76763, 4 / 1 (600) 1.23x; but 57563, 4 / 1 (450) 805 -> 928, 4 x 10000, 4 / 1 (316) 647 -> 773
-//   short rows: 5 x 1000, 8 / 8 1.07x; but 16 x 640, 16 / 16 264 -> 266, 64 x 256, 16 / 16 304 -> 319, 64 x 200, 16 / 4 250 -> 261
-//   and an accumulator past L2: 12 x 520, 32 / 8 (126 MB) 1.05x; but 64 x 512, 16 / 4 (268 MB) 614 -> 631
+//     6 copies and more, 2 units an SM: 4800, 32 / 8 heads (304) 416 -> 352, 2432, 16 / 16 (304) 130 -> 114
+//     3 to 5, 2.5: 17100, 48 / 3 (402) d = 120 2314 -> 2348; below 12763, 24 / 3 (300) 843 -> 740, 9563, 16 / 4 (300) 452 -> 390, d = 80 442 -> 366,
+//       d = 120 495 -> 457, 2 x 3001, 16 / 4 (192) 252 -> 244, 3001, 16 / 4 (96) 189 -> 189
+//     2, 3: 28763, 8 / 2 (450) 608 -> 510, 32000, 8 / 2 (500) d = 120 782 -> 728; below 25563, 8 / 2 (400) d = 120 570 -> 525, 19163 (300) 418 -> 374,
+//       32 / 2 1592 -> 1511
+//     1, 4: 76763, 4 / 1 (600) 1276 -> 1109; below 57563, 4 / 1 (450) 1092 -> 974, 4 x 10000, 4 / 1 (316) 525 -> 530
+//   short rows: 5 x 1000, 8 / 8 117 -> 101; below 16 x 640, 16 / 16 262 -> 250, 64 x 256, 16 / 16 303 -> 309, 64 x 200, 16 / 4 252 -> 253
+//   and an accumulator past L2: 12 x 520, 32 / 8 (126 MB) 315 -> 291; below 64 x 512, 16 / 4 (268 MB) 596 -> 613
 // Without a mask units are even, and the two kernels walk no tables:
-//   G >= 4, any length: 64 x 100, 32 / 8 causal 238 -> 225, 40 x 64, 64 / 8 211 -> 185; 4800, 32 / 8 949 -> 865
-//   G < 4: 8 x 1280, 16 / 16 causal (1280) 370 -> 349; but 64 x 256, 16 / 16 331 -> 336
-//   G = 1 in less than three waves, where the last is nearly empty: 2432, 16 / 16 (304) 173 -> 171; but 5 x 1000, 8 / 8 (320)
-//   114 -> 116, 4 x 1280, 8 / 8 (320) d = 120 135 -> 142
+//   G >= 4, any length: 64 x 100, 32 / 8 causal 242 -> 224, 40 x 64, 64 / 8 214 -> 181, 4800 full, 32 / 8 1699 -> 1438; below two units an SM
+//     2 x 1300 causal, 64 / 8 (176) d = 72 442 -> 397, 2000 causal, 16 / 4 (64) d = 120 202 -> 231
+//   G < 4: 8 x 1280 causal, 16 / 16 (1280) 374 -> 331; below 64 x 256 causal, 16 / 16 334 -> 327, 128 x 256 full d = 120 733 -> 744,
+//     12000 full, 4 / 2 (188) d = 80 1317 -> 1168
+//   G = 1 in less than three waves, where the last is nearly empty: 2432 causal, 16 / 16 (304) 173 -> 157; below 5 x 1000 causal, 8 / 8 (320)
+//     112 -> 108, 4 x 1280 full, 8 / 8 (320) d = 120 184 -> 179, 4000 full, 8 / 8 (256) 296 -> 236
 static bool one_kernel_pays(const fm_attn_args* a) {
   if (a->Hkv <= 0 || a->Sk <= 0 || a->Hq < a->Hkv) return false;
   const int64_t units = (int64_t)a->Hkv * a->B * ((a->Sk + 127) / 128), sms = sm_count();

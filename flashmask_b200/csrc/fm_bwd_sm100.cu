@@ -113,7 +113,7 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
 // leaves three 64-column score buffers instead of four: S^T (S) keeps one buffer per item parity, dP^T
 // (dP) has a single buffer, and the bf16 operands P^T / dS^T (dS) of an item are written over the
 // S^T buffer of that item, which is dead once its warpgroup holds the scores in registers.  The
-// issue order then is: accumulation MMAs of item k, S^T of item k+2 (after them in the pipe, so
+// issue order then is: accumulation MMAs of item k, S^T of item k+2 (after them in the pipe, see "Order of MMAs" in fm_sm100.cuh, so
 // the overlay is no longer read), dP^T of item k+2 as soon as dP^T of item k+1 has been read out of
 // the single buffer.  So the scores of item k+2 wait for item k from its own scores on, and the
 // exponentials are the longest link: the warpgroups share them (SHARE).  8192 documents, 32 / 8 heads:

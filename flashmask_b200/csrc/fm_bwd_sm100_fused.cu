@@ -29,10 +29,10 @@
 // alone; 32 with A in TMEM).  128-column variant: S^T, dP^T and dQ^T 1250 cycles an item, dV and dK 512, and the L2 takes 20
 // bytes per clock and SM of fp32 reductions (bulk or red.v4, measured alone), 1640 cycles for an item's 32 KB of dQ; it takes 2100.
 // 64-column variant: 860 cycles of MMAs, 1120 of the shared-memory pipe; it takes 1490 on full tiles.  There the chain scores -> P, dS
-// -> dV, dK -> next scores decided: both warpgroups work on the same item (the chain has half the exponentials; in turn, 535 instead
-// of 512 us), and two threads issue.
-// 2 x 8192 documents, 32 / 8 heads, this kernel alone: d = 64 622 -> 493 us, d = 128 815 -> 776, d = 96 731 -> 690, against one
-// buffer each for S^T and dP^T, P^T in columns of its own and dS^T read from shared memory.
+// -> dV, dK -> next scores decided: both warpgroups work on the same item (the chain has half the exponentials; in turn it was 4 %
+// slower when one thread issued everything), and two threads issue.
+// 2 x 8192 tokens, 32 / 8 heads, this kernel alone: documents d = 64 616 -> 483 us, d = 128 814 -> 780, d = 96 718 -> 691, full d = 64
+// 3.76 -> 2.92 ms, d = 128 4.93 -> 4.66, against one buffer each for S^T and dP^T, P^T in columns of its own, dS^T read from shared memory.
 //
 // Warp roles: 0-3 / 4-7 compute warpgroups, 8 TMA producer, 9 UMMA issuer
 // (owns TMEM), 10 scheduler + list builder, 11 second UMMA issuer, 12-15 dQ reduction + dK/dV epilogue.
@@ -50,8 +50,8 @@ __device__ int g_bwd_fused_status = 0;
 
 template <int D>
 struct BwdFusedCfg {
-  // (a slot is taken for about 6000 cycles, a load's 1000 to 2000 among them: with three the 64-column variant waited for Q and
-  // dO, 603 instead of 554 us on 2 x 8192 documents, 32 / 8 heads; the 128-column one has no room for a fourth)
+  // (a slot is taken for about 6000 cycles, a load's 1000 to 2000 among them: with three the 64-column variant waits for Q and
+  // dO, 886 instead of 485 us on 2 x 8192 documents, 32 / 8 heads; the 128-column one has no room for a fourth)
   static constexpr int NSLOT = D == 64 ? 6 : 3, LIST_MAX = 2048, NTHREADS = 512;
   static constexpr int TILE_BYTES = 128 * D * 2;       // 128 rows x D cols bf16
   static constexpr int SUB128 = 128 * 128;             // 128-row x 64-col sub-tile (bytes)
@@ -240,8 +240,8 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   constexpr uint32_t C_S = 0, C_DP = 128, DP_STEP = KV_T ? 64 : 0, C_DQ = KV_T ? 256 : 192, C_DV = KV_T ? 320 : 256,
                      C_DK = 384, C_K = 448, C_V = 480;
 
-  // 128: 512 threads start with 128 registers each; the compute warpgroups take what the others give up.  (168 / 80 / 96 left
-  // spills: 806 instead of 776 us.)  64: half the columns to a thread, 128 do.
+  // 128: 512 threads start with 128 registers each; the compute warpgroups take what the others give up.  (168 / 80 / 96 leaves
+  // spills: 799 instead of 784 us.)  64: half the columns to a thread, 128 do.
   if constexpr (!KV_T) {
     if (warp < 8) setmaxnreg_inc<160>();
     else setmaxnreg_dec<96>();
@@ -549,7 +549,7 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     }
   } else if (KV_T && warp == 9) {
     // =========================== UMMA issuer 1 (D = 64): dV, dK, S^T ===========================
-    // What runs in the order of issue needs no barrier: S^T of item k+2 follows the dV and dK GEMMs of item k, which read the P^T
+    // What runs in the order of issue needs no barrier (see "Order of MMAs" in fm_sm100.cuh): S^T of item k+2 follows the dV and dK GEMMs of item k, which read the P^T
     // and dS^T that it overwrites.  dP^T and dQ^T are issued by another thread: a thread that issues spends its time waiting for
     // the queue of the tensor pipe and, some 150 cycles each, for barriers, and one for all five GEMMs was busy for all of an
     // item's 1640 cycles.
@@ -809,9 +809,9 @@ bwd_sm100_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       // dQ^T of an item: this warp's lanes are 32 head-dim columns (D = 64: 16; an MMA of M = 64 leaves its row i in lane
       // 32 (i / 16) + i % 16), the 64 TMEM columns the item's queries.  A lane puts its column into the staging buffer four queries (16
       // bytes) at a time, [4 queries][columns][4 queries], and lane 0 hands the buffer to the copy engine, which adds it to
-      // the block of the fp32 accumulator that has the same order.  (Rows of 32 columns, four times as many stores: 814 instead
-      // of 806 us on 2 x 8192 documents, 32 / 8 heads, d = 128, 557 instead of 547 at 64; through a tensor map, 16 x 32 boxes,
-      // 815 and 554.  M = 128 at D = 64, half of it products nobody reads: 502 instead of 493.)
+      // the block of the fp32 accumulator that has the same order.  (When tried, against the form of
+      // that day: rows of 32 columns, four times as many stores, or boxes of 16 x 32 through a tensor map 1 to 2 % slower on 2 x 8192
+      // documents; M = 128 at D = 64, half of it products nobody reads, 2 %.)
       for (int k = 0; k < K_items && ok; ++k) {
         const int kk = kb + k;
         ok = group_all(mbar_wait_parked(bar(Cfg::B_DQFULL), (uint32_t)kk & 1u, wc), 2, 128);
