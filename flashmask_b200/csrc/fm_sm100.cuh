@@ -128,14 +128,15 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// Order of MMAs.  PTX promises the order of issue for MMAs of one thread with the same accumulator and shape.  Four places rely on it for
+// Order of MMAs.  PTX promises the order of issue for MMAs of one thread with the same accumulator and shape.  The kernels rely on it for
 // MMAs of ONE issuing thread, of the same cta_group and kind, with different accumulators: an MMA that writes the columns which an
 // earlier one reads as its A operand in tensor memory is issued behind it with no
 // barrier between (the tensor pipe takes the MMAs of a thread one after the other, and all outputs are compared against 64 bits):
 //   forward                    scores of the next tile over P, behind P V                      fm_fwd_sm100.cu
 //   CTA-pair forward           scores of tile i + 2 over P of tile i, behind its P V           fm_fwd_pair.cu
-//   192 / 128 backward         scores of item k + 2 over P and dS of item k, behind its dV, dK (dQ)   fm_bwd_sm100.cu
-//   one-kernel backward at 64  the same                                                        fm_bwd_sm100_fused.cu
+//   two-kernel backward        dP (up to head dim 128, dK / dV kernel) or the scores (192 / 128) of item k + 2 over P and dS of item k,
+//                              behind its dV and dK (dQ)                                       fm_bwd_sm100.cu, fm_bwd_sm100_persist.cu
+//   one-kernel backward at 64  scores of item k + 2 over P and dS of item k, behind its dV, dK  fm_bwd_sm100_fused.cu
 // MMAs of different threads have no order (the one-kernel backward at 128 issues its scores from another thread than dV and dK: B_PFREE
 // stands between), nor have an MMA and tensor-memory accesses of other warps (commit, barrier and the fences stand between).  A change that
 // deals such a pair to two threads, or to other cta_groups, needs a commit and a barrier there.
